@@ -59,6 +59,28 @@ __device__ __forceinline__ void load8(const T* p, float (&f)[8]) {
     f[2 * i + 1] = t.y;
   }
 }
+// The 8 values of a 16-byte register quad that was loaded earlier.
+template <typename T>
+__device__ __forceinline__ void unpack8(const uint4& q, float (&f)[8]) {
+  const typename Num<T>::T2* v = reinterpret_cast<const typename Num<T>::T2*>(&q);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float2 t = Num<T>::to_f2(v[i]);
+    f[2 * i] = t.x;
+    f[2 * i + 1] = t.y;
+  }
+}
+// Values n .. n + 7 of a row of N, zeros behind its end; `vec`: they may be read as one 16-byte piece.
+template <typename T>
+__device__ __forceinline__ uint4 vec8_upto(const T* row, int n, int N, bool vec) {
+  if (vec && n + 8 <= N) return *reinterpret_cast<const uint4*>(row + n);
+  uint4 q = make_uint4(0u, 0u, 0u, 0u);
+  T* v = reinterpret_cast<T*>(&q);
+#pragma unroll
+  for (int j = 0; j < 8; ++j)
+    if (n + j < N) v[j] = row[n + j];
+  return q;
+}
 template <typename T>
 __device__ __forceinline__ void store8(T* p, const float (&f)[8]) {
   Vec8<T> x;

@@ -47,8 +47,8 @@ struct GemmPsParams {
   int tiles_m, tiles_n;   // tiles_m counts tiles of 128*MT rows
   int band;               // row tiles per band of the tile order
   int pf_blocks;          // k blocks prefetched into L2 ahead of the ring
-  int tma_out;            // results leave through shared-memory staging: 1 tiled bulk stores, 2 bulk reduce-adds
-                          // into an output that already holds the residual (out == residual)
+  int aff_vec;            // bias and scale may be read as 16-byte vectors (see finish16)
+  int tma_out;            // results leave through shared-memory staging and tiled bulk stores
   // grouped form: grp[0] = number of row blocks, then {expert, row0, row_end, 0} per block (device memory)
   const int32_t* grp;
   int grp_rt_per_expert;  // row tiles of the weight image between two experts (projection whose N axis is split by expert)
@@ -100,8 +100,15 @@ struct alignas(8) GemmPsCtl {
   int32_t abort_flag;
 };
 
-template <typename T, bool DUAL, int MT>
-__global__ void __launch_bounds__(64 + 128 * MT)
+__device__ __forceinline__ uint4 shfl_u4(const uint4& q, int lane) {
+  return make_uint4(__shfl_sync(0xffffffffu, q.x, lane), __shfl_sync(0xffffffffu, q.y, lane), __shfl_sync(0xffffffffu, q.z, lane),
+                    __shfl_sync(0xffffffffu, q.w, lane));
+}
+
+// EXTRA: the epilogue has more to do than the activation (row scale, scale, bias, residual); without it their tests stay out of a
+// loop whose length delays the MMA-issuing lane (3072 x 6144 x 1152, nothing to add: 40.5 -> 36.6 us)
+template <typename T, bool DUAL, int MT, bool EXTRA>
+__global__ void __launch_bounds__(64 + 128 * MT, 1)
 gemm_ps_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmO, const GemmPsParams p) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   const uint32_t raw_addr = smem_u32(smem_raw);
@@ -179,7 +186,7 @@ gemm_ps_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
 #pragma unroll
           for (int wt = 0; wt < kW; ++wt)
             for (int sub = 0; sub < nsub; ++sub)
-              bulk_prefetch_l2(p.w_packed + ((size_t)(rt0 + sub + wt * p.dual_tiles) * p.k_blocks + pf_kb) * kPsBlock,
+              bulk_prefetch_l2(p.w_packed + ((size_t)(min(rt0 + sub, p.n_blocks - 1) + wt * p.dual_tiles) * p.k_blocks + pf_kb) * kPsBlock,
                                kPsBlock);
         }
         if (acts) {
@@ -286,12 +293,13 @@ gemm_ps_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     const int half = (warp - 2) >> 2;                      // which 128-row half of the tile it drains
     const int r = quarter * 32 + lane;
     const uint32_t lane_base = tmem_base + ((uint32_t)(quarter * 32) << 16);
-    const T* bias = reinterpret_cast<const T*>(p.bias);
-    const T* scale = reinterpret_cast<const T*>(p.scale);
-    const T* resid = reinterpret_cast<const T*>(p.residual);
+    const T* bias = EXTRA ? reinterpret_cast<const T*>(p.bias) : nullptr;
+    const T* scale = EXTRA ? reinterpret_cast<const T*>(p.scale) : nullptr;
+    const T* resid = EXTRA ? reinterpret_cast<const T*>(p.residual) : nullptr;
     T* out = reinterpret_cast<T*>(p.out);
     const int N = p.N;
-    const bool vec_ok = (p.ldo & 7) == 0 && (!resid || (p.ldr & 7) == 0);
+    const bool out_vec = (p.ldo & 7) == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0;
+    const bool res_vec = (p.ldr & 7) == 0 && (reinterpret_cast<uintptr_t>(resid) & 15) == 0;
     int lt = 0;
     const int tiles = tile_count();
     for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x, ++lt) {
@@ -299,28 +307,36 @@ gemm_ps_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
       const PsTile pt = ps_tile<MT>(p, tile);
       const int tn = pt.tn;
       const int M = pt.row_end;                            // rows at and past it are not this tile's to store
+      const int row = pt.row0 + half * kPsBM + r;
+      const int n_base = tn * bn;
+      // Bias and scale of the tile's columns, eight to a lane, and the row's first residual values are asked for before the accumulator
+      // is awaited: next to the operand ring there is no L1 to speak of, and a load inside the column loop is a trip to L2
+      // (3072 x 6144 x 1152 with a bias, us: sixteen two-byte loads per 16 columns 69.8, two 16-byte ones 48.0, this 42.3, no bias 35.9).
+      uint4 bias_g = {}, bias_u = {}, scale_g = {}, scale_u = {}, rv[DUAL ? 2 : 1][2] = {};
+      if constexpr (EXTRA) {
+        const int n = n_base + lane * 8;
+        if (lane * 8 < bn) {
+          if (bias) bias_g = vec8_upto(bias, n, N, p.aff_vec);
+          if (scale) scale_g = vec8_upto(scale, n, N, p.aff_vec);
+          if (DUAL && bias) bias_u = vec8_upto(bias + p.dual_offset, n, N, p.aff_vec);
+          if (DUAL && scale) scale_u = vec8_upto(scale + p.dual_offset, n, N, p.aff_vec);
+        }
+        if (resid && row < M) {
+#pragma unroll
+          for (int q = 0; q < (DUAL ? 4 : 2); ++q) rv[q >> 1][q & 1] = vec8_upto(resid + (size_t)row * p.ldr, n_base + q * 8, N, res_vec);
+        }
+      }
       if (!mbar_wait(&ctl->acc_full[b], (uint32_t)(lt / nbuf) & 1u) || *abort_flag) {
         if (!*abort_flag) report_status(p.status, kStatusEpilogueTimeout, kTagGemmTc, tile);
         ctl->abort_flag = 1;
         break;
       }
       tc_fence_after_sync();
-      const int row = pt.row0 + half * kPsBM + r;
-      const int n_base = tn * bn;
       const uint32_t acc = lane_base + (uint32_t)(b * acc_cols + half * half_cols);
-      const float rs = (p.row_scale && row < M) ? p.row_scale[row] : 1.f;
-      // Results go straight from registers to global memory, 16 columns (of each accumulator) per tensor-memory
-      // round trip for one accumulator and 32 for the GLU pair.  Measured alternatives on 8192 x 4096 x 4096:
-      // 64-column round trips 30 % slower, a shared-memory transpose for full-line stores 35 % slower - long
-      // instruction bursts of the epilogue warps delay the single MMA-issuing lane that shares their schedulers,
-      // so the loop is kept short: scale / bias work and the activation switch are hoisted out of the element loop.
-      const bool affine = scale || bias;                  // per-element scale / bias work, hoisted out of the loop
-      // Output path without a residual, or with the residual already in place (out == residual, the decoder's
-      // out-projection and down-projection): 64 finished columns of the warp's 32 rows are parked in a swizzled
-      // staging tile and leave as ONE tiled bulk store (or bulk reduce-add, which makes the residual add an L2
-      // operation) issued by lane 0 - whole 128-byte lines, asynchronous, no load or store instructions on the
-      // epilogue warps (16-byte stores to 32 rows per instruction kept the store queue saturated: 537 MB on the
-      // L1->L2 path for 67 MB of output).
+      const float rs = (EXTRA && p.row_scale && row < M) ? p.row_scale[row] : 1.f;
+      // Output path: 64 finished columns of the warp's 32 rows are parked in a swizzled staging tile and leave as ONE tiled bulk
+      // store issued by lane 0 - whole 128-byte lines, asynchronous, no store instructions on the epilogue warps (16-byte stores
+      // to 32 rows per instruction kept the store queue saturated: 537 MB on the L1->L2 path for 67 MB of output).
       uint8_t* stg = epi_stage + (size_t)(warp - 2) * kPsEpiBytes;
       const int row0 = pt.row0 + half * kPsBM + quarter * 32;
       // grouped form: rows behind the expert's last one are another expert's, so only whole 32-row pieces leave this way
@@ -333,99 +349,109 @@ gemm_ps_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         fence_proxy_async();
         __syncwarp();
         if (lane == 0 && row0 < M && n_base + c_first < N) {
-          if (p.tma_out == 2) tma_reduce_add_2d(&tmO, stg, n_base + c_first, row0);
-          else tma_store_2d(&tmO, stg, n_base + c_first, row0);
+          tma_store_2d(&tmO, stg, n_base + c_first, row0);
           bulk_commit_group();
         }
       };
-      auto finish16 = [&](int n0, const uint32_t* g16, const uint32_t* u16) {
+      // 16 residual values of this row (zeros where there are none): added in fp32 and rounded once
+      auto resid16 = [&](int n0, uint4 (&rv)[2]) {
+        rv[0] = rv[1] = make_uint4(0u, 0u, 0u, 0u);
+        if (!resid || row >= M) return;
+        rv[0] = vec8_upto(resid + (size_t)row * p.ldr, n0, N, res_vec);
+        rv[1] = vec8_upto(resid + (size_t)row * p.ldr, n0 + 8, N, res_vec);
+      };
+      // x <- x * scale + bias for 16 columns; every lane must take part (the tile's values lie eight to a lane)
+      auto affine16 = [&](int c0, float (&x)[16], const uint4& sq, const uint4& bq) {
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int src = (c0 >> 3) + h;
+          float f[8];
+          if (scale) {
+            const uint4 q = shfl_u4(sq, src);
+            unpack8<T>(q, f);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) x[h * 8 + j] *= f[j];
+          }
+          if (bias) {
+            const uint4 q = shfl_u4(bq, src);
+            unpack8<T>(q, f);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) x[h * 8 + j] += f[j];
+          }
+        }
+      };
+      auto finish16 = [&](int c0, const uint32_t* g16, const uint32_t* u16, const uint4 (&rv)[2]) {
+        const int n0 = n_base + c0;
         float g[16], u[16], v[16];
 #pragma unroll
         for (int j = 0; j < 16; ++j) {
           g[j] = __uint_as_float(g16[j]);
           u[j] = DUAL ? __uint_as_float(u16[j]) : 0.f;
         }
-        if (p.row_scale) {
+        if constexpr (EXTRA) {
+          if (p.row_scale) {
 #pragma unroll
-          for (int j = 0; j < 16; ++j) {
-            g[j] *= rs;
-            if (DUAL) u[j] *= rs;
-          }
-        }
-        if (affine) {
-#pragma unroll
-          for (int j = 0; j < 16; ++j) {
-            const int n = n0 + j;
-            if (n < N) {
-              if (scale) {
-                g[j] *= Num<T>::to_f(scale[n]);
-                if (DUAL) u[j] *= Num<T>::to_f(scale[p.dual_offset + n]);
-              }
-              if (bias) {
-                g[j] += Num<T>::to_f(bias[n]);
-                if (DUAL) u[j] += Num<T>::to_f(bias[p.dual_offset + n]);
-              }
+            for (int j = 0; j < 16; ++j) {
+              g[j] *= rs;
+              if (DUAL) u[j] *= rs;
             }
           }
+          affine16(c0, g, scale_g, bias_g);
+          if (DUAL) affine16(c0, u, scale_u, bias_u);
         }
+        if (!tma_out && (row >= M || n0 >= N)) return;
         apply_act_n<16>(p.act, g, u, v, p.act_args);
-        if (tma_out) {
-          // row `lane` of the warp's staging tile, 128-byte swizzled as the bulk store expects it
-          const int ch = ((n0 - n_base) >> 3) & 7;
-          float lo[8], hi[8];
+        float lo[8], hi[8];
 #pragma unroll
-          for (int j = 0; j < 8; ++j) { lo[j] = v[j]; hi[j] = v[8 + j]; }
-          store8(reinterpret_cast<T*>(stg + lane * 128 + ((ch ^ (lane & 7)) << 4)), lo);
-          store8(reinterpret_cast<T*>(stg + lane * 128 + (((ch + 1) ^ (lane & 7)) << 4)), hi);
-        } else if (vec_ok && n0 + 16 <= N) {
+        for (int j = 0; j < 8; ++j) { lo[j] = v[j]; hi[j] = v[8 + j]; }
+        if constexpr (EXTRA) {
           if (resid) {
             float r0[8], r1[8];
-            load8(resid + (size_t)row * p.ldr + n0, r0);
-            load8(resid + (size_t)row * p.ldr + n0 + 8, r1);
+            unpack8<T>(rv[0], r0);
+            unpack8<T>(rv[1], r1);
 #pragma unroll
-            for (int j = 0; j < 8; ++j) { v[j] += r0[j]; v[8 + j] += r1[j]; }
+            for (int j = 0; j < 8; ++j) { lo[j] += r0[j]; hi[j] += r1[j]; }
           }
-          float lo[8], hi[8];
-#pragma unroll
-          for (int j = 0; j < 8; ++j) { lo[j] = v[j]; hi[j] = v[8 + j]; }
+        }
+        if (tma_out) {
+          // row `lane` of the warp's staging tile, 128-byte swizzled as the bulk store expects it
+          const int ch = (c0 >> 3) & 7;
+          store8(reinterpret_cast<T*>(stg + lane * 128 + ((ch ^ (lane & 7)) << 4)), lo);
+          store8(reinterpret_cast<T*>(stg + lane * 128 + (((ch + 1) ^ (lane & 7)) << 4)), hi);
+        } else if (out_vec && n0 + 16 <= N) {
           store8(out + (size_t)row * p.ldo + n0, lo);
           store8(out + (size_t)row * p.ldo + n0 + 8, hi);
         } else {
-          for (int j = 0; j < 16; ++j) {
-            const int n = n0 + j;
-            if (n < N) {
-              float x = v[j];
-              if (resid) x += Num<T>::to_f(resid[(size_t)row * p.ldr + n]);
-              out[(size_t)row * p.ldo + n] = Num<T>::from_f(x);
-            }
-          }
+#pragma unroll
+          for (int j = 0; j < 16; ++j)
+            if (n0 + j < N) out[(size_t)row * p.ldo + n0 + j] = Num<T>::from_f(j < 8 ? lo[j & 7] : hi[j & 7]);
         }
       };
-      if constexpr (DUAL) {
-        for (int c0 = 0; c0 < bn; c0 += 32) {
-          uint32_t ra[32], rb[32];
-          tmem_ld32(acc + c0, ra);
-          tmem_ld32(acc + bn + c0, rb);
-          tmem_ld_wait();
-          if (tma_out && (c0 & 63) == 0) chunk_begin();
-          if (row < M || tma_out) {
-#pragma unroll
-            for (int q = 0; q < 2; ++q) {
-              const int n0 = n_base + c0 + q * 16;
-              if (n0 < N || tma_out) finish16(n0, ra + q * 16, rb + q * 16);
-            }
-          }
-          if (tma_out && (c0 & 63) == 32) chunk_end(c0 - 32);
+      // 16 columns (of each accumulator) per tensor-memory round trip for one accumulator and 32 for the GLU pair.  Measured
+      // alternatives: 32- and 64-column trips 1 - 5 % slower, a shared-memory transpose for full-line stores 35 % slower - long
+      // instruction bursts of the epilogue warps delay the single MMA-issuing lane that shares their schedulers.
+      constexpr int kTrip = DUAL ? 32 : 16;
+      for (int c0 = 0; c0 < bn; c0 += kTrip) {
+        uint32_t ra[kTrip], rb[kTrip];
+        uint4 rnext[kTrip / 16][2];
+        if constexpr (DUAL) {
+          tmem_ld32(acc + c0, *reinterpret_cast<uint32_t(*)[32]>(&ra[0]));
+          tmem_ld32(acc + bn + c0, *reinterpret_cast<uint32_t(*)[32]>(&rb[0]));
+        } else {
+          tmem_ld16(acc + c0, *reinterpret_cast<uint32_t(*)[16]>(&ra[0]));
         }
-      } else {
-        for (int c0 = 0; c0 < bn; c0 += 16) {
-          uint32_t ra[16];
-          tmem_ld16(acc + c0, ra);
-          tmem_ld_wait();
-          const int n0 = n_base + c0;
-          if (tma_out && (c0 & 63) == 0) chunk_begin();
-          if ((row < M && n0 < N) || tma_out) finish16(n0, ra, ra);
-          if (tma_out && (c0 & 63) == 48) chunk_end(c0 - 48);
+        if constexpr (EXTRA) {                         // the next trip's residual values
+#pragma unroll
+          for (int q = 0; q < kTrip / 16; ++q) resid16(c0 + kTrip < bn ? n_base + c0 + kTrip + q * 16 : N, rnext[q]);
+        }
+        tmem_ld_wait();
+        if (tma_out && (c0 & 63) == 0) chunk_begin();
+#pragma unroll
+        for (int q = 0; q < kTrip / 16; ++q) finish16(c0 + q * 16, ra + q * 16, DUAL ? rb + q * 16 : ra, rv[q]);
+        if (tma_out && ((c0 + kTrip) & 63) == 0) chunk_end(c0 + kTrip - 64);
+        if constexpr (EXTRA) {
+#pragma unroll
+          for (int q = 0; q < kTrip / 16; ++q) { rv[q][0] = rnext[q][0]; rv[q][1] = rnext[q][1]; }
         }
       }
       // this accumulator buffer may now be overwritten by a later tile
@@ -440,17 +466,15 @@ gemm_ps_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
   if (warp == 1) tmem_dealloc(tmem_base, 512u);
 }
 
-template <typename T, bool DUAL, int MT>
+template <typename T, bool DUAL, int MT, bool EXTRA>
 static int launch_ps(const RfGemm* g, int bn, cudaStream_t stream) {
-  auto kfn = gemm_ps_kernel<T, DUAL, MT>;
+  auto kfn = gemm_ps_kernel<T, DUAL, MT, EXTRA>;
   RF_ALLOW_SMEM_PER_DEVICE(kfn, 227 * 1024);
   CUtensorMap tmA, tmO;
   int rc = make_tmap_2d(&tmA, g->x, g->dtype, 2, g->K, g->M, g->ldx, kPsBK, kPsBM, true);
   if (rc) return rc;
   static const bool tma_out_enabled = [] { const char* e = getenv("RF_GEMM_PS_TMA_OUT"); return !(e && e[0] == '0'); }();
-  const bool inplace_resid = g->residual == g->out && g->ldr == g->ldo;
-  const bool tma_out = tma_out_enabled && (!g->residual || inplace_resid) && (g->ldo & 7) == 0 &&
-                       (reinterpret_cast<uintptr_t>(g->out) & 15) == 0;
+  const bool tma_out = tma_out_enabled && (g->ldo & 7) == 0 && (reinterpret_cast<uintptr_t>(g->out) & 15) == 0;
   if (tma_out) {
     rc = make_tmap_2d(&tmO, g->out, g->dtype, 2, g->N, g->M, g->ldo, 64, 32, true);
     if (rc) return rc;
@@ -462,7 +486,8 @@ static int launch_ps(const RfGemm* g, int bn, cudaStream_t stream) {
   p.bias = g->bias; p.scale = g->scale; p.row_scale = g->row_scale;
   p.w_packed = reinterpret_cast<const uint8_t*>(g->w);
   p.status = g->status;
-  p.tma_out = tma_out ? (g->residual ? 2 : 1) : 0;
+  p.aff_vec = ((reinterpret_cast<uintptr_t>(g->bias) | reinterpret_cast<uintptr_t>(g->scale)) & 15) == 0 && (g->dual_offset & 7) == 0;
+  p.tma_out = tma_out ? 1 : 0;
   p.M = g->M; p.N = g->N; p.k_blocks = ceil_div(g->K, kPsBK); p.bn = bn;
   p.kb_total = p.k_blocks; p.n_blocks = ceil_div(g->N, 128);
   p.act = g->act; p.act_args = {g->act_limit, g->act_alpha}; p.dual_offset = g->dual_offset; p.dual_tiles = ceil_div(g->N, 128);
@@ -487,43 +512,68 @@ static int launch_ps(const RfGemm* g, int bn, cudaStream_t stream) {
   return RF_OK;
 }
 
-// Rows per tile: 256 (MT = 2) once that still gives about one tile per SM, else 128 down to half a tile per SM;
-// 0 = not a persistent shape.
-static int ps_rows_per_tile(const RfGemm* g, int bn) {
-  static const int forced = [] { const char* e = getenv("RF_GEMM_PS_ROWS"); return e ? atoi(e) : 0; }();
-  const int t1 = ceil_div(g->M, kPsBM) * ceil_div(g->N, bn), t2 = ceil_div(g->M, 2 * kPsBM) * ceil_div(g->N, bn);
-  if (forced == 128 || forced == 256) return (forced == 256 ? t2 : t1) >= sm_count() / 2 ? forced : 0;
-  if (t2 * 4 >= sm_count() * 3) return 256;
-  return t1 * 2 >= sm_count() ? 128 : 0;   // half a wave of 128-row tiles still beats one-tile CTAs (Pi0.5 chunk 28.3 -> 26.6 ms)
-}
+// Tile shape of a launch and its estimated time.
+struct PsShape { int bn, rows; long ns; };
 
-// True when the persistent kernel takes this GEMM (called by rf_gemm after its argument checks).
-bool gemm_ps_eligible(const RfGemm* g, bool swap, int splits) {
-  static const bool enabled = [] { const char* e = getenv("RF_GEMM_PERSISTENT"); return !(e && e[0] == '0'); }();
-  if (!enabled || swap || splits != 1 || g->ar_world > 1 || !g->w_packed || g->w_int8) return false;
+// The main loop of a tile is bound by its operand stream, not by the tensor core: per 64-column k block and SM, with all SMs busy,
+// 128 x 128 tiles take 450 ns (32 KB), 256 x 128 and 128 x 256 tiles 595 ns (48 KB, twice the work), 256 x 256 tiles 800 ns
+// (64 KB, four times the work).  So larger tiles win unless they leave SMs without one: a launch takes as many waves of them as
+// the busiest SM has tiles.  Tiles that take all of tensor memory (512 columns) also wait for their epilogue, about 3.5 us, each;
+// the others only for the last one.  fp16, us, 128-row / 256-row tiles 128 wide (model in brackets): 3072 x 1152 x 4304 60.4 / 39.9
+// (65 / 44), 768 x 4304 x 1152 19.7 / 15.0 (21 / 15); 3072 x 6144 x 1152 with 256 x 256 tiles 37.3 (39).
+static PsShape ps_shape(const RfGemm* g) {
   const bool dual = g->dual_offset > 0;
-  const int bn = (!dual && g->N % 256 == 0) ? 256 : 128;
-  return ps_rows_per_tile(g, bn) != 0;
+  const int k_blocks = ceil_div(g->K, kPsBK), sms = sm_count();
+  static const int forced = [] { const char* e = getenv("RF_GEMM_PS_ROWS"); return e ? atoi(e) : 0; }();
+  PsShape best = {0, 0, 0};
+  for (int mt = 2; mt >= 1; --mt) {
+    if ((forced == 128 || forced == 256) && forced != mt * kPsBM) continue;
+    for (int bn = dual || g->N <= 128 ? 128 : 256; bn >= 128; bn -= 128) {   // a 256-wide tile may end in the middle
+      const long tiles = (long)ceil_div(g->M, mt * kPsBM) * ceil_div(g->N, bn), waves = (tiles + sms - 1) / sms;
+      const int pieces = mt + (dual ? 2 : bn / 128);                         // 16 KB operand pieces of a stage
+      const long kb_ns = pieces == 2 ? 450 : pieces == 3 ? 595 : 800;
+      const bool alone = mt * bn * (dual ? 2 : 1) > 256;
+      const long ns = 3000 + waves * k_blocks * kb_ns + (alone ? waves * 3500 : (dual ? 256 : bn) * 9);
+      if (best.bn == 0 || ns < best.ns) best = {bn, mt * kPsBM, ns};
+    }
+  }
+  return best;
 }
 
-template <typename T>
+// True when the persistent kernel takes this GEMM (called by rf_gemm after its argument checks): it is estimated to be no slower than
+// the one-tile kernel with `splits` K splits, whose CTAs pay the same per k block (two of them share an SM's operand stream), about
+// 4.5 us around it and 6.5 us more for the reduction of a split (fp16, us, persistent / split kernel: 825 x 2560 x 2048 20 / 26,
+// 825 x 2048 x 2048 20 / 30; 768 x 1152 x 4304 34 / 23, 825 x 2048 x 16384 119 / 96).
+bool gemm_ps_eligible(const RfGemm* g, bool swap, int splits, int bn, int tiles) {
+  static const bool enabled = [] { const char* e = getenv("RF_GEMM_PERSISTENT"); return !(e && e[0] == '0'); }();
+  if (!enabled || swap || g->ar_world > 1 || !g->w_packed || g->w_int8) return false;
+  const PsShape s = ps_shape(g);
+  if (s.bn == 0) return false;
+  const long sms = sm_count(), ctas = (long)tiles * splits, kb = ceil_div(ceil_div(g->K, kPsBK), splits);
+  const long kb_ns = (g->dual_offset > 0 || bn > 128) ? 595 : 450;
+  const long load = splits == 1 ? (ctas + sms - 1) / sms * 100 : std::max(100l, ctas * 100 / sms);    // busiest SM's CTAs, per cent
+  return s.ns <= 4500 + (splits > 1 ? 6500 : 0) + kb * kb_ns * load / 100;
+}
+
+template <typename T, bool EXTRA>
 static int launch_ps_t(const RfGemm* g, bool dual, int bn, int rows, cudaStream_t stream) {
-  if (rows == 256) return dual ? launch_ps<T, true, 2>(g, bn, stream) : launch_ps<T, false, 2>(g, bn, stream);
-  return dual ? launch_ps<T, true, 1>(g, bn, stream) : launch_ps<T, false, 1>(g, bn, stream);
+  if (rows == 256) return dual ? launch_ps<T, true, 2, EXTRA>(g, bn, stream) : launch_ps<T, false, 2, EXTRA>(g, bn, stream);
+  return dual ? launch_ps<T, true, 1, EXTRA>(g, bn, stream) : launch_ps<T, false, 1, EXTRA>(g, bn, stream);
 }
 
 int launch_gemm_ps(const RfGemm* g, cudaStream_t stream) {
   const bool dual = g->dual_offset > 0;
-  const int bn = (!dual && g->N % 256 == 0) ? 256 : 128;
-  const int rows = ps_rows_per_tile(g, bn);
-  if (g->dtype == 0) return launch_ps_t<__half>(g, dual, bn, rows, stream);
-  return launch_ps_t<__nv_bfloat16>(g, dual, bn, rows, stream);
+  const PsShape s = ps_shape(g);
+  const bool extra = g->bias || g->scale || g->row_scale || g->residual;
+  if (g->dtype == 0)
+    return extra ? launch_ps_t<__half, true>(g, dual, s.bn, s.rows, stream) : launch_ps_t<__half, false>(g, dual, s.bn, s.rows, stream);
+  return extra ? launch_ps_t<__nv_bfloat16, true>(g, dual, s.bn, s.rows, stream) : launch_ps_t<__nv_bfloat16, false>(g, dual, s.bn, s.rows, stream);
 }
 
 // Grouped (mixture-of-experts) launch: see the file comment.  One accumulator or a GLU pair, 128-row tiles.
-template <typename T, bool DUAL>
+template <typename T, bool DUAL, bool EXTRA>
 static int launch_ps_grouped(const RfMoeGroupedGemm* a, cudaStream_t stream) {
-  auto kfn = gemm_ps_kernel<T, DUAL, 1>;
+  auto kfn = gemm_ps_kernel<T, DUAL, 1, EXTRA>;
   RF_ALLOW_SMEM_PER_DEVICE(kfn, 227 * 1024);
   CUtensorMap tmA, tmO;
   int rc = make_tmap_2d(&tmA, a->x, a->dtype, 2, a->K, a->max_rows, a->ldx, kPsBK, kPsBM, true);
@@ -557,9 +607,14 @@ static int launch_ps_grouped(const RfMoeGroupedGemm* a, cudaStream_t stream) {
   return RF_OK;
 }
 
+template <typename T>
+static int launch_ps_grouped_t(const RfMoeGroupedGemm* a, cudaStream_t stream) {
+  if (a->row_scale) return a->dual ? launch_ps_grouped<T, true, true>(a, stream) : launch_ps_grouped<T, false, true>(a, stream);
+  return a->dual ? launch_ps_grouped<T, true, false>(a, stream) : launch_ps_grouped<T, false, false>(a, stream);
+}
+
 int launch_moe_grouped(const RfMoeGroupedGemm* a, cudaStream_t stream) {
-  if (a->dtype == 0) return a->dual ? launch_ps_grouped<__half, true>(a, stream) : launch_ps_grouped<__half, false>(a, stream);
-  return a->dual ? launch_ps_grouped<__nv_bfloat16, true>(a, stream) : launch_ps_grouped<__nv_bfloat16, false>(a, stream);
+  return a->dtype == 0 ? launch_ps_grouped_t<__half>(a, stream) : launch_ps_grouped_t<__nv_bfloat16>(a, stream);
 }
 
 // int8 tile-major weight image -> 16-bit tile-major image (the 128-byte-swizzled block layout the MMA reads).

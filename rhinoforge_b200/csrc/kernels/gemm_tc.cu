@@ -1346,7 +1346,7 @@ bool gemm_small_eligible(const RfGemm* g);                         // gemm_small
 int gemm_small_run(const RfGemm* g, cudaStream_t stream);
 void gemm_sk_scratch(const RfGemm* g, uint64_t* ws_bytes, int32_t* flags);
 int launch_gemm_sk(const RfGemm* g, cudaStream_t stream);
-bool gemm_ps_eligible(const RfGemm* g, bool swap, int splits);   // gemm_ps.cu: persistent kernel for large M
+bool gemm_ps_eligible(const RfGemm* g, bool swap, int splits, int bn, int tiles);   // gemm_ps.cu: persistent kernel for large M
 int launch_gemm_ps(const RfGemm* g, cudaStream_t stream);
 int widen_packed(const void* src, void* dst, int64_t blocks, int dtype, cudaStream_t stream);   // gemm_ps.cu
 }
@@ -1360,7 +1360,7 @@ static int run_gemm(const RfGemm* g, cudaStream_t stream, bool w8) {
   GemmPlan pl;
   rc = plan_gemm(g, &pl);
   if (rc) return rc;
-  if (!w8 && g->force_splits == 0 && g->force_bn == 0 && rf::gemm_ps_eligible(g, pl.swap != 0, pl.splits))
+  if (!w8 && g->force_splits == 0 && g->force_bn == 0 && rf::gemm_ps_eligible(g, pl.swap != 0, pl.splits, pl.bn, pl.grid_x * pl.grid_y))
     return rf::launch_gemm_ps(g, stream);
   if (w8 && g->w_bits != 4 && !pl.swap && g->M > 256 && g->w_packed && g->w_scratch && g->force_splits == 0 && g->force_bn == 0) {
     // Large token counts are compute-bound: widen the int8 weight image once into the caller's scratch (a pass
@@ -1408,7 +1408,7 @@ extern "C" int rf_gemm_plan_info(const RfGemm* g, int32_t* out) {
   if (rc) return rc;
   out[0] = pl.swap; out[1] = pl.bn; out[2] = pl.splits; out[3] = pl.stages; out[4] = pl.grid_x; out[5] = pl.grid_y;
   out[6] = (int32_t)pl.smem_bytes; out[7] = pl.k_blocks;
-  out[8] = (!g->w_int8 && g->force_splits == 0 && g->force_bn == 0 && rf::gemm_ps_eligible(g, pl.swap != 0, pl.splits)) ? 1 : 0;
+  out[8] = (!g->w_int8 && g->force_splits == 0 && g->force_bn == 0 && rf::gemm_ps_eligible(g, pl.swap != 0, pl.splits, pl.bn, pl.grid_x * pl.grid_y)) ? 1 : 0;
   if (!g->w_int8 && rf::gemm_sk_eligible(g, nullptr)) out[8] = 2;   // persistent stream-K kernel
   out[9] = (g->ar_world > 1 && !pl.swap && g->M > 256) ? 1 : 0;
   return RF_OK;

@@ -891,3 +891,28 @@ def test_gemm_small_dual_glu(dt, M, N, K, packed, status):
     ref = torch.nn.functional.silu(gte) * up
     got = K_.gemm(x, wk, bias=b, act="silu_mul", dual=True, **kw)
     _close(got, ref, dt, scale=max(1.0, float(ref.abs().max())))
+
+
+@pytest.mark.parametrize("dt", DT)
+@pytest.mark.parametrize("M,N,K", [(5000, 1152, 256), (4100, 4304, 128), (2500, 136, 520), (768, 4304, 1152), (825, 2560, 2048), (6000, 328, 64)])
+@pytest.mark.parametrize("vec", [True, False])
+def test_gemm_persistent_epilogue(dt, M, N, K, vec, status):
+    """Persistent kernel: column tiles that end in the middle of a weight block or before their second one, bias and scale from the lanes
+    of a warp, the residual added ahead of the staged store, operands that cannot be read as 16-byte vectors."""
+    from rhinoforge_b200.ops import kernels as K_
+    x = (torch.randn(M, K, device="cuda") * 0.5).to(dt)
+    w = (torch.randn(N, K, device="cuda") * 0.05).to(dt)
+    wp = K_.pack_weight(w)
+    off, pitch = (0, N + 8) if vec else (1, N + 3)
+    vector = lambda n, base: (base + 0.2 * torch.randn(n + 1, device="cuda")).to(dt)[off:off + n]
+    b, sc, r = vector(N, 0.0), vector(N, 1.0), torch.randn(M, pitch, device="cuda").to(dt)
+    rs = torch.rand(M, device="cuda") + 0.5
+    z = x.float() @ w.float().t()
+    ref = z * rs[:, None] * sc.float() + b.float() + r[:, :N].float()
+    scale = max(1.0, ref.abs().max().item())
+    _close(K_.gemm(x, wp, packed_shape=(N, K), bias=b, scale=sc, row_scale=rs, residual=r[:, :N], status=status), ref, dt, scale=scale)
+    acc = r.clone()
+    K_.gemm(x, wp, packed_shape=(N, K), bias=b, act="gelu_tanh", residual=acc[:, :N], out=acc[:, :N], status=status)
+    ref = torch.nn.functional.gelu(z + b.float(), approximate="tanh") + r[:, :N].float()
+    _close(acc[:, :N], ref, dt, scale=scale)
+    assert torch.equal(acc[:, N:], r[:, N:])
