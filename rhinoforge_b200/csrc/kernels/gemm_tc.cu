@@ -22,6 +22,7 @@
 // src/core/rpu_runtime_extras.cpp:1035-1092).
 #include <map>
 #include <mutex>
+#include <type_traits>
 
 #include "../common/dtype.cuh"
 #include "../common/host_util.h"
@@ -66,6 +67,7 @@ struct GemmTcParams {
   float* ss_out;           // per (128-column tile, token) sum of squares of the finished values (swap mode)
   const float* ss_in;      // per (tile, token) sums of squares of the input rows: the result is scaled by their rstd
   int ss_tiles, ss_ld;
+  int aff_vec, res_vec, out_vec;   // bias and scale / residual rows / output rows may be accessed as 16-byte vectors
   float ss_inv_dim, ss_eps;
 };
 constexpr uint32_t kPrefetchChunk = 8192;
@@ -80,10 +82,9 @@ struct alignas(8) GemmSmemCtl {
   uint32_t tmem_base;
   int32_t abort_flag;
 };
-// Scratch behind the control block, present only in launches with a folded RMSNorm (ss_in / ss_out):
-// rs[256] = reciprocal RMS of this tile's token columns, then ssw[4][256] = the four epilogue warps' partial sums of
-// squares per token column.
-constexpr int kSsScratchBytes = (256 + 4 * 256) * (int)sizeof(float);
+// Scratch behind the control block, present only in launches with a folded RMSNorm (ss_in): rs[256] = reciprocal RMS of this tile's
+// token columns.
+constexpr int kSsScratchBytes = 256 * (int)sizeof(float);
 
 // Converter warps of the quantised kernels: the block is 128 threads (producer, MMA issuer, epilogue) plus these.
 constexpr int kMaxConvWarps = 6;     // two CTAs of 128 + 192 threads still fit an SM's register file
@@ -430,17 +431,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
   const uint32_t crank = p.splits > 1 ? cluster_ctarank() : 0u;
 
   // folded RMSNorm: reciprocal RMS of every token column of this tile from the producer's per-tile sums of squares
-  float* ss_rs = reinterpret_cast<float*>(ctl + 1);
-  float (*ss_w)[256] = reinterpret_cast<float (*)[256]>(ss_rs + 256);
+  const float* ss_rs = reinterpret_cast<const float*>(ctl + 1);
   const bool use_rs = SWAP && p.ss_in != nullptr;   // ss_rs was filled by warps 2 and 3 while the main loop ran
-  const bool emit_ss = SWAP && p.ss_out != nullptr && p.ar_world <= 1;
-  // sum over this warp's 32 output features of the square of one finished value per lane, for token column c
-  auto ss_add = [&](int c, float v) {
-    float q = v * v;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) q += __shfl_xor_sync(0xffffffffu, q, o);
-    if (lane_id() == 0 && warp < 4) ss_w[warp][c] = q;
-  };
 
   // per-element epilogue math shared by both paths
   const bool affine = p.row_scale || scale || use_bias || use_rs;
@@ -465,6 +457,39 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
       if (DUAL) vu += Num<T>::to_f(bias[p.dual_offset + n]);
     }
     return apply_act(p.act, vg, vu, p.act_args);
+  };
+  // the same for eight neighbouring features of one token
+  auto finish8 = [&](int tok, int n0, float (&g)[8], float (&u)[8], float (&v)[8]) {
+    if (affine) {
+      float rs = use_rs ? ss_rs[tok - blockIdx.y * bn] : 1.f;
+      if (p.row_scale) rs *= p.row_scale[tok];
+      if (use_rs || p.row_scale) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) { g[j] *= rs; u[j] *= rs; }
+      }
+      float f[8];
+      if (scale) {
+        unpack8<T>(vec8_upto(scale, n0, N, p.aff_vec), f);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) g[j] *= f[j];
+        if (DUAL) {
+          unpack8<T>(vec8_upto(scale + p.dual_offset, n0, N, p.aff_vec), f);
+#pragma unroll
+          for (int j = 0; j < 8; ++j) u[j] *= f[j];
+        }
+      }
+      if (use_bias) {
+        unpack8<T>(vec8_upto(bias, n0, N, p.aff_vec), f);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) g[j] += f[j];
+        if (DUAL) {
+          unpack8<T>(vec8_upto(bias + p.dual_offset, n0, N, p.aff_vec), f);
+#pragma unroll
+          for (int j = 0; j < 8; ++j) u[j] += f[j];
+        }
+      }
+    }
+    apply_act_n<8>(p.act, g, u, v, p.act_args);
   };
   // Peer buffer addresses are read ONCE: the table lives in global memory and nothing tells the compiler
   // that the remote stores below cannot alias it, so a lookup per element would sit between every two stores.
@@ -499,7 +524,140 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
       if (d == owner) owner_buf = peer_buf[d];
   }
 
-  if (p.splits > 1) {
+  if (SWAP && p.ar_world <= 1) {
+    // ---- weights on the rows: the accumulator holds one feature per lane and one token per column, the output wants features side by
+    // side.  The fp32 partial is parked in shared memory as rows [token][128 features] (over the operand ring, which is idle); a thread
+    // then takes EIGHT neighbouring features of a token - of every split, over distributed shared memory, in split order - finishes
+    // them together and stores 16 bytes.  One value at a time, with a switch over the activations and a two-byte store each, this
+    // phase took longer than streaming the weights from 64 tokens on (fp16, us, before / now: 64 x 12288 x 4096 with SwiGLU
+    // 53.4 / 42.5, 64 x 6144 x 4096 20.5 / 14.9, 93 x 2048 x 2048 12.0 / 9.4, 1 x 4096 x 1024 5.9 / 5.6).
+    float* part = reinterpret_cast<float*>(smem);
+    const int S = p.splits;
+    const int step = S > 1 ? bn : min(bn, DUAL ? 32 : 64);        // token columns parked at a time
+    const int nthr = (int)blockDim.x;
+    for (int base = 0; base < ncols; base += step) {
+      const int here = min(step, ncols - base);                   // valid tokens of this pass
+      const int own = here > (int)crank ? (here - (int)crank + S - 1) / S : 0;   // ... that this CTA finishes: crank, crank + S, ...
+      const int items = own * 16;
+      if (!aborted && epi) {
+        for (int c = 0; c < here; c += 16) {
+          uint32_t rg[16], ru[16];
+          tmem_ld16(trow + base + c, rg);
+          if (DUAL) tmem_ld16(trow + bn + base + c, ru);
+          tmem_ld_wait();
+#pragma unroll
+          for (int j = 0; j < 16; ++j) {
+            if (c + j < here) {
+              part[(c + j) * kBM + tid] = __uint_as_float(rg[j]);
+              if (DUAL) part[(step + c + j) * kBM + tid] = __uint_as_float(ru[j]);
+            }
+          }
+        }
+      }
+      auto token_of = [&](int i) { return base + (int)crank + (i >> 4) * S; };   // token column of an item
+      const int fg = (tid & 15) * 8;                              // first feature of this thread's items inside the tile
+      const int n0 = a0 + fg;
+      // the residual is not part of anybody's partial: ask for it before the rendezvous
+      uint4 rv = make_uint4(0u, 0u, 0u, 0u);
+      if (resid && tid < items) rv = vec8_upto(resid + (size_t)(b0 + token_of(tid)) * p.ldr, n0, N, p.res_vec);
+      if (S > 1) {
+        // the splits' sums of this CTA's own tokens replace its own partial of them, which nobody else reads.  Four bytes a lane: a warp's
+        // 128 neighbouring bytes are one request between SMs (16-byte remote loads ran at a tenth of the rate)
+        cluster_sync_all();
+        if (!aborted && epi) {
+          // kS splits: 32 values of (token, split) in flight at a time (8 of the quantised kernels, which have fewer registers); a
+          // round trip per token made this part of 64 x 12288 x 4096 (two splits) 5 us longer
+          auto reduce = [&](auto kS_c) {
+            constexpr int kS = decltype(kS_c)::value, kTok = (W8 ? 16 : 32) / kS;
+            uint32_t peer[kS];
+#pragma unroll
+            for (int s = 0; s < kS; ++s) peer[s] = dsmem_addr(smem_u32(part) + (uint32_t)tid * 4u, (uint32_t)s);
+            for (int acc = 0; acc < kAcc; ++acc) {
+              for (int j0 = 0; j0 < own; j0 += kTok) {
+                float x[kTok][kS];
+#pragma unroll
+                for (int q = 0; q < kTok; ++q) {
+                  const int at = (acc * step + (int)crank + (j0 + q) * kS) * kBM;
+#pragma unroll
+                  for (int s = 0; s < kS; ++s)
+                    x[q][s] = j0 + q >= own ? 0.f : kS == 2 && s == (int)crank ? part[at + tid] : ld_dsmem_f32(peer[s] + (uint32_t)at * 4u);
+                }
+#pragma unroll
+                for (int q = 0; q < kTok; ++q) {
+                  float sum = 0.f;
+#pragma unroll
+                  for (int s = 0; s < kS; ++s) sum += x[q][s];
+                  if (j0 + q < own) part[(acc * step + (int)crank + (j0 + q) * kS) * kBM + tid] = sum;
+                }
+              }
+            }
+          };
+          // 2, 4 or 8 splits are the planner's; any other number can only be forced
+          if (S == 2) reduce(std::integral_constant<int, 2>{});
+          else if (S == 4) reduce(std::integral_constant<int, 4>{});
+          else if (S == 8) reduce(std::integral_constant<int, 8>{});
+          else {
+            for (int j = 0; j < own * kAcc; ++j) {
+              const int at = (j / own * step + (int)crank + (j % own) * S) * kBM;
+              float sum = 0.f;
+              for (int s = 0; s < S; ++s) sum += ld_dsmem_f32(dsmem_addr(smem_u32(part) + (uint32_t)(at + tid) * 4u, (uint32_t)s));
+              part[at + tid] = sum;
+            }
+          }
+        }
+      }
+      __syncthreads();
+      if (!aborted) {
+        for (int i0 = 0; i0 < items; i0 += nthr) {
+          const int i = i0 + tid;
+          const bool on = i < items;
+          const int c = on ? token_of(i) : base;
+          float g[8], u[8], v[8];
+          const float4* gp = reinterpret_cast<const float4*>(part + (c - base) * kBM + fg);
+          const float4 g0 = gp[0], g1 = gp[1];
+          g[0] = g0.x; g[1] = g0.y; g[2] = g0.z; g[3] = g0.w; g[4] = g1.x; g[5] = g1.y; g[6] = g1.z; g[7] = g1.w;
+          if (DUAL) {
+            const float4 u0 = gp[step * (kBM / 4)], u1 = gp[step * (kBM / 4) + 1];
+            u[0] = u0.x; u[1] = u0.y; u[2] = u0.z; u[3] = u0.w; u[4] = u1.x; u[5] = u1.y; u[6] = u1.z; u[7] = u1.w;
+          } else {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) u[j] = 0.f;
+          }
+          const int tok = b0 + c;
+          finish8(tok, n0, g, u, v);
+          if (resid) {
+            float r8[8];
+            unpack8<T>(rv, r8);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) v[j] += r8[j];
+            if (i + nthr < items) rv = vec8_upto(resid + (size_t)(b0 + token_of(i + nthr)) * p.ldr, n0, N, p.res_vec);
+          }
+          float sq = 0.f;                                         // squares of the values as stored
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            const float r = n0 + j < N ? Num<T>::to_f(Num<T>::from_f(v[j])) : 0.f;
+            sq += r * r;
+          }
+          if (on && n0 < N) {
+            T* dst = out + (size_t)tok * p.ldo + n0;
+            if (p.out_vec && n0 + 8 <= N) {
+              store8(dst, v);
+            } else {
+#pragma unroll
+              for (int j = 0; j < 8; ++j)
+                if (n0 + j < N) dst[j] = Num<T>::from_f(v[j]);
+            }
+          }
+          if (p.ss_out) {                                         // a token's 128 features sit in 16 neighbouring lanes
+#pragma unroll
+            for (int o = 8; o > 0; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
+            if (on && (tid & 15) == 0) p.ss_out[(size_t)blockIdx.x * p.ss_ld + tok] = sq;
+          }
+        }
+      }
+      if (base + step < ncols) __syncthreads();                   // the parked rows may be overwritten (one split only)
+    }
+  } else if (p.splits > 1) {
     // ---- split-K: the CTAs of one output tile form a cluster (cluster dim z =
     // splits).  Each parks its fp32 partial in its own shared memory
     // ([column][lane], conflict-free), then CTA r reduces columns r, r+S, ...
@@ -611,8 +769,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
           const int n0 = b0 + g0;
           if (a_idx < M) {
             float v[8];
-#pragma unroll
-            for (int j = 0; j < 8; ++j) v[j] = (n0 + j < N) ? finish(a_idx, n0 + j, ag[j], au[j]) : 0.f;
+            finish8(a_idx, n0, ag, au, v);
             if (p.ar_world > 1) {
 #pragma unroll
               for (int j = 0; j < 8; ++j)
@@ -668,28 +825,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
           if (pub) {
             if (epi) stage_put((c - (int)crank) / p.splits, (tok < M && n < N) ? finish(tok, n, g, u) : 0.f);
           } else {
-            float fin = 0.f;                       // the value as stored (0 outside the matrix)
-            if (tok < M && n < N) {
-              const float v = finish(tok, n, g, u);
-              if (p.ar_world > 1) {
-                push_partial(tok, n, v);
-              } else {
-                float r = v;
-                if (resid) r += Num<T>::to_f(resid[(size_t)tok * p.ldr + n]);
-                const T rt = Num<T>::from_f(r);
-                out[(size_t)tok * p.ldo + n] = rt;
-                fin = Num<T>::to_f(rt);
-              }
-            }
-            if (emit_ss) ss_add(c, fin);
+            if (tok < M && n < N) push_partial(tok, n, finish(tok, n, g, u));
           }
         }
-      }
-      if (emit_ss) {
-        // the columns this CTA finished (crank, crank + S, ...): one thread each adds the four warps' sums
-        __syncthreads();
-        for (int c = (int)crank + tid * p.splits; c < ncols; c += (int)blockDim.x * p.splits)
-          p.ss_out[(size_t)blockIdx.x * p.ss_ld + b0 + c] = ss_w[0][c] + ss_w[1][c] + ss_w[2][c] + ss_w[3][c];
       }
     }
   } else if (!aborted) {
@@ -699,13 +837,25 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
       if (DUAL) tmem_ld16(trow + bn + c, ru);
       tmem_ld_wait();
       float v[16];
+      if constexpr (SWAP) {
 #pragma unroll
-      for (int j = 0; j < 16; ++j) {
-        const int tok = SWAP ? (b0 + c + j) : a_idx;
-        const int n = SWAP ? a_idx : (b0 + c + j);
-        const float vg = __uint_as_float(rg[j]);
-        const float vu = DUAL ? __uint_as_float(ru[j]) : 0.f;
-        v[j] = (tok < M && n < N) ? finish(tok, n, vg, vu) : 0.f;
+        for (int j = 0; j < 16; ++j) {
+          const int tok = b0 + c + j;
+          v[j] = (tok < M && a_idx < N) ? finish(tok, a_idx, __uint_as_float(rg[j]), DUAL ? __uint_as_float(ru[j]) : 0.f) : 0.f;
+        }
+      } else {
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          float g8[8], u8[8], v8[8];
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            g8[j] = __uint_as_float(rg[h * 8 + j]);
+            u8[j] = DUAL ? __uint_as_float(ru[h * 8 + j]) : 0.f;
+          }
+          finish8(min(a_idx, M - 1), b0 + c + h * 8, g8, u8, v8);
+#pragma unroll
+          for (int j = 0; j < 8; ++j) v[h * 8 + j] = (a_idx < M && b0 + c + h * 8 + j < N) ? v8[j] : 0.f;
+        }
       }
       if (p.ar_world > 1 && p.ar_two_shot) {
         // The 16-bit partial of this tile is parked in the operand ring (idle once the accumulator is
@@ -733,26 +883,6 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
           const int tok = SWAP ? (b0 + c + j) : a_idx;
           const int n = SWAP ? a_idx : (b0 + c + j);
           if (tok < M && n < N) push_partial(tok, n, v[j]);
-        }
-      } else if (SWAP) {
-#pragma unroll
-        for (int j = 0; j < 16; ++j) {
-          const int tok = b0 + c + j;
-          float fin = 0.f;
-          if (tok < M && a_idx < N) {
-            float r = v[j];
-            if (resid) r += Num<T>::to_f(resid[(size_t)tok * p.ldr + a_idx]);
-            const T rt = Num<T>::from_f(r);
-            out[(size_t)tok * p.ldo + a_idx] = rt;
-            fin = Num<T>::to_f(rt);
-          }
-          if (emit_ss) ss_add(c + j, fin);
-        }
-        if (emit_ss && c + 16 >= bn) {
-          // last column group: one thread per token column adds the four warps' sums
-          __syncthreads();
-          for (int cc = tid; cc < ncols; cc += (int)blockDim.x)
-            p.ss_out[(size_t)blockIdx.x * p.ss_ld + b0 + cc] = ss_w[0][cc] + ss_w[1][cc] + ss_w[2][cc] + ss_w[3][cc];
         }
       } else {
         const int n0 = b0 + c;
@@ -1085,7 +1215,7 @@ static int plan_gemm(const RfGemm* g, GemmPlan* pl) {
     const int rows = swap ? kBM : pl->bn;
     stage_bytes += round_up((dual ? 2 : 1) * (g->w_bits == 4 ? ceil_div(rows, kBM) * rf_w4_block_bytes(g->w_group) : rows * kBK), 1024);
   }
-  const int ctl_bytes = (int)sizeof(GemmSmemCtl) + 64 + ((g->ss_in || g->ss_out) ? kSsScratchBytes : 0);
+  const int ctl_bytes = (int)sizeof(GemmSmemCtl) + 64 + (g->ss_in ? kSsScratchBytes : 0);
   const bool publish = g->ar_world > 1 && g->ar_publish && swap;
   static const int env_smem_kb = [] { const char* e = getenv("RF_GEMM_SMEM_KB"); return e ? atoi(e) : 0; }();
 
@@ -1133,9 +1263,13 @@ static int plan_gemm(const RfGemm* g, GemmPlan* pl) {
       for (int S = 8; S >= 2; S >>= 1) {
         if (S > max_by_k || tiles * S > cap) continue;
         int st, part;
-        const int b = tiles * S > sm_count() ? kTwoCtaSmem : 224 * 1024;
+        const int b = tiles * S > sm_count() || S == 8 ? kTwoCtaSmem : 224 * 1024;
         const size_t smem = layout(S, b, &st, &part);
         if (st < 2 || smem > 227 * 1024) continue;
+        // A parked partial that takes more than half of shared memory leaves one CTA to an SM: then a grid of more CTAs than SMs runs
+        // in two rounds, and clusters of eight do not all find a place (fp16, us, with / without this line: 128 x 12288 x 4096 SwiGLU
+        // 81 / 46, 256 x 4096 x 12288 78 / 33, 256 x 2048 x 8192 35 / 24).
+        if (smem > kTwoCtaSmem && (tiles * S > sm_count() || S == 8)) continue;
         splits = S;
         break;
       }
@@ -1143,7 +1277,9 @@ static int plan_gemm(const RfGemm* g, GemmPlan* pl) {
     {
       int st, part;
       layout(splits, kTwoCtaSmem, &st, &part);
-      budget = (tiles * splits > sm_count() && st >= 2) ? kTwoCtaSmem : 224 * 1024;
+      // clusters of eight that own their SMs do not all find a place at once (16 of them: 20.9 us for 1 x 2048 x 8192, 16.0 with half as
+      // many CTAs in clusters of four, 11.2 with two CTAs to an SM)
+      budget = ((tiles * splits > sm_count() || splits == 8) && st >= 2) ? kTwoCtaSmem : 224 * 1024;
     }
   }
   if (env_smem_kb > 0) budget = std::min(224, std::max(48, env_smem_kb)) * 1024;
@@ -1239,6 +1375,9 @@ static int launch_gemm(const RfGemm* g, const GemmPlan& pl, cudaStream_t stream)
   p.ss_out = SWAP ? g->ss_out : nullptr;
   p.ss_in = SWAP ? g->ss_in : nullptr;
   p.ss_tiles = g->ss_tiles; p.ss_ld = g->ss_ld;
+  p.aff_vec = ((reinterpret_cast<uintptr_t>(g->bias) | reinterpret_cast<uintptr_t>(g->scale)) & 15) == 0 && (g->dual_offset & 7) == 0;
+  p.res_vec = (g->ldr & 7) == 0 && (reinterpret_cast<uintptr_t>(g->residual) & 15) == 0;
+  p.out_vec = (g->ldo & 7) == 0 && (reinterpret_cast<uintptr_t>(g->out) & 15) == 0;
   p.ss_inv_dim = g->ss_dim > 0 ? 1.f / (float)g->ss_dim : 0.f;
   p.ss_eps = g->ss_eps;
   p.w4 = (W8 && g->w_bits == 4) ? 1 : 0;

@@ -894,6 +894,35 @@ def test_gemm_small_dual_glu(dt, M, N, K, packed, status):
 
 
 @pytest.mark.parametrize("dt", DT)
+@pytest.mark.parametrize("M,N,K,splits", [(1, 128, 512, 8), (16, 136, 576, 3), (17, 1000, 640, 2), (65, 264, 1024, 4), (93, 300, 1024, 8),
+                                          (33, 7, 256, 1), (130, 640, 512, 1), (256, 384, 256, 2)])
+@pytest.mark.parametrize("vec", [True, False])
+def test_gemm_weight_row_epilogue(dt, M, N, K, splits, vec, status, monkeypatch):
+    """Few tokens, weights on the MMA rows: parked partials, the splits' sums and the eight-feature finish against fp32 - one split in
+    passes of 64 (32 for a GLU) tokens, two to eight splits, token and feature counts that end inside a group, operands that cannot be
+    read as 16-byte vectors."""
+    from rhinoforge_b200.ops import kernels as K_
+    monkeypatch.setenv("RF_GEMM_SMALL", "0")
+    x = (torch.randn(M, K, device="cuda") * 0.5).to(dt)
+    w = (torch.randn(2 * N, K, device="cuda") * 0.05).to(dt)
+    off, pitch = (0, (N + 7) // 8 * 8) if vec else (1, N + 3)
+    vector = lambda n, base: (base + 0.2 * torch.randn(n + 1, device="cuda")).to(dt)[off:off + n]
+    b, sc, r = vector(N, 0.0), vector(N, 1.0), torch.randn(M, pitch, device="cuda").to(dt)[:, :N]
+    out = torch.full((M, pitch), 7.0, device="cuda").to(dt)
+    y = K_.gemm(x, K_.pack_weight(w[:N]), packed_shape=(N, K), bias=b, scale=sc, residual=r, out=out[:, :N], status=status, force_splits=splits, force_swap=1)
+    z = x.float() @ w.float().t()
+    ref = z[:, :N] * sc.float() + b.float() + r.float()
+    _close(y, ref, dt, scale=max(1.0, ref.abs().max().item()))
+    assert bool((out[:, N:] == 7.0).all())
+    try:
+        y = K_.gemm(x, K_.pack_weight(w, 2), packed_shape=(2 * N, K), act="silu_mul", dual=True, status=status, force_splits=splits, force_swap=1)
+    except Exception as e:
+        assert M > 128 and "partial" in str(e)                 # two parked accumulators of this many tokens do not fit
+    else:
+        _close(y, torch.nn.functional.silu(z[:, :N]) * z[:, N:], dt, scale=2.0)
+
+
+@pytest.mark.parametrize("dt", DT)
 @pytest.mark.parametrize("M,N,K", [(5000, 1152, 256), (4100, 4304, 128), (2500, 136, 520), (768, 4304, 1152), (825, 2560, 2048), (6000, 328, 64)])
 @pytest.mark.parametrize("vec", [True, False])
 def test_gemm_persistent_epilogue(dt, M, N, K, vec, status):
