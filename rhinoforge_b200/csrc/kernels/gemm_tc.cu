@@ -1483,6 +1483,8 @@ namespace rf {
 bool gemm_sk_eligible(const RfGemm* g, int* ctas);               // gemm_sk.cu: persistent stream-K kernel for small M
 bool gemm_small_eligible(const RfGemm* g);                         // gemm_small.cu: latency-bound shapes (few rows, small weight)
 int gemm_small_run(const RfGemm* g, cudaStream_t stream);
+bool gemm_rows_takes(const RfGemm* g);                             // gemm_rows.cu: very few rows, weights straight into MMA fragments
+int launch_gemm_rows(const RfGemm* g, cudaStream_t stream);
 void gemm_sk_scratch(const RfGemm* g, uint64_t* ws_bytes, int32_t* flags);
 int launch_gemm_sk(const RfGemm* g, cudaStream_t stream);
 bool gemm_ps_eligible(const RfGemm* g, bool swap, int splits, int bn, int tiles);   // gemm_ps.cu: persistent kernel for large M
@@ -1496,6 +1498,7 @@ static int run_gemm(const RfGemm* g, cudaStream_t stream, bool w8) {
   if (g->mul) RF_REQUIRE(!w8 && g->mul_row && rf::gemm_small_eligible(g), "GEMM %dx%dx%d has no gate-by-token epilogue (see rf_gemm_takes_mul)", g->M, g->N, g->K);
   if (!w8 && rf::gemm_small_eligible(g)) return rf::gemm_small_run(g, stream);      // latency-bound shapes: gemm_small.cu
   if (!w8 && rf::gemm_sk_eligible(g, nullptr)) return rf::launch_gemm_sk(g, stream);
+  if (rf::gemm_rows_takes(g)) return rf::launch_gemm_rows(g, stream);
   GemmPlan pl;
   rc = plan_gemm(g, &pl);
   if (rc) return rc;

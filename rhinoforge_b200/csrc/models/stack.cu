@@ -19,6 +19,8 @@
 
 namespace rf {
 
+bool gemm_rows_takes(const RfGemm* g);      // gemm_rows.cu
+
 struct Stack {
   RfStackConfig cfg;
   std::vector<RfLayerWeights> layers;
@@ -172,6 +174,18 @@ static void hint_next_weights(const Stack& s, const void* w, const void* scale, 
 static thread_local float* t_ss_out = nullptr;
 static thread_local const float* t_ss_in = nullptr;
 
+// Whether a linear layer of these sizes will run on the kernel that takes the squares of its input rows itself (gemm_rows.cu): then nobody
+// has to write their sums for it.
+static bool norms_itself(const Stack& s, const void* x, int M, int N, int K, int dual_offset) {
+  RfGemm g = {};
+  g.x = x;
+  g.M = M; g.N = N; g.K = K; g.dtype = s.cfg.dtype; g.dual_offset = dual_offset;
+  g.w_packed = s.cfg.weights_packed;
+  g.force_swap = -1;
+  g.streaming_only = s.cfg.gemm_streaming_only ? (s.cfg.tp_world > 1 ? 2 : 1) : 0;
+  return s.cfg.tp_world <= 1 && gemm_rows_takes(&g);
+}
+
 // One linear layer: picks GEMV / tcgen05 GEMM / W8A16 and wires the fused all-reduce.  pub_ctas != null asks for
 // the publish-and-exit form: *pub_ctas receives the CTA count the consumer must wait for, or 0 when the shape took
 // the in-kernel form after all (more than 256 tokens), in which case `out` and `residual` were used as given.
@@ -195,7 +209,8 @@ static int linear(const Stack& s, const void* x, int64_t ldx, const void* w, con
   }
   g.status = s.status();
   g.force_swap = -1;
-  g.streaming_only = s.cfg.gemm_streaming_only;
+  // the ranks of a tensor-parallel group stay with one kernel family, whatever their shards' shapes
+  g.streaming_only = s.cfg.gemm_streaming_only ? (s.cfg.tp_world > 1 ? 2 : 1) : 0;
   g.prefetch = t_pf_ptr; g.prefetch_bytes = t_pf_bytes;
   t_pf_ptr = nullptr; t_pf_bytes = 0;
   if (t_ss_out || t_ss_in) {
@@ -504,7 +519,7 @@ static int forward(Stack& s, const RfStackForward& f, cudaStream_t st) {
                        mix_dim, kActNone, 0, st);
       if (rc) return rc;
     } else if (!side) {
-      if (fuse_ss) t_ss_out = ss_attn;
+      if (fuse_ss && !norms_itself(s, f.hidden, T, I, H, s.glu() ? I : 0)) t_ss_out = ss_attn;
       rc = linear_ar(s, mix_out, mix_dim, w.wo, w.so, w.bo, f.hidden, f.hidden, T, mix_dim,
                      norm_rides ? w.norm2_w : nullptr, xn, &have_xn2, st, /*rows_stay=*/true);
       if (rc) return rc;
@@ -571,7 +586,7 @@ static int forward(Stack& s, const RfStackForward& f, cudaStream_t st) {
     const void* next_w = (norm_rides && l + 1 < le && !hook_after) ? s.layers[l + 1].norm1_w : nullptr;
     if (l + 1 < le && s.layers[l + 1].mixer != 1) hint_next_weights(s, s.layers[l + 1].wqkv, s.layers[l + 1].sqkv, QD, H, 1, T);
     if (fuse_ss && l + 1 < le && !hook_after) {
-      t_ss_out = ss_mlp;
+      if (!norms_itself(s, f.hidden, T, QD, H, 0)) t_ss_out = ss_mlp;
       ss_ready = true;
     }
     if (twin) {

@@ -95,7 +95,7 @@ typedef struct RfGemm {
   const float* ss_in;
   int32_t ss_ld, ss_dim;
   float ss_eps;
-  int32_t streaming_only;      // 1: never the latency-bound mma.sync kernel (gemm_small.cu), whatever the shape
+  int32_t streaming_only;      // 1: never the latency-bound mma.sync kernel (gemm_small.cu), whatever the shape; 2: only the tcgen05 kernels
   // Gate by token (shapes for which rf_gemm_takes_mul returns 1): the activated result of row m, column n is multiplied by
   // mul[mul_row[m] * mul_ld + n] (same dtype), a slice of an embedding table.
   const void* mul; const int32_t* mul_row; int64_t mul_ld;

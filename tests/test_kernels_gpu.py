@@ -945,3 +945,56 @@ def test_gemm_persistent_epilogue(dt, M, N, K, vec, status):
     ref = torch.nn.functional.gelu(z + b.float(), approximate="tanh") + r[:, :N].float()
     _close(acc[:, :N], ref, dt, scale=scale)
     assert torch.equal(acc[:, N:], r[:, N:])
+
+
+@pytest.mark.parametrize("dt", DT)
+@pytest.mark.parametrize("M,N,K", [(1, 16, 64), (1, 1000, 72), (7, 264, 520), (8, 40, 8), (9, 1536, 1024), (16, 5000, 1160), (3, 24, 4096), (16, 7, 2048)])
+@pytest.mark.parametrize("dual", [False, True])
+def test_gemm_very_few_rows(dt, M, N, K, dual, status):
+    """Up to 16 rows over 16-bit weights: strips of 16 features that end inside a weight block or past N, fewer k blocks than warps and
+    partial ones, every epilogue option, strided and odd-pitched outputs, a CTA that takes several strips; the RMSNorm that the kernel
+    folds in itself."""
+    from rhinoforge_b200.ops import kernels as K_
+    rows = 2 * N if dual else N
+    x = (torch.randn(M, K + 8, device="cuda") * 0.5).to(dt)[:, :K]
+    w = (torch.randn(rows, K, device="cuda") / K ** 0.5).to(dt)
+    wp = K_.pack_weight(w, 2 if dual else 1)
+    b, sc = torch.randn(rows, device="cuda").to(dt), (torch.rand(rows, device="cuda") + 0.5).to(dt)
+    rs, r = torch.rand(M, device="cuda") + 0.5, torch.randn(M, N, device="cuda").to(dt)
+    out = torch.full((M, N + 3), 7.0, device="cuda").to(dt)
+    kw = dict(packed_shape=(rows, K), status=status, **(dict(act="silu_mul", dual=True) if dual else {}))
+    finish = lambda z: torch.nn.functional.silu(z[:, :N]) * z[:, N:] if dual else z
+    K_.gemm(x, wp, bias=b, scale=sc, row_scale=rs, residual=r, out=out[:, :N], **kw)
+    z = x.float() @ w.float().t()
+    _close(out[:, :N], finish(z * rs[:, None] * sc.float() + b.float()) + r.float(), dt, scale=2.0)
+    assert bool((out[:, N:] == 7.0).all())
+    ss = torch.zeros((max(K // 128, 1), 256), device="cuda")
+    ss[0, :M] = x.float().pow(2).sum(1)
+    _close(K_.gemm(x, wp, ss_in=ss, ss_dim=K, ss_eps=1e-6, **kw), finish(z * torch.rsqrt(x.float().pow(2).mean(1, keepdim=True) + 1e-6)), dt, scale=4.0)
+
+
+@pytest.mark.parametrize("dt", DT)
+@pytest.mark.parametrize("M", [1, 8, 11, 16])
+@pytest.mark.parametrize("N,K,group,fp4", [(264, 320, 0, False), (1000, 1024, 64, False), (40, 2176, 32, False), (128, 192, 16, True), (5008, 512, None, False)])
+@pytest.mark.parametrize("dual", [False, True])
+def test_gemm_very_few_rows_quantised(dt, M, N, K, group, fp4, dual, status):
+    """Up to 16 rows over int8 (``group`` None) and 4-bit weights, against the product with the values that the image holds."""
+    from rhinoforge_b200.ops import kernels as K_
+    rows = 2 * N if dual else N
+    x = (torch.randn(M, K, device="cuda") / K ** 0.5).to(dt)
+    sc = (torch.rand(rows, device="cuda") * 0.2 + 0.1).to(dt)
+    kw = dict(packed_shape=(rows, K), status=status, **(dict(act="silu_mul", dual=True) if dual else {}))
+    sections = 2 if dual else 1
+    if group is None:
+        q = torch.randint(-127, 128, (rows, K), device="cuda", dtype=torch.int8)
+        y, w = K_.gemm(x, K_.pack_weight(q, sections), scale=sc, **kw), q.float() * sc.float()[:, None]
+    else:
+        q = torch.randint(-8, 8, (rows, K), device="cuda", dtype=torch.int8)
+        gs = (torch.rand(rows, K // group, device="cuda") * 0.2 + 0.1).to(dt) if group else None
+        value = torch.tensor([0, 0.5, 1, 1.5, 2, 3, 4, 6, -0.0, -0.5, -1, -1.5, -2, -3, -4, -6], device="cuda")[(q & 15).long()] if fp4 else q.float()
+        img = K_.pack_weight_int4(q, gs, group, sections=sections, dtype=dt)
+        y = K_.gemm(x, img, w_bits=4, w_group=group, w_fp4=fp4, scale=None if group else sc, **kw)
+        w = (value.view(rows, -1, group) * gs.float()[..., None]).view(rows, K).to(dt).float() if group else value * sc.float()[:, None]
+    z = x.float() @ w.t()
+    ref = torch.nn.functional.silu(z[:, :N]) * z[:, N:] if dual else z
+    _close(y, ref, dt, scale=max(1.0, ref.abs().max().item()))
