@@ -577,7 +577,7 @@ class DecoderEngine:
             cache.ensure(slots[s], starts[s] + L + decode_room)
         cache.sync_table()
         logits_all = torch.empty((B, self.vocab_local), dtype=self.dtype, device=self.device) if return_logits else None
-        first = torch.zeros(B, dtype=torch.int32, device=self.device)
+        first = torch.empty(B, dtype=torch.int32, device=self.device)
         chunk: List[tuple] = []
         used = 0
         items: List[List[tuple]] = []
@@ -609,16 +609,17 @@ class DecoderEngine:
         # decode state: the token to feed next is `first`, at position = new length
         self.ids[:B].copy_(first)
         new_len = torch.from_numpy(cache.lengths[:B].astype("int32"))
+        new_len = torch.stack((new_len, new_len + 1))
         if self.device.type == "cuda":
             new_len = new_len.pin_memory()
-        new_len = new_len.to(self.device, non_blocking=True)
+        new_len, next_len = new_len.to(self.device, non_blocking=True)
         if positions3 is not None:
             # generation continues one past the largest position on all three axes
             nxt = torch.stack([p.max().to(self.device) + 1 for p in positions3]).to(torch.int32)
             self.pos[:B].copy_(nxt[:, None].expand(B, self.pos_stride))
         else:
             self.pos[:B].copy_(new_len[:, None].expand(B, self.pos_stride))
-        self.kv_len[:B].copy_(new_len + 1)
+        self.kv_len[:B].copy_(next_len)
         return self._extend_result(first, logits_all, row_logits, return_logits)
 
     def _extend_result(self, first, logits_all, row_logits, return_logits):
@@ -646,22 +647,26 @@ class DecoderEngine:
                        deepstack=None, row_logits=None, slots=None) -> None:
         T = sum(c[2] for c in ch)
         n = len(ch)
-        meta = torch.empty((6, max(n, 1)), dtype=torch.int32)
-        tokmeta = torch.empty((2, T), dtype=torch.int32)
-        ids_host = torch.empty(T, dtype=torch.int32)
+        # Everything the launch reads from the host travels in one upload: six rows of n numbers (first row, new rows, K/V length, cache slot,
+        # last row, starts from an empty state), the sequences' page-table rows, three rows of T (sequence, position, token id).
+        # Reading anything back or making one of these on the device would wait for the launches before it.
+        pages = self.cache.page_table.shape[1]
+        up4 = lambda v: (v + 3) // 4 * 4           # every row of the upload starts on 16 bytes
+        sections = ((6, up4(n)), (n, up4(pages)), (3, up4(T)))
+        cut = lambda buf: [part.view(*shape) for part, shape in zip(buf.split([r * c for r, c in sections]), sections)]
+        host = torch.empty(sum(r * c for r, c in sections), dtype=torch.int32)
+        meta, table, tokmeta = cut(host)
         o = 0
         emb_rows = []
         pos3 = []
         ds_rows, ds_feats = [], None
         for j, (s, off, cnt) in enumerate(ch):
             base = starts[s]
-            meta[0, j], meta[1, j], meta[2, j] = o, cnt, base + off + cnt   # q_start, q_len, kv_len
-            meta[3, j] = slots[s]
-            meta[4, j] = o + cnt - 1
-            meta[5, j] = 1 if (base + off) == 0 else 0        # starts from an empty recurrent state
-            tokmeta[0, o:o + cnt] = s
+            meta[:, j] = torch.tensor((o, cnt, base + off + cnt, slots[s], o + cnt - 1, int(base + off == 0)), dtype=torch.int32)
+            table[j, :pages] = self.cache._pt_host[slots[s]]
+            tokmeta[0, o:o + cnt] = j
             tokmeta[1, o:o + cnt] = torch.arange(base + off, base + off + cnt, dtype=torch.int32)
-            ids_host[o:o + cnt] = prompts[s][off:off + cnt].to("cpu", torch.int32)
+            tokmeta[2, o:o + cnt] = prompts[s][off:off + cnt].to("cpu", torch.int32)
             if inputs_embeds is not None:
                 emb_rows.append(inputs_embeds[s][off:off + cnt])
             if positions3 is not None:
@@ -677,22 +682,18 @@ class DecoderEngine:
                     for l, ft in enumerate(feats_s):
                         ds_feats[l].append(ft.to(self.device, self.dtype)[sel.to(self.device)])
             o += cnt
-        meta_d = meta.pin_memory().to(self.device, non_blocking=True)
-        tok_d = tokmeta.pin_memory().to(self.device, non_blocking=True)
-        ids_d = ids_host.pin_memory().to(self.device, non_blocking=True)
-        # the page table the kernels see is indexed by chunk-local sequence number
-        pt = self.cache.page_table[meta_d[3].long()].contiguous()
-        seq_local = torch.repeat_interleave(torch.arange(n, dtype=torch.int32, device=self.device), meta_d[1].long())
+        dev = host.pin_memory().to(self.device, non_blocking=True)
+        meta_d, pt, tok_d = cut(dev)
+        qs, ql, kl, slot_d, last_d, fresh_d = meta_d[:, :n]
+        seq_local, cache_pos, ids_d = tok_d[:, :T]
         if inputs_embeds is not None:
             self.hidden[:T].copy_(torch.cat(emb_rows).to(self.device, self.dtype))
         else:
             self._embed(ids_d, T)
         if positions3 is not None:
             pos_d = torch.cat(pos3).to(self.device, torch.int32).contiguous()
-            cache_pos = tok_d[1].contiguous()
         else:
-            pos_d = tok_d[1].contiguous() if self.pos_stride == 1 else tok_d[1][:, None].expand(T, 3).contiguous()
-            cache_pos = tok_d[1].contiguous()
+            pos_d = cache_pos if self.pos_stride == 1 else cache_pos[:, None].expand(T, 3).contiguous()
         f = N.RfStackForward()
         f.hidden, f.tokens, f.decode = self.hidden.data_ptr(), T, 0
         f.pos, f.pos_stride = pos_d.data_ptr(), self.pos_stride
@@ -700,13 +701,11 @@ class DecoderEngine:
         f.axis_of_freq = None if self.axis is None else self.axis.data_ptr()
         f.seq_of_tok, f.cache_pos = seq_local.data_ptr(), cache_pos.data_ptr()
         f.num_seqs = n
-        qs, ql, kl = meta_d[0].contiguous(), meta_d[1].contiguous(), meta_d[2].contiguous()
         f.q_start, f.q_len, f.kv_len = qs.data_ptr(), ql.data_ptr(), kl.data_ptr()
         f.max_q_len = max(c[2] for c in ch)
         f.max_kv_len = max(starts[c[0]] + c[1] + c[2] for c in ch)
         f.page_table, f.pt_stride, f.pool_pages = pt.data_ptr(), pt.stride(0), self.cache.num_pages
         if self.gdn_layers:
-            slot_d, fresh_d = meta_d[3].contiguous(), meta_d[5].contiguous()
             f.state_slot, f.state_fresh = slot_d.data_ptr(), fresh_d.data_ptr()
         if ds_rows:
             ds_rows_d = torch.cat(ds_rows).to(torch.int32).pin_memory().to(self.device, non_blocking=True)
@@ -727,18 +726,13 @@ class DecoderEngine:
                     self._head(nr, idx, lg)
                     row_logits["out"][s].append(lg)
                 o2 += cnt
-        # sequences whose prompt ends in this chunk get their first token
-        done = [(j, s) for j, (s, off, cnt) in enumerate(ch) if off + cnt == lens[s]]
-        if done:
-            rows = meta_d[4][torch.tensor([j for j, _ in done], device=self.device)].contiguous()
-            for b0 in range(0, len(done), self.max_batch):
-                sub = done[b0:b0 + self.max_batch]
-                lg = torch.empty((len(sub), self.vocab_local), dtype=self.dtype, device=self.device) if logits_all is not None else None
-                self._head(len(sub), rows[b0:b0 + len(sub)].contiguous(), lg)
-                dst = torch.tensor([s for _, s in sub], device=self.device)
-                first[dst] = self.out_ids[:len(sub)]
-                if logits_all is not None:
-                    logits_all[dst] = lg
+        # sequences whose prompt ends in this chunk get their first token: a chunk takes them in order, so they are neighbours
+        done = [j for j, (s, off, cnt) in enumerate(ch) if off + cnt == lens[s]]
+        for b0 in range(0, len(done), self.max_batch):
+            j0, k = done[b0], min(self.max_batch, len(done) - b0)
+            s0 = ch[j0][0]
+            self._head(k, last_d[j0:j0 + k], None if logits_all is None else logits_all[s0:s0 + k])
+            first[s0:s0 + k].copy_(self.out_ids[:k])
 
     # ------------------------------------------------------------------- decode
     def _decode_step(self, B: int, logits_out: Optional[torch.Tensor] = None) -> None:
