@@ -1,15 +1,24 @@
 // Flash attention (prefill) on the 5th-generation tensor cores.
 //
-// One CTA owns 128 query rows of one head.  Both GEMMs of attention run as tcgen05.mma with
+// One CTA owns one or two tiles of 128 query rows of one head.  Both GEMMs of attention run as tcgen05.mma with
 // accumulators in tensor memory:
 //   S = Q . K^T   A = Q tile  [128 x HD]  (K-major, smem)   B = K tile [KVB x HD] (K-major, smem)   D = S in TMEM
 //   O += P . V    A = P tile  [128 x KVB] (K-major, smem)   B = V tile [KVB x HD] (MN-major, smem)  D = O in TMEM
-// Warp roles: warp 0 = TMA producer (K/V pages or rows, double buffered), warp 1 = MMA issuer (and
-// TMEM owner), warps 2-5 = softmax: thread r owns query row r, which is TMEM lane r, so row max and
+// Warp roles: warp 0 = TMA producer (K/V pages or rows through a ring), warp 1 = MMA issuer (and
+// TMEM owner), then four softmax warps per tile: thread r owns query row r, which is TMEM lane r, so row max and
 // row sum need no shuffles.  S is double buffered in TMEM: Q.K^T of block j+1 runs on the tensor core
 // while the softmax warps work on block j.  The running maximum is only raised when a block exceeds
 // it by more than 2^8 (the accumulator and the row sum share the stale maximum, so the final
 // O / l is exact); raising it rescales the O accumulator in TMEM (tcgen05.ld / tcgen05.st).
+//
+// What bounds it: a block of one tile is a chain - S from TMEM, maximum, 64 exponentials a thread (512 cycles of the special-function
+// unit for a warp), P to shared memory, P.V - of some 1100 cycles, so that an SM needs two tiles in different places of their chains, and K/V
+// must be under way earlier than that.  Two tiles in ONE CTA share the K/V blocks (half the copies, and they come in 2 KB boxes) and leave room for
+// a ring of four; two CTAs of one tile each with two-block rings waited for their copies (2.1 us a block).  One tile to a CTA is for short
+// inputs, where the CTAs would not fill the GPU otherwise, and for heads above 128.
+// fp16, us (one tile with a two-block ring / now), heads of 128 unless said: 128 queries x 2048 keys 76 / 41 (the chain alone: one CTA per SM);
+// 8192 causal, 32 + 8 heads 1324 / 951; 8192 queries on 16384 keys 3317 / 2522; 8 x 1024 causal 382 / 273; 6 x 1100, window 1024 194 / 141;
+// 2 x 4096, heads of 64 588 / 481; 12 x 256 full 45 / 41 (one tile each); 93 causal, heads of 64 14.2 / 13.6.
 // V needs no transpose: the [tokens x 64] slabs a TMA box leaves in shared memory are exactly the
 // MN-major 128-byte-swizzle operand layout.
 //
@@ -25,35 +34,42 @@ namespace rf {
 
 constexpr int kFaRows = 128;          // query rows per CTA
 constexpr int kFaBox = 16 * 128;      // one TMA box: 16 rows x 64 x 16-bit
-constexpr int kFaThreads = 192;
+constexpr int kFaMaxStages = 8;
 constexpr float kFaRaise = 8.0f;      // raise the reference maximum only beyond 2^8
 
 struct alignas(8) FaCtl {
-  uint64_t q_full, kv_full[2], kv_empty[2], s_full[2], s_empty[2], p_full, p_empty, o_full;
+  uint64_t q_full, kv_full[kFaMaxStages], kv_empty[kFaMaxStages], s_full[2][2], s_empty[2][2], p_full[2], p_empty[2], o_full[2];
   uint32_t tmem_base;
   int32_t abort_flag;
 };
 
-// HD: size of a query / key head, VD: of a value head
-template <int HD, int VD> struct FaGeom {
+// HD: size of a query / key head, VD: of a value head, NQ: query tiles of a CTA
+template <int HD, int VD, int NQ> struct FaGeom {
   static constexpr int J = HD / 64, JV = VD / 64;        // 64-column chunks of the heads
-  static constexpr int KVB = 64;                         // kv tokens per block: small enough for TWO CTAs per SM
-                                                         // (HD <= 128), whose softmax and MMA phases interleave
+  static constexpr int KVB = 64;                         // kv tokens per block
   static constexpr int PC = KVB / 64;                    // 64-token chunks of P
-  static constexpr int kQBytes = J * kFaRows * 128;
+  static constexpr int kQTile = J * kFaRows * 128;
   static constexpr int kKBytes = J * KVB * 128;          // K of one stage, V behind it
   static constexpr int kStageBytes = kKBytes + JV * KVB * 128;
-  static constexpr int kPBytes = PC * kFaRows * 128;
-  static constexpr int kSmem = kQBytes + 2 * kStageBytes + kPBytes;
-  static constexpr int kTmemCols = VD == 256 ? 512 : 256; // 2 x KVB (S) + VD (O), rounded up to a power of two
-  static constexpr int kOCol = 2 * KVB;
+  static constexpr int kPTile = PC * kFaRows * 128;
+  static constexpr int kFixed = NQ * (kQTile + kPTile);  // the ring lies behind Q and P
+  static constexpr int kSCols = NQ * 2 * KVB;            // S: two buffers per tile, then O per tile
+  static constexpr int kTmemCols = kSCols + NQ * VD > 256 ? 512 : 256;
+  static constexpr int kThreads = 64 + NQ * 128;
+  static_assert(kSCols + NQ * VD <= 512, "accumulators do not fit tensor memory");
 };
+// 2^x on the special-function unit, results below 2^-126 flushed to zero
+__device__ __forceinline__ float ex2(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
 
-template <typename T, int HD, int VD>
-__global__ void __launch_bounds__(kFaThreads)
+template <typename T, int HD, int VD, int NQ>
+__global__ void __launch_bounds__(FaGeom<HD, VD, NQ>::kThreads, NQ == 1 && HD <= 128 ? 2 : 1)
 attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
-                       const __grid_constant__ CUtensorMap tmV, const AttnParams p) {
-  using G = FaGeom<HD, VD>;
+                       const __grid_constant__ CUtensorMap tmV, const AttnParams p, const int stages) {
+  using G = FaGeom<HD, VD, NQ>;
   constexpr int J = G::J, JV = G::JV, KVB = G::KVB;
   // No alignment slack: two CTAs of the HD <= 128 configuration fill the SM's shared memory to within 2 KB.
   // The swizzled tiles need a 1024-byte aligned base, which the runtime provides when the kernel has no
@@ -65,42 +81,56 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
     return;
   }
   uint8_t* qsm = smem;
-  uint8_t* kvsm = smem + G::kQBytes;
-  uint8_t* psm = kvsm + 2 * G::kStageBytes;
-  FaCtl* ctl = reinterpret_cast<FaCtl*>(psm + G::kPBytes);
+  uint8_t* psm = smem + NQ * G::kQTile;
+  uint8_t* kvsm = smem + G::kFixed;
+  FaCtl* ctl = reinterpret_cast<FaCtl*>(kvsm + (size_t)stages * G::kStageBytes);
 
-  const int qt = blockIdx.x, h = blockIdx.y, seq = blockIdx.z;
+  // heads run fastest, the last rows of a sequence first: under a causal mask they have the most keys, and what is left for the end is short
+  const int h = blockIdx.x, seq = blockIdx.z;
+  const int qt0 = (int)(gridDim.y - 1 - blockIdx.y) * NQ;   // first query tile of this CTA
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int qlen = p.q_len[seq];
-  if (qt * kFaRows >= qlen) return;                       // before any barrier or allocation
+  if (qt0 * kFaRows >= qlen) return;                      // before any barrier or allocation
   const int kvlen = p.kv_len[seq];
   const int kvh = h / p.G;
   const int pt_row = p.slot ? p.slot[seq] : seq;
   const int qpos0 = kvlen - qlen;                         // position of query row 0 on the kv axis
-  const int q_row0 = p.q_start[seq] + qt * kFaRows;
-  const int rows_here = min(kFaRows, qlen - qt * kFaRows);
-  int kv_hi = kvlen;
-  if (p.causal) kv_hi = min(kvlen, qpos0 + qt * kFaRows + rows_here);
+  const int q_row0 = p.q_start[seq] + qt0 * kFaRows;
+  const int tiles = NQ == 1 ? 1 : min(NQ, (qlen - qt0 * kFaRows + kFaRows - 1) / kFaRows);   // tiles that have rows
+  const int first = qpos0 + qt0 * kFaRows;                // position of the CTA's first query row
   int kv_lo = 0;
-  if (p.window > 0) kv_lo = max(0, qpos0 + qt * kFaRows - p.window + 1);
-  if (p.chunk > 0) kv_lo = max(kv_lo, (qpos0 + qt * kFaRows) / p.chunk * p.chunk);   // the first row's chunk
+  if (p.window > 0) kv_lo = max(0, first - p.window + 1);
+  if (p.chunk > 0) kv_lo = max(kv_lo, first / p.chunk * p.chunk);   // the first row's chunk
   kv_lo &= ~(KVB - 1);
   // blocks of the kept first positions come first, then those from the first row's window or chunk on
   const int keep_blk = min((p.keep_first + KVB - 1) / KVB, kv_lo / KVB);
-  const int nblk = kv_hi > kv_lo ? keep_blk + (kv_hi - kv_lo + KVB - 1) / KVB : 0;
   auto block_start = [&](int j) { return j < keep_blk ? j * KVB : kv_lo + (j - keep_blk) * KVB; };
+  // a tile's blocks: up to the last key its last row sees (the CTA's tiles walk the same list, the first one may stop earlier)
+  auto blocks_of = [&](int t) {
+    const int rows = min(kFaRows, qlen - (qt0 + t) * kFaRows);
+    const int hi = p.causal ? min(kvlen, first + t * kFaRows + rows) : kvlen;
+    return hi > kv_lo ? keep_blk + (hi - kv_lo + KVB - 1) / KVB : 0;
+  };
+  int nblk_t[NQ];
+#pragma unroll
+  for (int t = 0; t < NQ; ++t) nblk_t[t] = t < tiles ? blocks_of(t) : 0;
+  const int nblk = NQ == 1 ? nblk_t[0] : max(nblk_t[0], nblk_t[NQ - 1]);
 
   if (tid == 0) {
     mbar_init(&ctl->q_full, 1);
-    for (int s = 0; s < 2; ++s) {
+    for (int s = 0; s < stages; ++s) {
       mbar_init(&ctl->kv_full[s], 1);
       mbar_init(&ctl->kv_empty[s], 1);
-      mbar_init(&ctl->s_full[s], 1);
-      mbar_init(&ctl->s_empty[s], 4);
     }
-    mbar_init(&ctl->p_full, 4);
-    mbar_init(&ctl->p_empty, 1);
-    mbar_init(&ctl->o_full, 1);
+    for (int t = 0; t < NQ; ++t) {
+      for (int b = 0; b < 2; ++b) {
+        mbar_init(&ctl->s_full[t][b], 1);
+        mbar_init(&ctl->s_empty[t][b], 4);
+      }
+      mbar_init(&ctl->p_full[t], 4);
+      mbar_init(&ctl->p_empty[t], 1);
+      mbar_init(&ctl->o_full[t], 1);
+    }
     ctl->abort_flag = 0;
     fence_barrier_init();
     tma_prefetch_desc(&tmQ);
@@ -124,12 +154,11 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
     // the warp reads 32 page numbers at a time, one lane issues the copies
     constexpr int kPagesPerBlock = KVB / 16, kBlocksPerFetch = 32 / kPagesPerBlock;
     if (lane == 0) {
-      mbar_arrive_expect_tx(&ctl->q_full, (uint32_t)G::kQBytes);
+      mbar_arrive_expect_tx(&ctl->q_full, (uint32_t)(tiles * G::kQTile));
+      for (int t = 0; t < tiles; ++t)
 #pragma unroll
-      for (int c = 0; c < J; ++c)
-#pragma unroll
-        for (int rg = 0; rg < kFaRows / 16; ++rg)
-          tma_load_2d(qsm + c * (kFaRows * 128) + rg * kFaBox, &tmQ, &ctl->q_full, h * HD + c * 64, q_row0 + rg * 16);
+        for (int c = 0; c < J; ++c)
+          tma_load_2d(qsm + t * G::kQTile + c * (kFaRows * 128), &tmQ, &ctl->q_full, h * HD + c * 64, q_row0 + t * kFaRows);
     }
     {
       int issued = 0, pages = 0;
@@ -140,10 +169,10 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
 #pragma unroll
         for (int w = 0; w < kPagesPerBlock; ++w) block_pages[w] = __shfl_sync(0xffffffffu, pages, (j % kBlocksPerFetch) * kPagesPerBlock + w);
         int go = 1;
-        const int s = j & 1;
-        const uint32_t ph = (uint32_t)(j >> 1) & 1u;
+        const int s = j % stages;
+        const uint32_t ph = (uint32_t)(j / stages) & 1u;
         if (lane == 0) {
-          if (!mbar_wait(&ctl->kv_empty[s], ph ^ 1u, kLocalWaitNs, 64)) {
+          if (!mbar_wait(&ctl->kv_empty[s], ph ^ 1u, kLocalWaitNs, 32)) {
             report_status(p.status, kStatusTmaTimeout, kTagAttnPrefill, j);
             ctl->abort_flag = 1;
           }
@@ -157,29 +186,30 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
         mbar_arrive_expect_tx(&ctl->kv_full[s], (uint32_t)G::kStageBytes);
         // Whole blocks are always loaded: rows past the sequence end are other (finite) cache rows or the
         // zero fill beyond the tensor, and their probabilities are forced to zero.
+        if (p.paged) {
 #pragma unroll
-        for (int w = 0; w < kPagesPerBlock; ++w) {
-          int row, colk, colv;
-          if (p.paged) {
-            row = (block_pages[w] * p.Hkv + kvh) * 16;
-            colk = colv = 0;
-          } else {
-            row = p.kv_start[seq] + t0 + w * 16;
-            colk = kvh * HD;
-            colv = kvh * VD;
+          for (int w = 0; w < kPagesPerBlock; ++w) {
+            const int row = (block_pages[w] * p.Hkv + kvh) * 16;
+#pragma unroll
+            for (int c = 0; c < J; ++c) {
+              tma_load_2d(ks + c * (KVB * 128) + w * kFaBox, &tmK, &ctl->kv_full[s], c * 64, row);
+              if (c < JV) tma_load_2d(vs + c * (KVB * 128) + w * kFaBox, &tmV, &ctl->kv_full[s], c * 64, row);
+            }
           }
+        } else {
+          const int row = p.kv_start[seq] + t0;
 #pragma unroll
           for (int c = 0; c < J; ++c) {
-            tma_load_2d(ks + c * (KVB * 128) + w * kFaBox, &tmK, &ctl->kv_full[s], colk + c * 64, row);
-            if (c < JV) tma_load_2d(vs + c * (KVB * 128) + w * kFaBox, &tmV, &ctl->kv_full[s], colv + c * 64, row);
+            tma_load_2d(ks + c * (KVB * 128), &tmK, &ctl->kv_full[s], kvh * HD + c * 64, row);
+            if (c < JV) tma_load_2d(vs + c * (KVB * 128), &tmV, &ctl->kv_full[s], kvh * VD + c * 64, row);
           }
         }
         issued = j + 1;
       }
       if (lane == 0 && *abort_flag) {   // let every copy that was issued land before the CTA can exit
         mbar_wait(&ctl->q_full, 0, 20ull * 1000 * 1000);
-        for (int j = max(0, issued - 2); j < issued; ++j)
-          mbar_wait(&ctl->kv_full[j & 1], (uint32_t)(j >> 1) & 1u, 20ull * 1000 * 1000);
+        for (int j = max(0, issued - stages); j < issued; ++j)
+          mbar_wait(&ctl->kv_full[j % stages], (uint32_t)(j / stages) & 1u, 20ull * 1000 * 1000);
       }
     }
   } else if (warp == 1) {
@@ -187,38 +217,47 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
     if (lane == 0 && nblk > 0) {
       const uint32_t idesc_qk = umma_idesc_f16(kFaRows, KVB, Num<T>::kFmt, 0);
       const uint32_t idesc_pv = umma_idesc_f16(kFaRows, VD, Num<T>::kFmt, 1);
-      const uint32_t q_addr = smem_u32(qsm), p_addr = smem_u32(psm);
-      bool ok = mbar_wait(&ctl->q_full, 0, kLocalWaitNs, 32);
-      auto issue_qk = [&](int j) -> bool {
-        const int s = j & 1, b = j & 1;
-        if (!mbar_wait(&ctl->kv_full[s], (uint32_t)(j >> 1) & 1u, kLocalWaitNs, 32)) return false;
-        if (!mbar_wait(&ctl->s_empty[b], ((uint32_t)(j >> 1) & 1u) ^ 1u, kLocalWaitNs, 32)) return false;
+      // One lane issues every MMA, twelve per tile and block: the operand descriptors are made once and advance by constants (16-byte units)
+      const uint64_t q_desc = umma_desc_k128(smem_u32(qsm)), p_desc = umma_desc_k128(smem_u32(psm));
+      const uint64_t k_desc0 = umma_desc_k128(smem_u32(kvsm)), v_desc0 = umma_desc_mn128(smem_u32(kvsm) + G::kKBytes, (uint32_t)(KVB * 128));
+      bool ok = mbar_wait(&ctl->q_full, 0);
+      auto issue_qk = [&](int t, int j) -> bool {
+        const int s = j % stages, b = j & 1;
+        if (!mbar_wait(&ctl->kv_full[s], (uint32_t)(j / stages) & 1u)) return false;
+        if (!mbar_wait(&ctl->s_empty[t][b], ((uint32_t)(j >> 1) & 1u) ^ 1u)) return false;
         tc_fence_after_sync();
-        const uint32_t k_addr = smem_u32(kvsm + (size_t)s * G::kStageBytes);
+        const uint64_t qd = q_desc + (uint32_t)(t * (G::kQTile >> 4)), kd = k_desc0 + (uint32_t)(s * (G::kStageBytes >> 4));
+        const uint32_t d = tmem_base + (uint32_t)((t * 2 + b) * KVB);
 #pragma unroll
         for (int c = 0; c < J; ++c)
 #pragma unroll
           for (int kk = 0; kk < 4; ++kk)
-            umma_f16(tmem_base + (uint32_t)(b * KVB), umma_desc_k128(q_addr + c * (kFaRows * 128) + kk * 32),
-                     umma_desc_k128(k_addr + c * (KVB * 128) + kk * 32), idesc_qk, (c | kk) ? 1u : 0u);
-        umma_commit(&ctl->s_full[b]);
+            umma_f16(d, qd + (uint32_t)((c * kFaRows * 128 + kk * 32) >> 4), kd + (uint32_t)((c * KVB * 128 + kk * 32) >> 4), idesc_qk, (c | kk) ? 1u : 0u);
+        umma_commit(&ctl->s_full[t][b]);
         return true;
       };
-      if (ok) ok = issue_qk(0);
-      for (int j = 0; ok && j < nblk; ++j) {
-        if (j + 1 < nblk) ok = issue_qk(j + 1);          // runs while the softmax warps work on block j
-        if (!ok) break;
-        if (!mbar_wait(&ctl->p_full, (uint32_t)j & 1u, kLocalWaitNs, 32)) { ok = false; break; }
-        tc_fence_after_sync();
-        const int s = j & 1;
-        const uint32_t v_addr = smem_u32(kvsm + (size_t)s * G::kStageBytes + G::kKBytes);
 #pragma unroll
-        for (int t = 0; t < KVB / 16; ++t)
-          umma_f16(tmem_base + (uint32_t)G::kOCol, umma_desc_k128(p_addr + (t >> 2) * (kFaRows * 128) + (t & 3) * 32),
-                   umma_desc_mn128(v_addr + t * kFaBox, (uint32_t)(KVB * 128)), idesc_pv, (j | t) ? 1u : 0u);
-        umma_commit(&ctl->kv_empty[s]);
-        umma_commit(&ctl->p_empty);
-        if (j + 1 == nblk) umma_commit(&ctl->o_full);
+      for (int t = 0; t < NQ; ++t)
+        if (ok && nblk_t[t] > 0) ok = issue_qk(t, 0);
+      for (int j = 0; ok && j < nblk; ++j) {
+#pragma unroll
+        for (int t = 0; t < NQ; ++t)
+          if (ok && j + 1 < nblk_t[t]) ok = issue_qk(t, j + 1);      // runs while the softmax warps work on block j
+        const int s = j % stages;
+        const uint64_t vd = v_desc0 + (uint32_t)(s * (G::kStageBytes >> 4));
+#pragma unroll
+        for (int t = 0; t < NQ; ++t) {
+          if (!ok || j >= nblk_t[t]) continue;
+          if (!mbar_wait(&ctl->p_full[t], (uint32_t)j & 1u)) { ok = false; continue; }
+          tc_fence_after_sync();
+#pragma unroll
+          for (int k = 0; k < KVB / 16; ++k)
+            umma_f16(tmem_base + (uint32_t)(G::kSCols + t * VD), p_desc + (uint32_t)((t * G::kPTile + (k >> 2) * (kFaRows * 128) + (k & 3) * 32) >> 4),
+                     vd + (uint32_t)((k * kFaBox) >> 4), idesc_pv, (j | k) ? 1u : 0u);
+          umma_commit(&ctl->p_empty[t]);
+          if (j + 1 == nblk_t[t]) umma_commit(&ctl->o_full[t]);
+        }
+        if (ok) umma_commit(&ctl->kv_empty[s]);                     // every tile's products with this block
       }
       if (!ok) {
         if (!*abort_flag) report_status(p.status, kStatusMmaTimeout, kTagAttnPrefill, 1000);
@@ -227,16 +266,19 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
     }
   } else {
     // ------------------------------------------------- softmax / correction / epilogue ----
+    const int t = NQ == 1 ? 0 : (warp - 2) >> 2;          // this warp's query tile
+    const int nblk = t == 0 ? nblk_t[0] : nblk_t[NQ - 1];
     const int quarter = warp & 3;                         // TMEM lanes this warp may touch
     const int r = quarter * 32 + lane;                    // query row of this thread inside the tile
-    const int qi = qt * kFaRows + r;                      // row index inside the sequence
+    const int qi = (qt0 + t) * kFaRows + r;               // row index inside the sequence
+    const uint32_t o_col = (uint32_t)(G::kSCols + t * VD);
     const uint32_t lane_base = tmem_base + ((uint32_t)(quarter * 32) << 16);
     const uint8_t* mrow = p.mask ? p.mask + (size_t)seq * p.mask_seq_stride + (size_t)min(qi, qlen - 1) * p.mask_ld : nullptr;
     const int sq = (p.seg_q && qi < qlen) ? p.seg_q[p.q_start[seq] + qi] : 0;
     const int kv0 = p.paged ? 0 : p.kv_start[seq];
     float m_ref = -INFINITY, l = 0.f;
     bool ok = true;
-    uint8_t* prow = psm + r * 128;
+    uint8_t* prow = psm + t * G::kPTile + r * 128;
     // bounds of the valid kv positions of this row that do not depend on data: [lo, hi]
     const int hi_row = min(kvlen - 1, p.causal ? qpos0 + qi : 0x7fffffff);
     int lo_row = p.window > 0 ? qpos0 + qi - p.window + 1 : 0;
@@ -246,10 +288,10 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
     const float score_mul = p.slopes ? 1.f : p.scale_log2;
     for (int j = 0; j < nblk; ++j) {
       const int b = j & 1;
-      if (!mbar_wait(&ctl->s_full[b], (uint32_t)(j >> 1) & 1u) || *abort_flag) { ok = false; break; }
+      if (!mbar_wait(&ctl->s_full[t][b], (uint32_t)(j >> 1) & 1u) || *abort_flag) { ok = false; break; }
       tc_fence_after_sync();
       const int t0 = block_start(j);
-      const uint32_t s_addr = lane_base + (uint32_t)(b * KVB);
+      const uint32_t s_addr = lane_base + (uint32_t)((t * 2 + b) * KVB);
       // the whole row of S for this block: all loads in flight, one wait
       uint32_t sv[KVB];
 #pragma unroll
@@ -258,7 +300,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
       // S[b] may now be overwritten by Q.K^T of block j+2
       tc_fence_before_sync();
       __syncwarp();
-      if (lane == 0) mbar_arrive(&ctl->s_empty[b]);
+      if (lane == 0) mbar_arrive(&ctl->s_empty[t][b]);
       // masking: interior blocks need none; edge blocks compare against the row's [lo, hi]; boolean
       // masks and segment ids (rare) take the per-element path
       const bool edge = __any_sync(0xffffffffu, (t0 < lo_row && t0 + KVB > p.keep_first) || t0 + KVB - 1 > hi_row) || data_mask;
@@ -273,13 +315,21 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
         for (int i = 0; i < KVB; ++i)
           sv[i] = __float_as_uint(fmaf(fall, past + (float)i, __uint_as_float(sv[i]) * p.scale_log2));
       }
-      float mx = -INFINITY;
-      if (!edge) {
+      // Inside the mask the scores stay as they came and `mul` goes into the exponent's multiply-add; elsewhere they are finished here.
+      // Four running maxima (and sums below): one would be a chain of 64 dependent instructions.
+      float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY}, mul = 1.f;
+      if (!edge && score_mul > 0.f) {
+        mul = score_mul;
+#pragma unroll
+        for (int i = 0; i < KVB; ++i) mx4[i & 3] = fmaxf(mx4[i & 3], __uint_as_float(sv[i]));
+#pragma unroll
+        for (int i = 0; i < 4; ++i) mx4[i] *= score_mul;
+      } else if (!edge) {
 #pragma unroll
         for (int i = 0; i < KVB; ++i) {
           const float v = __uint_as_float(sv[i]) * score_mul;
           sv[i] = __float_as_uint(v);
-          mx = fmaxf(mx, v);
+          mx4[i & 3] = fmaxf(mx4[i & 3], v);
         }
       } else if (mrow != nullptr && p.seg_q == nullptr && ((reinterpret_cast<uintptr_t>(mrow) + (uintptr_t)t0) & 15u) == 0 &&
                  t0 + KVB <= p.mask_ld) {
@@ -297,7 +347,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
           const bool v = tk >= lo_row && tk <= hi_row && ((word >> ((i & 3) * 8)) & 0xffu) != 0;
           const float x = v ? __uint_as_float(sv[i]) * score_mul : -INFINITY;
           sv[i] = __float_as_uint(x);
-          mx = fmaxf(mx, x);
+          mx4[i & 3] = fmaxf(mx4[i & 3], x);
         }
       } else {
 #pragma unroll
@@ -310,11 +360,12 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
           }
           const float x = v ? __uint_as_float(sv[i]) * score_mul : -INFINITY;
           sv[i] = __float_as_uint(x);
-          mx = fmaxf(mx, x);
+          mx4[i & 3] = fmaxf(mx4[i & 3], x);
         }
       }
+      const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
       // P and O belong to the tensor core until P.V of the previous block has finished
-      if (j > 0 && !mbar_wait(&ctl->p_empty, (uint32_t)(j - 1) & 1u)) { ok = false; break; }
+      if (j > 0 && !mbar_wait(&ctl->p_empty[t], (uint32_t)(j - 1) & 1u)) { ok = false; break; }
       tc_fence_after_sync();
       const bool raise = mx > m_ref + kFaRaise || (m_ref == -INFINITY && mx > -INFINITY);
       if (__any_sync(0xffffffffu, raise)) {               // tcgen05.ld/st are warp-wide
@@ -324,11 +375,11 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
 #pragma unroll 1
           for (int c0 = 0; c0 < VD; c0 += 32) {
             uint32_t ov[32];
-            tmem_ld32(lane_base + (uint32_t)(G::kOCol + c0), ov);
+            tmem_ld32(lane_base + o_col + (uint32_t)c0, ov);
             tmem_ld_wait();
 #pragma unroll
             for (int i = 0; i < 32; ++i) ov[i] = __float_as_uint(__uint_as_float(ov[i]) * (raise ? alpha : 1.f));
-            tmem_st32(lane_base + (uint32_t)(G::kOCol + c0), ov);
+            tmem_st32(lane_base + o_col + (uint32_t)c0, ov);
           }
           tmem_st_wait();
         }
@@ -339,27 +390,27 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
       }
       // probabilities against the reference maximum -> 16-bit P tile (K-major, 128-byte swizzle)
       const float mref = m_ref == -INFINITY ? 0.f : m_ref;
-      float rs = 0.f;
+      float rs[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
       for (int u = 0; u < KVB / 8; ++u) {                 // 16-byte units of 8 values
         float f8[8];
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
-          f8[i] = exp2f(__uint_as_float(sv[u * 8 + i]) - mref);   // masked entries are -inf -> 0
-          rs += f8[i];
+          f8[i] = ex2(fmaf(__uint_as_float(sv[u * 8 + i]), mul, -mref));   // masked entries are -inf -> 0
+          rs[i & 3] += f8[i];
         }
         uint8_t* chunk_base = prow + (u >> 3) * (kFaRows * 128);
         store8(reinterpret_cast<T*>(chunk_base + (((u & 7) ^ (r & 7)) << 4)), f8);
       }
-      l += rs;
+      l += (rs[0] + rs[1]) + (rs[2] + rs[3]);
       // P (and a rescaled O) are ready for the tensor core
       tc_fence_before_sync();
       fence_proxy_async();
       __syncwarp();
-      if (lane == 0) mbar_arrive(&ctl->p_full);
+      if (lane == 0) mbar_arrive(&ctl->p_full[t]);
     }
     // epilogue: O / l
-    if (ok && nblk > 0) ok = mbar_wait(&ctl->o_full, 0);
+    if (ok && nblk > 0) ok = mbar_wait(&ctl->o_full[t], 0);
     if (!ok) {
       if (!*abort_flag) report_status(p.status, kStatusEpilogueTimeout, kTagAttnPrefill, r);
       ctl->abort_flag = 1;
@@ -378,7 +429,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
       for (int c0 = 0; c0 < VD; c0 += 32) {
         uint32_t ov[32];
         if (nblk > 0) {
-          tmem_ld32(lane_base + (uint32_t)(G::kOCol + c0), ov);
+          tmem_ld32(lane_base + o_col + (uint32_t)c0, ov);
           tmem_ld_wait();
         } else {
 #pragma unroll
@@ -408,9 +459,9 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
   if (warp == 1) tmem_dealloc(tmem_base, (uint32_t)G::kTmemCols);
 }
 
-template <typename T, int HD, int VD = HD>
-static int launch_prefill_tc_t(const RfAttn* a, const AttnParams& p, cudaStream_t s) {
-  using G = FaGeom<HD, VD>;
+template <typename T, int HD, int VD, int NQ>
+static int launch_prefill_tc_n(const RfAttn* a, const AttnParams& p, cudaStream_t s) {
+  using G = FaGeom<HD, VD, NQ>;
   CUtensorMap tmQ, tmK, tmV;
   int rc;
   if (a->k_pool) {
@@ -419,20 +470,38 @@ static int launch_prefill_tc_t(const RfAttn* a, const AttnParams& p, cudaStream_
     if (rc) return rc;
     rc = make_tmap_2d(&tmV, a->v_pool, a->dtype, 2, a->hd, rows, a->hd, 64, 16, true);
   } else {
-    rc = make_tmap_2d(&tmK, a->k, a->dtype, 2, (uint64_t)a->Hkv * a->hd, a->kv_rows_total, a->ldk, 64, 16, true);
+    rc = make_tmap_2d(&tmK, a->k, a->dtype, 2, (uint64_t)a->Hkv * a->hd, a->kv_rows_total, a->ldk, 64, G::KVB, true);
     if (rc) return rc;
-    rc = make_tmap_2d(&tmV, a->v, a->dtype, 2, (uint64_t)a->Hkv * VD, a->kv_rows_total, a->ldv, 64, 16, true);
+    rc = make_tmap_2d(&tmV, a->v, a->dtype, 2, (uint64_t)a->Hkv * VD, a->kv_rows_total, a->ldv, 64, G::KVB, true);
   }
   if (rc) return rc;
-  rc = make_tmap_2d(&tmQ, a->q, a->dtype, 2, (uint64_t)a->Hq * a->hd, a->q_rows_total, a->ldq, 64, 16, true);
+  rc = make_tmap_2d(&tmQ, a->q, a->dtype, 2, (uint64_t)a->Hq * a->hd, a->q_rows_total, a->ldq, 64, kFaRows, true);
   if (rc) return rc;
-  const size_t smem = (size_t)G::kSmem + sizeof(FaCtl);
-  auto kfn = attn_prefill_tc_kernel<T, HD, VD>;
+  dim3 grid(a->Hq, ceil_div(a->max_q_len, kFaRows * NQ), a->num_seqs);
+  RF_REQUIRE(grid.y <= 65535 && grid.z <= 65535, "prefill attention: %u row tiles of %u sequences", grid.y, grid.z);
+  // One-tile CTAs of heads up to 128 sit two to an SM with a ring of two blocks once there are more of them than SMs; a CTA that has its SM to
+  // itself takes what shared memory there is.
+  const bool pair = NQ == 1 && HD <= 128 && (long)grid.x * grid.y * grid.z > sm_count();
+  const int room = (pair ? 113 : 226) * 1024 - G::kFixed - (int)sizeof(FaCtl);
+  const int stages = std::min(kFaMaxStages, room / G::kStageBytes);
+  RF_REQUIRE(stages >= 2, "prefill attention: heads of %d / %d do not fit shared memory", HD, VD);
+  const size_t smem = (size_t)G::kFixed + (size_t)stages * G::kStageBytes + sizeof(FaCtl);
+  auto kfn = attn_prefill_tc_kernel<T, HD, VD, NQ>;
   RF_ALLOW_SMEM_PER_DEVICE(kfn, 227 * 1024);
-  dim3 grid(ceil_div(a->max_q_len, kFaRows), a->Hq, a->num_seqs);
-  RF_CUDA_CHECK(::rf::launch_k(kfn, grid, dim3(kFaThreads), smem, s, 1, tmQ, tmK, tmV, p));
+  RF_CUDA_CHECK(::rf::launch_k(kfn, grid, dim3(G::kThreads), smem, s, 1, tmQ, tmK, tmV, p, stages));
   ::rf::count_launch();
   return RF_OK;
+}
+
+template <typename T, int HD, int VD = HD>
+static int launch_prefill_tc_t(const RfAttn* a, const AttnParams& p, cudaStream_t s) {
+  if constexpr (HD <= 128) {
+    // Two tiles to a CTA where that still makes about one CTA per SM and the tiles have more than a few blocks to share (12 x 256 rows and keys,
+    // 16 heads of 128: 47 us with two tiles, 42 with one)
+    if (a->max_q_len > 2 * kFaRows && 4l * ceil_div(a->max_q_len, 2 * kFaRows) * a->Hq * a->num_seqs >= 3l * sm_count())
+      return launch_prefill_tc_n<T, HD, VD, 2>(a, p, s);
+  }
+  return launch_prefill_tc_n<T, HD, VD, 1>(a, p, s);
 }
 
 // Entry used by rf_attn_prefill (attention.cu): `p` is already filled from `a`.

@@ -998,3 +998,35 @@ def test_gemm_very_few_rows_quantised(dt, M, N, K, group, fp4, dual, status):
     z = x.float() @ w.t()
     ref = torch.nn.functional.silu(z[:, :N]) * z[:, N:] if dual else z
     _close(y, ref, dt, scale=max(1.0, ref.abs().max().item()))
+
+
+@pytest.mark.parametrize("dt", DT)
+@pytest.mark.parametrize("hd,Hq,Hkv", [(64, 32, 8), (128, 32, 4)])
+@pytest.mark.parametrize("mode", ["causal", "window", "full", "mask"])
+def test_attn_prefill_two_tiles(dt, hd, Hq, Hkv, mode, status):
+    """Enough heads and rows that a CTA takes two query tiles: second tiles that are empty, partial and full, keys ahead of the new rows, tiles that
+    stop at different blocks, and the masks that leave a tile's first blocks empty - paged against fp32, contiguous against paged."""
+    from rhinoforge_b200.ops import kernels as K_
+    q_lens, kv_lens = [257, 100, 384, 129], [257, 420, 400, 129]
+    k_pool, v_pool, pt, ks, vs = _paged(Hkv, hd, kv_lens, dt)
+    i32 = lambda l: torch.tensor(l, dtype=torch.int32, device="cuda")
+    starts = [sum(q_lens[:i]) for i in range(len(q_lens))]
+    q = torch.randn(sum(q_lens), Hq * hd, device="cuda").to(dt)
+    kw = dict(Hq=Hq, Hkv=Hkv, hd=hd, q_start=i32(starts), q_len=i32(q_lens), kv_len=i32(kv_lens), max_q_len=max(q_lens), causal=mode in ("causal", "window"),
+              window=70 if mode == "window" else 0, status=status)
+    given = torch.rand(len(q_lens), max(q_lens), 432, device="cuda") > 0.4
+    given[:, :, 0] = True
+    if mode == "mask":
+        kw["mask"] = given
+    out = K_.attention_prefill(q, torch.zeros_like(q), k_pool=k_pool, v_pool=v_pool, page_table=pt, **kw)
+    flat = lambda parts: torch.cat([t.transpose(0, 1).reshape(t.shape[1], Hkv * hd) for t in parts])
+    rows = K_.attention_prefill(q, torch.zeros_like(q), k=flat(ks), v=flat(vs), kv_start=i32([sum(kv_lens[:i]) for i in range(len(kv_lens))]), **kw)
+    assert torch.equal(out, rows)
+    for s, (Lq, Lk) in enumerate(zip(q_lens, kv_lens)):
+        qs = q[starts[s]:starts[s] + Lq].view(Lq, Hq, hd).transpose(0, 1)
+        i, j = torch.arange(Lq, device="cuda")[:, None] + (Lk - Lq), torch.arange(Lk, device="cuda")[None]
+        mask = torch.ones(Lq, Lk, dtype=torch.bool, device="cuda") if mode == "full" else given[s, :Lq, :Lk] if mode == "mask" else j <= i
+        if mode == "window":
+            mask = mask & (j > i - 70)
+        ref = _sdpa_ref(qs, ks[s], vs[s], mask).transpose(0, 1).reshape(Lq, Hq * hd)
+        _close(out[starts[s]:starts[s] + Lq], ref, dt)
