@@ -3,6 +3,8 @@
 // Replaces the reference's llama_rms_norm*, layer_norm* and l2norm operators
 // (src/ops/rpu_rmsnorm.cpp, src/ops/rpu_layernorm.cpp, src/ops/rpu_l2norm.cpp)
 // and the adaRMS SUB/MUL/ADD chain (src/fused/rpu_pi05_denoise_step_model.cpp:848-857).
+#include <type_traits>
+
 #include "../common/dtype.cuh"
 #include "../common/host_util.h"
 #include "../common/ptx.cuh"
@@ -128,6 +130,139 @@ __global__ void layernorm_kernel(const T* __restrict__ x, const T* __restrict__ 
   }
 }
 
+// Many rows: a warp per row that holds it in registers, 16-byte pieces 256 values apart, all of them on their way at once; nothing but shuffles
+// between the two passes.  The kernels above keep the row in shared memory (eight-way bank conflicts) and meet at three to six block barriers,
+// which few rows hide no worse.  us, before / now: LayerNorm 3072 x 1152 9.0 / 6.8, 6000 x 2048 25.3 / 15.5; RMSNorm 5400 x 4096 31.5 / 21.6, 768 x 1152 4.4 / 3.3.
+template <typename T, int NC>
+__global__ void __launch_bounds__(128)
+rmsnorm_warp_kernel(const T* __restrict__ x, const T* __restrict__ residual, const T* __restrict__ w, T* __restrict__ y,
+                    T* __restrict__ residual_out, const T* __restrict__ mod, int rows_per_mod, int rows, int H, int64_t ldx, int64_t ldy, float eps,
+                    int mode) {
+  pdl_prologue();
+  const int row = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (row >= rows) return;
+  const T* xr = x + (size_t)row * ldx;
+  uint4 v[NC];
+#pragma unroll
+  for (int c = 0; c < NC; ++c) {
+    const int i = c * 256 + lane * 8;
+    v[c] = i < H ? *reinterpret_cast<const uint4*>(xr + i) : make_uint4(0u, 0u, 0u, 0u);
+  }
+  float ss = 0.f;
+#pragma unroll
+  for (int c = 0; c < NC; ++c) {
+    const int i = c * 256 + lane * 8;
+    float f[8];
+    unpack8<T>(v[c], f);
+    if (residual && i < H) {
+      float r[8];
+      load8(residual + (size_t)row * ldx + i, r);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) f[j] += r[j];
+      store8(reinterpret_cast<T*>(&v[c]), f);
+      unpack8<T>(v[c], f);                       // the sum as it is stored
+      if (residual_out) *reinterpret_cast<uint4*>(residual_out + (size_t)row * ldx + i) = v[c];
+    }
+#pragma unroll
+    for (int j = 0; j < 8; ++j) ss += f[j] * f[j];
+  }
+  const float rstd = rsqrtf(warp_sum(ss) / (float)H + eps);
+  const T* mrow = mod ? mod + (size_t)(row / rows_per_mod) * 3 * H : nullptr;
+#pragma unroll
+  for (int c = 0; c < NC; ++c) {
+    const int i = c * 256 + lane * 8;
+    if (i >= H) continue;
+    float f[8], o[8];
+    unpack8<T>(v[c], f);
+    if (mrow) {
+      float sc[8], sh[8];
+      load8(mrow + i, sc);
+      load8(mrow + H + i, sh);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) o[j] = f[j] * rstd * (1.f + sc[j]) + sh[j];
+    } else {
+      float wf[8];
+      if (w) {
+        load8(w + i, wf);
+      } else {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) wf[j] = (mode & 1) ? 0.f : 1.f;
+      }
+#pragma unroll
+      for (int j = 0; j < 8; ++j) o[j] = (mode & 1) ? f[j] * rstd * (1.f + wf[j]) : wf[j] * Num<T>::to_f(Num<T>::from_f(f[j] * rstd));
+    }
+    store8(y + (size_t)row * ldy + i, o);
+  }
+}
+
+template <typename T, int NC>
+__global__ void __launch_bounds__(128)
+layernorm_warp_kernel(const T* __restrict__ x, const T* __restrict__ w, const T* __restrict__ b, T* __restrict__ y, int rows, int H, int64_t ldx,
+                      int64_t ldy, float eps) {
+  pdl_prologue();
+  const int row = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (row >= rows) return;
+  const T* xr = x + (size_t)row * ldx;
+  uint4 v[NC];
+#pragma unroll
+  for (int c = 0; c < NC; ++c) {
+    const int i = c * 256 + lane * 8;
+    v[c] = i < H ? *reinterpret_cast<const uint4*>(xr + i) : make_uint4(0u, 0u, 0u, 0u);
+  }
+  float s = 0.f, q = 0.f;
+#pragma unroll
+  for (int c = 0; c < NC; ++c) {
+    float f[8];
+    unpack8<T>(v[c], f);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) s += f[j];
+  }
+  const float mean = warp_sum(s) / (float)H;
+#pragma unroll
+  for (int c = 0; c < NC; ++c) {
+    if (c * 256 + lane * 8 >= H) continue;
+    float f[8];
+    unpack8<T>(v[c], f);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) q += (f[j] - mean) * (f[j] - mean);
+  }
+  const float rstd = rsqrtf(warp_sum(q) / (float)H + eps);
+#pragma unroll
+  for (int c = 0; c < NC; ++c) {
+    const int i = c * 256 + lane * 8;
+    if (i >= H) continue;
+    float f[8], wf[8], bf[8], o[8];
+    unpack8<T>(v[c], f);
+    load8(w + i, wf);
+    if (b) load8(b + i, bf);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) o[j] = (f[j] - mean) * rstd * wf[j] + (b ? bf[j] : 0.f);
+    store8(y + (size_t)row * ldy + i, o);
+  }
+}
+
+// 256-value pieces of a row that the warp kernels hold (0: the row is too long, or the rows are too few to fill the GPU with a warp each)
+static int warp_pieces(int rows, int H) {
+  if (rows < 2 * sm_count() || H > 4096) return 0;
+  const int nc = ceil_div(H, 256);
+  return nc <= 4 ? 4 : nc <= 5 ? 5 : nc <= 8 ? 8 : nc <= 12 ? 12 : 16;
+}
+
+// Calls `run` with the piece count and the element type as types.
+template <typename Run>
+static cudaError_t with_pieces(int nc, int dtype, Run run) {
+  auto typed = [&](auto zero) -> cudaError_t {
+    switch (nc) {
+      case 4: return run(std::integral_constant<int, 4>{}, zero);
+      case 5: return run(std::integral_constant<int, 5>{}, zero);
+      case 8: return run(std::integral_constant<int, 8>{}, zero);
+      case 12: return run(std::integral_constant<int, 12>{}, zero);
+      default: return run(std::integral_constant<int, 16>{}, zero);
+    }
+  };
+  return dtype == 0 ? typed(__half{}) : typed(__nv_bfloat16{});
+}
+
 template <typename T>
 __global__ void l2norm_kernel(const T* __restrict__ x, T* __restrict__ y, int rows, int H,
                               float eps, float out_scale) {
@@ -181,6 +316,16 @@ extern "C" int rf_rmsnorm(const void* x, const void* residual, const void* w, vo
   const size_t smem = (size_t)(H + 32) * sizeof(float);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (rows_per_mod <= 0) rows_per_mod = 1;
+  if (const int nc = warp_pieces(rows, H)) {
+    auto run = [&](auto kNC, auto zero) -> cudaError_t {
+      using T = decltype(zero);
+      return ::rf::launch_k(rmsnorm_warp_kernel<T, decltype(kNC)::value>, dim3(ceil_div(rows, 4)), dim3(128), 0, s, 1, (const T*)x, (const T*)residual, (const T*)w,
+                            (T*)y, (T*)residual_out, (const T*)mod, rows_per_mod, rows, H, ldx, ldy, eps, mode);
+    };
+    RF_CUDA_CHECK(with_pieces(nc, dtype, run));
+    ::rf::count_launch();
+    return RF_OK;
+  }
   if (dtype == 0)
     RF_CUDA_CHECK(::rf::launch_k(rmsnorm_kernel<__half>, dim3(rows), dim3(threads), smem, s, 1, 
         (const __half*)x, (const __half*)residual, (const __half*)w, (__half*)y,
@@ -203,6 +348,16 @@ extern "C" int rf_layernorm(const void* x, const void* w, const void* b, void* y
   const int threads = H >= 2048 ? 256 : 128;
   const size_t smem = (size_t)(H + 32) * sizeof(float);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
+  if (const int nc = warp_pieces(rows, H)) {
+    auto run = [&](auto kNC, auto zero) -> cudaError_t {
+      using T = decltype(zero);
+      return ::rf::launch_k(layernorm_warp_kernel<T, decltype(kNC)::value>, dim3(ceil_div(rows, 4)), dim3(128), 0, s, 1, (const T*)x, (const T*)w, (const T*)b,
+                            (T*)y, rows, H, ldx, ldy, eps);
+    };
+    RF_CUDA_CHECK(with_pieces(nc, dtype, run));
+    ::rf::count_launch();
+    return RF_OK;
+  }
   if (dtype == 0)
     RF_CUDA_CHECK(::rf::launch_k(layernorm_kernel<__half>, dim3(rows), dim3(threads), smem, s, 1, (const __half*)x, (const __half*)w,
                                                         (const __half*)b, (__half*)y, H, ldx, ldy,
