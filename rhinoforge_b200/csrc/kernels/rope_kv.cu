@@ -113,13 +113,16 @@ __global__ void qk_norm_rope_kv_kernel(const RfRopeKv a) {
   }
 }
 
-// Prefill-sized launches: the same computation with 16-byte accesses.  A head of 64 / 128 / 256 elements is held by 8 / 16 /
+// The common geometries: the same computation with 16-byte accesses.  A head of 64 / 128 / 256 elements is held by 8 / 16 /
 // 32 lanes with eight consecutive elements each, so one warp instruction moves four / two / one head(s); sums of squares
 // are reduced inside the lane group and the rotate-half partner comes from the lane rot_dim / 16 away (rot_dim % 16 == 0).
 // The scalar kernel above keeps a warp on 64 - 128 bytes per load and runs at a fraction of memory speed on thousands of
-// tokens (6 272 vision patches x 48 heads of 64: 53 us); it stays for decode-sized launches and odd geometries.
+// tokens (6 272 vision patches x 48 heads of 64: 53 us); at decode sizes it is a chain of five trips to memory (position, page, row,
+// position again, angles), where this one asks for the row and the positions together and then for page and angles together
+// (1 token, 16 + 2 x 8 heads of 128: 3.3 -> 2.4 us; 64 tokens, 32 + 2 x 8: 4.9 -> 3.3).  It stays for odd geometries.  Few tokens spread their heads over
+// blockIdx.y.
 template <typename T, int HD>
-__global__ void __launch_bounds__(256) qk_norm_rope_kv_vec_kernel(const RfRopeKv a) {
+__global__ void __launch_bounds__(256) qk_norm_rope_kv_vec_kernel(const RfRopeKv a, const int angle_vec) {
   pdl_prologue();
   constexpr int GROUP = HD / 8;                  // lanes per head
   constexpr int HPW = 32 / GROUP;                // heads per warp instruction
@@ -129,15 +132,16 @@ __global__ void __launch_bounds__(256) qk_norm_rope_kv_vec_kernel(const RfRopeKv
   const int heads = a.Hq + 2 * a.Hkv;
   const int gl = lane % GROUP, o = gl * 8;       // this lane's first element inside its head
   T* row = reinterpret_cast<T*>(a.qkv) + (size_t)tok * a.ld;
-  int page = -1, slot = 0;
-  if (a.k_pool) {
-    const int seq = a.seq_of_tok ? a.seq_of_tok[tok] : tok;
-    const int cpos = a.cache_pos ? a.cache_pos[tok] : a.pos[(size_t)tok * a.pos_stride];
-    if (seq >= 0 && cpos >= 0) {
-      page = a.page_table[(size_t)seq * a.pt_stride + (cpos >> 4)];
-      slot = cpos & 15;
-    }
-  }
+  const int first = (blockIdx.y * nwarps + warp) * HPW;
+  // asked for before anything is waited for: the first head's row, the positions, the sequence
+  const int h_first = first + lane / GROUP;
+  uint4 ahead = *reinterpret_cast<const uint4*>(row + (size_t)(h_first < heads ? h_first : 0) * HD + o);
+  const int pos0 = a.pos[(size_t)tok * a.pos_stride];
+  const int seq = a.k_pool && a.seq_of_tok ? a.seq_of_tok[tok] : tok;
+  const int cpos = a.k_pool && a.cache_pos ? a.cache_pos[tok] : pos0;
+  int page = -1;
+  const int slot = cpos & 15;
+  if (a.k_pool && seq >= 0 && cpos >= 0) page = a.page_table[(size_t)seq * a.pt_stride + (cpos >> 4)];
   const bool do_rope = a.cos != nullptr && rot > 0;
   const int region = o < half ? 0 : (o < rot ? 1 : 2);           // first half, second half, not rotated
   const int partner = lane + (region == 0 ? hl : (region == 1 ? -hl : 0));
@@ -145,6 +149,13 @@ __global__ void __launch_bounds__(256) qk_norm_rope_kv_vec_kernel(const RfRopeKv
   float cs[8], sn[8];
   if (do_rope && region < 2) {
     const int i0 = region == 0 ? o : o - half;
+    if (angle_vec) {                             // one axis, 16-byte aligned tables
+      const float4* c4 = reinterpret_cast<const float4*>(a.cos + (size_t)pos0 * half + i0);
+      const float4* s4 = reinterpret_cast<const float4*>(a.sin + (size_t)pos0 * half + i0);
+      const float4 c0 = c4[0], c1 = c4[1], s0 = s4[0], s1 = s4[1];
+      cs[0] = c0.x; cs[1] = c0.y; cs[2] = c0.z; cs[3] = c0.w; cs[4] = c1.x; cs[5] = c1.y; cs[6] = c1.z; cs[7] = c1.w;
+      sn[0] = s0.x; sn[1] = s0.y; sn[2] = s0.z; sn[3] = s0.w; sn[4] = s1.x; sn[5] = s1.y; sn[6] = s1.z; sn[7] = s1.w;
+    } else
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
       const int i = i0 + j;
@@ -157,17 +168,20 @@ __global__ void __launch_bounds__(256) qk_norm_rope_kv_vec_kernel(const RfRopeKv
 #pragma unroll
     for (int j = 0; j < 8; ++j) { cs[j] = 1.f; sn[j] = 0.f; }
   }
-  for (int h0 = warp * HPW; h0 < heads; h0 += nwarps * HPW) {
+  for (int h0 = first; h0 < heads; h0 += nwarps * HPW * gridDim.y) {
     const int h = h0 + lane / GROUP;
     const bool live = h < heads;
     const bool is_q = live && h < a.Hq, is_k = live && !is_q && h < a.Hq + a.Hkv, is_v = live && !is_q && !is_k;
     T* src = row + (size_t)(live ? h : 0) * HD + o;
     float x[8];
-    if (live) load8(src, x);
-    else {
+    const uint4 own_row = ahead;
+    unpack8<T>(own_row, x);
+    if (!live) {
 #pragma unroll
       for (int j = 0; j < 8; ++j) x[j] = 0.f;
     }
+    const int h_next = h + nwarps * HPW * (int)gridDim.y;
+    if (h_next < heads) ahead = *reinterpret_cast<const uint4*>(row + (size_t)h_next * HD + o);
     const T* nw = reinterpret_cast<const T*>(is_q ? a.q_norm_w : (is_k ? a.k_norm_w : nullptr));
     auto group_sum = [&](float v) {
 #pragma unroll
@@ -226,7 +240,7 @@ __global__ void __launch_bounds__(256) qk_norm_rope_kv_vec_kernel(const RfRopeKv
       const int vh = h - a.Hq - a.Hkv;
       T* dst = reinterpret_cast<T*>(a.v_pool) + (((size_t)page * a.Hkv + vh) * 16 + slot) * HD + o;
       if (a.v_norm) store8(dst, x);
-      else *reinterpret_cast<uint4*>(dst) = *reinterpret_cast<const uint4*>(src);
+      else *reinterpret_cast<uint4*>(dst) = own_row;
     }
   }
 }
@@ -254,19 +268,23 @@ extern "C" int rf_qk_norm_rope_kv(const RfRopeKv* a, rf_stream_t stream) {
   }
   const size_t smem = (size_t)warps * a->hd * sizeof(float);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  // prefill-sized launches on the common geometries take the 16-byte kernel (RF_ROPE_VEC=0: never)
+  // the common geometries take the 16-byte kernel (RF_ROPE_VEC=0: never)
   static const bool vec_on = [] { const char* e = getenv("RF_ROPE_VEC"); return !(e && e[0] == '0'); }();
   const bool aligned = a->ld % 8 == 0 && (reinterpret_cast<uintptr_t>(a->qkv) & 15) == 0 &&
                        (!a->q_out || (a->ldq % 8 == 0 && (reinterpret_cast<uintptr_t>(a->q_out) & 15) == 0)) &&
                        (!a->k_pool || ((reinterpret_cast<uintptr_t>(a->k_pool) | reinterpret_cast<uintptr_t>(a->v_pool)) & 15) == 0) &&
                        (!a->q_norm_w || (reinterpret_cast<uintptr_t>(a->q_norm_w) & 15) == 0) &&
                        (!a->k_norm_w || (reinterpret_cast<uintptr_t>(a->k_norm_w) & 15) == 0);
-  if (vec_on && a->tokens >= 512 && aligned && a->rot_dim % 16 == 0 && (a->hd == 64 || a->hd == 128 || a->hd == 256)) {
+  if (vec_on && aligned && a->rot_dim % 16 == 0 && (a->hd == 64 || a->hd == 128 || a->hd == 256)) {
     cudaError_t e;
+    const int angle_vec = !a->axis_of_freq && ((reinterpret_cast<uintptr_t>(a->cos) | reinterpret_cast<uintptr_t>(a->sin)) & 15) == 0;
+    // few tokens: one pass over the heads, in blocks of two warps
+    const int per_warp = 256 / a->hd, threads = a->tokens < 512 ? 64 : 256;
+    const dim3 grid(a->tokens, a->tokens < 512 ? ceil_div(heads, 2 * per_warp) : 1);
 #define RF_ROPE_VEC(T)                                                                                              \
-    e = a->hd == 64 ? ::rf::launch_k(qk_norm_rope_kv_vec_kernel<T, 64>, dim3(a->tokens), dim3(256), 0, s, 1, *a)    \
-      : a->hd == 128 ? ::rf::launch_k(qk_norm_rope_kv_vec_kernel<T, 128>, dim3(a->tokens), dim3(256), 0, s, 1, *a)  \
-                     : ::rf::launch_k(qk_norm_rope_kv_vec_kernel<T, 256>, dim3(a->tokens), dim3(256), 0, s, 1, *a);
+    e = a->hd == 64 ? ::rf::launch_k(qk_norm_rope_kv_vec_kernel<T, 64>, grid, dim3(threads), 0, s, 1, *a, angle_vec)    \
+      : a->hd == 128 ? ::rf::launch_k(qk_norm_rope_kv_vec_kernel<T, 128>, grid, dim3(threads), 0, s, 1, *a, angle_vec)  \
+                     : ::rf::launch_k(qk_norm_rope_kv_vec_kernel<T, 256>, grid, dim3(threads), 0, s, 1, *a, angle_vec);
     if (a->dtype == 0) { RF_ROPE_VEC(__half) } else { RF_ROPE_VEC(__nv_bfloat16) }
 #undef RF_ROPE_VEC
     RF_CUDA_CHECK(e);

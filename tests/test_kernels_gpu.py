@@ -217,3 +217,889 @@ def test_qk_norm_rope_kv_insert(dt, hd, rot):
         page = int(page_table[s, p // 16])
         _close(k_pool[page, :, p % 16], k_ref[t], dt)
         _close(v_pool[page, :, p % 16], v_ref[t], dt)
+
+
+@pytest.mark.parametrize("dt", DT)
+@pytest.mark.parametrize("hd,rot,Hq,Hkv", [(64, 64, 6, 6), (128, 128, 5, 2), (256, 64, 3, 1), (128, 64, 4, 4)])
+@pytest.mark.parametrize("variant", ["plain", "norm", "gemma_rope_first", "mrope_vnorm", "pool"])
+def test_qk_norm_rope_kv_prefill_sized(dt, hd, rot, Hq, Hkv, variant):
+    """Launches of 512 tokens or more take the 16-byte kernel: the same rows through one 640-token launch and through
+    two launches of 320 (below the switch, the scalar kernel) must agree to one rounding step, in every mode."""
+    from rhinoforge_b200.ops import kernels as K_
+    torch.manual_seed(3)
+    T, half = 640, rot // 2
+    W = (Hq + 2 * Hkv) * hd
+    qkv = (torch.randn(T, W, device="cuda") * 0.7).to(dt)
+    axes = 3 if variant == "mrope_vnorm" else 1
+    pos = torch.randint(0, 900, (T, axes), device="cuda", dtype=torch.int32)
+    ang = torch.arange(1024, device="cuda", dtype=torch.float32)[:, None] * (1.0 / 10000 ** (torch.arange(half, device="cuda") / half))[None]
+    kw = dict(pos=pos, cos=ang.cos().contiguous(), sin=ang.sin().contiguous(), rot_dim=rot)
+    if variant in ("norm", "gemma_rope_first", "mrope_vnorm", "pool"):
+        kw.update(q_norm_w=(1 + 0.1 * torch.randn(hd, device="cuda")).to(dt), k_norm_w=(1 + 0.1 * torch.randn(hd, device="cuda")).to(dt))
+    if variant == "gemma_rope_first":
+        kw.update(gemma=True, rope_before_norm=True)
+    if variant == "mrope_vnorm":
+        kw.update(axis_of_freq=torch.randint(0, 3, (half,), device="cuda", dtype=torch.int8), v_norm=True)
+    outs = []
+    pt = torch.randperm(T // 16 + 2, device="cuda").to(torch.int32)[None].contiguous()     # one shuffled page table for both runs
+    for chunks in (1, 2):
+        buf = qkv.clone()
+        q_out = torch.zeros(T, Hq * hd, device="cuda", dtype=dt) if variant == "pool" else None
+        pools = None
+        if variant == "pool":
+            pages = T // 16 + 2
+            pools = (torch.zeros(pages, Hkv, 16, hd, device="cuda", dtype=dt), torch.zeros(pages, Hkv, 16, hd, device="cuda", dtype=dt))
+        n = T // chunks
+        for c in range(chunks):
+            sl = slice(c * n, (c + 1) * n)
+            extra = {}
+            if variant == "pool":
+                extra = dict(k_pool=pools[0], v_pool=pools[1], page_table=pt, seq_of_tok=torch.zeros(n, device="cuda", dtype=torch.int32),
+                             cache_pos=torch.arange(c * n, (c + 1) * n, device="cuda", dtype=torch.int32), q_out=q_out[sl])
+            K_.qk_norm_rope_kv(buf[sl], Hq, Hkv, hd, **{**kw, "pos": pos[sl].contiguous()}, **extra)
+        torch.cuda.synchronize()
+        outs.append((buf, q_out, pools))
+    (b1, q1, p1), (b2, q2, p2) = outs
+
+    def same(x, y):            # one rounding step of the 16-bit type at most (the two kernels may contract their FMAs differently)
+        tol = (2.0 ** -10 if dt == torch.float16 else 2.0 ** -7) * max(1.0, float(y.float().abs().max()))
+        return float((x.float() - y.float()).abs().max()) <= tol
+    assert same(b1, b2)
+    if variant == "pool":
+        assert same(q1, q2) and same(p1[0], p2[0]) and same(p1[1], p2[1])
+        assert float(p1[0].abs().max()) > 0 and float(q1.abs().max()) > 0
+    else:
+        assert not torch.equal(b1, qkv)
+
+
+def test_mrope_axis_select():
+    from rhinoforge_b200.ops import kernels as K_
+    dt, hd, T = torch.float16, 128, 9
+    qkv = torch.randn(T, 3 * hd, device="cuda").to(dt)
+    orig = qkv.clone()
+    cos, sin = _rope_tables(256, hd, 1e6, "cuda")
+    pos = torch.randint(0, 200, (T, 3), device="cuda", dtype=torch.int32)
+    sec = [24, 20, 20]
+    axis = torch.zeros(hd // 2, dtype=torch.int8)
+    for dim, off in ((1, 1), (2, 2)):
+        axis[off:sec[dim] * 3:3] = dim
+    K_.qk_norm_rope_kv(qkv, 1, 1, hd, pos=pos, cos=cos, sin=sin, axis_of_freq=axis.cuda(), write_k_inplace=True)
+    idx = pos.long()[:, axis.long().cuda()]  # [T, hd/2]
+    f = torch.arange(hd // 2, device="cuda")
+    c = cos[idx, f].repeat(1, 2)
+    s = sin[idx, f].repeat(1, 2)
+    for h in range(2):
+        x = orig.float().view(T, 3, hd)[:, h]
+        _close(qkv.view(T, 3, hd)[:, h], x * c + _rot_half(x) * s, dt)
+
+
+def _sdpa_ref(q, k, v, mask):
+    # q [Hq, Lq, hd], k/v [Hkv, Lk, hd], mask [Lq, Lk] bool
+    G = q.shape[0] // k.shape[0]
+    k = k.repeat_interleave(G, 0)
+    v = v.repeat_interleave(G, 0)
+    s = (q.float() @ k.float().transpose(1, 2)) / math.sqrt(q.shape[-1])
+    s = s.masked_fill(~mask[None], float("-inf"))
+    p = torch.softmax(s, -1)
+    p = torch.nan_to_num(p)
+    return p @ v.float()
+
+
+def _paged(Hkv, hd, kv_lens, dt, extra_pages=3):
+    seqs = len(kv_lens)
+    maxp = max((l + 15) // 16 for l in kv_lens) + 1
+    total = seqs * maxp + extra_pages
+    perm = torch.randperm(total)[: seqs * maxp].to(torch.int32).view(seqs, maxp)
+    k_pool = torch.zeros(total, Hkv, 16, hd, device="cuda", dtype=dt)
+    v_pool = torch.zeros_like(k_pool)
+    ks, vs = [], []
+    for s, L in enumerate(kv_lens):
+        k = torch.randn(Hkv, L, hd, device="cuda").to(dt)
+        v = torch.randn(Hkv, L, hd, device="cuda").to(dt)
+        for t in range(L):
+            pg = int(perm[s, t // 16])
+            k_pool[pg, :, t % 16] = k[:, t]
+            v_pool[pg, :, t % 16] = v[:, t]
+        ks.append(k)
+        vs.append(v)
+    return k_pool, v_pool, perm.cuda().contiguous(), ks, vs
+
+
+@pytest.mark.parametrize("dt", DT)
+@pytest.mark.parametrize("hd,Hq,Hkv", [(128, 8, 2), (64, 4, 4), (256, 8, 1)])
+def test_attn_prefill_paged_causal(dt, hd, Hq, Hkv, status):
+    from rhinoforge_b200.ops import kernels as K_
+    q_lens, kv_lens = [70, 33, 128], [70, 97, 128]
+    k_pool, v_pool, pt, ks, vs = _paged(Hkv, hd, kv_lens, dt)
+    q_start = [0, 70, 103]
+    Tq = sum(q_lens)
+    q = torch.randn(Tq, Hq * hd, device="cuda").to(dt)
+    out = torch.zeros_like(q)
+    i32 = lambda l: torch.tensor(l, dtype=torch.int32, device="cuda")
+    K_.attention_prefill(q, out, Hq=Hq, Hkv=Hkv, hd=hd, q_start=i32(q_start), q_len=i32(q_lens), kv_len=i32(kv_lens),
+                         max_q_len=max(q_lens), k_pool=k_pool, v_pool=v_pool, page_table=pt, causal=True,
+                         status=status)
+    for s in range(3):
+        Lq, Lk = q_lens[s], kv_lens[s]
+        qs = q[q_start[s]:q_start[s] + Lq].view(Lq, Hq, hd).transpose(0, 1)
+        qi = torch.arange(Lq, device="cuda")[:, None] + (Lk - Lq)
+        mask = torch.arange(Lk, device="cuda")[None] <= qi
+        ref = _sdpa_ref(qs, ks[s], vs[s], mask).transpose(0, 1).reshape(Lq, Hq * hd)
+        _close(out[q_start[s]:q_start[s] + Lq], ref, dt)
+
+
+@pytest.mark.parametrize("mode", ["bidir", "mask", "segments", "window"])
+def test_attn_prefill_contiguous_masks(mode, status):
+    from rhinoforge_b200.ops import kernels as K_
+    dt, hd, H = torch.float16, 64, 4
+    L = 201
+    qkv = torch.randn(L, 3 * H * hd, device="cuda").to(dt)
+    q, k, v = qkv[:, :H * hd], qkv[:, H * hd:2 * H * hd], qkv[:, 2 * H * hd:]
+    out = torch.zeros(L, H * hd, device="cuda", dtype=dt)
+    i32 = lambda l: torch.tensor(l, dtype=torch.int32, device="cuda")
+    kw = dict(Hq=H, Hkv=H, hd=hd, q_start=i32([0]), q_len=i32([L]), kv_len=i32([L]), max_q_len=L, k=k, v=v,
+              kv_start=i32([0]), causal=False, status=status)
+    full = torch.ones(L, L, dtype=torch.bool, device="cuda")
+    if mode == "bidir":
+        mask = full
+    elif mode == "mask":
+        mask = torch.rand(L, L, device="cuda") > 0.3
+        mask[:, 0] = True
+        kw["mask"] = mask.contiguous()
+    elif mode == "segments":
+        seg = (torch.arange(L, device="cuda") // 37).to(torch.int32)
+        mask = seg[:, None] == seg[None]
+        kw["seg_q"], kw["seg_k"] = seg, seg
+    else:
+        kw["causal"], kw["window"] = True, 48
+        i = torch.arange(L, device="cuda")
+        mask = (i[None] <= i[:, None]) & (i[None] > i[:, None] - 48)
+    K_.attention_prefill(q, out, **kw)
+    tr = lambda t: t.reshape(L, H, hd).transpose(0, 1)
+    ref = _sdpa_ref(tr(q), tr(k), tr(v), mask).transpose(0, 1).reshape(L, H * hd)
+    _close(out, ref, dt)
+
+
+@pytest.mark.parametrize("dt", DT)
+@pytest.mark.parametrize("hd,Hq,Hkv", [(128, 32, 8), (128, 8, 1), (64, 4, 2), (256, 8, 1)])
+@pytest.mark.parametrize("split", [False, True])
+def test_attn_decode_paged(dt, hd, Hq, Hkv, split, status):
+    from rhinoforge_b200.ops import kernels as K_
+    kv_lens = [1, 17, 300, 1025, 64]
+    k_pool, v_pool, pt, ks, vs = _paged(Hkv, hd, kv_lens, dt)
+    B = len(kv_lens)
+    q = torch.randn(B, Hq * hd, device="cuda").to(dt)
+    out = torch.zeros_like(q)
+    ws = K_.attn_decode_scratch(B, Hq, hd, "cuda") if split else None
+    K_.attention_decode(q, out, Hq=Hq, Hkv=Hkv, hd=hd, kv_len=torch.tensor(kv_lens, dtype=torch.int32, device="cuda"),
+                        max_kv_len=max(kv_lens), k_pool=k_pool, v_pool=v_pool, page_table=pt, ws=ws, status=status)
+    for s in range(B):
+        L = kv_lens[s]
+        ref = _sdpa_ref(q[s].view(Hq, 1, hd), ks[s], vs[s], torch.ones(1, L, dtype=torch.bool, device="cuda"))
+        _close(out[s], ref.reshape(Hq * hd), dt)
+
+
+def test_embedding_scatter_eltwise_cast_argmax():
+    from rhinoforge_b200.ops import kernels as K_
+    dt = torch.float16
+    table = torch.randn(1000, 256, device="cuda").to(dt)
+    ids = torch.tensor([3, 999, -1, 0, 17], dtype=torch.int32, device="cuda")
+    e = K_.embedding(table, ids, scale=2.0)
+    ref = table[ids.clamp(min=0).long()].float() * 2.0
+    ref[2] = 0
+    _close(e, ref, dt)
+    dst = torch.zeros(10, 256, device="cuda", dtype=dt)
+    K_.scatter_rows(dst, e, torch.tensor([9, 1, -1, 4, 0], dtype=torch.int32, device="cuda"))
+    assert torch.equal(dst[9], e[0]) and torch.equal(dst[0], e[4]) and dst[2].abs().sum() == 0
+    a, b = torch.randn(77, 256, device="cuda").to(dt), torch.randn(77, 256, device="cuda").to(dt)
+    _close(K_.eltwise("silu_mul", a, b), torch.nn.functional.silu(a.float()) * b.float(), dt)
+    _close(K_.eltwise("axpy", a, b, alpha=-0.1), a.float() - 0.1 * b.float(), dt)
+    _close(K_.eltwise("mul_row", a, b[0].contiguous()), a.float() * b[0].float(), dt)
+    u8 = torch.randint(0, 256, (3, 64), dtype=torch.uint8, device="cuda")
+    _close(K_.cast_u8(u8, dt, 1 / 127.5, -1.0), u8.float() / 127.5 - 1.0, dt)
+    logits = torch.randn(5, 151936, device="cuda").to(dt)
+    logits[2, 77] = 100.0
+    logits[3, 151935] = 100.0
+    ids2, vals = K_.argmax(logits, offset=10, return_vals=True)
+    assert torch.equal(ids2.long() - 10, logits.float().argmax(-1))
+    _close(vals, logits.float().max(-1).values, dt)
+
+
+@pytest.mark.parametrize("dt", DT)
+@pytest.mark.parametrize("M,N,K,swap,splits", [(16, 384, 1024, -1, 0), (64, 1000, 2048, 1, 4), (9, 256, 512, 1, 1),
+                                               (300, 640, 1024, 0, 1), (1024, 512, 2048, 0, 1), (130, 256, 4096, 1, 2)])
+def test_gemm_w8a16_tensor_core(dt, M, N, K, swap, splits, status):
+    """int8 weights widened in the mainloop, (X . Q^T) * scale in the epilogue."""
+    from rhinoforge_b200.ops import kernels as K_
+    x = (torch.randn(M, K, device="cuda") * 0.5).to(dt)
+    q = torch.randint(-127, 128, (N, K), device="cuda", dtype=torch.int8)
+    sc = (torch.rand(N, device="cuda") * 0.004 + 0.001).to(dt)
+    r = torch.randn(M, N, device="cuda").to(dt)
+    y = K_.gemm(x, q, scale=sc, residual=r, status=status, force_swap=swap, force_splits=splits)
+    ref = (x.float() @ q.float().t()) * sc.float() + r.float()
+    _close(y, ref, dt, scale=max(1.0, ref.abs().max().item()) * (4 if dt == torch.bfloat16 else 1))
+
+
+@pytest.mark.parametrize("M,swap", [(24, 1), (300, 0)])
+def test_gemm_w8a16_dual_glu(M, swap, status):
+    from rhinoforge_b200.ops import kernels as K_
+    dt, N, K = torch.float16, 384, 1024
+    x = (torch.randn(M, K, device="cuda") * 0.5).to(dt)
+    q = torch.randint(-127, 128, (2 * N, K), device="cuda", dtype=torch.int8)
+    sc = (torch.rand(2 * N, device="cuda") * 0.002 + 0.0005).to(dt)
+    y = K_.gemm(x, q, scale=sc, act="silu_mul", dual=True, status=status, force_swap=swap)
+    z = (x.float() @ q.float().t()) * sc.float()
+    _close(y, torch.nn.functional.silu(z[:, :N]) * z[:, N:], dt, scale=2.0)
+
+
+def test_engine_w8a16_matches_dequantised_oracle():
+    """Whole decoder with int8 weights: greedy tokens follow the oracle run on the dequantised weights."""
+    from rhinoforge_b200.models.decoder import TorchDecoder, random_state_dict, tiny_config
+    from rhinoforge_b200.quant._common import dequantize_linear_per_channel, quantize_linear_per_channel
+    from rhinoforge_b200.runtime.engine import DecoderEngine
+    cfg = tiny_config(num_layers=2)
+    sd = random_state_dict(cfg, seed=0, dtype=torch.float16, norm_jitter=0.05)
+    deq = {}
+    for k, v in sd.items():
+        if v.dim() == 2 and "embed" not in k:
+            qq, s = quantize_linear_per_channel(v)
+            deq[k] = dequantize_linear_per_channel(qq, s)
+        else:
+            deq[k] = v
+    if "lm_head.weight" not in sd:            # tied embeddings: the head is the quantised embedding matrix
+        deq["lm_head.weight"] = dequantize_linear_per_channel(*quantize_linear_per_channel(sd["model.embed_tokens.weight"]))
+    oracle = TorchDecoder(cfg, deq, dtype=torch.float32, device="cuda")
+    eng = DecoderEngine(cfg, lambda n: sd[n] if n in sd else sd["model.embed_tokens.weight"], dtype=torch.float16,
+                        max_batch=2, max_seq_len=96, quant="w8a16")
+    g = torch.Generator().manual_seed(7)
+    prompts = [torch.randint(0, cfg.vocab_size, (L,), generator=g) for L in (19, 40)]
+    _, logits = eng.prefill(prompts, return_logits=True)
+    for b, p in enumerate(prompts):
+        oracle.reset()
+        ref = oracle.forward(p[None].cuda())[0, -1]
+        torch.testing.assert_close(logits[b].float(), ref.float(), rtol=1e-2, atol=1e-2)
+    toks = eng.generate(prompts, 6)
+    assert toks.shape == (2, 6)
+    eng.check_status()
+    eng.close()
+
+
+@pytest.mark.parametrize("dt", DT)
+@pytest.mark.parametrize("M,N,K,swap,splits", [(16, 384, 1024, -1, 0), (64, 1000, 2048, 1, 4), (9, 200, 520, 1, 1),
+                                               (300, 640, 1024, 0, 1), (1024, 512, 2048, 0, 1), (700, 130, 264, 0, 1)])
+def test_gemm_packed_weights(dt, M, N, K, swap, splits, status):
+    """Tile-major (bulk-copy) weight layout gives the same result as row-major weights."""
+    from rhinoforge_b200.ops import kernels as K_
+    x = (torch.randn(M, K, device="cuda") * 0.5).to(dt)
+    w = (torch.randn(N, K, device="cuda") * 0.05).to(dt)
+    b = torch.randn(N, device="cuda").to(dt)
+    r = torch.randn(M, N, device="cuda").to(dt)
+    wp = K_.pack_weight(w)
+    y = K_.gemm(x, wp, packed_shape=(N, K), bias=b, residual=r, status=status, force_swap=swap, force_splits=splits)
+    ref = x.float() @ w.float().t() + b.float() + r.float()
+    _close(y, ref, dt, scale=max(1.0, ref.abs().max().item()))
+
+
+@pytest.mark.parametrize("M,swap", [(24, 1), (300, 0)])
+def test_gemm_packed_dual_and_int8(M, swap, status):
+    from rhinoforge_b200.ops import kernels as K_
+    dt, N, K = torch.float16, 200, 1024                    # N not a multiple of 128: sections are padded separately
+    x = (torch.randn(M, K, device="cuda") * 0.5).to(dt)
+    w = (torch.randn(2 * N, K, device="cuda") * 0.05).to(dt)
+    y = K_.gemm(x, K_.pack_weight(w, 2), packed_shape=(2 * N, K), act="silu_mul", dual=True, status=status, force_swap=swap)
+    z = x.float() @ w.float().t()
+    _close(y, torch.nn.functional.silu(z[:, :N]) * z[:, N:], dt, scale=2.0)
+    q = torch.randint(-127, 128, (2 * N, K), device="cuda", dtype=torch.int8)
+    sc = (torch.rand(2 * N, device="cuda") * 0.002 + 0.0005).to(dt)
+    y = K_.gemm(x, K_.pack_weight(q, 2), packed_shape=(2 * N, K), scale=sc, act="silu_mul", dual=True, status=status,
+                force_swap=swap)
+    z = (x.float() @ q.float().t()) * sc.float()
+    _close(y, torch.nn.functional.silu(z[:, :N]) * z[:, N:], dt, scale=2.0)
+
+
+@pytest.mark.parametrize("dt", DT)
+@pytest.mark.parametrize("M,N,K,dual", [(2500, 2048, 520, False), (4100, 1280, 1024, False), (2304, 2560, 512, True),
+                                        (20000, 256, 128, False), (1152, 2560, 512, True), (5000, 2048, 520, False),
+                                        (4900, 1152, 256, False), (4900, 2048, 4096, False)])
+def test_gemm_persistent_kernel(dt, M, N, K, dual, status):
+    """Large token counts take the persistent kernel (one CTA per SM walking tiles): 128-row tiles with two
+    accumulator buffers (the first, second, fourth and fifth shapes) and 256-row tiles (the others); ragged M
+    (a last half-tile partly or wholly past the end), N not a multiple of the tile, several tiles per CTA,
+    a ring shorter and longer than K, bias + residual, GLU epilogue."""
+    from rhinoforge_b200.ops import kernels as K_
+    torch.manual_seed(M)
+    x = (torch.randn(M, K, device="cuda") * 0.5).to(dt)
+    rows = 2 * N if dual else N
+    w = (torch.randn(rows, K, device="cuda") * 0.05).to(dt)
+    wp = K_.pack_weight(w, 2 if dual else 1)
+    if dual:
+        y = K_.gemm(x, wp, packed_shape=(rows, K), act="silu_mul", dual=True, status=status)
+        z = x.float() @ w.float().t()
+        ref = torch.nn.functional.silu(z[:, :N]) * z[:, N:]
+    else:
+        b = torch.randn(N, device="cuda").to(dt)
+        r = torch.randn(M, N, device="cuda").to(dt)
+        y = K_.gemm(x, wp, packed_shape=(rows, K), bias=b, residual=r, status=status)
+        ref = x.float() @ w.float().t() + b.float() + r.float()
+    _close(y, ref, dt, scale=max(1.0, ref.abs().max().item()))
+    y2 = K_.gemm(x, wp, packed_shape=(rows, K), act="silu_mul", dual=True, status=status) if dual else \
+        K_.gemm(x, wp, packed_shape=(rows, K), bias=b, residual=r, status=status)
+    assert torch.equal(y, y2), "two launches of the same GEMM must agree bit for bit"
+    if not dual:
+        # without a residual the results leave through staging tiles and tiled bulk stores
+        y3 = K_.gemm(x, wp, packed_shape=(rows, K), bias=b, status=status)
+        _close(y3, x.float() @ w.float().t() + b.float(), dt, scale=max(1.0, ref.abs().max().item()))
+        view = torch.zeros(M, N + 8, device="cuda", dtype=dt)           # strided output rows
+        K_.gemm(x, wp, packed_shape=(rows, K), out=view[:, :N], status=status)
+        _close(view[:, :N], x.float() @ w.float().t(), dt, scale=max(1.0, ref.abs().max().item()))
+        assert float(view[:, N:].abs().max()) == 0.0, "columns past N must stay untouched"
+        # residual already in the output buffer (out == residual): the add happens in the bulk reduce
+        acc = r.clone()
+        K_.gemm(x, wp, packed_shape=(rows, K), residual=acc, out=acc, status=status)
+        _close(acc, x.float() @ w.float().t() + r.float(), dt, scale=max(1.0, ref.abs().max().item()))
+
+
+def test_manual_graph_capture_replays_with_refilled_inputs(status):
+    """``graph.capture``: one recording run, then replays that refill the static input buffers; a changed shape is refused."""
+    from rhinoforge_b200.graph import capture
+    from rhinoforge_b200.ops import kernels as K_
+    w = (1.0 + 0.1 * torch.randn(256, device="cuda")).half()
+    x = torch.randn(40, 256, device="cuda").half()
+    out = torch.empty_like(x)
+
+    def fn(inp):
+        K_.rmsnorm(inp, w, 1e-6, out=out)
+        return out
+
+    g = capture(fn, x)
+    assert g.replayable, g.non_replayable_reason
+    ref = lambda t: (w.float() * (t.float() * torch.rsqrt(t.float().pow(2).mean(-1, keepdim=True) + 1e-6)))
+    torch.cuda.synchronize()
+    _close(g.cached_output, ref(x), torch.float16)
+    x2 = torch.randn(40, 256, device="cuda").half()
+    y = g.replay(x2)
+    torch.cuda.synchronize()
+    _close(y, ref(x2), torch.float16)
+    st = g.stats()
+    assert st["replays"] == 1 and st["build_count"] == 1 and st["node_count"] >= 1
+    with pytest.raises(RuntimeError, match="shape_bucket"):
+        g.replay(torch.randn(41, 256, device="cuda").half())
+    g.invalidate()
+
+
+@pytest.mark.parametrize("dt", DT)
+@pytest.mark.parametrize("dual", [False, True])
+def test_gemm_w8a16_large_m_widens_once_and_matches(dt, dual, status):
+    """W8A16 with a prefill-sized token count and caller scratch: the int8 image is widened once and the 16-bit
+    (persistent) kernel runs; the result equals ``(x . q^T) * scale`` like the in-loop path without scratch."""
+    from rhinoforge_b200.ops import kernels as K_
+    torch.manual_seed(3)
+    M, N, K = 2304, 2560, 512
+    x = (torch.randn(M, K, device="cuda") * 0.5).to(dt)
+    rows = 2 * N if dual else N
+    q = torch.randint(-127, 128, (rows, K), device="cuda", dtype=torch.int8)
+    sc = (torch.rand(rows, device="cuda") * 0.002 + 0.0005).to(dt)
+    qp = K_.pack_weight(q, 2 if dual else 1)
+    scratch = torch.empty(2 * qp.numel(), dtype=torch.uint8, device="cuda")
+    kw = dict(packed_shape=(rows, K), scale=sc, status=status)
+    if dual:
+        kw.update(act="silu_mul", dual=True)
+    y = K_.gemm(x, qp, w_scratch=scratch, **kw)
+    y0 = K_.gemm(x, qp, **kw)
+    z = (x.float() @ q.float().t()) * sc.float()
+    ref = torch.nn.functional.silu(z[:, :N]) * z[:, N:] if dual else z
+    _close(y, ref, dt, scale=max(1.0, ref.abs().max().item()))
+    _close(y0, ref, dt, scale=max(1.0, ref.abs().max().item()))
+
+
+@pytest.mark.parametrize("dt", DT)
+@pytest.mark.parametrize("M,N,K", [(64, 4096, 512), (64, 4096, 1024), (50, 1024, 192), (8, 2048, 64)])
+def test_gemm_short_k_splits_down_to_one_block_per_cta(dt, M, N, K, status):
+    """Short-K weight-streaming shapes (tensor-parallel out-projections): the planner may give every CTA of the
+    cluster a single k block (or fewer splits than blocks when K is tiny); bias, residual and the rotated K start are
+    all in play."""
+    from rhinoforge_b200.ops import kernels as K_
+    x = (torch.randn(M, K, device="cuda") * 0.5).to(dt)
+    w = (torch.randn(N, K, device="cuda") * 0.05).to(dt)
+    b = torch.randn(N, device="cuda").to(dt)
+    r = torch.randn(M, N, device="cuda").to(dt)
+    ref = x.float() @ w.float().t() + b.float() + r.float()
+    y = K_.gemm(x, K_.pack_weight(w), packed_shape=(N, K), bias=b, residual=r, status=status)
+    _close(y, ref, dt, scale=max(1.0, ref.abs().max().item()))
+    y2 = K_.gemm(x, w, bias=b, residual=r, status=status)                  # row-major weights, same planner
+    _close(y2, ref, dt, scale=max(1.0, ref.abs().max().item()))
+    for s in (1, 8):
+        if s * 64 <= max(K, 64) or s == 1:
+            y3 = K_.gemm(x, K_.pack_weight(w), packed_shape=(N, K), bias=b, residual=r, status=status, force_splits=s)
+            _close(y3, ref, dt, scale=max(1.0, ref.abs().max().item()))
+
+
+def _close_elementwise(y, ref, dt):
+    """Every element within fp16 / bf16 rounding of ITS OWN reference value (plus a small absolute floor), so a
+    wrong low-magnitude column cannot hide behind the largest entry of the matrix."""
+    rel = 2.0 ** -7 if dt == torch.bfloat16 else 2.0 ** -10
+    err = (y.float() - ref.float()).abs()
+    bound = rel * ref.float().abs() * 2.0 + (6e-2 if dt == torch.bfloat16 else 6e-3)
+    bad = (err > bound).nonzero()
+    assert bad.numel() == 0, f"{bad.shape[0]} elements off; first {bad[0].tolist()}: {y[tuple(bad[0])].item()} vs {ref[tuple(bad[0])].item()}"
+
+
+@pytest.mark.parametrize("dt", DT)
+@pytest.mark.parametrize("M,N,K,dual", [(1, 4096, 4096, False), (7, 384, 2048, False), (16, 1000, 1024, False),
+                                        (64, 2048, 4096, True), (64, 4096, 12288, False), (33, 1280, 512, True),
+                                        (200, 640, 2560, False), (256, 1152, 1024, False), (96, 8192, 1024, True),
+                                        (64, 151936, 1024, False)])
+def test_gemm_stream_k(dt, M, N, K, dual, status):
+    """The persistent stream-K kernel (tile-major weights, at most 256 tokens): shares that start and end inside a
+    tile (partials parked in scratch and added by the tile's finisher), several tiles per CTA, ragged N, one token,
+    a full 256-token tile, GLU pairs, a vocabulary-sized N; bias, per-channel scale, per-row scale and residual;
+    two launches agree bit for bit."""
+    from rhinoforge_b200 import _native as N_
+    from rhinoforge_b200.ops import kernels as K_
+    old_mode = N_.lib().rf_gemm_streamk_mode(2)          # every shape that fits, not only the large-N ones
+    try:
+        _stream_k_case(dt, M, N, K, dual, status)
+    finally:
+        N_.lib().rf_gemm_streamk_mode(old_mode)
+
+
+def _stream_k_case(dt, M, N, K, dual, status):
+    from rhinoforge_b200.ops import kernels as K_
+    torch.manual_seed(M * 7 + N)
+    rows = 2 * N if dual else N
+    plan = K_.gemm_plan(M, N, K, dtype=dt, dual=dual, packed=True)
+    x = (torch.randn(M, K, device="cuda") * 0.5).to(dt)
+    w = (torch.randn(rows, K, device="cuda") * (1.0 / math.sqrt(K))).to(dt)
+    wp = K_.pack_weight(w, 2 if dual else 1)
+    z = x.float() @ w.float().t()
+    if dual:
+        y = K_.gemm(x, wp, packed_shape=(rows, K), act="silu_mul", dual=True, status=status)
+        ref = torch.nn.functional.silu(z[:, :N]) * z[:, N:]
+        y2 = K_.gemm(x, wp, packed_shape=(rows, K), act="silu_mul", dual=True, status=status)
+    else:
+        b = torch.randn(N, device="cuda").to(dt)
+        sc = (torch.rand(N, device="cuda") + 0.5).to(dt)
+        rs = torch.rand(M, device="cuda") + 0.5
+        r = torch.randn(M, N, device="cuda").to(dt)
+        y = K_.gemm(x, wp, packed_shape=(rows, K), bias=b, scale=sc, row_scale=rs, residual=r, status=status)
+        ref = z * rs[:, None] * sc.float() + b.float() + r.float()
+        y2 = K_.gemm(x, wp, packed_shape=(rows, K), bias=b, scale=sc, row_scale=rs, residual=r, status=status)
+        # in place: the residual already sits in the output buffer
+        acc = r.clone()
+        K_.gemm(x, wp, packed_shape=(rows, K), residual=acc, out=acc, status=status)
+        _close_elementwise(acc, z + r.float(), dt)
+    _close_elementwise(y, ref, dt)
+    assert torch.equal(y, y2), "two launches of the same GEMM must agree bit for bit"
+    assert plan is None or plan["persistent"] in (0, 2)
+
+
+@pytest.mark.parametrize("dt", DT)
+@pytest.mark.parametrize("M,N,K,group,dual", [(1, 1024, 4096, 64, False), (16, 1000, 1024, 32, False), (64, 384, 2048, 128, False),
+                                              (64, 2048, 1024, 0, False), (33, 1280, 512, 64, True), (200, 640, 2560, 32, False),
+                                              (300, 512, 1024, 64, False), (300, 768, 512, 128, True), (8, 256, 192, 64, False)])
+def test_gemm_w4a16(dt, M, N, K, group, dual, status):
+    """int4 weights in the tile-major image: nibbles widened and group scales applied by the converter warps of the
+    main loop (per-channel scales in the epilogue when group = 0); reference = x @ dequantised weights in fp32."""
+    from rhinoforge_b200.ops import kernels as K_
+    torch.manual_seed(N + K + group)
+    rows = 2 * N if dual else N
+    x = (torch.randn(M, K, device="cuda") * 0.5).to(dt)
+    q = torch.randint(-8, 8, (rows, K), device="cuda", dtype=torch.int8)
+    r = torch.randn(M, N, device="cuda").to(dt)
+    kw = dict(packed_shape=(rows, K), w_bits=4, w_group=group, status=status)
+    if group:
+        sc = (torch.rand(rows, K // group, device="cuda") * 0.03 + 0.005).to(dt)
+        img = K_.pack_weight_int4(q, sc, group, sections=2 if dual else 1, dtype=dt)
+        wd = q.float().view(rows, K // group, group) * sc.float()[..., None]
+        wd = wd.view(rows, K)
+    else:
+        sc = (torch.rand(rows, device="cuda") * 0.03 + 0.005).to(dt)
+        img = K_.pack_weight_int4(q, sections=2 if dual else 1)
+        kw["scale"] = sc
+        wd = q.float() * sc.float()[:, None]
+    assert img.numel() == K_.N.lib().rf_pack_w4_bytes(rows, K, 2 if dual else 1, group)
+    z = x.float() @ wd.t()
+    if dual:
+        y = K_.gemm(x, img, act="silu_mul", dual=True, **kw)
+        ref = torch.nn.functional.silu(z[:, :N]) * z[:, N:]
+    else:
+        y = K_.gemm(x, img, residual=r, **kw)
+        ref = z + r.float()
+    _close(y, ref, dt, scale=max(1.0, ref.abs().max().item()) * (4 if dt == torch.bfloat16 else 1))
+
+
+@pytest.mark.parametrize("group,from_packed", [(64, False), (32, True), (0, False)])
+def test_engine_w4a16_matches_dequantised_oracle(group, from_packed):
+    """Whole decoder with int4 projections (lm_head 16-bit): prefill logits follow the oracle run on the dequantised
+    weights, whether the engine quantises 16-bit weights itself or reads a packed 4-bit checkpoint."""
+    from rhinoforge_b200.models.decoder import TorchDecoder, random_state_dict, tiny_config
+    from rhinoforge_b200.quant.int4_pack import pack_int4
+    from rhinoforge_b200.runtime.engine import DecoderEngine
+    cfg = tiny_config(num_layers=2)
+    sd = random_state_dict(cfg, seed=0, dtype=torch.float16, norm_jitter=0.05)
+
+    def quant(w):
+        wf = w.float()
+        grp = wf.view(wf.shape[0], -1, group) if group else wf.view(wf.shape[0], 1, -1)
+        sc = (grp.abs().amax(-1) / 7.0).clamp_min(1e-8)
+        q = torch.round(grp / sc[..., None]).clamp_(-8, 7)
+        return q.to(torch.int8).view_as(wf), sc, (q * sc[..., None].half().float()).view_as(wf)
+
+    deq, packed, scales = {}, {}, {}
+    for k, v in sd.items():
+        if v.dim() == 2 and "embed" not in k and "lm_head" not in k:
+            q, sc, d = quant(v)
+            deq[k], packed[k], scales[k] = d, pack_int4(q), sc.half()
+        else:
+            deq[k] = v
+    oracle = TorchDecoder(cfg, deq, dtype=torch.float32, device="cuda")
+
+    def get(n):
+        if n not in sd:
+            return sd["model.embed_tokens.weight"]
+        return packed[n] if (from_packed and n in packed) else sd[n]
+    get.scale = lambda n: scales.get(n)
+    eng = DecoderEngine(cfg, get, dtype=torch.float16, max_batch=2, max_seq_len=96, quant="w4a16", w4_group=group)
+    g = torch.Generator().manual_seed(7)
+    prompts = [torch.randint(0, cfg.vocab_size, (L,), generator=g) for L in (19, 40)]
+    _, logits = eng.prefill(prompts, return_logits=True)
+    for b, p in enumerate(prompts):
+        oracle.reset()
+        ref = oracle.forward(p[None].cuda())[0, -1]
+        torch.testing.assert_close(logits[b].float(), ref.float(), rtol=2e-2, atol=2e-2)
+    toks = eng.generate(prompts, 6)
+    assert toks.shape == (2, 6)
+    eng.check_status()
+    eng.close()
+
+
+@pytest.mark.parametrize("dt", DT)
+@pytest.mark.parametrize("M,N,K,dual", [(1, 1024, 2048, False), (48, 520, 1024, False), (64, 768, 512, True), (300, 512, 1024, False)])
+def test_gemm_nvfp4(dt, M, N, K, dual, status):
+    """NVFP4 weights (e2m1 codes, e4m3 block scale per 16 columns, fp32 tensor scale) through the 4-bit main loop;
+    reference = x @ the exact fp32 weight the codes stand for."""
+    from rhinoforge_b200.ops import kernels as K_
+    from rhinoforge_b200.quant.nvfp4_pack import dequantize_nvfp4, quantize_nvfp4
+    torch.manual_seed(N + K)
+    rows = 2 * N if dual else N
+    w = torch.randn(rows, K, device="cuda") * 0.05
+    codes, sc, ts = quantize_nvfp4(w)
+    wd = dequantize_nvfp4(codes, sc, ts)
+    img = K_.pack_weight_nvfp4(codes, sc, ts, sections=2 if dual else 1, dtype=dt)
+    x = (torch.randn(M, K, device="cuda") * 0.5).to(dt)
+    kw = dict(packed_shape=(rows, K), w_bits=4, w_group=16, w_fp4=True, status=status)
+    z = x.float() @ wd.t()
+    if dual:
+        y = K_.gemm(x, img, act="silu_mul", dual=True, **kw)
+        ref = torch.nn.functional.silu(z[:, :N]) * z[:, N:]
+    else:
+        y = K_.gemm(x, img, **kw)
+        ref = z
+    _close(y, ref, dt, scale=max(1.0, ref.abs().max().item()) * (4 if dt == torch.bfloat16 else 1))
+
+
+@pytest.mark.parametrize("dt", DT)
+@pytest.mark.parametrize("M,H,I,splits", [(1, 1024, 2048, 0), (64, 1024, 3072, 0), (16, 512, 1024, 1), (200, 768, 1536, 0),
+                                           (33, 1280, 512, 4)])
+def test_gemm_folded_rmsnorm(dt, M, H, I, splits, status):
+    """RMSNorm without a kernel of its own: the residual GEMM writes per-tile sums of squares of its finished rows, the
+    next projection (norm weights multiplied into its columns) scales its rows by their reciprocal RMS.  Reference:
+    rmsnorm(hidden) * w @ W2^T on the rows the first GEMM stored."""
+    from rhinoforge_b200.ops import kernels as K_
+    torch.manual_seed(M + H)
+    x = (torch.randn(M, I, device="cuda") * 0.5).to(dt)
+    w1 = (torch.randn(H, I, device="cuda") * 0.05).to(dt)
+    resid = torch.randn(M, H, device="cuda").to(dt)
+    nw = (1.0 + 0.2 * torch.randn(H, device="cuda")).to(dt)
+    w2 = (torch.randn(2 * I, H, device="cuda") * 0.05).to(dt)
+    bias = (torch.randn(2 * I, device="cuda") * 0.1).to(dt)
+    tiles = (H + 127) // 128
+    ss = torch.full((tiles, 256), float("nan"), device="cuda")
+    hidden = resid.clone()
+    K_.gemm(x, K_.pack_weight(w1), packed_shape=(H, I), residual=hidden, out=hidden, ss_out=ss, status=status,
+            force_splits=splits)
+    ref_h = (x.float() @ w1.float().t() + resid.float())
+    _close(hidden, ref_h, dt, scale=max(1.0, ref_h.abs().max().item()))
+    want_ss = hidden.float().pow(2).view(M, tiles, -1).sum(-1).t()             # [tiles, M] of the rows as stored
+    torch.testing.assert_close(ss[:, :M], want_ss, rtol=1e-4, atol=1e-3)
+    w2f = (w2.float() * nw.float()[None]).to(dt)                                # norm weights folded into the columns
+    y = K_.gemm(hidden, K_.pack_weight(w2f, 2), packed_shape=(2 * I, H), bias=bias, act="silu_mul", dual=True, ss_in=ss,
+                ss_dim=H, ss_eps=1e-6, status=status)
+    hn = hidden.float() * torch.rsqrt(hidden.float().pow(2).mean(-1, keepdim=True) + 1e-6) * nw.float()
+    z = hn @ w2.float().t() + bias.float()
+    ref = torch.nn.functional.silu(z[:, :I]) * z[:, I:]
+    _close(y, ref, dt, scale=max(1.0, ref.abs().max().item()) * (4 if dt == torch.bfloat16 else 1))
+
+
+@pytest.mark.parametrize("dt", DT)
+@pytest.mark.parametrize("M,N,K", [(128, 384, 1536), (128, 1536, 384), (41, 1536, 2048), (50, 1024, 4096), (31, 1024, 1024),
+                                   (7, 72, 136), (130, 200, 72), (256, 512, 640), (1, 384, 384), (1028, 1152, 384), (600, 384, 1536)])
+@pytest.mark.parametrize("packed", [False, True])
+def test_gemm_small_latency_kernel(dt, M, N, K, packed, status, monkeypatch):
+    """Shapes the latency-bound kernel takes (few rows, small weight): every epilogue option against fp32 PyTorch, and the
+    same call with the kernel switched off (the streaming kernel) within rounding."""
+    from rhinoforge_b200.ops import kernels as K_
+    x = (torch.randn(M, K, device="cuda") * 0.5).to(dt)
+    w = (torch.randn(N, K, device="cuda") * 0.05).to(dt)
+    b = torch.randn(N, device="cuda").to(dt)
+    r = torch.randn(M, N, device="cuda").to(dt)
+    wk = K_.pack_weight(w) if packed else w
+    kw = dict(packed_shape=(N, K)) if packed else {}
+    ref = x.float() @ w.float().t()
+    _close(K_.gemm(x, wk, **kw), ref, dt, scale=max(1.0, float(ref.abs().max())))
+    full = torch.nn.functional.gelu(ref + b.float(), approximate="tanh") + r.float()
+    got = K_.gemm(x, wk, bias=b, act="gelu_tanh", residual=r, **kw)
+    _close(got, full, dt, scale=max(1.0, float(full.abs().max())))
+    # per-column factor before the bias (the gate of a gated residual): r + (x.w^T * s + b)
+    sc = (torch.randn(N, device="cuda") * 0.5).to(dt)
+    gated = ref * sc.float() + b.float() + r.float()
+    _close(K_.gemm(x, wk, scale=sc, bias=b, residual=r, **kw), gated, dt, scale=max(1.0, float(gated.abs().max())))
+    # strided output / input views
+    buf = torch.zeros(M, N + 16, device="cuda", dtype=dt)
+    K_.gemm(x, wk, out=buf[:, 8:8 + N], **kw)
+    _close(buf[:, 8:8 + N], ref, dt, scale=max(1.0, float(ref.abs().max())))
+    assert float(buf[:, :8].abs().max()) == 0 and float(buf[:, 8 + N:].abs().max()) == 0
+
+
+def test_gemm_forced_wide_tile_over_odd_block_count(status):
+    """A forced 256-wide tile on a tile-major weight with an odd number of 128-row blocks (N = 1152: nine) falls back to
+    128-wide tiles instead of copying a tenth block that is not there; token-row split K (pushed partial slices) on
+    the same shape at 2 and 4 splits."""
+    from rhinoforge_b200.ops import kernels as K_
+    M, N, K = 768, 1152, 1152
+    x = (torch.randn(M, K, device="cuda") * 0.5).half()
+    w = (torch.randn(N, K, device="cuda") * 0.05).half()
+    r = torch.randn(M, N, device="cuda").half()
+    wp = K_.pack_weight(w)
+    ref = x.float() @ w.float().t() + r.float()
+    for kw in (dict(force_bn=256), dict(force_bn=256, force_splits=2), dict(force_bn=128, force_splits=4), dict(force_splits=3)):
+        got = K_.gemm(x, wp, packed_shape=(N, K), residual=r, status=status, **kw)
+        _close(got, ref, torch.float16, scale=max(1.0, float(ref.abs().max())))
+
+
+@pytest.mark.parametrize("dt", DT)
+@pytest.mark.parametrize("M,N,K", [(50, 4096, 1024), (128, 1536, 384), (31, 136, 200)])
+@pytest.mark.parametrize("packed", [False, True])
+def test_gemm_small_dual_glu(dt, M, N, K, packed, status):
+    from rhinoforge_b200.ops import kernels as K_
+    x = (torch.randn(M, K, device="cuda") * 0.5).to(dt)
+    w = (torch.randn(2 * N, K, device="cuda") * 0.05).to(dt)
+    b = (torch.randn(2 * N, device="cuda") * 0.1).to(dt)
+    wk = K_.pack_weight(w, sections=2) if packed else w
+    kw = dict(packed_shape=(2 * N, K)) if packed else {}
+    gte, up = x.float() @ w[:N].float().t() + b[:N].float(), x.float() @ w[N:].float().t() + b[N:].float()
+    ref = torch.nn.functional.silu(gte) * up
+    got = K_.gemm(x, wk, bias=b, act="silu_mul", dual=True, **kw)
+    _close(got, ref, dt, scale=max(1.0, float(ref.abs().max())))
+
+
+@pytest.mark.parametrize("dt", DT)
+@pytest.mark.parametrize("M,N,K,splits", [(1, 128, 512, 8), (16, 136, 576, 3), (17, 1000, 640, 2), (65, 264, 1024, 4), (93, 300, 1024, 8),
+                                          (33, 7, 256, 1), (130, 640, 512, 1), (256, 384, 256, 2)])
+@pytest.mark.parametrize("vec", [True, False])
+def test_gemm_weight_row_epilogue(dt, M, N, K, splits, vec, status, monkeypatch):
+    """Few tokens, weights on the MMA rows: parked partials, the splits' sums and the eight-feature finish against fp32 - one split in
+    passes of 64 (32 for a GLU) tokens, two to eight splits, token and feature counts that end inside a group, operands that cannot be
+    read as 16-byte vectors."""
+    from rhinoforge_b200.ops import kernels as K_
+    monkeypatch.setenv("RF_GEMM_SMALL", "0")
+    x = (torch.randn(M, K, device="cuda") * 0.5).to(dt)
+    w = (torch.randn(2 * N, K, device="cuda") * 0.05).to(dt)
+    off, pitch = (0, (N + 7) // 8 * 8) if vec else (1, N + 3)
+    vector = lambda n, base: (base + 0.2 * torch.randn(n + 1, device="cuda")).to(dt)[off:off + n]
+    b, sc, r = vector(N, 0.0), vector(N, 1.0), torch.randn(M, pitch, device="cuda").to(dt)[:, :N]
+    out = torch.full((M, pitch), 7.0, device="cuda").to(dt)
+    y = K_.gemm(x, K_.pack_weight(w[:N]), packed_shape=(N, K), bias=b, scale=sc, residual=r, out=out[:, :N], status=status, force_splits=splits, force_swap=1)
+    z = x.float() @ w.float().t()
+    ref = z[:, :N] * sc.float() + b.float() + r.float()
+    _close(y, ref, dt, scale=max(1.0, ref.abs().max().item()))
+    assert bool((out[:, N:] == 7.0).all())
+    try:
+        y = K_.gemm(x, K_.pack_weight(w, 2), packed_shape=(2 * N, K), act="silu_mul", dual=True, status=status, force_splits=splits, force_swap=1)
+    except Exception as e:
+        assert M > 128 and "partial" in str(e)                 # two parked accumulators of this many tokens do not fit
+    else:
+        _close(y, torch.nn.functional.silu(z[:, :N]) * z[:, N:], dt, scale=2.0)
+
+
+@pytest.mark.parametrize("dt", DT)
+@pytest.mark.parametrize("M,N,K", [(5000, 1152, 256), (4100, 4304, 128), (2500, 136, 520), (768, 4304, 1152), (825, 2560, 2048), (6000, 328, 64)])
+@pytest.mark.parametrize("vec", [True, False])
+def test_gemm_persistent_epilogue(dt, M, N, K, vec, status):
+    """Persistent kernel: column tiles that end in the middle of a weight block or before their second one, bias and scale from the lanes
+    of a warp, the residual added ahead of the staged store, operands that cannot be read as 16-byte vectors."""
+    from rhinoforge_b200.ops import kernels as K_
+    x = (torch.randn(M, K, device="cuda") * 0.5).to(dt)
+    w = (torch.randn(N, K, device="cuda") * 0.05).to(dt)
+    wp = K_.pack_weight(w)
+    off, pitch = (0, N + 8) if vec else (1, N + 3)
+    vector = lambda n, base: (base + 0.2 * torch.randn(n + 1, device="cuda")).to(dt)[off:off + n]
+    b, sc, r = vector(N, 0.0), vector(N, 1.0), torch.randn(M, pitch, device="cuda").to(dt)
+    rs = torch.rand(M, device="cuda") + 0.5
+    z = x.float() @ w.float().t()
+    ref = z * rs[:, None] * sc.float() + b.float() + r[:, :N].float()
+    scale = max(1.0, ref.abs().max().item())
+    _close(K_.gemm(x, wp, packed_shape=(N, K), bias=b, scale=sc, row_scale=rs, residual=r[:, :N], status=status), ref, dt, scale=scale)
+    acc = r.clone()
+    K_.gemm(x, wp, packed_shape=(N, K), bias=b, act="gelu_tanh", residual=acc[:, :N], out=acc[:, :N], status=status)
+    ref = torch.nn.functional.gelu(z + b.float(), approximate="tanh") + r[:, :N].float()
+    _close(acc[:, :N], ref, dt, scale=scale)
+    assert torch.equal(acc[:, N:], r[:, N:])
+
+
+@pytest.mark.parametrize("dt", DT)
+@pytest.mark.parametrize("M,N,K", [(1, 16, 64), (1, 1000, 72), (7, 264, 520), (8, 40, 8), (9, 1536, 1024), (16, 5000, 1160), (3, 24, 4096), (16, 7, 2048)])
+@pytest.mark.parametrize("dual", [False, True])
+def test_gemm_very_few_rows(dt, M, N, K, dual, status):
+    """Up to 16 rows over 16-bit weights: strips of 16 features that end inside a weight block or past N, fewer k blocks than warps and
+    partial ones, every epilogue option, strided and odd-pitched outputs, a CTA that takes several strips; the RMSNorm that the kernel
+    folds in itself."""
+    from rhinoforge_b200.ops import kernels as K_
+    rows = 2 * N if dual else N
+    x = (torch.randn(M, K + 8, device="cuda") * 0.5).to(dt)[:, :K]
+    w = (torch.randn(rows, K, device="cuda") / K ** 0.5).to(dt)
+    wp = K_.pack_weight(w, 2 if dual else 1)
+    b, sc = torch.randn(rows, device="cuda").to(dt), (torch.rand(rows, device="cuda") + 0.5).to(dt)
+    rs, r = torch.rand(M, device="cuda") + 0.5, torch.randn(M, N, device="cuda").to(dt)
+    out = torch.full((M, N + 3), 7.0, device="cuda").to(dt)
+    kw = dict(packed_shape=(rows, K), status=status, **(dict(act="silu_mul", dual=True) if dual else {}))
+    finish = lambda z: torch.nn.functional.silu(z[:, :N]) * z[:, N:] if dual else z
+    K_.gemm(x, wp, bias=b, scale=sc, row_scale=rs, residual=r, out=out[:, :N], **kw)
+    z = x.float() @ w.float().t()
+    _close(out[:, :N], finish(z * rs[:, None] * sc.float() + b.float()) + r.float(), dt, scale=2.0)
+    assert bool((out[:, N:] == 7.0).all())
+    ss = torch.zeros((max(K // 128, 1), 256), device="cuda")
+    ss[0, :M] = x.float().pow(2).sum(1)
+    _close(K_.gemm(x, wp, ss_in=ss, ss_dim=K, ss_eps=1e-6, **kw), finish(z * torch.rsqrt(x.float().pow(2).mean(1, keepdim=True) + 1e-6)), dt, scale=4.0)
+
+
+@pytest.mark.parametrize("dt", DT)
+@pytest.mark.parametrize("M", [1, 8, 11, 16])
+@pytest.mark.parametrize("N,K,group,fp4", [(264, 320, 0, False), (1000, 1024, 64, False), (40, 2176, 32, False), (128, 192, 16, True), (5008, 512, None, False)])
+@pytest.mark.parametrize("dual", [False, True])
+def test_gemm_very_few_rows_quantised(dt, M, N, K, group, fp4, dual, status):
+    """Up to 16 rows over int8 (``group`` None) and 4-bit weights, against the product with the values that the image holds."""
+    from rhinoforge_b200.ops import kernels as K_
+    rows = 2 * N if dual else N
+    x = (torch.randn(M, K, device="cuda") / K ** 0.5).to(dt)
+    sc = (torch.rand(rows, device="cuda") * 0.2 + 0.1).to(dt)
+    kw = dict(packed_shape=(rows, K), status=status, **(dict(act="silu_mul", dual=True) if dual else {}))
+    sections = 2 if dual else 1
+    if group is None:
+        q = torch.randint(-127, 128, (rows, K), device="cuda", dtype=torch.int8)
+        y, w = K_.gemm(x, K_.pack_weight(q, sections), scale=sc, **kw), q.float() * sc.float()[:, None]
+    else:
+        q = torch.randint(-8, 8, (rows, K), device="cuda", dtype=torch.int8)
+        gs = (torch.rand(rows, K // group, device="cuda") * 0.2 + 0.1).to(dt) if group else None
+        value = torch.tensor([0, 0.5, 1, 1.5, 2, 3, 4, 6, -0.0, -0.5, -1, -1.5, -2, -3, -4, -6], device="cuda")[(q & 15).long()] if fp4 else q.float()
+        img = K_.pack_weight_int4(q, gs, group, sections=sections, dtype=dt)
+        y = K_.gemm(x, img, w_bits=4, w_group=group, w_fp4=fp4, scale=None if group else sc, **kw)
+        w = (value.view(rows, -1, group) * gs.float()[..., None]).view(rows, K).to(dt).float() if group else value * sc.float()[:, None]
+    z = x.float() @ w.t()
+    ref = torch.nn.functional.silu(z[:, :N]) * z[:, N:] if dual else z
+    _close(y, ref, dt, scale=max(1.0, ref.abs().max().item()))
+
+
+@pytest.mark.parametrize("dt", DT)
+@pytest.mark.parametrize("hd,Hq,Hkv", [(64, 32, 8), (128, 32, 4)])
+@pytest.mark.parametrize("mode", ["causal", "window", "full", "mask"])
+def test_attn_prefill_two_tiles(dt, hd, Hq, Hkv, mode, status):
+    """Enough heads and rows that a CTA takes two query tiles: second tiles that are empty, partial and full, keys ahead of the new rows, tiles that
+    stop at different blocks, and the masks that leave a tile's first blocks empty - paged against fp32, contiguous against paged."""
+    from rhinoforge_b200.ops import kernels as K_
+    q_lens, kv_lens = [257, 100, 384, 129], [257, 420, 400, 129]
+    k_pool, v_pool, pt, ks, vs = _paged(Hkv, hd, kv_lens, dt)
+    i32 = lambda l: torch.tensor(l, dtype=torch.int32, device="cuda")
+    starts = [sum(q_lens[:i]) for i in range(len(q_lens))]
+    q = torch.randn(sum(q_lens), Hq * hd, device="cuda").to(dt)
+    kw = dict(Hq=Hq, Hkv=Hkv, hd=hd, q_start=i32(starts), q_len=i32(q_lens), kv_len=i32(kv_lens), max_q_len=max(q_lens), causal=mode in ("causal", "window"),
+              window=70 if mode == "window" else 0, status=status)
+    given = torch.rand(len(q_lens), max(q_lens), 432, device="cuda") > 0.4
+    given[:, :, 0] = True
+    if mode == "mask":
+        kw["mask"] = given
+    out = K_.attention_prefill(q, torch.zeros_like(q), k_pool=k_pool, v_pool=v_pool, page_table=pt, **kw)
+    flat = lambda parts: torch.cat([t.transpose(0, 1).reshape(t.shape[1], Hkv * hd) for t in parts])
+    rows = K_.attention_prefill(q, torch.zeros_like(q), k=flat(ks), v=flat(vs), kv_start=i32([sum(kv_lens[:i]) for i in range(len(kv_lens))]), **kw)
+    assert torch.equal(out, rows)
+    for s, (Lq, Lk) in enumerate(zip(q_lens, kv_lens)):
+        qs = q[starts[s]:starts[s] + Lq].view(Lq, Hq, hd).transpose(0, 1)
+        i, j = torch.arange(Lq, device="cuda")[:, None] + (Lk - Lq), torch.arange(Lk, device="cuda")[None]
+        mask = torch.ones(Lq, Lk, dtype=torch.bool, device="cuda") if mode == "full" else given[s, :Lq, :Lk] if mode == "mask" else j <= i
+        if mode == "window":
+            mask = mask & (j > i - 70)
+        ref = _sdpa_ref(qs, ks[s], vs[s], mask).transpose(0, 1).reshape(Lq, Hq * hd)
+        _close(out[starts[s]:starts[s] + Lq], ref, dt)
+
+
+@pytest.mark.parametrize("dt", DT)
+@pytest.mark.parametrize("H", [8, 264, 1024, 1152, 2040, 3072, 4096, 4104])
+@pytest.mark.parametrize("rows", [295, 1301])
+def test_norms_of_many_rows(dt, H, rows):
+    """A warp per row (296 rows and more, up to 4096 values): rows that end inside a piece, a last block with idle warps, residual and modulation,
+    pitched rows, in place - and one size past each end of that range on the block kernels."""
+    from rhinoforge_b200.ops import kernels as K_
+    x = torch.randn(rows, H, device="cuda").to(dt)
+    r = torch.randn(rows, H, device="cuda").to(dt)
+    w, b = (1 + 0.1 * torch.randn(H, device="cuda")).to(dt), torch.randn(H, device="cuda").to(dt)
+    mod = torch.randn((rows + 6) // 7, 3 * H, device="cuda").to(dt)
+    rms = lambda t: t.float() * torch.rsqrt(t.float().pow(2).mean(-1, keepdim=True) + 1e-6)
+    _close(K_.layernorm(x, w, b, 1e-6), torch.nn.functional.layer_norm(x.float(), (H,), w.float(), b.float(), 1e-6), dt, scale=2.0)
+    total, out = torch.empty_like(x), torch.empty(rows, H + 8, device="cuda", dtype=dt)
+    K_.rmsnorm(x, w, 1e-6, residual=r, residual_out=total, out=out[:, :H])
+    assert torch.equal(total, (x.float() + r.float()).to(dt))
+    _close(out[:, :H], rms(total) * w.float(), dt, scale=2.0)
+    _close(K_.rmsnorm(x, w, 1e-6, gemma=True), rms(x) * (1 + w.float()), dt, scale=4.0)
+    m = mod.float().repeat_interleave(7, 0)[:rows]
+    _close(K_.rmsnorm(x, None, 1e-6, mod=mod, rows_per_mod=7), rms(x) * (1 + m[:, :H]) + m[:, H:2 * H], dt, scale=6.0)
+    y = x.clone()
+    K_.rmsnorm(y, None, 1e-6, out=y)
+    _close(y, rms(x), dt, scale=2.0)
+
+
+@pytest.mark.parametrize("dt", DT)
+@pytest.mark.parametrize("hd,rot,Hq,Hkv", [(64, 64, 3, 1), (128, 64, 5, 2), (128, 128, 16, 8), (256, 96, 2, 1), (64, 24, 4, 4)])
+@pytest.mark.parametrize("T", [1, 3, 77, 600])
+def test_rope_kv_few_and_many_tokens_agree(dt, hd, rot, Hq, Hkv, T):
+    """Norm, rotation and page insertion of the same rows at every launch size (and on the scalar kernel, which takes rotations that are no multiple
+    of 16): heads that do not fill the last warp, tables that are and are not 16-byte aligned, one and three position axes, in place and paged."""
+    from rhinoforge_b200.ops import kernels as K_
+    width = (Hq + 2 * Hkv) * hd
+    qkv = torch.randn(T, width, device="cuda").to(dt)
+    w = [(1 + 0.1 * torch.randn(hd, device="cuda")).to(dt) for _ in range(2)]
+    ang = torch.rand(T + 9, rot // 2, device="cuda") * 6.0
+    table = torch.stack((ang.cos(), ang.sin()))
+    shifted = torch.empty(table.numel() + 1, device="cuda")[1:].view_as(table).copy_(table)          # 4-byte aligned only
+    pos3 = torch.randint(0, T + 9, (T, 3), dtype=torch.int32, device="cuda")
+    axis = (torch.arange(rot // 2) % 3).to(torch.int8).cuda()
+    pt = torch.randperm((T + 15) // 16 + 2, device="cuda").to(torch.int32)[None].repeat(T, 1).contiguous()
+    seq, cpos = torch.zeros(T, dtype=torch.int32, device="cuda"), torch.arange(T, dtype=torch.int32, device="cuda")
+
+    def ref(pos_of):
+        x = qkv.view(T, -1, hd).float()
+        parts = []
+        for heads, wt in ((x[:, :Hq], w[0]), (x[:, Hq:Hq + Hkv], w[1])):
+            n = wt.float() * (heads * torch.rsqrt(heads.pow(2).mean(-1, keepdim=True) + 1e-6)).to(dt).float()
+            n = n.to(dt).float()
+            c, s = (torch.gather(t, 0, pos_of.long())[:, None] for t in table)
+            u, v = n[..., :rot // 2], n[..., rot // 2:rot]
+            parts.append(torch.cat((u * c - v * s, v * c + u * s, n[..., rot:]), -1))
+        return parts
+
+    for cos_sin, three in ((table, False), (shifted, False), (table, True)):
+        pos = pos3 if three else pos3[:, 0].contiguous()
+        pos_of = pos3[:, axis.long()] if three else pos3[:, :1].expand(T, rot // 2)
+        q_ref, k_ref = ref(pos_of)
+        k_pool = torch.zeros(pt.shape[1], Hkv, 16, hd, device="cuda", dtype=dt)
+        v_pool, rows = torch.zeros_like(k_pool), qkv.clone()
+        K_.qk_norm_rope_kv(rows, Hq, Hkv, hd, pos=pos, cos=cos_sin[0], sin=cos_sin[1], rot_dim=rot, q_norm_w=w[0], k_norm_w=w[1], k_pool=k_pool, v_pool=v_pool,
+                           page_table=pt, seq_of_tok=seq, cache_pos=cpos, axis_of_freq=axis if three else None)
+        got = rows.view(T, -1, hd)
+        at = lambda pool: pool[pt[0][(cpos // 16).long()].long(), :, (cpos % 16).long()]
+        _close(got[:, :Hq], q_ref, dt, scale=3.0)
+        _close(at(k_pool), k_ref, dt, scale=3.0)
+        assert torch.equal(at(v_pool), qkv.view(T, -1, hd)[:, Hq + Hkv:])
+        assert torch.equal(got[:, Hq:], qkv.view(T, -1, hd)[:, Hq:])
+        flat = qkv.clone()
+        K_.qk_norm_rope_kv(flat, Hq, Hkv, hd, pos=pos, cos=cos_sin[0], sin=cos_sin[1], rot_dim=rot, q_norm_w=w[0], k_norm_w=w[1], axis_of_freq=axis if three else None)
+        _close(flat.view(T, -1, hd)[:, Hq:Hq + Hkv], k_ref, dt, scale=3.0)
