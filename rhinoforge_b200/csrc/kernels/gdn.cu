@@ -15,6 +15,7 @@
 // and a batch-1 decode step still fills Hv * Dv/32 SMs.
 #include "../common/dtype.cuh"
 #include "../common/host_util.h"
+#include "../common/mma.cuh"
 #include "../common/ptx.cuh"
 #include "../rf_api.h"
 
@@ -205,23 +206,29 @@ gdn_recurrent_kernel(const RfGdn p) {
 //     (I + L) U = beta * (V - e^G * (K S0))
 //     O  = e^G * (Q S0) + tril(e^{G_i - G_j} (q_i . k_j)) U
 //     S' = e^{G_C} S0 + K^T (e^{G_C - G} * U)
-// One CTA owns 32 state columns of one value head of one sequence (the same split as the recurrent kernel) and walks
-// the sequence's chunks with its [128 x 32] state slice resident in shared memory.  Every product is an fp32-accumulate
+// One CTA owns 32 or 64 state columns of one value head of one sequence and walks the sequence's chunks with its
+// [128 x NV] state slice resident in shared memory.  Every product is an fp32-accumulate
 // TF32 mma.sync (operands rounded to nearest): the state stays fp32 between chunks, and every decay factor that appears
 // is e^{G_i - G_j} with j <= i, at most one.  The unit-triangular system is solved in 16-row blocks: the four diagonal
-// blocks are inverted by forward substitution (one warp each), the rest is block forward substitution on the 32
-// right-hand-side columns.  Rows past the end of a sequence are zero tokens with beta = 0 and no decay, which leave both
+// blocks are inverted by forward substitution (a column per lane), the rest is block forward substitution on the
+// right-hand-side columns: a thread keeps its rows of all four blocks in registers and takes a finished block off the later ones at
+// once, so that a value of U read from shared memory serves up to three rows.  Rows past the end of a sequence are zero tokens with beta = 0 and no decay, which leave both
 // the outputs of the real rows and the state untouched.
+// What bounds it: the chain of a chunk - normalise, L and P, substitution, state - on one CTA per SM, most of it shared-memory accesses.  Tiles
+// are written 16 bytes a lane without bank conflicts and read as fragments by ldmatrix (a 32-bit element is a pair of its 16-bit ones).
+// Half the work of a chunk does not depend on the columns, so 64 of them cost a CTA little more than 32.  4 x 1500 tokens, 16 heads of 128:
+// 577 us with scalar tiles and 32 columns, 318 now; 1 x 1500 (64 CTAs of 32 columns, one wave) 287 and 248.
 constexpr int kGcC = 64;          // tokens per chunk
 constexpr int kGcThreads = 256;
 constexpr int kGcLdQK = 132;      // fp32 row pitch of the q / k tiles: (4 * row + col) mod 32 is distinct over a fragment
-constexpr int kGcLdS = 40;        // row pitch of the state slice and of the v / rhs / u tile
 constexpr int kGcLdL = 68;        // row pitch of the two chunk x chunk matrices
-constexpr int kGcLdD = 17;
-constexpr int kGcSmemFloats = 2 * kGcC * kGcLdQK + 128 * kGcLdS + 2 * kGcC * kGcLdS + 2 * kGcC * kGcLdL + 4 * 16 * kGcLdD + 3 * kGcC;
-// + the raw 16-bit q | k rows and v slice of the NEXT chunk, fetched with cp.async while this chunk is computed
-constexpr int kGcRawElems = kGcC * 256 + kGcC * kGdnCols;
-constexpr size_t kGcSmemBytes = (size_t)kGcSmemFloats * sizeof(float) + (size_t)kGcRawElems * 2;
+constexpr int kGcLdD = 20;
+// NV state columns: row pitch NV + 8 of the state slice and of the v / rhs / u tiles; + the raw 16-bit q | k rows and v slice of the NEXT chunk,
+// fetched with cp.async while this chunk is computed
+constexpr size_t gc_smem_bytes(int nv) {
+  return (size_t)(2 * kGcC * kGcLdQK + (128 + 2 * kGcC) * (nv + 8) + 2 * kGcC * kGcLdL + 4 * 16 * kGcLdD + 3 * kGcC) * sizeof(float) +
+         (size_t)kGcC * (256 + nv) * 2;
+}
 
 __device__ __forceinline__ void cp_async16(void* smem_dst, const void* gsrc, bool valid) {
   const uint32_t d = (uint32_t)__cvta_generic_to_shared(smem_dst);
@@ -241,27 +248,34 @@ __device__ __forceinline__ void mma_tf32(float (&d)[4], const uint32_t (&a)[4], 
                : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
                : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
 }
-// A fragment of a row-major fp32 tile: rows r0 + {g, g + 8}, columns c0 + {t, t + 4}
-__device__ __forceinline__ void frag_a(uint32_t (&a)[4], const float* m, int ld, int r0, int c0, int g, int t) {
-  a[0] = to_tf32(m[(r0 + g) * ld + c0 + t]);
-  a[1] = to_tf32(m[(r0 + g + 8) * ld + c0 + t]);
-  a[2] = to_tf32(m[(r0 + g) * ld + c0 + t + 4]);
-  a[3] = to_tf32(m[(r0 + g + 8) * ld + c0 + t + 4]);
+// Four 8 x 4 blocks of a row-major tile of TF32 bits whose pitch is 4 (mod 32) words, without bank conflicts: rows r0 .. and r0 + 8 .. of columns
+// c0 .. c0 + 3, then of c0 + 4 .. c0 + 7; lane 4 g + t gets element (g, t) of each.  That is the A fragment of rows r0 .. r0 + 15, and
+// (a[0], a[2]), (a[1], a[3]) are the B fragments of the two groups of eight rows.
+__device__ __forceinline__ void frag_x4(uint32_t (&a)[4], const float* m, int ld, int r0, int c0, int lane) {
+  ldsm_x4(smem_u32(m + (r0 + (lane & 15)) * ld + c0 + (lane >> 4) * 4), a[0], a[1], a[2], a[3]);
+}
+template <int N> __device__ __forceinline__ void ld_row(const float* src, float (&v)[N]) {
+  if constexpr (N == 2) { const float2 x = *reinterpret_cast<const float2*>(src); v[0] = x.x; v[1] = x.y; }
+  else { const float4 x = *reinterpret_cast<const float4*>(src); v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w; }
+}
+template <int N> __device__ __forceinline__ void st_row(float* dst, const float (&v)[N]) {
+  if constexpr (N == 2) *reinterpret_cast<float2*>(dst) = make_float2(v[0], v[1]);
+  else *reinterpret_cast<float4*>(dst) = make_float4(v[0], v[1], v[2], v[3]);
+}
+// four 16-bit values as floats (8-byte aligned)
+template <typename T> __device__ __forceinline__ float4 load4(const T* src) {
+  const uint2 u = *reinterpret_cast<const uint2*>(src);
+  const T* e = reinterpret_cast<const T*>(&u);
+  return make_float4(Num<T>::to_f(e[0]), Num<T>::to_f(e[1]), Num<T>::to_f(e[2]), Num<T>::to_f(e[3]));
 }
 
-// the same for a tile whose values were rounded to TF32 when they were stored
-__device__ __forceinline__ void frag_a_bits(uint32_t (&a)[4], const float* m, int ld, int r0, int c0, int g, int t) {
-  a[0] = __float_as_uint(m[(r0 + g) * ld + c0 + t]);
-  a[1] = __float_as_uint(m[(r0 + g + 8) * ld + c0 + t]);
-  a[2] = __float_as_uint(m[(r0 + g) * ld + c0 + t + 4]);
-  a[3] = __float_as_uint(m[(r0 + g + 8) * ld + c0 + t + 4]);
-}
-
-template <typename T>
+template <typename T, int NV>
 __global__ void __launch_bounds__(kGcThreads, 1)
 gdn_chunked_kernel(const RfGdn p) {
   pdl_prologue();
-  constexpr int DK = 128, C = kGcC, NV = kGdnCols;
+  constexpr int DK = 128, C = kGcC, kGcLdS = NV + 8;
+  constexpr int NT = NV / 16;                          // 8-column tiles of a warp in the products with the state and with U
+  constexpr int CPT = NV / 16;                         // columns of a thread in the substitution
   extern __shared__ __align__(16) float gsm[];
   float* sQ = gsm;
   float* sK = sQ + C * kGcLdQK;
@@ -275,7 +289,7 @@ gdn_chunked_kernel(const RfGdn p) {
   float* sBeta = sG + C;
   float* sg = sBeta + C;
   T* rawQK = reinterpret_cast<T*>(sg + C);             // [C][q 128 | k 128]
-  T* rawV = rawQK + C * 256;                           // [C][32]
+  T* rawV = rawQK + C * 256;                           // [C][NV]
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
   const int seq = blockIdx.z, hv = blockIdx.y, j0 = blockIdx.x * NV;
@@ -308,8 +322,9 @@ gdn_chunked_kernel(const RfGdn p) {
         const size_t row = (size_t)(s0 + (valid ? cn + i : 0));
         cp_async16(rawQK + i * 256 + part * 8, qkv + row * p.ld + (part < 16 ? q_off + part * 8 : k_off + (part - 16) * 8), valid);
       }
-      {
-        const int i = tid >> 2, part = tid & 3;
+#pragma unroll
+      for (int k = 0; k < NV / 32; ++k) {
+        const int idx = tid + kGcThreads * k, i = idx / (NV / 8), part = idx % (NV / 8);
         const bool valid = cn + i < n;
         const size_t row = (size_t)(s0 + (valid ? cn + i : 0));
         cp_async16(rawV + i * NV + part * 8, qkv + row * p.ld + v_off + part * 8, valid);
@@ -332,24 +347,21 @@ gdn_chunked_kernel(const RfGdn p) {
     for (int rr = 0; rr < 8; ++rr) {
       const int i = warp * 8 + rr;
       const int half = lane >> 4, l16 = lane & 15;
-      float f[8];
-      load8(rawQK + i * 256 + half * 128 + l16 * 8, f);
-      float ss = 0.f;
-#pragma unroll
-      for (int e = 0; e < 8; ++e) ss += f[e] * f[e];
+      // four neighbouring values and the four 64 further on: every 16-byte store of the warp covers whole rows of banks
+      const T* src = rawQK + i * 256 + half * 128 + l16 * 4;
+      const float4 lo = load4(src), hi = load4(src + 64);
+      float ss = lo.x * lo.x + lo.y * lo.y + lo.z * lo.z + lo.w * lo.w + hi.x * hi.x + hi.y * hi.y + hi.z * hi.z + hi.w * hi.w;
 #pragma unroll
       for (int o = 8; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
       const float sc = rsqrtf(ss + 1e-6f) * (half ? 1.f : qscale);
-      float* dst = (half ? sK : sQ) + i * kGcLdQK + l16 * 8;
-#pragma unroll
-      for (int e = 0; e < 8; ++e) dst[e] = __uint_as_float(to_tf32(f[e] * sc));   // rounded once here, read as TF32 bits below
+      uint4* dst = reinterpret_cast<uint4*>((half ? sK : sQ) + i * kGcLdQK + l16 * 4);   // rounded once here, read as TF32 bits below
+      dst[0] = make_uint4(to_tf32(lo.x * sc), to_tf32(lo.y * sc), to_tf32(lo.z * sc), to_tf32(lo.w * sc));
+      dst[16] = make_uint4(to_tf32(hi.x * sc), to_tf32(hi.y * sc), to_tf32(hi.z * sc), to_tf32(hi.w * sc));
     }
-    {
-      const int i = tid >> 2, part = tid & 3;
-      float vv[8];
-      load8(rawV + i * NV + part * 8, vv);
 #pragma unroll
-      for (int e = 0; e < 8; ++e) sV[i * kGcLdS + part * 8 + e] = vv[e];
+    for (int k = 0; k < C * NV / 4 / kGcThreads; ++k) {
+      const int idx = tid + kGcThreads * k, i = idx / (NV / 4), part = idx % (NV / 4);
+      *reinterpret_cast<float4*>(sV + i * kGcLdS + part * 4) = load4(rawV + i * NV + part * 4);
     }
     if (tid < C) {
       float beta = 0.f, lg = 0.f;
@@ -387,17 +399,20 @@ gdn_chunked_kernel(const RfGdn p) {
 #pragma unroll 4
       for (int ks = 0; ks < DK / 8; ++ks) {
         uint32_t aK[4], aQ[4];
-        frag_a_bits(aK, sK, kGcLdQK, rt * 16, ks * 8, g, t);
-        frag_a_bits(aQ, sQ, kGcLdQK, rt * 16, ks * 8, g, t);
+        frag_x4(aK, sK, kGcLdQK, rt * 16, ks * 8, lane);
+        frag_x4(aQ, sQ, kGcLdQK, rt * 16, ks * 8, lane);
 #pragma unroll
-        for (int ti = 0; ti < 4; ++ti) {
-          if (ti < cnt) {
-            const int col = (nt0 + ti) * 8 + g;
-            uint32_t b[2];
-            b[0] = __float_as_uint(sK[col * kGcLdQK + ks * 8 + t]);
-            b[1] = __float_as_uint(sK[col * kGcLdQK + ks * 8 + t + 4]);
-            mma_tf32(accL[ti], aK, b);
-            mma_tf32(accP[ti], aQ, b);
+        for (int ti = 0; ti < 4; ti += 2) {
+          if (ti < cnt) {                              // an odd count reads rows of the tile behind and leaves them (at most row 63)
+            uint32_t bb[4];
+            frag_x4(bb, sK, kGcLdQK, (nt0 + ti) * 8, ks * 8, lane);
+            const uint32_t b0[2] = {bb[0], bb[2]}, b1[2] = {bb[1], bb[3]};
+            mma_tf32(accL[ti], aK, b0);
+            mma_tf32(accP[ti], aQ, b0);
+            if (ti + 1 < cnt) {
+              mma_tf32(accL[ti + 1], aK, b1);
+              mma_tf32(accP[ti + 1], aQ, b1);
+            }
           }
         }
       }
@@ -416,36 +431,38 @@ gdn_chunked_kernel(const RfGdn p) {
     }
     __syncthreads();
 
-    // ---- inverses of the four 16 x 16 diagonal blocks of I + L (warps 0..3, one column per lane)
-    if (warp < 4 && lane < 16) {
+    // ---- inverses of the four 16 x 16 diagonal blocks of I + L (warps 0 and 1, one column per lane): a finished row is taken off all later ones
+    if (warp < 2) {
+      const int blk = warp * 2 + (lane >> 4), col = lane & 15;
+      const float* Lb = sL + blk * 16 * kGcLdL + blk * 16;
       float x[16];
 #pragma unroll
-      for (int i = 0; i < 16; ++i) {
-        float acc = i == lane ? 1.f : 0.f;
+      for (int i = 0; i < 16; ++i) x[i] = i == col ? 1.f : 0.f;
 #pragma unroll
-        for (int j = 0; j < i; ++j) acc -= sL[(warp * 16 + i) * kGcLdL + warp * 16 + j] * x[j];
-        x[i] = acc;
-        sD[(warp * 16 + i) * kGcLdD + lane] = acc;
-      }
+      for (int j = 0; j < 15; ++j)
+#pragma unroll
+        for (int i = j + 1; i < 16; ++i) x[i] -= Lb[i * kGcLdL + j] * x[j];
+#pragma unroll
+      for (int i = 0; i < 16; ++i) sD[(blk * 16 + i) * kGcLdD + col] = x[i];
     }
 
     // ---- rhs = beta (V - e^G (K S0)) in place of V;  accO = e^G (Q S0)
     const int rt = warp & 3, nh = warp >> 2;
-    float accO[2][4];
+    float accO[NT][4];
     {
-      float accR[2][4];
+      float accR[NT][4];
 #pragma unroll
-      for (int a = 0; a < 2; ++a)
+      for (int a = 0; a < NT; ++a)
 #pragma unroll
         for (int b = 0; b < 4; ++b) accR[a][b] = accO[a][b] = 0.f;
 #pragma unroll 4
       for (int ks = 0; ks < DK / 8; ++ks) {
         uint32_t aK[4], aQ[4];
-        frag_a_bits(aK, sK, kGcLdQK, rt * 16, ks * 8, g, t);
-        frag_a_bits(aQ, sQ, kGcLdQK, rt * 16, ks * 8, g, t);
+        frag_x4(aK, sK, kGcLdQK, rt * 16, ks * 8, lane);
+        frag_x4(aQ, sQ, kGcLdQK, rt * 16, ks * 8, lane);
 #pragma unroll
-        for (int a = 0; a < 2; ++a) {
-          const int col = (nh * 2 + a) * 8 + g;
+        for (int a = 0; a < NT; ++a) {
+          const int col = (nh * NT + a) * 8 + g;
           uint32_t b[2];
           b[0] = to_tf32(sS[(ks * 8 + t) * kGcLdS + col]);
           b[1] = to_tf32(sS[(ks * 8 + t + 4) * kGcLdS + col]);
@@ -454,51 +471,78 @@ gdn_chunked_kernel(const RfGdn p) {
         }
       }
 #pragma unroll
-      for (int a = 0; a < 2; ++a)
+      for (int h = 0; h < 2; ++h) {
+        const int i = rt * 16 + g + h * 8;
+        const float eg = __expf(sG[i]), beta = sBeta[i];
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const int i = rt * 16 + g + (e >> 1) * 8, j = (nh * 2 + a) * 8 + 2 * t + (e & 1);
-          const float eg = __expf(sG[i]);
-          sV[i * kGcLdS + j] = sBeta[i] * (sV[i * kGcLdS + j] - eg * accR[a][e]);
-          accO[a][e] *= eg;
+        for (int a = 0; a < NT; ++a) {
+          float2* v = reinterpret_cast<float2*>(sV + i * kGcLdS + (nh * NT + a) * 8 + 2 * t);
+          const float2 x = *v;
+          *v = make_float2(beta * (x.x - eg * accR[a][2 * h]), beta * (x.y - eg * accR[a][2 * h + 1]));
+          accO[a][2 * h] *= eg;
+          accO[a][2 * h + 1] *= eg;
         }
+      }
     }
     __syncthreads();
 
-    // ---- U = (I + L)^-1 rhs by block forward substitution: rhs rows in sV, finished rows in sU
+    // ---- U = (I + L)^-1 rhs by block forward substitution: a thread has row r of every block in registers, a block's right-hand side meets the
+    // others' through sV, finished rows are in sU
     {
-      const int r = tid >> 4, cc = (tid & 15) * 2;
+      const int r = tid >> 4, cc = (tid & 15) * CPT;
+      float a[4][CPT];
+#pragma unroll
+      for (int b = 0; b < 4; ++b) ld_row(sV + (b * 16 + r) * kGcLdS + cc, a[b]);
+#pragma unroll
       for (int b = 0; b < 4; ++b) {
-        const int i = b * 16 + r;
-        float a0 = sV[i * kGcLdS + cc], a1 = sV[i * kGcLdS + cc + 1];
-#pragma unroll 4
-        for (int j = 0; j < b * 16; ++j) {
-          const float l = sL[i * kGcLdL + j];
-          a0 -= l * sU[j * kGcLdS + cc];
-          a1 -= l * sU[j * kGcLdS + cc + 1];
+        if (b > 0) {
+          st_row(sV + (b * 16 + r) * kGcLdS + cc, a[b]);
+          __syncthreads();
         }
-        sV[i * kGcLdS + cc] = a0;          // a row of block b is touched by its owner only until the barrier
-        sV[i * kGcLdS + cc + 1] = a1;
-        __syncthreads();
-        float u0 = 0.f, u1 = 0.f;
-        for (int r2 = 0; r2 <= r; ++r2) {
-          const float d = sD[i * kGcLdD + r2];
-          u0 += d * sV[(b * 16 + r2) * kGcLdS + cc];
-          u1 += d * sV[(b * 16 + r2) * kGcLdS + cc + 1];
+        float u[CPT] = {};
+#pragma unroll
+        for (int r4 = 0; r4 < 16; r4 += 4) {
+          float d[4];
+          ld_row(sD + (b * 16 + r) * kGcLdD + r4, d);
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            float v[CPT];
+            ld_row(sV + (b * 16 + r4 + k) * kGcLdS + cc, v);
+            if (r4 + k <= r) {                         // rows behind this one stay out of it, whatever they hold
+#pragma unroll
+              for (int e = 0; e < CPT; ++e) u[e] += d[k] * v[e];
+            }
+          }
         }
-        sU[i * kGcLdS + cc] = u0;
-        sU[i * kGcLdS + cc + 1] = u1;
+        st_row(sU + (b * 16 + r) * kGcLdS + cc, u);
         __syncthreads();
+        if (b < 3) {
+#pragma unroll
+          for (int j4 = 0; j4 < 16; j4 += 4) {
+            float l[3][4];
+#pragma unroll
+            for (int k = b + 1; k < 4; ++k) ld_row(sL + (k * 16 + r) * kGcLdL + b * 16 + j4, l[k - 1]);
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+              float v[CPT];
+              ld_row(sU + (b * 16 + j4 + q) * kGcLdS + cc, v);
+#pragma unroll
+              for (int k = b + 1; k < 4; ++k)
+#pragma unroll
+                for (int e = 0; e < CPT; ++e) a[k][e] -= l[k - 1][q] * v[e];
+            }
+          }
+        }
       }
     }
 
     // ---- O = accO + P U
     for (int ks = 0; ks <= 2 * rt + 1; ++ks) {
       uint32_t aP[4];
-      frag_a_bits(aP, sP, kGcLdL, rt * 16, ks * 8, g, t);
+      frag_x4(aP, sP, kGcLdL, rt * 16, ks * 8, lane);
 #pragma unroll
-      for (int a = 0; a < 2; ++a) {
-        const int col = (nh * 2 + a) * 8 + g;
+      for (int a = 0; a < NT; ++a) {
+        const int col = (nh * NT + a) * 8 + g;
         uint32_t b[2];
         b[0] = to_tf32(sU[(ks * 8 + t) * kGcLdS + col]);
         b[1] = to_tf32(sU[(ks * 8 + t + 4) * kGcLdS + col]);
@@ -506,19 +550,19 @@ gdn_chunked_kernel(const RfGdn p) {
       }
     }
 #pragma unroll
-    for (int a = 0; a < 2; ++a)
+    for (int a = 0; a < NT; ++a)
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
-        const int i = rt * 16 + g + (e >> 1) * 8, j = (nh * 2 + a) * 8 + 2 * t + (e & 1);
+        const int i = rt * 16 + g + (e >> 1) * 8, j = (nh * NT + a) * 8 + 2 * t + (e & 1);
         if (c0 + i < n) out[(size_t)(s0 + c0 + i) * p.ldo + hv * p.Dv + j0 + j] = Num<T>::from_f(accO[a][e]);
       }
 
     // ---- S' = e^{G_C} S0 + K^T (e^{G_C - G} * U): warp w owns state rows 16 w .. 16 w + 15
     {
       const float gl = sG[C - 1], egl = __expf(gl);
-      float accS[4][4];
+      float accS[NV / 8][4];
 #pragma unroll
-      for (int a = 0; a < 4; ++a)
+      for (int a = 0; a < NV / 8; ++a)
 #pragma unroll
         for (int e = 0; e < 4; ++e)
           accS[a][e] = egl * sS[(warp * 16 + g + (e >> 1) * 8) * kGcLdS + a * 8 + 2 * t + (e & 1)];
@@ -532,7 +576,7 @@ gdn_chunked_kernel(const RfGdn p) {
         aT[3] = __float_as_uint(sK[cb * kGcLdQK + warp * 16 + g + 8]);
         const float wa = __expf(gl - sG[ca]), wb = __expf(gl - sG[cb]);
 #pragma unroll
-        for (int a = 0; a < 4; ++a) {
+        for (int a = 0; a < NV / 8; ++a) {
           uint32_t b[2];
           b[0] = to_tf32(wa * sU[ca * kGcLdS + a * 8 + g]);
           b[1] = to_tf32(wb * sU[cb * kGcLdS + a * 8 + g]);
@@ -540,7 +584,7 @@ gdn_chunked_kernel(const RfGdn p) {
         }
       }
 #pragma unroll
-      for (int a = 0; a < 4; ++a)
+      for (int a = 0; a < NV / 8; ++a)
 #pragma unroll
         for (int e = 0; e < 4; ++e)
           sS[(warp * 16 + g + (e >> 1) * 8) * kGcLdS + a * 8 + 2 * t + (e & 1)] = accS[a][e];
@@ -702,15 +746,22 @@ extern "C" int rf_gdn_chunked(const RfGdn* a, rf_stream_t stream) {
   RF_REQUIRE(a->ld % 8 == 0 && (a->Hk * a->Dk) % 8 == 0 && a->Dv % 8 == 0, "gdn: the chunked form reads 16-byte vectors (pitch %lld)", (long long)a->ld);
   RF_REQUIRE(a->num_seqs > 0, "gdn: no sequences");
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  const dim3 grid(a->Dv / kGdnCols, a->Hv, a->num_seqs);
-  constexpr size_t smem = kGcSmemBytes;
-  if (a->dtype == 0) {
-    RF_ALLOW_SMEM_PER_DEVICE(gdn_chunked_kernel<__half>, smem);
-    RF_CUDA_CHECK(::rf::launch_k(gdn_chunked_kernel<__half>, grid, dim3(kGcThreads), smem, s, 1, *a));
-  } else {
-    RF_ALLOW_SMEM_PER_DEVICE(gdn_chunked_kernel<__nv_bfloat16>, smem);
-    RF_CUDA_CHECK(::rf::launch_k(gdn_chunked_kernel<__nv_bfloat16>, grid, dim3(kGcThreads), smem, s, 1, *a));
-  }
+  // 64 columns to a CTA where 32 would make more CTAs than there are SMs (one sits on an SM): half of a chunk's work is the same for any number of
+  // columns (1500 tokens, 16 heads of 128: a wave of 32 columns takes 248 us, which 4 sequences need twice, a wave of 64 columns 318)
+  const bool wide = a->Dv % 64 == 0 && (long)(a->Dv / kGdnCols) * a->Hv * a->num_seqs > sm_count();
+  auto run = [&](auto kfn, int nv) -> cudaError_t {
+    return ::rf::launch_k(kfn, dim3(a->Dv / nv, a->Hv, a->num_seqs), dim3(kGcThreads), gc_smem_bytes(nv), s, 1, *a);
+  };
+#define RF_GDN_CHUNKED(T, NV)                                                    \
+  do {                                                                           \
+    RF_ALLOW_SMEM_PER_DEVICE((gdn_chunked_kernel<T, NV>), gc_smem_bytes(NV));    \
+    RF_CUDA_CHECK(run(gdn_chunked_kernel<T, NV>, NV));                           \
+  } while (0)
+  if (a->dtype == 0 && wide) RF_GDN_CHUNKED(__half, 64);
+  else if (a->dtype == 0) RF_GDN_CHUNKED(__half, 32);
+  else if (wide) RF_GDN_CHUNKED(__nv_bfloat16, 64);
+  else RF_GDN_CHUNKED(__nv_bfloat16, 32);
+#undef RF_GDN_CHUNKED
   ::rf::count_launch();
   return RF_OK;
 }

@@ -164,6 +164,28 @@ def test_gdn_chunked_prefill_matches_recurrence(dt):
     assert _rel(o2.view(L2, Hv, Dv), ref) < tol and _rel(state[3], S) < 1e-3
 
 
+@pytest.mark.parametrize("dt", DT)
+@pytest.mark.parametrize("Dv,seqs", [(128, 3), (64, 12), (96, 12), (192, 5)])
+def test_gdn_chunked_many_heads_matches_recurrence(dt, Dv, seqs):
+    """More 32-column slices than SMs, where a CTA takes 64 columns (unless the heads are no multiple of it), and fewer: sequences that end at every
+    place of a chunk's row blocks, fresh and carried states, against the token-by-token kernel."""
+    from rhinoforge_b200.ops import kernels as K
+    torch.manual_seed(7)
+    Hk, Hv, Dk = 4, 16, 128
+    lens = [65, 64, 17, 128, 1, 95, 33, 16, 63, 100, 2, 49][:seqs]
+    width = 2 * Hk * Dk + Hv * Dv
+    qkv = torch.randn(sum(lens), width, device="cuda").to(dt)
+    ba = torch.randn(sum(lens), 2 * Hv, device="cuda").to(dt)
+    A_log, dtb = torch.log(torch.rand(Hv, device="cuda") * 4 + 0.5), torch.rand(Hv, device="cuda")
+    ql = torch.tensor(lens, dtype=torch.int32, device="cuda")
+    kw = dict(Hk=Hk, Hv=Hv, Dk=Dk, Dv=Dv, q_start=(torch.cumsum(ql, 0) - ql).to(torch.int32), q_len=ql, fresh=(torch.arange(seqs, device="cuda") % 2).to(torch.int32))
+    a = torch.randn(seqs, Hv, Dk, Dv, device="cuda") * 0.1
+    b = a.clone()
+    out = K.gdn_recurrent(qkv, ba[:, :Hv], ba[:, Hv:], a, A_log, dtb, chunked=True, **kw)
+    ref = K.gdn_recurrent(qkv, ba[:, :Hv], ba[:, Hv:], b, A_log, dtb, **kw)
+    assert _rel(out, ref) < (5e-3 if dt == torch.float16 else 3e-2) and _rel(a, b) < 1e-3      # TF32 products: the bounds of the test above
+
+
 def test_gdn_chunked_is_faster_than_token_serial_on_a_long_prompt():
     """Qwen3.5 geometry (16 key heads, 32 value heads of 128) over 4096 tokens: the chunked kernel has to beat the
     token-by-token kernel by a wide margin and leave the same state."""
