@@ -17,8 +17,8 @@
 // a ring of four; two CTAs of one tile each with two-block rings waited for their copies (2.1 us a block).  One tile to a CTA is for short
 // inputs, where the CTAs would not fill the GPU otherwise, and for heads above 128.
 // fp16, us (one tile with a two-block ring / now), heads of 128 unless said: 128 queries x 2048 keys 76 / 41 (the chain alone: one CTA per SM);
-// 8192 causal, 32 + 8 heads 1324 / 951; 8192 queries on 16384 keys 3317 / 2522; 8 x 1024 causal 382 / 273; 6 x 1100, window 1024 194 / 141;
-// 2 x 4096, heads of 64 588 / 481; 12 x 256 full 45 / 41 (one tile each); 93 causal, heads of 64 14.2 / 13.6.
+// 8192 causal, 32 + 8 heads 1324 / 890; 8192 queries on 16384 keys 3317 / 2462; 8 x 1024 causal 382 / 209; 6 x 1100, window 1024 194 / 104;
+// 2 x 4096, heads of 64 588 / 417; 12 x 256 full 45 / 41 (one tile each); 93 causal, heads of 64 14.2 / 6.9.
 // V needs no transpose: the [tokens x 64] slabs a TMA box leaves in shared memory are exactly the
 // MN-major 128-byte-swizzle operand layout.
 //
@@ -58,6 +58,8 @@ template <int HD, int VD, int NQ> struct FaGeom {
   static constexpr int kThreads = 64 + NQ * 128;
   static_assert(kSCols + NQ * VD <= 512, "accumulators do not fit tensor memory");
 };
+// bits a .. 63 set (all of them from a <= 0, none from a >= 64)
+__device__ __forceinline__ uint64_t bits_from(int a) { return a >= 64 ? 0ull : ~0ull << max(a, 0); }
 // 2^x on the special-function unit, results below 2^-126 flushed to zero
 __device__ __forceinline__ float ex2(float x) {
   float y;
@@ -322,6 +324,20 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
         mul = score_mul;
 #pragma unroll
         for (int i = 0; i < KVB; ++i) mx4[i & 3] = fmaxf(mx4[i & 3], __uint_as_float(sv[i]));
+#pragma unroll
+        for (int i = 0; i < 4; ++i) mx4[i] *= score_mul;
+      } else if (!data_mask && score_mul > 0.f) {
+        // a block on the diagonal or on the edge of a window: the row's keys as one bit each.  The general loop below, with its tests for data masks
+        // behind every key, took some 3 us a block (128 x 128 causal, 32 + 8 heads of 128: 17.1 us, 10.4 with this), and a causal tile has two such blocks.
+        mul = score_mul;
+        const uint64_t bits = (bits_from(lo_row - t0) | ~bits_from(p.keep_first - t0)) & ~bits_from(hi_row - t0 + 1);
+        const uint32_t w32[2] = {(uint32_t)bits, (uint32_t)(bits >> 32)};
+#pragma unroll
+        for (int i = 0; i < KVB; ++i) {
+          const float x = (w32[i >> 5] & (1u << (i & 31))) ? __uint_as_float(sv[i]) : -INFINITY;
+          sv[i] = __float_as_uint(x);
+          mx4[i & 3] = fmaxf(mx4[i & 3], x);
+        }
 #pragma unroll
         for (int i = 0; i < 4; ++i) mx4[i] *= score_mul;
       } else if (!edge) {
