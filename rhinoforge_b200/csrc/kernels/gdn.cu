@@ -307,12 +307,23 @@ gdn_chunked_kernel(const RfGdn p) {
   const float A = -__expf(p.A_log[hv]), dtb = p.dt_bias[hv];
   const float qscale = rsqrtf((float)DK);
 
-  for (int i = tid; i < DK * NV; i += kGcThreads) {
-    const int m = i / NV, c = i % NV;
-    sS[m * kGcLdS + c] = fresh ? 0.f : S[(size_t)m * p.Dv + c];
-  }
+  // the fp32 state stays in registers - warp w has rows 16 w .. 16 w + 15 -, sS holds it rounded to TF32 for the products
+  float st[NV / 8][4];
+  auto state_row = [&](int e) { return warp * 16 + g + (e >> 1) * 8; };
+  auto publish_state = [&] {
+#pragma unroll
+    for (int a = 0; a < NV / 8; ++a)
+#pragma unroll
+      for (int e = 0; e < 4; e += 2)
+        *reinterpret_cast<uint2*>(sS + state_row(e) * kGcLdS + a * 8 + 2 * t) = make_uint2(to_tf32(st[a][e]), to_tf32(st[a][e + 1]));
+  };
+#pragma unroll
+  for (int a = 0; a < NV / 8; ++a)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) st[a][e] = fresh ? 0.f : S[(size_t)state_row(e) * p.Dv + a * 8 + 2 * t + (e & 1)];
+  publish_state();
 
-  float nb = 0.f, na = 0.f;                            // beta / decay inputs of row `tid` of the chunk in flight
+  T nb = Num<T>::from_f(0.f), na = nb;                 // beta / decay inputs of row `tid` of the chunk in flight, not looked at before they are needed
   auto prefetch = [&](int cn) {
     if (cn < n) {
 #pragma unroll
@@ -331,8 +342,8 @@ gdn_chunked_kernel(const RfGdn p) {
       }
       if (tid < C && cn + tid < n) {
         const size_t row = (size_t)(s0 + cn + tid);
-        nb = Num<T>::to_f(bp[row * p.ld_ba + hv]);
-        na = Num<T>::to_f(ap[row * p.ld_ba + hv]);
+        nb = bp[row * p.ld_ba + hv];
+        na = ap[row * p.ld_ba + hv];
       }
     }
     cp_async_commit();
@@ -366,8 +377,8 @@ gdn_chunked_kernel(const RfGdn p) {
     if (tid < C) {
       float beta = 0.f, lg = 0.f;
       if (c0 + tid < n) {
-        beta = 1.f / (1.f + __expf(-nb));
-        const float ar = na + dtb;
+        beta = 1.f / (1.f + __expf(-Num<T>::to_f(nb)));
+        const float ar = Num<T>::to_f(na) + dtb;
         lg = A * (ar > 20.f ? ar : log1pf(__expf(ar)));
       }
       sBeta[tid] = beta;
@@ -388,43 +399,55 @@ gdn_chunked_kernel(const RfGdn p) {
     }
     __syncthreads();
 
-    // ---- L = beta_i e^{G_i - G_j} (k_i . k_j) [j < i],  P = e^{G_i - G_j} (q_i . k_j) [j <= i]
+    // ---- L = beta_i e^{G_i - G_j} (k_i . k_j) [j < i],  P = e^{G_i - G_j} (q_i . k_j) [j <= i].  Row tile rt has 2 (rt + 1) column tiles on or below
+    // the diagonal, 20 in all and as many of P: five to a warp (even warps L, odd ones P), from at most two row tiles.
     {
-      const int rt = warp >> 1, cnt = rt + 1, nt0 = (warp & 1) * cnt;   // row tile rt has 2 (rt + 1) column tiles on or below the diagonal
-      float accL[4][4], accP[4][4];
+      const bool isP = warp & 1;
+      const int pair = warp >> 1, rt0 = pair < 2 ? 3 : 2, first = (pair & 1) * 5, n0 = pair == 1 ? 3 : pair == 3 ? 1 : 5, rt1 = pair == 1 ? 0 : 1;
+      const float* sA = isP ? sQ : sK;
+      float acc[5][4];
 #pragma unroll
-      for (int a = 0; a < 4; ++a)
+      for (int a = 0; a < 5; ++a)
 #pragma unroll
-        for (int b = 0; b < 4; ++b) accL[a][b] = accP[a][b] = 0.f;
-#pragma unroll 4
-      for (int ks = 0; ks < DK / 8; ++ks) {
-        uint32_t aK[4], aQ[4];
-        frag_x4(aK, sK, kGcLdQK, rt * 16, ks * 8, lane);
-        frag_x4(aQ, sQ, kGcLdQK, rt * 16, ks * 8, lane);
+        for (int b = 0; b < 4; ++b) acc[a][b] = 0.f;
+#pragma unroll 2
+      for (int ks = 0; ks < DK / 8; ks += 2) {
+        uint32_t a0[2][4], a1[2][4] = {};
+        frag_x4(a0[0], sA, kGcLdQK, rt0 * 16, ks * 8, lane);
+        frag_x4(a0[1], sA, kGcLdQK, rt0 * 16, ks * 8 + 8, lane);
+        if (n0 < 5) {
+          frag_x4(a1[0], sA, kGcLdQK, rt1 * 16, ks * 8, lane);
+          frag_x4(a1[1], sA, kGcLdQK, rt1 * 16, ks * 8 + 8, lane);
+        }
 #pragma unroll
-        for (int ti = 0; ti < 4; ti += 2) {
-          if (ti < cnt) {                              // an odd count reads rows of the tile behind and leaves them (at most row 63)
-            uint32_t bb[4];
-            frag_x4(bb, sK, kGcLdQK, (nt0 + ti) * 8, ks * 8, lane);
-            const uint32_t b0[2] = {bb[0], bb[2]}, b1[2] = {bb[1], bb[3]};
-            mma_tf32(accL[ti], aK, b0);
-            mma_tf32(accP[ti], aQ, b0);
-            if (ti + 1 < cnt) {
-              mma_tf32(accL[ti + 1], aK, b1);
-              mma_tf32(accP[ti + 1], aQ, b1);
-            }
+        for (int i = 0; i < 5; ++i) {
+          const int ct = i < n0 ? first + i : i - n0;
+          uint32_t b[4];                               // the tile's B fragments of both k steps
+          ldsm_x4(smem_u32(sK + (ct * 8 + (lane & 7)) * kGcLdQK + ks * 8 + (lane >> 3) * 4), b[0], b[1], b[2], b[3]);
+          const uint32_t b0[2] = {b[0], b[1]}, b1[2] = {b[2], b[3]};
+          if (i < n0) {
+            mma_tf32(acc[i], a0[0], b0);
+            mma_tf32(acc[i], a0[1], b1);
+          } else {
+            mma_tf32(acc[i], a1[0], b0);
+            mma_tf32(acc[i], a1[1], b1);
           }
         }
       }
 #pragma unroll
-      for (int ti = 0; ti < 4; ++ti) {
-        if (ti < cnt) {
+      for (int k = 0; k < 5; ++k) {
+        const int rt = k < n0 ? rt0 : rt1, j = (k < n0 ? first + k : k - n0) * 8 + 2 * t;
+        const float g0 = sG[j], g1 = sG[j + 1];
 #pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const int i = rt * 16 + g + (e >> 1) * 8, j = (nt0 + ti) * 8 + 2 * t + (e & 1);
-            const float dec = j <= i ? __expf(sG[i] - sG[j]) : 0.f;
-            sL[i * kGcLdL + j] = j < i ? sBeta[i] * dec * accL[ti][e] : 0.f;
-            sP[i * kGcLdL + j] = __uint_as_float(to_tf32(dec * accP[ti][e]));
+        for (int h = 0; h < 2; ++h) {
+          const int i = rt * 16 + g + h * 8;
+          const float gi = sG[i];
+          const float d0 = j <= i ? __expf(gi - g0) : 0.f, d1 = j + 1 <= i ? __expf(gi - g1) : 0.f;
+          if (isP) {
+            *reinterpret_cast<uint2*>(sP + i * kGcLdL + j) = make_uint2(to_tf32(d0 * acc[k][2 * h]), to_tf32(d1 * acc[k][2 * h + 1]));
+          } else {
+            const float beta = sBeta[i];
+            *reinterpret_cast<float2*>(sL + i * kGcLdL + j) = make_float2(j < i ? beta * d0 * acc[k][2 * h] : 0.f, j + 1 < i ? beta * d1 * acc[k][2 * h + 1] : 0.f);
           }
         }
       }
@@ -464,8 +487,8 @@ gdn_chunked_kernel(const RfGdn p) {
         for (int a = 0; a < NT; ++a) {
           const int col = (nh * NT + a) * 8 + g;
           uint32_t b[2];
-          b[0] = to_tf32(sS[(ks * 8 + t) * kGcLdS + col]);
-          b[1] = to_tf32(sS[(ks * 8 + t + 4) * kGcLdS + col]);
+          b[0] = __float_as_uint(sS[(ks * 8 + t) * kGcLdS + col]);
+          b[1] = __float_as_uint(sS[(ks * 8 + t + 4) * kGcLdS + col]);
           mma_tf32(accR[a], aK, b);
           mma_tf32(accO[a], aQ, b);
         }
@@ -516,6 +539,13 @@ gdn_chunked_kernel(const RfGdn p) {
         }
         st_row(sU + (b * 16 + r) * kGcLdS + cc, u);
         __syncthreads();
+        {                                              // e^{G_C - G} U as TF32 for the state, where the right-hand side was
+          const float w = __expf(sG[C - 1] - sG[b * 16 + r]);
+          float v[CPT];
+#pragma unroll
+          for (int e = 0; e < CPT; ++e) v[e] = __uint_as_float(to_tf32(w * u[e]));
+          st_row(sV + (b * 16 + r) * kGcLdS + cc, v);
+        }
         if (b < 3) {
 #pragma unroll
           for (int j4 = 0; j4 < 16; j4 += 4) {
@@ -557,15 +587,14 @@ gdn_chunked_kernel(const RfGdn p) {
         if (c0 + i < n) out[(size_t)(s0 + c0 + i) * p.ldo + hv * p.Dv + j0 + j] = Num<T>::from_f(accO[a][e]);
       }
 
+    __syncthreads();                                   // the last block of e^{G_C - G} U
     // ---- S' = e^{G_C} S0 + K^T (e^{G_C - G} * U): warp w owns state rows 16 w .. 16 w + 15
     {
-      const float gl = sG[C - 1], egl = __expf(gl);
-      float accS[NV / 8][4];
+      const float egl = __expf(sG[C - 1]);
 #pragma unroll
       for (int a = 0; a < NV / 8; ++a)
 #pragma unroll
-        for (int e = 0; e < 4; ++e)
-          accS[a][e] = egl * sS[(warp * 16 + g + (e >> 1) * 8) * kGcLdS + a * 8 + 2 * t + (e & 1)];
+        for (int e = 0; e < 4; ++e) st[a][e] *= egl;
 #pragma unroll
       for (int ks = 0; ks < C / 8; ++ks) {
         const int ca = ks * 8 + t, cb = ks * 8 + t + 4;
@@ -574,28 +603,21 @@ gdn_chunked_kernel(const RfGdn p) {
         aT[1] = __float_as_uint(sK[ca * kGcLdQK + warp * 16 + g + 8]);
         aT[2] = __float_as_uint(sK[cb * kGcLdQK + warp * 16 + g]);
         aT[3] = __float_as_uint(sK[cb * kGcLdQK + warp * 16 + g + 8]);
-        const float wa = __expf(gl - sG[ca]), wb = __expf(gl - sG[cb]);
 #pragma unroll
         for (int a = 0; a < NV / 8; ++a) {
-          uint32_t b[2];
-          b[0] = to_tf32(wa * sU[ca * kGcLdS + a * 8 + g]);
-          b[1] = to_tf32(wb * sU[cb * kGcLdS + a * 8 + g]);
-          mma_tf32(accS[a], aT, b);
+          const uint32_t b[2] = {__float_as_uint(sV[ca * kGcLdS + a * 8 + g]), __float_as_uint(sV[cb * kGcLdS + a * 8 + g])};
+          mma_tf32(st[a], aT, b);
         }
       }
-#pragma unroll
-      for (int a = 0; a < NV / 8; ++a)
-#pragma unroll
-        for (int e = 0; e < 4; ++e)
-          sS[(warp * 16 + g + (e >> 1) * 8) * kGcLdS + a * 8 + 2 * t + (e & 1)] = accS[a][e];
+      publish_state();
     }
     __syncthreads();
   }
 
-  for (int i = tid; i < DK * NV; i += kGcThreads) {
-    const int m = i / NV, c = i % NV;
-    S[(size_t)m * p.Dv + c] = sS[m * kGcLdS + c];
-  }
+#pragma unroll
+  for (int a = 0; a < NV / 8; ++a)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) S[(size_t)state_row(e) * p.Dv + a * 8 + 2 * t + (e & 1)] = st[a][e];
 }
 
 // ------------------------------------------------- gated RMSNorm over Dv ----
