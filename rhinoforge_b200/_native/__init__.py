@@ -110,7 +110,7 @@ class RfAttn(C.Structure):
         ("status", C.c_void_p), ("dtype", C.c_int32),
         ("slot", C.c_void_p), ("chunk", C.c_int32), ("sink", C.c_void_p), ("gate", C.c_void_p), ("ld_gate", C.c_int64),
         ("gate_by_head", C.c_int32), ("keep_first", C.c_int32), ("slopes", C.c_void_p), ("rates", C.c_void_p),
-        ("seq_of_row", C.c_void_p), ("pos", C.c_void_p), ("vd", C.c_int32),
+        ("seq_of_row", C.c_void_p), ("pos", C.c_void_p), ("vd", C.c_int32), ("rows_per_seq", C.c_int32),
     ]
 
 
@@ -173,7 +173,7 @@ class RfStackForward(C.Structure):
         ("n_deepstack_rows", C.c_int32),
         ("taps", C.c_void_p), ("tap_layers", C.c_void_p), ("n_taps", C.c_int32),
         ("state_slot", C.c_void_p), ("state_fresh", C.c_void_p),
-        ("twin_split", C.c_int32), ("reserved0", C.c_int32),
+        ("twin_split", C.c_int32), ("rows_per_seq", C.c_int32),
     ]
 
 

@@ -11,13 +11,21 @@
 //    bidirectional, sliding-window, boolean 2-D mask and segment-id (block
 //    diagonal / packed images) masking; GQA by kv head = q head / group.
 //  * decode: one CTA per (KV split, kv head, sequence), over the whole sequence,
-//    a chunk or a window with kept first tokens; the GQA group's query heads are the MMA rows, every consumer warp owns one page per stage, warps
-//    and splits are merged with log-sum-exp weights.
+//    a chunk or a window with kept first tokens; the GQA group's query heads are the MMA rows, every consumer warp owns one page per stage.  A
+//    sequence may have several query rows that see the same keys (a block of action tokens): (row, head) pairs then fill the MMA rows, so that
+//    two rows of eight heads read the pages once.  Warps are merged through shared memory with log-sum-exp weights, splits over the
+//    thread-block cluster that they form (up to eight) or, beyond that, by a second kernel.
+//
+// Decode, fp16, us, with one lane that copies page by page, merges in rows of bank conflicts and a second kernel / now: 1 x 300 keys, 16 + 2 x 8
+// heads of 128 9.4 / 7.2; 64 x 1024, 32 + 2 x 8 54.8 / 49.6 (K/V at the copy rate: 40.4); 8 x 8000 53.3 / 45.9 (39.4); 32 x 260, 16 + 2 x 4
+// 12.3 / 9.4; 50 rows on 880 keys, 8 + 2 x 1 heads of 256 22.0 as 50 sequences / 13.8 as one.
 //
 // Replaces llm_fp16_32b_prefill_flash_attn_univ_* and its vctxlen / minibatch
 // variants (src/ops/rpu_sdpa.cpp:30-37,202-203, src/ops/rpu_sdpa_vctxlen.cpp,
 // src/ops/rpu_sdpa_minibatch.cpp) and the per-sequence decode SDPA loop
 // (src/fused/rpu_qwen3_model.h:3504-3513).
+#include <atomic>
+
 #include "../common/dtype.cuh"
 #include "../common/host_util.h"
 #include "../common/mma.cuh"
@@ -35,6 +43,8 @@ struct alignas(8) AttnCtl {
   uint64_t empty[kAttnMaxStages];
   uint64_t qbar;
   int32_t abort_flag;
+  // decode, per MMA row: the warps' maxima and (scaled) sums of weights, this split's own
+  float warp_max[4][16], warp_sum[4][16], row_max[16], row_sum[16];
 };
 
 // STREAM: the page is read once in this launch (decode): it takes the L2 evict-first policy, so that a step's KV
@@ -99,7 +109,7 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
   constexpr int kStageBytes = 4 * kPageBytes;
   AttnCtl* ctl = reinterpret_cast<AttnCtl*>(smem + (size_t)p.stages * kStageBytes);
 
-  const int split = blockIdx.x, kvh = (int)blockIdx.y / p.g_tiles, g_first = ((int)blockIdx.y % p.g_tiles) * 16, seq = blockIdx.z;
+  const int split = blockIdx.z, kvh = (int)blockIdx.x / p.g_tiles, r_first = ((int)blockIdx.x % p.g_tiles) * 16, seq = blockIdx.y;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   // by row: the row's own position bounds its keys and its sequence's slot owns the pages
   const int owner = p.pos && p.seq_of_row ? p.seq_of_row[seq] : seq;
@@ -115,8 +125,9 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
   const int npg = max(0, pg_end - pg_begin);
   auto page_at = [&](int i) { return i < keep_pages ? i : i + skipped; };
   const int iters = (npg + 3) >> 2;
-  const int G = min(p.G - g_first, 16);          // query heads of this CTA
-  const int head0 = kvh * p.G + g_first;
+  const int R = min(p.rows_per_seq * p.G - r_first, 16);          // MMA rows of this CTA: (query row, head of the group) pairs
+  auto head_of = [&](int r) { return kvh * p.G + (p.rows_per_seq == 1 ? r_first + r : (r_first + r) % p.G); };
+  auto row_of = [&](int r) { return p.rows_per_seq == 1 ? seq : seq * p.rows_per_seq + (r_first + r) / p.G; };
 
   if (tid == 0) {
     for (int s = 0; s < p.stages; ++s) {
@@ -136,33 +147,36 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
   for (int i = 0; i < HD / 8; ++i) { o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f; }
 
   if (warp == 4) {
-    if (lane == 0) {
+    // Four lanes, one for each page of a stage, that fetch their page numbers a stage ahead: one lane that looked a page up and copied it four
+    // times over had eight (heads of 256: 32) copies and a table look-up in a row in front of every stage.
+    if (lane < 4) {
+      auto row_of_page = [&](int i) -> int {
+        if (i >= npg) return 0;
+        const int pg = page_at(pg_begin + i);
+        return p.paged ? (p.page_table[(size_t)pt_row * p.pt_stride + pg] * p.Hkv + kvh) * 16 : p.kv_start[seq] + pg * 16;
+      };
+      const int col0 = p.paged ? 0 : kvh * HD;
+      int row = row_of_page(lane);
       for (int it = 0; it < iters; ++it) {
-        const int s = it % p.stages;
+        const int s = it % p.stages, next = row_of_page((it + 1) * 4 + lane);
         const uint32_t ph = (uint32_t)(it / p.stages) & 1u;
-        if (!mbar_wait(&ctl->empty[s], ph ^ 1u)) {
-          report_status(p.status, kStatusTmaTimeout, kTagAttnDecode, it);
+        const bool ok = mbar_wait(&ctl->empty[s], ph ^ 1u);
+        if (!__all_sync(0xfu, ok)) {
+          if (lane == 0) report_status(p.status, kStatusTmaTimeout, kTagAttnDecode, it);
           ctl->abort_flag = 1;
           break;
         }
         const int nvalid = min(4, npg - it * 4);
-        mbar_arrive_expect_tx(&ctl->full[s], (uint32_t)(nvalid * kPageBytes));
-        for (int w = 0; w < nvalid; ++w) {
-          const int pg = page_at(pg_begin + it * 4 + w);
-          int row, col0;
-          if (p.paged) {
-            const int page_id = p.page_table[(size_t)pt_row * p.pt_stride + pg];
-            row = (page_id * p.Hkv + kvh) * 16;
-            col0 = 0;
-          } else {
-            row = p.kv_start[seq] + pg * 16;
-            col0 = kvh * HD;
-          }
+        if (lane == 0) mbar_arrive_expect_tx(&ctl->full[s], (uint32_t)(nvalid * kPageBytes));
+        __syncwarp(0xfu);
+        if (lane < nvalid) {
+          uint8_t* dst = smem + (size_t)s * kStageBytes + lane * kPageBytes;
           if (p.kv_stream)
-            load_kv_page<HD, true>(&tmK, &tmV, smem + (size_t)s * kStageBytes + w * kPageBytes, &ctl->full[s], col0, row);
+            load_kv_page<HD, true>(&tmK, &tmV, dst, &ctl->full[s], col0, row);
           else
-            load_kv_page<HD>(&tmK, &tmV, smem + (size_t)s * kStageBytes + w * kPageBytes, &ctl->full[s], col0, row);
+            load_kv_page<HD>(&tmK, &tmV, dst, &ctl->full[s], col0, row);
         }
+        row = next;
       }
     }
   } else {
@@ -171,24 +185,25 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
     float fall0 = 0.f, fall1 = 0.f;                // what the two rows' scores lose per token of distance
     if (p.slopes) {
       const float unit = p.rates ? 1.f : kLog2e;   // with rates the logarithm is one to the base of two already
-      if ((lane >> 2) < G) fall0 = p.slopes[head0 + (lane >> 2)] * unit;
-      if ((lane >> 2) + 8 < G) fall1 = p.slopes[head0 + (lane >> 2) + 8] * unit;
+      if ((lane >> 2) < R) fall0 = p.slopes[head_of(lane >> 2)] * unit;
+      if ((lane >> 2) + 8 < R) fall1 = p.slopes[head_of((lane >> 2) + 8)] * unit;
     }
     float rate0 = 0.f, rate1 = 0.f;
     if (p.rates) {
-      if ((lane >> 2) < G) rate0 = p.rates[head0 + (lane >> 2)];
-      if ((lane >> 2) + 8 < G) rate1 = p.rates[head0 + (lane >> 2) + 8];
+      if ((lane >> 2) < R) rate0 = p.rates[head_of(lane >> 2)];
+      if ((lane >> 2) + 8 < R) rate1 = p.rates[head_of((lane >> 2) + 8)];
     }
     {
       const int g0 = lane >> 2, g1 = g0 + 8;
-      const T* qbase = reinterpret_cast<const T*>(p.q) + (size_t)seq * p.ldq + (size_t)head0 * HD;
+      const T* q0 = reinterpret_cast<const T*>(p.q) + (size_t)row_of(g0 < R ? g0 : 0) * p.ldq + (size_t)head_of(g0 < R ? g0 : 0) * HD;
+      const T* q1 = reinterpret_cast<const T*>(p.q) + (size_t)row_of(g1 < R ? g1 : 0) * p.ldq + (size_t)head_of(g1 < R ? g1 : 0) * HD;
 #pragma unroll
       for (int ks = 0; ks < HD / 16; ++ks) {
         const int col = ks * 16 + (lane & 3) * 2;
-        qf[ks][0] = g0 < G ? *reinterpret_cast<const uint32_t*>(qbase + (size_t)g0 * HD + col) : 0u;
-        qf[ks][1] = g1 < G ? *reinterpret_cast<const uint32_t*>(qbase + (size_t)g1 * HD + col) : 0u;
-        qf[ks][2] = g0 < G ? *reinterpret_cast<const uint32_t*>(qbase + (size_t)g0 * HD + col + 8) : 0u;
-        qf[ks][3] = g1 < G ? *reinterpret_cast<const uint32_t*>(qbase + (size_t)g1 * HD + col + 8) : 0u;
+        qf[ks][0] = g0 < R ? *reinterpret_cast<const uint32_t*>(q0 + col) : 0u;
+        qf[ks][1] = g1 < R ? *reinterpret_cast<const uint32_t*>(q1 + col) : 0u;
+        qf[ks][2] = g0 < R ? *reinterpret_cast<const uint32_t*>(q0 + col + 8) : 0u;
+        qf[ks][3] = g1 < R ? *reinterpret_cast<const uint32_t*>(q1 + col + 8) : 0u;
       }
     }
     for (int it = 0; it < iters; ++it) {
@@ -249,63 +264,116 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
     l0 = quad_sum(l0);
     l1 = quad_sum(l1);
   }
+  const int r0 = lane >> 2, r1 = r0 + 8;
+  if (warp < 4 && (lane & 3) == 0) {
+    ctl->warp_max[warp][r0] = m0;
+    ctl->warp_max[warp][r1] = m1;
+  }
   __syncthreads();  // every issued copy has landed and been consumed
 
-  // merge the four warps (stage memory is free now)
-  float* mo = reinterpret_cast<float*>(smem);            // [4][16][HD]
-  float* mm = mo + 4 * 16 * HD;                          // [4][16]
-  float* ml = mm + 4 * 16;                               // [4][16]
+  // merge the four warps (stage memory is free now): each scales its sums to the common maximum and leaves them in rows of pitch LDO (conflict-free)
+  constexpr int LDO = HD + 8;
+  float* mo = reinterpret_cast<float*>(smem);            // [4][16][LDO]
+  auto max_of = [&](int g) { return fmaxf(fmaxf(ctl->warp_max[0][g], ctl->warp_max[1][g]), fmaxf(ctl->warp_max[2][g], ctl->warp_max[3][g])); };
+  auto sum_of = [&](int g) { return (ctl->warp_sum[0][g] + ctl->warp_sum[1][g]) + (ctl->warp_sum[2][g] + ctl->warp_sum[3][g]); };
+  auto out_of = [&](int g, int col) {
+    const float* at = mo + g * LDO + col;
+    return (at[0] + at[16 * LDO]) + (at[32 * LDO] + at[48 * LDO]);
+  };
   if (warp < 4) {
-    const int r0 = lane >> 2, r1 = r0 + 8, c = (lane & 3) * 2;
+    const int c = (lane & 3) * 2;
+    const float f0 = m0 == -INFINITY ? 0.f : exp2f(m0 - max_of(r0)), f1 = m1 == -INFINITY ? 0.f : exp2f(m1 - max_of(r1));
+    float* d0 = mo + (warp * 16 + r0) * LDO + c;
+    float* d1 = mo + (warp * 16 + r1) * LDO + c;
+    if (r0 < R) {
 #pragma unroll
-    for (int i = 0; i < HD / 8; ++i) {
-      float* d0 = mo + ((size_t)warp * 16 + r0) * HD + i * 8 + c;
-      float* d1 = mo + ((size_t)warp * 16 + r1) * HD + i * 8 + c;
-      d0[0] = o[i][0]; d0[1] = o[i][1];
-      d1[0] = o[i][2]; d1[1] = o[i][3];
+      for (int i = 0; i < HD / 8; ++i) *reinterpret_cast<float2*>(d0 + i * 8) = make_float2(o[i][0] * f0, o[i][1] * f0);
+    }
+    if (r1 < R) {
+#pragma unroll
+      for (int i = 0; i < HD / 8; ++i) *reinterpret_cast<float2*>(d1 + i * 8) = make_float2(o[i][2] * f1, o[i][3] * f1);
     }
     if ((lane & 3) == 0) {
-      mm[warp * 16 + r0] = m0; mm[warp * 16 + r1] = m1;
-      ml[warp * 16 + r0] = l0; ml[warp * 16 + r1] = l1;
+      ctl->warp_sum[warp][r0] = l0 * f0;
+      ctl->warp_sum[warp][r1] = l1 * f1;
     }
   }
   __syncthreads();
-  if (ctl->abort_flag) {
-    // A bounded wait ran out (the status word says where).  The merge pass still runs after this kernel, so this
-    // CTA's slots must not keep an earlier call's partials: mark them empty (weight 0 in the merge).
+  auto store = [&](int r, int col, float val) {
+    const int row = row_of(r), head = head_of(r);
+    const size_t at = (size_t)head * HD + col;
+    if (p.gate) val *= sigmoid_fast(Num<T>::to_f(reinterpret_cast<const T*>(p.gate)[(size_t)row * p.ld_gate + (p.gate_by_head ? head : at)]));
+    reinterpret_cast<T*>(p.out)[(size_t)row * p.ldo + at] = Num<T>::from_f(val);
+  };
+  const bool aborted = ctl->abort_flag != 0;   // a bounded wait ran out (the status word says where)
+  if (p.cluster) {
+    // The splits of a (sequence, K/V head) are one cluster: every CTA leaves its sums in its own shared memory and finishes a share of them.
+    // A CTA that gave up counts as empty (maximum -inf): its sums are not used.
+    if (!aborted) {
+      for (int idx = tid; idx < R * HD; idx += blockDim.x) {
+        float* at = mo + idx / HD * LDO + idx % HD;        // read and written by this thread alone
+        *at = (at[0] + at[16 * LDO]) + (at[32 * LDO] + at[48 * LDO]);
+      }
+    }
+    if (tid < R) {
+      ctl->row_max[tid] = aborted ? -INFINITY : max_of(tid);
+      ctl->row_sum[tid] = sum_of(tid);
+    }
+    cluster_sync_all();
+    const int share = (R * HD / 32 + p.splits - 1) / p.splits * 32, lo = split * share, hi = min(lo + share, R * HD);   // whole warps: one row to a warp
+    const uint32_t a_o = smem_u32(mo), a_m = smem_u32(ctl->row_max), a_s = smem_u32(ctl->row_sum);
+    for (int idx = lo + tid; idx < hi; idx += blockDim.x) {
+      const int g = idx / HD;
+      const uint32_t at = a_o + (uint32_t)(g * LDO + idx % HD) * 4u;
+      float m[8], l[8], part[8];
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {              // all on their way before the first is used
+        m[k] = -INFINITY; l[k] = 0.f; part[k] = 0.f;
+        if (k < p.splits) {
+          m[k] = ld_dsmem_f32(dsmem_addr(a_m + g * 4u, k));
+          l[k] = ld_dsmem_f32(dsmem_addr(a_s + g * 4u, k));
+          part[k] = ld_dsmem_f32(dsmem_addr(at, k));
+        }
+      }
+      float M = -INFINITY, num = 0.f, den = 0.f;
+#pragma unroll
+      for (int k = 0; k < 8; ++k) M = fmaxf(M, m[k]);
+      if (M != -INFINITY) {
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+          const float f = exp2f(m[k] - M);
+          num += m[k] == -INFINITY ? 0.f : f * part[k];
+          den += m[k] == -INFINITY ? 0.f : f * l[k];
+        }
+        if (p.sink) den += exp2f(p.sink[head_of(g)] * kLog2e - M);
+      }
+      store(g, idx % HD, den > 0.f ? num / den : 0.f);
+    }
+    cluster_sync_relaxed();                      // peers may still be reading this CTA's sums
+    return;
+  }
+  if (aborted) {
+    // The merge pass still runs after this kernel, so this CTA's slots must not keep an earlier call's partials: mark them empty (weight 0).
     if (p.splits > 1) {
-      for (int idx = tid; idx < G * HD; idx += blockDim.x) {
+      for (int idx = tid; idx < R * HD; idx += blockDim.x) {
         const int g = idx / HD, col = idx % HD;
-        const size_t base = ((size_t)seq * p.Hq + head0 + g) * p.splits + split;
+        const size_t base = ((size_t)row_of(g) * p.Hq + head_of(g)) * p.splits + split;
         p.ws_o[base * HD + col] = 0.f;
         if (col == 0) p.ws_lse[base] = -INFINITY;
       }
     }
     return;
   }
-  for (int idx = tid; idx < G * HD; idx += blockDim.x) {
+  for (int idx = tid; idx < R * HD; idx += blockDim.x) {
     const int g = idx / HD, col = idx % HD;
-    float M = -INFINITY;
-#pragma unroll
-    for (int w = 0; w < 4; ++w) M = fmaxf(M, mm[w * 16 + g]);
-    float num = 0.f, den = 0.f;
-    if (M != -INFINITY) {
-#pragma unroll
-      for (int w = 0; w < 4; ++w) {
-        const float f = exp2f(mm[w * 16 + g] - M);
-        num += f * mo[((size_t)w * 16 + g) * HD + col];
-        den += f * ml[w * 16 + g];
-      }
-    }
-    const int head = head0 + g;
-    if (p.splits == 1 && p.sink && M != -INFINITY) den += exp2f(p.sink[head] * kLog2e - M);
-    float val = den > 0.f ? num / den : 0.f;
+    const float M = max_of(g), num = out_of(g, col);
+    float den = sum_of(g);
+    if (p.splits == 1 && p.sink && M != -INFINITY) den += exp2f(p.sink[head_of(g)] * kLog2e - M);
+    const float val = den > 0.f ? num / den : 0.f;
     if (p.splits == 1) {
-      const size_t col_of_row = (size_t)head * HD + col;
-      if (p.gate) val *= sigmoid_fast(Num<T>::to_f(reinterpret_cast<const T*>(p.gate)[(size_t)seq * p.ld_gate + (p.gate_by_head ? head : col_of_row)]));
-      reinterpret_cast<T*>(p.out)[(size_t)seq * p.ldo + col_of_row] = Num<T>::from_f(val);
+      store(g, col, val);
     } else {
-      const size_t base = ((size_t)seq * p.Hq + head) * p.splits + split;
+      const size_t base = ((size_t)row_of(g) * p.Hq + head_of(g)) * p.splits + split;
       p.ws_o[base * HD + col] = val;
       if (col == 0) p.ws_lse[base] = den > 0.f ? M + log2f(den) : -INFINITY;
     }
@@ -563,7 +631,8 @@ static int fill_params(const RfAttn* a, AttnParams* p) {
   if (a->slopes || a->keep_first > 0) RF_REQUIRE(!a->mask && !a->seg_q, "distance slopes and kept first positions do not go with data-dependent masks");
   p->slot = a->slot; p->chunk = a->chunk; p->sink = a->sink; p->gate = a->gate; p->ld_gate = a->ld_gate;
   p->gate_by_head = a->gate_by_head; p->keep_first = a->window > 0 || a->chunk > 0 ? std::max(a->keep_first, 0) : 0; p->slopes = a->slopes; p->rates = a->rates;
-  p->seq_of_row = a->seq_of_row; p->pos = a->pos; p->g_tiles = ceil_div(p->G, 16);
+  p->seq_of_row = a->seq_of_row; p->pos = a->pos; p->rows_per_seq = std::max(a->rows_per_seq, 1); p->g_tiles = ceil_div(p->rows_per_seq * p->G, 16);
+  p->cluster = 0;
   p->ws_o = nullptr; p->ws_lse = nullptr; p->splits = 1; p->pages_per_split = 1 << 28; p->stages = 2;
   p->status = a->status;
   return RF_OK;
@@ -586,12 +655,13 @@ static int kv_tmaps(const RfAttn* a, CUtensorMap* tmK, CUtensorMap* tmV) {
 // takes.  Small batches are split until about two CTAs per SM exist; a split covers at least 8 pages and a multiple
 // of 4 (one ring stage).  `allow_split` is false when the caller gave no scratch for the partials.
 struct DecodeSplitPlan {
-  int splits, pages_per_split;
+  int splits, pages_per_split, max_pages;
   uint64_t scratch_bytes;   // fp32 partial outputs + one log-sum-exp per (sequence, head, split); 0 when unsplit
 };
-static DecodeSplitPlan plan_decode_split(int num_seqs, int Hq, int Hkv, int hd, int max_kv_len, bool allow_split) {
+static DecodeSplitPlan plan_decode_split(int num_seqs, int rows_per_seq, int Hq, int Hkv, int hd, int max_kv_len, bool allow_split) {
   const int max_pages = std::max(1, (max_kv_len + 15) / 16);
-  const int ctas = num_seqs * Hkv;
+  // one query row per sequence: a group of more than 16 heads counts as one CTA
+  const int ctas = num_seqs * Hkv * (rows_per_seq > 1 ? ceil_div(rows_per_seq * (Hq / Hkv), 16) : 1);
   int splits = 1;
   // RF_ATTN_DECODE_CTAS_PER_SM (default 2; 1 for heads of 256): CTAs per SM the split aims at; RF_ATTN_DECODE_MIN_PAGES (default 8): fewest
   // pages a split may cover
@@ -605,10 +675,37 @@ static DecodeSplitPlan plan_decode_split(int num_seqs, int Hq, int Hkv, int hd, 
     splits = std::min(splits, 64);
   }
   DecodeSplitPlan pl;
+  pl.max_pages = max_pages;
   pl.pages_per_split = round_up(ceil_div(max_pages, splits), 4);
   pl.splits = std::max(1, ceil_div(max_pages, pl.pages_per_split));
-  pl.scratch_bytes = pl.splits > 1 ? (uint64_t)num_seqs * Hq * pl.splits * (hd + 1) * sizeof(float) : 0;
+  pl.scratch_bytes = pl.splits > 1 ? (uint64_t)num_seqs * rows_per_seq * Hq * pl.splits * (hd + 1) * sizeof(float) : 0;
   return pl;
+}
+
+// Clusters of `size` CTAs of the kernel that the current device holds at once (asked once per kernel, device and size)
+template <typename T, int HD>
+static long clusters_resident(int size, size_t smem) {
+  static std::atomic<int> known[64][9];
+  auto kfn = attn_decode_kernel<T, HD>;
+  const int dev = device_ordinal();
+  const bool track = dev >= 0 && dev < 64;
+  if (track) {
+    const int n = known[dev][size].load(std::memory_order_relaxed);
+    if (n > 0) return n - 1;
+  }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(1, 1, size); cfg.blockDim = dim3(160); cfg.dynamicSmemBytes = smem;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 1; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = (unsigned)size;
+  cfg.attrs = attr; cfg.numAttrs = 1;
+  int n = 0;
+  if (cudaOccupancyMaxActiveClusters(&n, kfn, &cfg) != cudaSuccess) {
+    (void)cudaGetLastError();
+    n = 0;
+  }
+  if (track) known[dev][size].store(n + 1, std::memory_order_relaxed);
+  return n;
 }
 
 template <typename T, int HD>
@@ -617,7 +714,7 @@ static int launch_decode(const RfAttn* a, AttnParams& p, cudaStream_t s) {
   int rc = kv_tmaps(a, &tmK, &tmV);
   if (rc) return rc;
   constexpr int kStageBytes = 4 * 2 * (HD / 64) * kBoxBytes;
-  const int merge_bytes = (4 * 16 * HD + 128) * 4;
+  const int merge_bytes = 4 * 16 * (HD + 8) * 4;
   int stages = HD == 256 ? 2 : (HD == 128 ? 3 : 4);
   while (stages * kStageBytes < merge_bytes) ++stages;
   p.stages = stages;
@@ -629,29 +726,39 @@ static int launch_decode(const RfAttn* a, AttnParams& p, cudaStream_t s) {
   int max_kv = a->max_kv_len;
   if (a->chunk > 0) max_kv = std::min(max_kv, a->chunk + 15 + p.keep_first + 15);
   if (a->window > 0) max_kv = std::min(max_kv, a->window + 15 + p.keep_first + 15);
-  const DecodeSplitPlan pl = plan_decode_split(a->num_seqs, a->Hq, a->Hkv, HD, max_kv, a->ws != nullptr);
-  const int splits = pl.splits;
+  const DecodeSplitPlan pl = plan_decode_split(a->num_seqs, p.rows_per_seq, a->Hq, a->Hkv, HD, max_kv, a->ws != nullptr);
+  int splits = pl.splits;
+  p.pages_per_split = pl.pages_per_split;
+  // Up to eight splits are one cluster and merged inside the launch: the second kernel cost 2.2 us (1 x 300 keys) to 3.5 us (50 rows, heads of
+  // 256) behind every layer's attention.  Where so many clusters would not all be resident, fewer splits, down to half, are tried before the
+  // second kernel is taken (12 x 517 keys, 8 K/V heads: 3 splits and the second kernel 14.0 us, 2 splits 11.4).
+  for (int n = splits; splits <= 8 && n > 1 && 2 * n >= splits; --n) {
+    const int pages = n == splits ? pl.pages_per_split : round_up(ceil_div(pl.max_pages, n), 4), parts = ceil_div(pl.max_pages, pages);
+    if (parts > 1 && (long)a->Hkv * p.g_tiles * a->num_seqs <= clusters_resident<T, HD>(parts, smem)) {
+      p.cluster = 1;
+      splits = parts;
+      p.pages_per_split = pages;
+      break;
+    }
+  }
   if (splits > 1) {
     RF_REQUIRE(pl.scratch_bytes <= a->ws_bytes, "decode attention scratch too small: need %llu B",
                (unsigned long long)pl.scratch_bytes);
     p.ws_o = a->ws;
-    p.ws_lse = a->ws + (size_t)a->num_seqs * a->Hq * splits * HD;
+    p.ws_lse = a->ws + (size_t)a->num_seqs * p.rows_per_seq * a->Hq * splits * HD;
   }
   p.splits = splits;
-  p.pages_per_split = pl.pages_per_split;
   {
     static const int ef = [] { const char* e = getenv("RF_ATTN_KV_EVICT_FIRST"); return e ? atoi(e) : 1; }();
-    p.kv_stream = ef;
+    p.kv_stream = ef && p.g_tiles == 1;      // pages that several CTAs of the launch read stay
   }
-  dim3 grid(splits, a->Hkv * p.g_tiles, a->num_seqs);
-  RF_CUDA_CHECK(::rf::launch_k(kfn, dim3(grid), dim3(160), smem, s, 1, tmK, tmV, p));
-  RF_CUDA_CHECK(cudaGetLastError());
+  const dim3 grid(a->Hkv * p.g_tiles, a->num_seqs, splits);
+  RF_CUDA_CHECK(::rf::launch_k(kfn, grid, dim3(160), smem, s, p.cluster ? splits : 1, tmK, tmV, p));
   ::rf::count_launch();
-  if (splits > 1) {
-    dim3 g2(a->Hq, a->num_seqs);
+  if (splits > 1 && !p.cluster) {
+    const dim3 g2(a->Hq, a->num_seqs * p.rows_per_seq);
     RF_CUDA_CHECK(::rf::launch_k(attn_decode_combine_kernel<T>, dim3(g2), dim3(HD < 128 ? HD : 128), 0, s, 1, p.ws_o, p.ws_lse, (T*)a->out, a->ldo, a->Hq, HD, splits, a->sink, (const T*)a->gate, a->ld_gate, a->gate_by_head));
-    RF_CUDA_CHECK(cudaGetLastError());
-  ::rf::count_launch();
+    ::rf::count_launch();
   }
   return RF_OK;
 }
@@ -709,7 +816,8 @@ extern "C" int rf_attn_decode(const RfAttn* a, rf_stream_t stream) {
   AttnParams p;
   int rc = fill_params(a, &p);
   if (rc) return rc;
-  RF_REQUIRE(a->num_seqs <= 65535, "decode attention: %d rows in one launch", a->num_seqs);
+  RF_REQUIRE(a->num_seqs <= 65535 && (int64_t)a->num_seqs * p.rows_per_seq <= 65535, "decode attention: %d x %d rows in one launch", a->num_seqs, p.rows_per_seq);
+  RF_REQUIRE(p.rows_per_seq == 1 || !a->pos, "decode attention by row takes one row per sequence");
   RF_REQUIRE(a->max_kv_len > 0, "decode attention needs max_kv_len");
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   RF_ATTN_DISPATCH(launch_decode)
@@ -773,7 +881,7 @@ static int static_scratch_ptr(void** out) {
 
 // Bytes of split-KV partials the launcher will ask for: the launcher's own plan, with splitting allowed.
 static uint64_t decode_scratch_need(const RfAttn* a) {
-  return plan_decode_split(a->num_seqs, a->Hq, a->Hkv, a->hd, a->max_kv_len, true).scratch_bytes;
+  return plan_decode_split(a->num_seqs, std::max(a->rows_per_seq, 1), a->Hq, a->Hkv, a->hd, a->max_kv_len, true).scratch_bytes;
 }
 
 }  // namespace rf

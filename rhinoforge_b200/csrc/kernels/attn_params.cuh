@@ -29,7 +29,9 @@ struct AttnParams {
   const float* slopes;    // natural-log units per token of distance, or per unit of ln(1 + rate * distance)
   const float* rates;
   const int32_t* seq_of_row; const int32_t* pos;
-  int32_t g_tiles;        // decode: CTAs that share one K/V head (16 query heads each)
+  int32_t g_tiles;        // decode: CTAs that share one K/V head (16 (query row, head) pairs each)
+  int32_t rows_per_seq;   // decode: query rows of a sequence, all of which see its keys
+  int32_t cluster;        // decode: the splits of a (sequence, K/V head) are one thread-block cluster
 };
 
 constexpr float kLog2e = 1.4426950408889634f;

@@ -217,7 +217,7 @@ gdn_recurrent_kernel(const RfGdn p) {
 // What bounds it: the chain of a chunk - normalise, L and P, substitution, state - on one CTA per SM, most of it shared-memory accesses.  Tiles
 // are written 16 bytes a lane without bank conflicts and read as fragments by ldmatrix (a 32-bit element is a pair of its 16-bit ones).
 // Half the work of a chunk does not depend on the columns, so 64 of them cost a CTA little more than 32.  4 x 1500 tokens, 16 heads of 128:
-// 577 us with scalar tiles and 32 columns, 318 now; 1 x 1500 (64 CTAs of 32 columns, one wave) 287 and 248.
+// 577 us with scalar tiles and 32 columns, 306 now; 1 x 1500 (64 CTAs of 32 columns, one wave) 287 and 240.
 constexpr int kGcC = 64;          // tokens per chunk
 constexpr int kGcThreads = 256;
 constexpr int kGcLdQK = 132;      // fp32 row pitch of the q / k tiles: (4 * row + col) mod 32 is distinct over a fragment
@@ -769,7 +769,7 @@ extern "C" int rf_gdn_chunked(const RfGdn* a, rf_stream_t stream) {
   RF_REQUIRE(a->num_seqs > 0, "gdn: no sequences");
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   // 64 columns to a CTA where 32 would make more CTAs than there are SMs (one sits on an SM): half of a chunk's work is the same for any number of
-  // columns (1500 tokens, 16 heads of 128: a wave of 32 columns takes 248 us, which 4 sequences need twice, a wave of 64 columns 318)
+  // columns (1500 tokens, 16 heads of 128: a wave of 32 columns takes 240 us, which 4 sequences need twice, a wave of 64 columns 306)
   const bool wide = a->Dv % 64 == 0 && (long)(a->Dv / kGdnCols) * a->Hv * a->num_seqs > sm_count();
   auto run = [&](auto kfn, int nv) -> cudaError_t {
     return ::rf::launch_k(kfn, dim3(a->Dv / nv, a->Hv, a->num_seqs), dim3(kGcThreads), gc_smem_bytes(nv), s, 1, *a);

@@ -112,7 +112,7 @@ typedef struct RfStackComm {
 typedef struct RfStackForward {
   void* hidden;                  // [tokens, hidden] residual stream, updated in place
   int32_t tokens;
-  int32_t decode;                // 1: one token per sequence
+  int32_t decode;                // 1: one token (rows_per_seq tokens) per sequence
   const int32_t* pos; int32_t pos_stride;
   const float* cos; const float* sin; const int8_t* axis_of_freq;
   const int32_t* seq_of_tok; const int32_t* cache_pos;
@@ -135,7 +135,7 @@ typedef struct RfStackForward {
   // [twin_split, tokens) through its twin set (rf_stack_set_twin_layer).  0: no routing.  The caller orders the rows
   // accordingly; positions, cache rows and the attention mask are per row, so the order is free.
   int32_t twin_split;
-  int32_t reserved0;
+  int32_t rows_per_seq;                    // decode: query rows of every sequence (0: 1), which all see its kv_len keys
 } RfStackForward;
 
 int64_t rf_stack_create(const RfStackConfig* cfg);

@@ -367,21 +367,15 @@ class Pi05Engine:
         self.h = torch.zeros(Bm * n, e.hidden, dtype=dtype, device=dev)
         self.hn = torch.zeros_like(self.h)
         self.s_pos = torch.zeros(Bm * n, **i32)
-        # Every action row is its own one-query "sequence" for the split-KV decode attention kernel: it sees the
-        # whole prefix plus all action rows of its sample (their K/V are inserted before attention runs), which
-        # is exactly the bidirectional suffix mask, and the KV range is split over many CTAs instead of one.
-        self.s_seq = torch.arange(Bm * n, **i32)
-        self.s_kvlen = torch.zeros(Bm * n, **i32)
-        self.s_pt = torch.zeros((Bm * n, self.cache.pages_per_seq), **i32)
-        # the same suffix as one query block per sample (prefill form of the attention launch)
+        # Every action row sees the whole prefix plus all action rows of its sample (their K/V are inserted before attention
+        # runs): one sequence per sample with `horizon` query rows, on either attention kernel
         self.b_qstart = torch.arange(Bm, **i32) * n
         self.b_qlen = torch.full((Bm,), n, **i32)
         self.b_kvlen = torch.zeros(Bm, **i32)
         self.b_seq = torch.arange(Bm, **i32).repeat_interleave(n).contiguous()
-        # RF_PI05_SUFFIX_ATTN: `decode` = every suffix row is its own one-token sequence over the sample's pages (split-KV
-        # decode kernel: many small CTAs, best at one or two samples); `block` = one bidirectional query block of
-        # `horizon` rows per sample (tensor-core prefill kernel: one CTA per sample and head, reads the pages once per
-        # sample instead of once per row).  `auto` (default) takes `block` from four samples up: measured denoise loop
+        # RF_PI05_SUFFIX_ATTN: `decode` = split-KV decode kernel, 16 (row, head) pairs to a CTA (many small CTAs, best at one
+        # or two samples); `block` = one bidirectional query block of `horizon` rows per sample (tensor-core prefill kernel:
+        # one CTA per sample and head, reads the pages once per sample and head).  `auto` (default) takes `block` from four samples up: measured denoise loop
         # 14.2 / 51.1 / 97.0 ms (decode) against 20.7 / 45.5 / 58.7 ms (block) at 1 / 8 / 32 samples.
         self.suffix_attn = os.environ.get("RF_PI05_SUFFIX_ATTN", "auto")
         self.prefix_hidden = torch.zeros(Bm * self.max_prefix, v.hidden, dtype=dtype, device=dev)
@@ -505,9 +499,9 @@ class Pi05Engine:
                                           seq_of_tok=self.b_seq[:T], cache_pos=self.s_pos[:T], page_table=self.cache.page_table[:B],
                                           mod=sch["mod"][s], rows_per_mod=T)
             else:
-                self.expert_stack.forward(h, decode=True, kv_len=self.s_kvlen[:T], max_kv_len=self.max_seq, pos=self.s_pos[:T],
-                                          cos=self.cos, sin=self.sin, seq_of_tok=self.s_seq[:T], cache_pos=self.s_pos[:T],
-                                          page_table=self.s_pt[:T], mod=sch["mod"][s], rows_per_mod=T)
+                self.expert_stack.forward(h, decode=True, rows_per_seq=n, kv_len=self.b_kvlen[:B], max_kv_len=self.max_seq, pos=self.s_pos[:T],
+                                          cos=self.cos, sin=self.sin, seq_of_tok=self.b_seq[:T], cache_pos=self.s_pos[:T],
+                                          page_table=self.cache.page_table[:B], mod=sch["mod"][s], rows_per_mod=T)
             K.rmsnorm(h, None, cfg.expert.eps, out=hn, mod=sch["final"][s:s + 1], rows_per_mod=T)
             K.gemm(hn, sch["out_w"], bias=sch["out_b"], residual=x, out=x)        # x <- x + dt * v
 
@@ -517,9 +511,7 @@ class Pi05Engine:
         B, n = noise.shape[0], cfg.horizon
         T = B * n
         pl = torch.tensor(list(prefix_lens), dtype=torch.int32)
-        self.s_kvlen[:T].copy_((pl + n).repeat_interleave(n).to(dev), non_blocking=True)
         self.b_kvlen[:B].copy_((pl + n).to(dev), non_blocking=True)
-        self.s_pt[:T].copy_(self.cache.page_table[:B].repeat_interleave(n, 0))
         self.s_pos[:T].copy_((pl[:, None] + torch.arange(n, dtype=torch.int32)[None]).flatten().to(dev), non_blocking=True)
         self.x[:T].copy_(noise.reshape(T, -1).to(dev, self.dtype))
         if not use_graph:

@@ -461,12 +461,12 @@ def attention_prefill(q: torch.Tensor, out: torch.Tensor, *, Hq: int, Hkv: int, 
 def attention_decode(q: torch.Tensor, out: torch.Tensor, *, Hq: int, Hkv: int, hd: int, kv_len: torch.Tensor,
                      max_kv_len: int, k_pool: torch.Tensor, v_pool: torch.Tensor, page_table: torch.Tensor,
                      scale: float = 0.0, ws: Optional[torch.Tensor] = None,
-                     status: Optional[torch.Tensor] = None) -> torch.Tensor:
-    """One query token per sequence against the paged KV pool (split-KV when ``ws`` is given)."""
+                     status: Optional[torch.Tensor] = None, rows_per_seq: int = 1) -> torch.Tensor:
+    """One query token (``rows_per_seq`` that all see the sequence's keys) per sequence against the paged KV pool (split-KV when ``ws`` is given)."""
     a = N.RfAttn()
     a.q, a.ldq, a.out, a.ldo = q.data_ptr(), q.stride(0), out.data_ptr(), out.stride(0)
     a.q_rows_total = q.shape[0]
-    a.num_seqs, a.Hq, a.Hkv, a.hd = q.shape[0], Hq, Hkv, hd
+    a.num_seqs, a.rows_per_seq, a.Hq, a.Hkv, a.hd = q.shape[0] // rows_per_seq, rows_per_seq, Hq, Hkv, hd
     a.k_pool, a.v_pool, a.pool_pages = k_pool.data_ptr(), v_pool.data_ptr(), k_pool.shape[0]
     a.page_table, a.pt_stride = _i32(page_table), page_table.stride(0)
     a.kv_len = _i32(kv_len)

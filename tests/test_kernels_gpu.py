@@ -1103,3 +1103,25 @@ def test_rope_kv_few_and_many_tokens_agree(dt, hd, rot, Hq, Hkv, T):
         flat = qkv.clone()
         K_.qk_norm_rope_kv(flat, Hq, Hkv, hd, pos=pos, cos=cos_sin[0], sin=cos_sin[1], rot_dim=rot, q_norm_w=w[0], k_norm_w=w[1], axis_of_freq=axis if three else None)
         _close(flat.view(T, -1, hd)[:, Hq:Hq + Hkv], k_ref, dt, scale=3.0)
+
+
+@pytest.mark.parametrize("dt", DT)
+@pytest.mark.parametrize("hd,Hq,Hkv", [(64, 6, 2), (128, 32, 8), (128, 40, 2), (256, 8, 1)])
+@pytest.mark.parametrize("rows", [1, 2, 7, 50])
+@pytest.mark.parametrize("lens", [[1, 300, 131], [5000]])
+def test_attn_decode_rows_of_a_sequence(dt, hd, Hq, Hkv, rows, lens, status):
+    """Several query rows of a sequence over all its keys: (row, head) pairs that fill, share and end inside a tile of 16, splits merged over a cluster
+    (with and without empty ones) and, for 5000 keys, by the second kernel - against fp32 and against the unsplit kernel."""
+    from rhinoforge_b200.ops import kernels as K_
+    k_pool, v_pool, pt, ks, vs = _paged(Hkv, hd, lens, dt)
+    q = torch.randn(len(lens) * rows, Hq * hd, device="cuda").to(dt)
+    kw = dict(Hq=Hq, Hkv=Hkv, hd=hd, kv_len=torch.tensor(lens, dtype=torch.int32, device="cuda"), max_kv_len=max(lens), k_pool=k_pool, v_pool=v_pool, page_table=pt,
+              status=status, rows_per_seq=rows)
+    out = K_.attention_decode(q, torch.full_like(q, float("nan")), ws=K_.attn_decode_scratch(q.shape[0], Hq, hd, "cuda"), **kw)
+    whole = K_.attention_decode(q, torch.full_like(q, float("nan")), **kw)
+    for s, L in enumerate(lens):
+        at = slice(s * rows, (s + 1) * rows)
+        ref = _sdpa_ref(q[at].view(rows, Hq, hd).transpose(0, 1), ks[s], vs[s], torch.ones(rows, L, dtype=torch.bool, device="cuda"))
+        ref = ref.transpose(0, 1).reshape(rows, Hq * hd)
+        _close(out[at], ref, dt)
+        _close(whole[at], ref, dt)
