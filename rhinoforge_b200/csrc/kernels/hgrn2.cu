@@ -681,12 +681,13 @@ extern "C" int rf_hgrn2_chunked(const RfHgrn2* a, rf_stream_t stream) {
   RF_REQUIRE(a->rows.q_start && a->rows.q_len, "hgrn2: the block form works on portions");
   if (a->rows.num_seqs == 0) return RF_OK;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  // value channels per CTA: as few as still share a head between at most eight CTAs, more once the GPU is full
+  // Value channels per CTA: 64 as long as all CTAs are resident at once (two to an SM, one with more than 128 key channels) and a head is shared
+  // by at most eight, then 128.  What a CTA does for the gates and the in-block scores does not depend on its channels, and two CTAs hide each
+  // other's barriers.  bf16, heads of 128 x 128, us with 32 / 64 / 128 channels: 16 x 1100 tokens 265 / 248 / 290, 64 x 1100 306 / 329 / 408,
+  // 96 x 1100 579 / 336 / 482, 144 x 1000 752 / 307 / 456, 192 x 500 426 / 266 / 244.
   int vt = a->vdim <= 32 ? 32 : a->vdim <= 64 ? 64 : 128;
-  for (int t : {32, 64}) {
-    const int tiles = ceil_div(a->vdim, t);
-    if (tiles <= 8 && (long)a->rows.num_seqs * a->heads * tiles <= sm_count()) { vt = std::min(vt, t); break; }
-  }
+  const int halves = ceil_div(a->vdim, 64);
+  if (vt == 128 && halves <= 8 && (long)a->rows.num_seqs * a->heads * halves <= (a->dim <= 128 ? 2l : 1l) * sm_count()) vt = 64;
   const int tiles = ceil_div(a->vdim, vt);
   if (vt == 32) return launch_chunked<2>(a, tiles, s);
   if (vt == 64) return launch_chunked<4>(a, tiles, s);

@@ -235,6 +235,23 @@ def test_hgrn2_against_the_recurrence(dtype, chunked, heads, D, VD, vdim):
     torch.testing.assert_close(state.double().cpu(), want_state, rtol=1e-4, atol=1e-4)
 
 
+@pytest.mark.parametrize("heads,D,VD", [(20, 16, 72), (26, 16, 72), (26, 40, 128), (26, 136, 72)])
+def test_hgrn2_portions_of_many_heads(heads, D, VD):
+    """The block form on both sides of the line where its CTAs of 64 value channels are more than the GPU holds at once (128 to a CTA then), against
+    the token-by-token kernel."""
+    lens, pos0, slots = [1, 40, 2, 16, 17, 33], [4, 0, 33, 64, 0, 9], [5, 2, 0, 1, 4, 6]
+    d, _, _ = pack(lens, pos0, slots)
+    g = torch.Generator().manual_seed(heads + D)
+    x = torch.randn(sum(lens), heads * (2 * D + VD), generator=g).to("cuda", torch.bfloat16)
+    fb, lower, nw = torch.randn(heads * D, generator=g).cuda(), torch.rand(heads * D, generator=g).cuda() ** 3, torch.randn(VD, generator=g).cuda()
+    a = torch.randn(7, heads, D, VD, generator=g).cuda()
+    b = a.clone()
+    got = K().hgrn2(x, fb, lower, nw, a, K().rows(**d), eps=1e-5, chunked=True)
+    want = K().hgrn2(x, fb, lower, nw, b, K().rows(**d), eps=1e-5)
+    close(got, want.double().cpu(), torch.bfloat16, 4)
+    torch.testing.assert_close(a, b, rtol=1e-4, atol=1e-4)
+
+
 def test_hgrn2_keeps_a_value_written_long_ago():
     """A channel whose gate stays open carries one token's value over hundreds of others."""
     D = VD = 64
