@@ -1,24 +1,27 @@
 // GEMM of very few rows (at most 16) over tile-major weights:  out[M,N] = epilogue( x[M,K] . w[N,K]^T ).
 //
 // At these sizes the time is a pass over the weights plus what a launch adds around it, and the tcgen05 kernel (gemm_tc.cu) adds a lot:
-// barriers, tensor-memory allocation, a ring through shared memory, and a cluster rendezvous on both sides of the split-K reduction.
-// Here a weight goes from memory into the registers that feed the MMA and nowhere else.
+// barriers, tensor-memory allocation, a ring whose stages are handed from warp to warp, and a cluster rendezvous on both sides of the split-K
+// reduction.  Here every warp has a ring of its own and feeds its own MMAs.
 //
 //  * A CTA of eight warps takes strips of 16 output features; its warps share a strip's 64-column k blocks.  Inside a block a lane
-//    (g = lane / 4, t = lane % 4) loads 16 bytes of rows g and g + 8: eight values (16-bit), sixteen (int8) or, with 8 bytes, sixteen
+//    (g = lane / 4, t = lane % 4) holds 16 bytes of rows g and g + 8: eight values (16-bit), sixteen (int8) or, with 8 bytes, sixteen
 //    (int4), all neighbours along k.  mma.sync does not care which k a slot stands for as long as both operands agree, so the lane's
-//    words are the A fragments as they come, and the same k range of token g is the B fragment: no shared memory, no shuffles.
+//    words are the A fragments as they come, and the same k range of token g is the B fragment: no shuffles, and no meeting of warps.
 //    int8 and int4 are widened in registers on the way.
-//  * Two to four blocks of weights per warp are always on their way, over the ends of strips too; the first ones are asked for ahead of
-//    the dependency wait.  x comes from L2 or L1, one block ahead.
+//  * Four to eight blocks of weights per warp (64 KB a CTA, two CTAs an SM) are on their way in the warp's ring, over the ends of strips too; the
+//    first ones are asked for ahead of the dependency wait.  cp.async, and not loads into registers: a warp waits for its loads on a handful of
+//    counters, and with weights and x on the same ones every block waited for the newest (12 x 151936 x 4096 int8 215 us in registers, 160 now;
+//    1 x 12288 x 4096 int8 SwiGLU 24.7 / 18.2).  Each lane copies what it will read; only int4 blocks, 512 bytes, are shared by the warp.
+//  * x comes from L2 or L1, one block ahead; what the epilogue adds and multiplies by ahead of a strip's products.
 //  * The warps' sums meet in shared memory once per strip; one thread finishes one value.
 //  * A folded RMSNorm needs no sums of squares from the kernel before: every CTA reads all of x anyway and squares it on the way.
 //
-// fp16, us, this kernel / gemm_tc.cu: 1 x 4096 x 1024 3.1 / 5.7, 1 x 1024 x 2048 2.9 / 5.5, 8 x 2048 x 2048 3.7 / 6.2, 16 x 3072 x 2048 5.0 / 6.5,
-// 1 x 4096 x 4096 8.0 / 10.0, 8 x 8192 x 2048 SwiGLU 13.0 / 15.1; not taken: 1 x 2048 x 8192 13.0 / 11.2, 1 x 6144 x 4096 14.3 / 13.0,
-// 16 x 8192 x 2048 SwiGLU 16.3 / 15.3.  int8: 1 x 4096 x 4096 6.6 / 11.9, 12 x 12288 x 4096 SwiGLU 26.8 / 44.4, 12 x 151936 x 4096 215 / 242;
-// int4: 12 x 12288 x 4096 SwiGLU 40.4 / 52.8.  (Row tiles that start their k blocks at different places, as gemm_tc.cu has them: up to a quarter
-// slower.  The strips of a row tile then still share its blocks, but the blocks that are read side by side are no longer neighbours.)
+// fp16, us, this kernel / gemm_tc.cu: 1 x 4096 x 1024 3.1 / 5.7, 1 x 1024 x 2048 3.0 / 5.5, 8 x 2048 x 2048 4.1 / 6.2, 1 x 6144 x 4096 10.5 / 12.9,
+// 1 x 4096 x 12288 17.0 / 19.5, 16 x 3072 x 2048 5.1 / 6.6, 16 x 4096 x 4096 9.2 / 10.5; SwiGLU 1 x 12288 x 4096 31.5 / 35.3 (30.3 at the copy
+// rate), 16 x 8192 x 2048 13.9 / 15.2.  int8: 1 x 4096 x 4096 6.3 / 11.9, 12 x 12288 x 4096 SwiGLU 24.0 / 44.4, 12 x 151936 x 4096 160 / 242; int4:
+// 12 x 12288 x 4096 SwiGLU 38.5 / 52.8, 12 x 4096 x 12288 18.7 / 29.4.  (Row tiles that start their k blocks at different places, as gemm_tc.cu has
+// them: up to a quarter slower.  The strips of a row tile then still share its blocks, but the blocks read side by side are no longer neighbours.)
 #include "../common/dtype.cuh"
 #include "../common/host_util.h"
 #include "../common/mma.cuh"
@@ -43,141 +46,175 @@ struct GemmRowsParams {
 };
 
 // weights are read once and never written while the library runs: around L1, and allowed ahead of the dependency wait
-__device__ __forceinline__ uint4 ldw16(const void* p) {
+__device__ __forceinline__ void copy16(uint32_t dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ uint4 lds16(uint32_t a) {
   uint4 v;
-  asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+  asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a) : "memory");
   return v;
 }
-__device__ __forceinline__ uint2 ldw8(const void* p) {
+__device__ __forceinline__ uint2 lds8(uint32_t a) {
   uint2 v;
-  asm volatile("ld.global.nc.L1::no_allocate.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p));
+  asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(a) : "memory");
+  return v;
+}
+__device__ __forceinline__ uint16_t lds2(uint32_t a) {
+  uint16_t v;
+  asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(a) : "memory");
   return v;
 }
 
-// What a lane holds of one k block of a strip: rows g and g + 8.
-template <int BITS> struct RowsA;
-template <> struct RowsA<16> { uint4 q[2][2]; };                    // [32-column half][row]
-template <> struct RowsA<8> { uint4 q[2]; };                        // [row]
-template <> struct RowsA<4> { uint2 q[2]; uint32_t s[2]; };         // [row]; s: scales of the two words, 16 bits each
+// Ring of a warp: `depth` blocks of weights, each `bytes` (of every accumulator) long: 16 rows of 64 columns, behind int4 up to four scales a row.
+template <int BITS, bool DUAL> struct RowsRing {
+  static constexpr int bytes = BITS == 16 ? 2048 : BITS == 8 ? 1024 : 512 + kRowsStrip * 8;
+  static constexpr int depth = (BITS == 16 ? 4 : 8) / (DUAL && BITS > 4 ? 2 : 1);
+  static constexpr int warp_bytes = depth * bytes * (DUAL ? 2 : 1);
+  static constexpr int total = warp_bytes * kRowsWarps;
+};
 
 template <typename T, int BITS, bool DUAL, int NT>
 __global__ void __launch_bounds__(kRowsWarps * 32, 2)
 gemm_rows_kernel(const GemmRowsParams p) {
+  using Ring = RowsRing<BITS, DUAL>;
   constexpr int kAcc = DUAL ? 2 : 1;
-  // Blocks of weights on their way per warp (2 KB of 16-bit values, 1 KB of int8, 0.5 KB of int4 each and accumulator).  x comes one block ahead
-  // and not with its weights: a warp waits for its loads on a handful of counters, and with x four blocks ahead as well, blocks began to wait for
-  // one another's (12 x 12288 x 4096 int8 SwiGLU 26.8 -> 33.3 us).
-  constexpr int U = BITS == 16 && DUAL ? 2 : 4;                     // even: the x ring of two turns with it
   constexpr int kPitch = kRowsStrip + 1;
+  extern __shared__ __align__(128) uint8_t ring_mem[];
   __shared__ float sums[2][kRowsWarps][kAcc][NT * 8][kPitch];
   __shared__ float squares[kRowsWarps][NT * 8];
   __shared__ float rstd[NT * 8];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
   const int KB = p.k_blocks, nk = (KB - warp + kRowsWarps - 1) / kRowsWarps;      // this warp's blocks of a strip: warp, warp + 8, ...
-  const int turns = (nk + U - 1) / U * U;                           // ... rounded up to whole turns of the ring
+  const uint32_t ring = smem_u32(ring_mem) + warp * Ring::warp_bytes;
   pdl_launch_dependents();
 
-  RowsA<BITS> a[U][kAcc];
-  // asks for block j of a strip, or past the strip's last turn for one of this CTA's next strip
-  auto ask = [&](RowsA<BITS> (&d)[kAcc], int strip, int j) {
-    if (j >= turns) { j -= turns; strip += gridDim.x; }
-    if (j >= nk || strip >= p.strips) return;
-    const int rt = strip >> 3, r0 = (strip & 7) * kRowsStrip;       // 128-row tile, first row inside it
+  // the next block to ask for: block aj of strip `as`, into slot `aslot`; one group per call, also behind the last block
+  int as = blockIdx.x, aj = 0, aslot = 0;
+  auto ask = [&] {
+    if (nk > 0 && as < p.strips) {
+      const int rt = as >> 3, r0 = (as & 7) * kRowsStrip;           // 128-row tile, first row inside it
 #pragma unroll
-    for (int c = 0; c < kAcc; ++c) {
-      const uint8_t* blk = p.w + ((size_t)(rt + c * p.dual_tiles) * KB + warp + j * kRowsWarps) * p.blk_bytes;
+      for (int c = 0; c < kAcc; ++c) {
+        const uint8_t* blk = p.w + ((size_t)(rt + c * p.dual_tiles) * KB + warp + aj * kRowsWarps) * p.blk_bytes;
+        const uint32_t dst = ring + (uint32_t)((aslot * kAcc + c) * Ring::bytes + lane * 16);
+        if constexpr (BITS == 16) {                                 // a lane copies what it will read: 16-byte pieces t and 4 + t of rows g and g + 8
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const int r = r0 + g + 8 * h;                               // r % 8 == g: the swizzle of 16-bit rows
-        if constexpr (BITS == 16) {
-          d[c].q[0][h] = ldw16(blk + r * 128 + ((t ^ g) << 4));
-          d[c].q[1][h] = ldw16(blk + r * 128 + (((4 + t) ^ g) << 4));
-        } else if constexpr (BITS == 8) {
-          d[c].q[h] = ldw16(blk + r * 64 + t * 16);
+          for (int h = 0; h < 2; ++h) {
+            const uint8_t* row = blk + (r0 + g + 8 * h) * 128;      // swizzled by row % 8 == g
+            copy16(dst + (0 + h) * 512, row + ((t ^ g) << 4));
+            copy16(dst + (2 + h) * 512, row + (((4 + t) ^ g) << 4));
+          }
+        } else if constexpr (BITS == 8) {                           // here too: lane 4 g + t has 16 values of rows g and g + 8
+          copy16(dst, blk + r0 * 64 + lane * 16);
+          copy16(dst + 512, blk + r0 * 64 + 512 + lane * 16);
         } else {
-          d[c].q[h] = ldw8(blk + r * 32 + t * 8);
-          const T* sr = reinterpret_cast<const T*>(blk + 4096) + r * p.ns;         // word w covers columns 8 w .. 8 w + 7
-          const T one = Num<T>::from_f(1.f);
-          const T s0 = p.ns ? sr[(2 * t) * p.ns >> 3] : one, s1 = p.ns ? sr[(2 * t + 1) * p.ns >> 3] : one;
-          d[c].s[h] = (uint32_t)*reinterpret_cast<const uint16_t*>(&s0) | ((uint32_t)*reinterpret_cast<const uint16_t*>(&s1) << 16);
+          copy16(dst, blk + r0 * 32 + lane * 16);
+          if (lane < 2 * p.ns) copy16(dst + 512, blk + 4096 + r0 * p.ns * 2 + lane * 16);
         }
       }
+      if (++aj == nk) { aj = 0; as += gridDim.x; }
+      if (++aslot == Ring::depth) aslot = 0;
     }
+    asm volatile("cp.async.commit_group;" ::: "memory");
   };
-  if (nk > 0) {
 #pragma unroll
-    for (int u = 0; u < U; ++u) ask(a[u], blockIdx.x, u);
-  }
+  for (int u = 0; u < Ring::depth; ++u) ask();
   pdl_wait();
 
   // x of a block: 16 values of token g of every group of eight, in two 16-byte pieces that match the weights' k order
   const T* x = reinterpret_cast<const T*>(p.x);
-  uint4 xb[2][NT][2];
-  auto load_x = [&](int j, uint4 (&d)[NT][2]) {
+  uint4 xn[NT][2];
+  auto load_x = [&](int j) {
 #pragma unroll
     for (int n = 0; n < NT; ++n) {
       const int tok = n * 8 + g;
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
         const int k = (warp + j * kRowsWarps) * kRowsBK + (BITS == 16 ? (h * 4 + t) * 8 : t * 16 + h * 8);
-        d[n][h] = make_uint4(0u, 0u, 0u, 0u);
-        if (tok < p.M && k < p.K) d[n][h] = *reinterpret_cast<const uint4*>(x + (size_t)tok * p.ldx + k);
+        xn[n][h] = make_uint4(0u, 0u, 0u, 0u);
+        if (tok < p.M && k < p.K) xn[n][h] = *reinterpret_cast<const uint4*>(x + (size_t)tok * p.ldx + k);
       }
     }
   };
+  if (nk > 0) load_x(0);
+  const int tok = tid >> 4, r = tid & 15;        // the value that this thread finishes in every strip
+  const T* bias = reinterpret_cast<const T*>(p.bias);
+  const T* scale = reinterpret_cast<const T*>(p.scale);
+  const T* resid = reinterpret_cast<const T*>(p.residual);
+  const float row_scale = p.row_scale && tok < p.M ? p.row_scale[tok] : 1.f;
   float sq[NT] = {};
-  int buf = 0;
+  int buf = 0, slot = 0;
   for (int strip = blockIdx.x; strip < p.strips; strip += gridDim.x, buf ^= 1) {
     const bool first = strip == (int)blockIdx.x;
+    // what the epilogue adds and multiplies by is asked for ahead of the products
+    const int n_out = strip * kRowsStrip + r;
+    const bool mine = tok < p.M && n_out < p.N;
+    const T one = Num<T>::from_f(1.f), zero = Num<T>::from_f(0.f);
+    T sc[2] = {one, one}, bi[2] = {zero, zero}, re = zero;
+    if (mine) {
+      if (scale) { sc[0] = scale[n_out]; if (DUAL) sc[1] = scale[p.dual_offset + n_out]; }
+      if (bias) { bi[0] = bias[n_out]; if (DUAL) bi[1] = bias[p.dual_offset + n_out]; }
+      if (resid) re = resid[(size_t)tok * p.ldr + n_out];
+    }
     float acc[kAcc][NT][4] = {};
-    if (nk > 0) load_x(0, xb[0]);
-    for (int j = 0; j < turns; j += U) {
+    for (int j = 0; j < nk; ++j) {
+      uint4 b[NT][2];
 #pragma unroll
-      for (int u = 0; u < U; ++u) {
-        if (j + u < nk) {
-          if (j + u + 1 < nk) load_x(j + u + 1, xb[(u + 1) & 1]);
-          const auto& b = xb[u & 1];
-          if (p.norm && first) {
+      for (int n = 0; n < NT; ++n) { b[n][0] = xn[n][0]; b[n][1] = xn[n][1]; }
+      load_x(j + 1 < nk ? j + 1 : 0);            // x is the same for every strip
+      asm volatile("cp.async.wait_group %0;" ::"n"(Ring::depth - 1) : "memory");
+      if constexpr (BITS == 4) __syncwarp();     // its pieces were copied by other lanes
+      if (p.norm && first) {
 #pragma unroll
-            for (int n = 0; n < NT; ++n)
+        for (int n = 0; n < NT; ++n)
 #pragma unroll
-              for (int h = 0; h < 2; ++h) {
-                float f[8];
-                unpack8<T>(b[n][h], f);
+          for (int h = 0; h < 2; ++h) {
+            float f[8];
+            unpack8<T>(b[n][h], f);
 #pragma unroll
-                for (int i = 0; i < 8; ++i) sq[n] = fmaf(f[i], f[i], sq[n]);
-              }
+            for (int i = 0; i < 8; ++i) sq[n] = fmaf(f[i], f[i], sq[n]);
           }
-          const RowsA<BITS> (&w)[kAcc] = a[u];
+      }
 #pragma unroll
-          for (int c = 0; c < kAcc; ++c) {
+      for (int c = 0; c < kAcc; ++c) {
+        const uint32_t src = ring + (uint32_t)((slot * kAcc + c) * Ring::bytes);
+        uint4 q[2];
+        uint2 q4[2];
+        if constexpr (BITS == 8) { q[0] = lds16(src + lane * 16); q[1] = lds16(src + 512 + lane * 16); }
+        if constexpr (BITS == 4) { q4[0] = lds8(src + lane * 8); q4[1] = lds8(src + 256 + lane * 8); }
 #pragma unroll
-            for (int h = 0; h < 2; ++h) {
-              uint4 lo, hi;                                         // eight values along k of row g, of row g + 8
-              if constexpr (BITS == 16) {
-                lo = w[c].q[h][0];
-                hi = w[c].q[h][1];
-              } else if constexpr (BITS == 8) {
-                lo = widen_i8x8<T>(h ? make_uint2(w[c].q[0].z, w[c].q[0].w) : make_uint2(w[c].q[0].x, w[c].q[0].y));
-                hi = widen_i8x8<T>(h ? make_uint2(w[c].q[1].z, w[c].q[1].w) : make_uint2(w[c].q[1].x, w[c].q[1].y));
-              } else {
-                const uint16_t s0 = (uint16_t)(w[c].s[0] >> (16 * h)), s1 = (uint16_t)(w[c].s[1] >> (16 * h));
-                const T t0 = *reinterpret_cast<const T*>(&s0), t1 = *reinterpret_cast<const T*>(&s1);
-                const uint32_t q0 = h ? w[c].q[0].y : w[c].q[0].x, q1 = h ? w[c].q[1].y : w[c].q[1].x;
-                lo = p.fp4 ? widen_e2m1x8<T>(q0, t0) : widen_i4x8<T>(q0, t0);
-                hi = p.fp4 ? widen_e2m1x8<T>(q1, t1) : widen_i4x8<T>(q1, t1);
-              }
-              const uint32_t a01[4] = {lo.x, hi.x, lo.y, hi.y}, a23[4] = {lo.z, hi.z, lo.w, hi.w};
+        for (int h = 0; h < 2; ++h) {
+          uint4 lo, hi;                                             // eight values along k of row g, of row g + 8
+          if constexpr (BITS == 16) {
+            lo = lds16(src + (2 * h) * 512 + lane * 16);
+            hi = lds16(src + (2 * h + 1) * 512 + lane * 16);
+          } else if constexpr (BITS == 8) {
+            lo = widen_i8x8<T>(h ? make_uint2(q[0].z, q[0].w) : make_uint2(q[0].x, q[0].y));
+            hi = widen_i8x8<T>(h ? make_uint2(q[1].z, q[1].w) : make_uint2(q[1].x, q[1].y));
+          } else {
+            T s[2] = {one, one};                                    // word w of a row covers columns 8 w .. 8 w + 7
+            if (p.ns) {
 #pragma unroll
-              for (int n = 0; n < NT; ++n) {
-                MmaOp<T>::mma(acc[c][n], a01, b[n][h].x, b[n][h].y);
-                MmaOp<T>::mma(acc[c][n], a23, b[n][h].z, b[n][h].w);
+              for (int row = 0; row < 2; ++row) {
+                const uint16_t bits = lds2(src + 512 + (uint32_t)((g + 8 * row) * p.ns + ((2 * t + h) * p.ns >> 3)) * 2);
+                s[row] = *reinterpret_cast<const T*>(&bits);
               }
             }
+            const uint32_t w0 = h ? q4[0].y : q4[0].x, w1 = h ? q4[1].y : q4[1].x;
+            lo = p.fp4 ? widen_e2m1x8<T>(w0, s[0]) : widen_i4x8<T>(w0, s[0]);
+            hi = p.fp4 ? widen_e2m1x8<T>(w1, s[1]) : widen_i4x8<T>(w1, s[1]);
+          }
+          const uint32_t a01[4] = {lo.x, hi.x, lo.y, hi.y}, a23[4] = {lo.z, hi.z, lo.w, hi.w};
+#pragma unroll
+          for (int n = 0; n < NT; ++n) {
+            MmaOp<T>::mma(acc[c][n], a01, b[n][h].x, b[n][h].y);
+            MmaOp<T>::mma(acc[c][n], a23, b[n][h].z, b[n][h].w);
           }
         }
-        ask(a[u], strip, j + u + U);
       }
+      if constexpr (BITS == 4) __syncwarp();
+      ask();                                     // into the slot just read
+      if (++slot == Ring::depth) slot = 0;
     }
     // ---- the warps' sums: token rows of 16 features; two buffers, so one rendezvous per strip is enough
 #pragma unroll
@@ -204,35 +241,24 @@ gemm_rows_kernel(const GemmRowsParams p) {
       }
       __syncthreads();
     }
-    const T* bias = reinterpret_cast<const T*>(p.bias);
-    const T* scale = reinterpret_cast<const T*>(p.scale);
-    const T* resid = reinterpret_cast<const T*>(p.residual);
-    for (int i = tid; i < p.M * kRowsStrip; i += kRowsWarps * 32) {
-      const int tok = i >> 4, r = i & 15, n = strip * kRowsStrip + r;
-      if (n >= p.N) continue;
+    if (mine) {
       float gate = 0.f, up = 0.f;
 #pragma unroll
       for (int w = 0; w < kRowsWarps; ++w) {
         gate += sums[buf][w][0][tok][r];
         if (DUAL) up += sums[buf][w][kAcc - 1][tok][r];
       }
-      float rs = p.norm ? rstd[tok] : 1.f;
-      if (p.row_scale) rs *= p.row_scale[tok];
+      const float rs = p.norm ? rstd[tok] * row_scale : row_scale;
       gate *= rs;
       up *= rs;
-      if (scale) {
-        gate *= Num<T>::to_f(scale[n]);
-        if (DUAL) up *= Num<T>::to_f(scale[p.dual_offset + n]);
-      }
-      if (bias) {
-        gate += Num<T>::to_f(bias[n]);
-        if (DUAL) up += Num<T>::to_f(bias[p.dual_offset + n]);
-      }
+      if (scale) { gate *= Num<T>::to_f(sc[0]); up *= Num<T>::to_f(sc[1]); }
+      if (bias) { gate += Num<T>::to_f(bi[0]); up += Num<T>::to_f(bi[1]); }
       float v = apply_act(p.act, gate, up, p.act_args);
-      if (resid) v += Num<T>::to_f(resid[(size_t)tok * p.ldr + n]);
-      reinterpret_cast<T*>(p.out)[(size_t)tok * p.ldo + n] = Num<T>::from_f(v);
+      if (resid) v += Num<T>::to_f(re);
+      reinterpret_cast<T*>(p.out)[(size_t)tok * p.ldo + n_out] = Num<T>::from_f(v);
     }
   }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
 }
 
 // ------------------------------------------------------------------ host side ----
@@ -241,17 +267,19 @@ static int rows_limit() {
   return v >= 0 ? std::min(v, 16) : 16;
 }
 
-// Shapes this kernel takes: see the table at the top of the file.  What it saves is the fixed part of a launch; what it pays are an uneven last
-// round (a third more strips than places) and long walks along K by few warps.  Quantised weights, widened in registers instead of through
-// shared memory, win at every size.
+// Shapes this kernel takes.  Quantised weights, widened in registers instead of through the warps of another kernel, and GLU pairs win at every size
+// (fp16, us, this kernel / gemm_tc.cu: 16 x 12288 x 4096 SwiGLU 35.4 / 35.9, 16 x 9728 x 2560 21.7 / 22.3).  Up to 8 rows what it pays is x, which
+// every CTA reads, on long rows (8 x 2560 x 9728 13.3 / 14.0, 4 x 4096 x 12288 19.0 / 19.8, 8 x 4096 x 12288 20.8 / 20.0).  With 9 to 16 rows the
+// products are twice as many, and long rows and an uneven last round of strips lose (16 x 4096 x 4096 9.2 / 10.5, 16 x 2560 x 4096 8.0 / 8.7;
+// 16 x 6144 x 4096 14.7 / 13.5, 16 x 6144 x 2560 10.5 / 9.8, 16 x 2048 x 8192 12.2 / 11.7).
 bool gemm_rows_takes(const RfGemm* g) {
   if (g->M > rows_limit() || !g->w_packed || g->ar_world > 1 || g->streaming_only == 2 || g->ss_out || g->mul || g->force_splits || g->force_bn || g->force_swap >= 0)
     return false;
   if ((reinterpret_cast<uintptr_t>(g->x) & 15) != 0) return false;
   if (g->w_int8) return true;
-  const bool dual = g->dual_offset > 0;
-  const int64_t values = (int64_t)g->N * g->K * (dual ? 2 : 1);
-  return values <= (8 << 20) || (g->K <= 4096 && g->N <= 2 * kRowsStrip * sm_count() && !dual) || (dual && g->M <= 8 && g->K <= (g->M <= 2 ? 4096 : 2048));
+  if (g->dual_offset > 0) return true;
+  if (g->M <= 8) return (int64_t)g->M * g->K <= (80 << 10);
+  return (int64_t)g->N * g->K <= (8 << 20) || (g->K <= 4096 && g->N <= 2 * kRowsStrip * sm_count());
 }
 
 template <typename T, int BITS, bool DUAL, int NT>
@@ -269,7 +297,9 @@ static int launch_rows(const RfGemm* g, cudaStream_t stream) {
   p.norm = g->ss_in != nullptr;
   p.inv_dim = g->ss_dim > 0 ? 1.f / (float)g->ss_dim : 0.f;
   p.eps = g->ss_eps;
-  RF_CUDA_CHECK(::rf::launch_k(kfn, dim3(std::min(p.strips, 2 * sm_count())), dim3(kRowsWarps * 32), 0, stream, 1, p));
+  constexpr int smem = RowsRing<BITS, DUAL>::total;
+  RF_ALLOW_SMEM_PER_DEVICE(kfn, smem);
+  RF_CUDA_CHECK(::rf::launch_k(kfn, dim3(std::min(p.strips, 2 * sm_count())), dim3(kRowsWarps * 32), smem, stream, 1, p));
   ::rf::count_launch();
   return RF_OK;
 }

@@ -1496,9 +1496,12 @@ static int run_gemm(const RfGemm* g, cudaStream_t stream, bool w8) {
   int rc = check_gemm(g);
   if (rc) return rc;
   if (g->mul) RF_REQUIRE(!w8 && g->mul_row && rf::gemm_small_eligible(g), "GEMM %dx%dx%d has no gate-by-token epilogue (see rf_gemm_takes_mul)", g->M, g->N, g->K);
-  if (!w8 && rf::gemm_small_eligible(g)) return rf::gemm_small_run(g, stream);      // latency-bound shapes: gemm_small.cu
+  const bool rows = rf::gemm_rows_takes(g);
+  // latency-bound shapes: gemm_small.cu, but for very few rows (fp16, us, gemm_rows.cu / gemm_small.cu: 1 x 4096 x 1024 3.1 / 7.8,
+  // 8 x 1024 x 3072 4.4 / 7.0, 16 x 2048 x 2048 4.7 / 8.4)
+  if (!w8 && !rows && rf::gemm_small_eligible(g)) return rf::gemm_small_run(g, stream);
   if (!w8 && rf::gemm_sk_eligible(g, nullptr)) return rf::launch_gemm_sk(g, stream);
-  if (rf::gemm_rows_takes(g)) return rf::launch_gemm_rows(g, stream);
+  if (rows) return rf::launch_gemm_rows(g, stream);
   GemmPlan pl;
   rc = plan_gemm(g, &pl);
   if (rc) return rc;

@@ -975,7 +975,7 @@ def test_gemm_very_few_rows(dt, M, N, K, dual, status):
 
 @pytest.mark.parametrize("dt", DT)
 @pytest.mark.parametrize("M", [1, 8, 11, 16])
-@pytest.mark.parametrize("N,K,group,fp4", [(264, 320, 0, False), (1000, 1024, 64, False), (40, 2176, 32, False), (128, 192, 16, True), (5008, 512, None, False)])
+@pytest.mark.parametrize("N,K,group,fp4", [(264, 320, 0, False), (1000, 1024, 64, False), (40, 2176, 32, False), (128, 192, 16, True), (5008, 512, None, False), (24, 4672, 0, False), (40, 4672, 32, False)])
 @pytest.mark.parametrize("dual", [False, True])
 def test_gemm_very_few_rows_quantised(dt, M, N, K, group, fp4, dual, status):
     """Up to 16 rows over int8 (``group`` None) and 4-bit weights, against the product with the values that the image holds."""
