@@ -136,7 +136,7 @@ __global__ void __launch_bounds__(256) qk_norm_rope_kv_vec_kernel(const RfRopeKv
   // asked for before anything is waited for: the first head's row, the positions, the sequence
   const int h_first = first + lane / GROUP;
   uint4 ahead = *reinterpret_cast<const uint4*>(row + (size_t)(h_first < heads ? h_first : 0) * HD + o);
-  const int pos0 = a.pos[(size_t)tok * a.pos_stride];
+  const int pos0 = a.pos ? a.pos[(size_t)tok * a.pos_stride] : 0;      // norms and insertion by cache_pos need no positions
   const int seq = a.k_pool && a.seq_of_tok ? a.seq_of_tok[tok] : tok;
   const int cpos = a.k_pool && a.cache_pos ? a.cache_pos[tok] : pos0;
   int page = -1;
@@ -258,6 +258,7 @@ extern "C" int rf_qk_norm_rope_kv(const RfRopeKv* a, rf_stream_t stream) {
              "rope_kv: head_dim %d / rot_dim %d", a->hd, a->rot_dim);
   RF_REQUIRE(a->pos_stride >= 1, "rope_kv: pos_stride");
   if (a->k_pool) RF_REQUIRE(a->v_pool && a->page_table && a->hd % 8 == 0, "rope_kv: KV pool arguments");
+  RF_REQUIRE(a->pos || !((a->cos && a->rot_dim > 0) || (a->k_pool && !a->cache_pos)), "rope_kv: rotation, and insertion without cache_pos, need positions");
   if (a->tokens == 0) return RF_OK;
   const int heads = a->Hq + 2 * a->Hkv;
   int warps = heads < 8 ? heads : 8;

@@ -1125,3 +1125,36 @@ def test_attn_decode_rows_of_a_sequence(dt, hd, Hq, Hkv, rows, lens, status):
         ref = ref.transpose(0, 1).reshape(rows, Hq * hd)
         _close(out[at], ref, dt)
         _close(whole[at], ref, dt)
+
+
+@pytest.mark.parametrize("dt", DT)
+@pytest.mark.parametrize("hd,T", [(64, 3), (128, 77), (128, 600), (80, 5)])
+def test_rope_kv_without_positions(dt, hd, T):
+    """Norm and page insertion by ``cache_pos`` alone: no tables, no positions (a null pointer), on the 16-byte and the scalar kernel."""
+    import ctypes as C
+    from rhinoforge_b200 import _native as N
+    from rhinoforge_b200.ops import kernels as K_
+    Hq, Hkv = 3, 2
+    qkv = torch.randn(T, (Hq + 2 * Hkv) * hd, device="cuda").to(dt)
+    w = (1 + 0.1 * torch.randn(hd, device="cuda")).to(dt)
+    pt = torch.arange((T + 15) // 16 + 1, dtype=torch.int32, device="cuda").flip(0).contiguous()[None]
+    seq, cpos = torch.zeros(T, dtype=torch.int32, device="cuda"), torch.arange(T, dtype=torch.int32, device="cuda")
+    got = []
+    for pos in (None, cpos):
+        rows = qkv.clone()
+        pools = torch.zeros(2, pt.shape[1], Hkv, 16, hd, device="cuda", dtype=dt)
+        a = N.RfRopeKv()
+        a.qkv, a.ld, a.tokens, a.Hq, a.Hkv, a.hd, a.rot_dim = rows.data_ptr(), rows.stride(0), T, Hq, Hkv, hd, 0
+        a.q_norm_w, a.k_norm_w, a.eps, a.dtype = w.data_ptr(), w.data_ptr(), 1e-6, K_.dtype_code(dt)
+        a.pos, a.pos_stride = None if pos is None else pos.data_ptr(), 1
+        a.k_pool, a.v_pool, a.page_table, a.pt_stride = pools[0].data_ptr(), pools[1].data_ptr(), pt.data_ptr(), pt.stride(0)
+        a.seq_of_tok, a.cache_pos = seq.data_ptr(), cpos.data_ptr()
+        N.check(N.lib().rf_qk_norm_rope_kv(C.byref(a), C.c_void_p(torch.cuda.current_stream().cuda_stream)), "rf_qk_norm_rope_kv")
+        got.append((rows, pools))
+    assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
+    x = qkv.view(T, -1, hd).float()
+    ref = w.float() * (x[:, :Hq + Hkv] * torch.rsqrt(x[:, :Hq + Hkv].pow(2).mean(-1, keepdim=True) + 1e-6)).to(dt).float()
+    at = lambda pool: pool[pt[0][(cpos // 16).long()].long(), :, (cpos % 16).long()]
+    _close(got[0][0].view(T, -1, hd)[:, :Hq], ref[:, :Hq], dt, scale=3.0)
+    _close(at(got[0][1][0]), ref[:, Hq:], dt, scale=3.0)
+    assert torch.equal(at(got[0][1][1]), qkv.view(T, -1, hd)[:, Hq + Hkv:])
