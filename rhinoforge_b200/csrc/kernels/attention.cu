@@ -818,6 +818,8 @@ extern "C" int rf_attn_decode(const RfAttn* a, rf_stream_t stream) {
   if (rc) return rc;
   RF_REQUIRE(a->num_seqs <= 65535 && (int64_t)a->num_seqs * p.rows_per_seq <= 65535, "decode attention: %d x %d rows in one launch", a->num_seqs, p.rows_per_seq);
   RF_REQUIRE(p.rows_per_seq == 1 || !a->pos, "decode attention by row takes one row per sequence");
+  RF_REQUIRE(p.rows_per_seq == 1 || (int64_t)a->num_seqs * p.rows_per_seq == a->q_rows_total, "decode attention: %d sequences of %d rows are not the %d query rows",
+             a->num_seqs, p.rows_per_seq, a->q_rows_total);
   RF_REQUIRE(a->max_kv_len > 0, "decode attention needs max_kv_len");
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   RF_ATTN_DISPATCH(launch_decode)

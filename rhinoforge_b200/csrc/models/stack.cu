@@ -344,6 +344,10 @@ static int forward(Stack& s, const RfStackForward& f, cudaStream_t st) {
   RF_REQUIRE(f.hidden && f.tokens >= 0 && f.tokens <= c.max_tokens, "forward: %d tokens (max %d)", f.tokens, c.max_tokens);
   RF_REQUIRE(f.num_seqs > 0 && f.num_seqs <= c.max_seqs, "forward: %d sequences (max %d)", f.num_seqs, c.max_seqs);
   if (f.tokens == 0) return RF_OK;
+  if (f.decode && f.rows_per_seq > 1) {
+    RF_REQUIRE((int64_t)f.num_seqs * f.rows_per_seq == f.tokens, "forward: %d sequences of %d rows are not the %d tokens", f.num_seqs, f.rows_per_seq, f.tokens);
+    RF_REQUIRE(c.gdn_Hv == 0, "forward: recurrent layers decode one row per sequence (got %d)", f.rows_per_seq);
+  }
   if (c.norm_kind == RF_NORM_ADARMS) RF_REQUIRE(f.mod && f.rows_per_mod > 0, "adaRMS stack needs mod");
   const int T = f.tokens, H = c.hidden, QD = s.qkv_dim(), AD = c.Hq * c.hd, I = c.inter;
   const int lb = f.layer_end > 0 ? f.layer_begin : 0, le = f.layer_end > 0 ? f.layer_end : c.layers;

@@ -135,7 +135,7 @@ typedef struct RfStackForward {
   // [twin_split, tokens) through its twin set (rf_stack_set_twin_layer).  0: no routing.  The caller orders the rows
   // accordingly; positions, cache rows and the attention mask are per row, so the order is free.
   int32_t twin_split;
-  int32_t rows_per_seq;                    // decode: query rows of every sequence (0: 1), which all see its kv_len keys
+  int32_t rows_per_seq;                    // decode: query rows of every sequence (0: 1), which all see its kv_len keys (attention layers only)
 } RfStackForward;
 
 int64_t rf_stack_create(const RfStackConfig* cfg);

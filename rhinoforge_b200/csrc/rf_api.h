@@ -265,7 +265,8 @@ typedef struct RfAttn {
   // chunk or window leaves of everything up to itself; kv_len is not used and num_seqs counts rows.
   const int32_t* seq_of_row; const int32_t* pos;
   int32_t vd;               // size of a value head (0: hd); contiguous rows with hd = 192 take 128, out is [rows, Hq * vd]
-  int32_t rows_per_seq;     // rf_attn_decode: query rows of every sequence (0: 1), rows [s * n, (s + 1) * n), all of which see its kv_len keys
+  int32_t rows_per_seq;     // rf_attn_decode: query rows of every sequence (0: 1), rows [s * n, (s + 1) * n), all of which see its kv_len keys;
+                            // q_rows_total is their number, num_seqs * n
 } RfAttn;
 int rf_attn_prefill(const RfAttn* a, rf_stream_t stream);
 int rf_attn_decode(const RfAttn* a, rf_stream_t stream);

@@ -463,6 +463,8 @@ def attention_decode(q: torch.Tensor, out: torch.Tensor, *, Hq: int, Hkv: int, h
                      scale: float = 0.0, ws: Optional[torch.Tensor] = None,
                      status: Optional[torch.Tensor] = None, rows_per_seq: int = 1) -> torch.Tensor:
     """One query token (``rows_per_seq`` that all see the sequence's keys) per sequence against the paged KV pool (split-KV when ``ws`` is given)."""
+    if rows_per_seq < 1 or q.shape[0] % rows_per_seq:
+        raise ValueError(f"{q.shape[0]} query rows are no whole number of sequences of {rows_per_seq}")
     a = N.RfAttn()
     a.q, a.ldq, a.out, a.ldo = q.data_ptr(), q.stride(0), out.data_ptr(), out.stride(0)
     a.q_rows_total = q.shape[0]
