@@ -663,7 +663,8 @@ class DecoderEngine:
         for j, (s, off, cnt) in enumerate(ch):
             base = starts[s]
             meta[:, j] = torch.tensor((o, cnt, base + off + cnt, slots[s], o + cnt - 1, int(base + off == 0)), dtype=torch.int32)
-            table[j, :pages] = self.cache._pt_host[slots[s]]
+            row = self.cache._pt_host[slots[s]]
+            table[j, :pages], table[j, pages:] = row, row[-1]          # a whole block of keys is fetched up to the row's end: a page there too
             tokmeta[0, o:o + cnt] = j
             tokmeta[1, o:o + cnt] = torch.arange(base + off, base + off + cnt, dtype=torch.int32)
             tokmeta[2, o:o + cnt] = prompts[s][off:off + cnt].to("cpu", torch.int32)
