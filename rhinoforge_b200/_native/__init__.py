@@ -47,7 +47,7 @@ class RfGemm(C.Structure):
         ("ss_out", C.c_void_p), ("ss_in", C.c_void_p), ("ss_ld", C.c_int32), ("ss_dim", C.c_int32),
         ("ss_eps", C.c_float), ("streaming_only", C.c_int32),
         ("mul", C.c_void_p), ("mul_row", C.c_void_p), ("mul_ld", C.c_int64),
-        ("act_limit", C.c_float), ("act_alpha", C.c_float),
+        ("act_limit", C.c_float), ("act_alpha", C.c_float), ("norm_x", C.c_int32),
     ]
 
 

@@ -1415,6 +1415,7 @@ static int check_gemm(const RfGemm* g) {
     if (g->ss_in) RF_REQUIRE(g->ss_tiles > 0 && g->ss_dim > 0, "ss_in needs ss_tiles and ss_dim");
     if (g->ss_out) RF_REQUIRE(g->ar_world <= 1, "ss_out is not available together with the fused all-reduce");
   }
+  if (g->norm_x) RF_REQUIRE(!g->ss_in && g->ss_dim > 0, "norm_x needs ss_dim and goes without ss_in");
   if (g->w_bits == 4) {
     RF_REQUIRE(g->w_int8 && g->w_packed, "int4 weights come as the tile-major image (w_int8 = 1, w_packed = 1)");
     RF_REQUIRE(g->w_group == 0 || g->w_group == 32 || g->w_group == 64 || g->w_group == 128 || (g->w_fp4 && g->w_group == 16),
@@ -1497,6 +1498,10 @@ static int run_gemm(const RfGemm* g, cudaStream_t stream, bool w8) {
   if (rc) return rc;
   if (g->mul) RF_REQUIRE(!w8 && g->mul_row && rf::gemm_small_eligible(g), "GEMM %dx%dx%d has no gate-by-token epilogue (see rf_gemm_takes_mul)", g->M, g->N, g->K);
   const bool rows = rf::gemm_rows_takes(g);
+  if (g->norm_x) {                    // no other kernel takes the squares of x
+    RF_REQUIRE(rows, "GEMM %dx%dx%d does not take the squares of its rows itself (see rf_gemm_takes_norm)", g->M, g->N, g->K);
+    return rf::launch_gemm_rows(g, stream);
+  }
   // latency-bound shapes: gemm_small.cu, but for very few rows (fp16, us, gemm_rows.cu / gemm_small.cu: 1 x 4096 x 1024 3.1 / 7.8,
   // 8 x 1024 x 3072 4.4 / 7.0, 16 x 2048 x 2048 4.7 / 8.4)
   if (!w8 && !rows && rf::gemm_small_eligible(g)) return rf::gemm_small_run(g, stream);
@@ -1543,6 +1548,8 @@ static int run_gemm(const RfGemm* g, cudaStream_t stream, bool w8) {
 }
 
 extern "C" int rf_gemm_takes_mul(const RfGemm* g) { return g && check_gemm(g) == RF_OK && !g->w_int8 && rf::gemm_small_eligible(g); }
+
+extern "C" int rf_gemm_takes_norm(const RfGemm* g) { return g && check_gemm(g) == RF_OK && rf::gemm_rows_takes(g); }
 
 extern "C" int rf_gemm_plan_info(const RfGemm* g, int32_t* out) {
   RF_REQUIRE(g && out, "rf_gemm_plan_info: null argument");

@@ -156,6 +156,7 @@ extern "C" int rf_gemv(const RfGemm* g, rf_stream_t stream) {
              "gemv K=%d / pitches must be multiples of %d", g->K, vec);
   RF_REQUIRE(!g->w_int8 || g->scale, "int8 weights need a scale vector");
   RF_REQUIRE(g->ar_world <= 1, "gemv has no fused all-reduce");
+  RF_REQUIRE(!g->norm_x, "gemv does not take the squares of its rows");
   RF_REQUIRE(act_is_dual(g->act) == (g->dual_offset > 0), "dual_offset and an activation of two operands go together");
   GemvParams p;
   p.x = g->x; p.ldx = g->ldx; p.w = g->w; p.ldw = g->ldw; p.out = g->out; p.ldo = g->ldo;

@@ -19,8 +19,6 @@
 
 namespace rf {
 
-bool gemm_rows_takes(const RfGemm* g);      // gemm_rows.cu
-
 struct Stack {
   RfStackConfig cfg;
   std::vector<RfLayerWeights> layers;
@@ -170,20 +168,23 @@ static void hint_next_weights(const Stack& s, const void* w, const void* scale, 
 }
 
 // Folded RMSNorm wiring of the next linear() call on this thread (set by the layer loop right before the call, consumed
-// by it): the buffer it writes its per-tile sums of squares to, and / or the buffer whose sums give its row scale.
+// by it): the buffer it writes its per-tile sums of squares to, and / or where its row scale comes from: a buffer of such sums, or the
+// squares of its input that the kernel takes itself.
 static thread_local float* t_ss_out = nullptr;
 static thread_local const float* t_ss_in = nullptr;
+static thread_local bool t_norm_x = false;
 
-// Whether a linear layer of these sizes will run on the kernel that takes the squares of its input rows itself (gemm_rows.cu): then nobody
-// has to write their sums for it.
+// Whether a linear layer of these sizes can take the squares of its input rows itself: then nobody has to write their sums for it, and it is
+// told so (t_norm_x), so that a GEMM which would need sums after all is refused and does not read those of an earlier call.
 static bool norms_itself(const Stack& s, const void* x, int M, int N, int K, int dual_offset) {
   RfGemm g = {};
-  g.x = x;
-  g.M = M; g.N = N; g.K = K; g.dtype = s.cfg.dtype; g.dual_offset = dual_offset;
+  g.x = x; g.ldx = K;
+  g.w = g.out = reinterpret_cast<void*>(4096);      // placeholders: alignment is all that is looked at
+  g.M = M; g.N = N; g.K = K; g.dtype = s.cfg.dtype; g.dual_offset = dual_offset; g.act = dual_offset > 0 ? kActSiluMul : kActNone;
   g.w_packed = s.cfg.weights_packed;
   g.force_swap = -1;
   g.streaming_only = s.cfg.gemm_streaming_only ? (s.cfg.tp_world > 1 ? 2 : 1) : 0;
-  return s.cfg.tp_world <= 1 && gemm_rows_takes(&g);
+  return s.cfg.tp_world <= 1 && rf_gemm_takes_norm(&g);
 }
 
 // One linear layer: picks GEMV / tcgen05 GEMM / W8A16 and wires the fused all-reduce.  pub_ctas != null asks for
@@ -213,10 +214,10 @@ static int linear(const Stack& s, const void* x, int64_t ldx, const void* w, con
   g.streaming_only = s.cfg.gemm_streaming_only ? (s.cfg.tp_world > 1 ? 2 : 1) : 0;
   g.prefetch = t_pf_ptr; g.prefetch_bytes = t_pf_bytes;
   t_pf_ptr = nullptr; t_pf_bytes = 0;
-  if (t_ss_out || t_ss_in) {
-    g.ss_out = t_ss_out; g.ss_in = t_ss_in;
+  if (t_ss_out || t_ss_in || t_norm_x) {
+    g.ss_out = t_ss_out; g.ss_in = t_ss_in; g.norm_x = t_norm_x;
     g.ss_ld = s.ss_ld; g.ss_tiles = s.ss_tiles; g.ss_dim = s.cfg.hidden; g.ss_eps = s.cfg.eps;
-    t_ss_out = nullptr; t_ss_in = nullptr;
+    t_ss_out = nullptr; t_ss_in = nullptr; t_norm_x = false;
   }
   g.ws = s.at<float>(s.off_sk_ws); g.ws_bytes = s.sk_ws_bytes;
   g.sem = s.at<uint32_t>(s.off_sk_flags); g.sem_count = Stack::kSkFlags;
@@ -383,7 +384,8 @@ static int forward(Stack& s, const RfStackForward& f, cudaStream_t st) {
   }
   float* ss_attn = s.at<float>(s.off_ss);                               // sums of squares of hidden after attention
   float* ss_mlp = ss_attn + (size_t)s.ss_tiles * s.ss_ld;               // ... after the MLP (the next layer's input)
-  bool ss_ready = false;    // ss_mlp describes f.hidden as it is now
+  bool ss_ready = false;    // the next layer's QKV GEMM can take its first norm: from ss_mlp, or
+  bool qkv_norms = false;   // ... from the squares of f.hidden itself
 
   for (int l = lb; l < le; ++l) {
     const RfLayerWeights& w = s.layers[l];
@@ -439,7 +441,10 @@ static int forward(Stack& s, const RfStackForward& f, cudaStream_t st) {
       mix_dim = VD;
     } else {
     hint_next_weights(s, w.wo, w.so, H, AD, 1, T);
-    if (qkv_from_hidden) t_ss_in = ss_mlp;
+    if (qkv_from_hidden) {
+      if (qkv_norms) t_norm_x = true;
+      else t_ss_in = ss_mlp;
+    }
     if (twin)
       rc = linear_twin(s, xn, H, w.wqkv, w.sqkv, w.bqkv, tw->wqkv, tw->sqkv, tw->bqkv, wide, QD, nullptr, 0, T, split, QD, H,
                        kActNone, 0, st);
@@ -517,13 +522,14 @@ static int forward(Stack& s, const RfStackForward& f, cudaStream_t st) {
     // residual) and the separate gated-residual launch disappears.
     const bool fuse_gate = c.gated_residual && !c.sandwich_norm && f.rows_per_mod >= T && !c.weights_int8 &&
                            c.tp_world == 1 && f.mod != nullptr;
+    const bool up_norms = fuse_ss && norms_itself(s, f.hidden, T, I, H, s.glu() ? I : 0);
     hint_next_weights(s, w.w_up, w.s_up, s.glu() ? 2 * (int64_t)I : I, H, s.glu() ? 2 : 1, T);
     if (twin) {
       rc = linear_twin(s, mix_out, mix_dim, w.wo, w.so, w.bo, tw->wo, tw->so, tw->bo, f.hidden, H, f.hidden, H, T, split, H,
                        mix_dim, kActNone, 0, st);
       if (rc) return rc;
     } else if (!side) {
-      if (fuse_ss && !norms_itself(s, f.hidden, T, I, H, s.glu() ? I : 0)) t_ss_out = ss_attn;
+      if (fuse_ss && !up_norms) t_ss_out = ss_attn;
       rc = linear_ar(s, mix_out, mix_dim, w.wo, w.so, w.bo, f.hidden, f.hidden, T, mix_dim,
                      norm_rides ? w.norm2_w : nullptr, xn, &have_xn2, st, /*rows_stay=*/true);
       if (rc) return rc;
@@ -573,7 +579,8 @@ static int forward(Stack& s, const RfStackForward& f, cudaStream_t st) {
       if (rc) return rc;
     }
     hint_next_weights(s, w.w_down, w.s_down, H, I, 1, T);
-    if (fuse_ss) t_ss_in = ss_attn;
+    if (up_norms) t_norm_x = true;
+    else if (fuse_ss) t_ss_in = ss_attn;
     if (twin)
       rc = linear_twin(s, xn, H, w.w_up, w.s_up, w.b_up, tw->w_up, tw->s_up, tw->b_up, wide, I, nullptr, 0, T, split, I, H,
                        act_of(c.mlp_kind), s.glu() ? I : 0, st);
@@ -590,7 +597,8 @@ static int forward(Stack& s, const RfStackForward& f, cudaStream_t st) {
     const void* next_w = (norm_rides && l + 1 < le && !hook_after) ? s.layers[l + 1].norm1_w : nullptr;
     if (l + 1 < le && s.layers[l + 1].mixer != 1) hint_next_weights(s, s.layers[l + 1].wqkv, s.layers[l + 1].sqkv, QD, H, 1, T);
     if (fuse_ss && l + 1 < le && !hook_after) {
-      if (!norms_itself(s, f.hidden, T, QD, H, 0)) t_ss_out = ss_mlp;
+      qkv_norms = norms_itself(s, f.hidden, T, QD, H, 0);
+      if (!qkv_norms) t_ss_out = ss_mlp;
       ss_ready = true;
     }
     if (twin) {

@@ -100,6 +100,9 @@ typedef struct RfGemm {
   // mul[mul_row[m] * mul_ld + n] (same dtype), a slice of an embedding table.
   const void* mul; const int32_t* mul_row; int64_t mul_ld;
   float act_limit, act_alpha;  // constants of the activations that have some (rf::ActArgs)
+  // 1: the result is scaled per token by rsqrt(sum of squares of its K values of x / ss_dim + ss_eps), which the kernel takes itself: a folded
+  // RMSNorm like ss_in's, without anybody's sums.  Only for GEMMs for which rf_gemm_takes_norm returns 1; others are refused.
+  int32_t norm_x;
 } RfGemm;
 // bytes of the tile-major image of a [rows, K] weight with `sections` equal row sections
 uint64_t rf_pack_weight_bytes(int64_t rows, int64_t K, int32_t sections, int32_t elem_bytes);
@@ -109,6 +112,7 @@ int32_t rf_w4_block_bytes(int32_t group);
 
 int rf_gemm(const RfGemm* g, rf_stream_t stream);
 int rf_gemm_takes_mul(const RfGemm* g);   // host-only: can this GEMM apply RfGemm.mul in its epilogue?
+int rf_gemm_takes_norm(const RfGemm* g);  // host-only: can this GEMM take the squares of its rows of x itself (RfGemm.norm_x)?
 // Launch plan of a shape without launching: out[10] = {swap, bn, splits, stages, grid_x, grid_y, smem bytes, k_blocks,
 // persistent kernel, two-shot all-reduce}.  Host-only.
 int rf_gemm_plan_info(const RfGemm* g, int32_t* out);

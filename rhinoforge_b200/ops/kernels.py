@@ -86,7 +86,7 @@ def gemm(x: torch.Tensor, w: torch.Tensor, *, out: Optional[torch.Tensor] = None
          norm_eps: float = 1e-6, norm_gemma: bool = False, w_bits: int = 0, w_group: int = 0,
          w_fp4: bool = False, ss_out: Optional[torch.Tensor] = None, ss_in: Optional[torch.Tensor] = None,
          ss_dim: int = 0, ss_eps: float = 1e-6, mul: Optional[torch.Tensor] = None,
-         mul_row: Optional[torch.Tensor] = None, limit: float = 0.0, alpha: float = 0.0) -> torch.Tensor:
+         mul_row: Optional[torch.Tensor] = None, limit: float = 0.0, alpha: float = 0.0, norm_x: bool = False) -> torch.Tensor:
     """``out = epilogue(x @ w.T)`` on the tcgen05 kernel (or the CUDA-core GEMV).
 
     ``dual=True``: ``w`` stacks ``[gate; up]`` (2N rows) and ``act`` is a ``*_mul``
@@ -104,7 +104,8 @@ def gemm(x: torch.Tensor, w: torch.Tensor, *, out: Optional[torch.Tensor] = None
     ``ss_out`` (fp32 ``[ceil(N / 128), ld >= M]``, at most 256 rows): also receives the sum of squares of the finished
     output values per 128-column tile and token.  ``ss_in`` (the ``ss_out`` of the GEMM that produced ``x``): the result
     is scaled per token by ``rsqrt(sum(ss_in[:, token]) / ss_dim + ss_eps)``: an RMSNorm of ``x`` whose weights were
-    multiplied into the columns of ``w`` beforehand.
+    multiplied into the columns of ``w`` beforehand.  ``norm_x``: the same with the squares of ``x`` that the kernel takes itself (at most
+    16 rows over packed weights; other GEMMs refuse it).
     ``mul`` / ``mul_row`` (few rows, small weights): row ``m`` of the activated result is multiplied by ``mul[mul_row[m], :N]``.
     ``limit`` / ``alpha``: constants of ``act="clipped_glu"`` (``dual``) and ``"soft_cap"`` (``limit``).
     """
@@ -147,6 +148,8 @@ def gemm(x: torch.Tensor, w: torch.Tensor, *, out: Optional[torch.Tensor] = None
         g.ss_out = ss_out.data_ptr()
     if ss_in is not None:
         g.ss_in, g.ss_tiles, g.ss_dim, g.ss_eps = ss_in.data_ptr(), ss_in.shape[0], ss_dim or K, ss_eps
+    if norm_x:
+        g.norm_x, g.ss_dim, g.ss_eps = 1, ss_dim or K, ss_eps
     g.force_splits, g.force_swap, g.force_bn = force_splits, force_swap, force_bn
     if mul is not None:
         g.mul, g.mul_row, g.mul_ld = mul.data_ptr(), _i32(mul_row), mul.stride(0)

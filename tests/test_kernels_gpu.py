@@ -1158,3 +1158,29 @@ def test_rope_kv_without_positions(dt, hd, T):
     _close(got[0][0].view(T, -1, hd)[:, :Hq], ref[:, :Hq], dt, scale=3.0)
     _close(at(got[0][1][0]), ref[:, Hq:], dt, scale=3.0)
     assert torch.equal(at(got[0][1][1]), qkv.view(T, -1, hd)[:, Hq + Hkv:])
+
+
+@pytest.mark.parametrize("dt", DT)
+@pytest.mark.parametrize("M", [1, 8, 11, 16, 17, 40])
+@pytest.mark.parametrize("dual", [False, True])
+def test_gemm_scaled_by_given_sums_or_by_its_own_squares(dt, M, dual, status):
+    """``ss_in`` scales by the caller's sums at every row count, whatever x holds; ``norm_x`` by the squares of x, where there is a kernel for it."""
+    from rhinoforge_b200.ops import kernels as K_
+    N, K = 264, 640
+    rows = 2 * N if dual else N
+    x = (torch.randn(M, K, device="cuda") * 0.5).to(dt)
+    w = (torch.randn(rows, K, device="cuda") / K ** 0.5).to(dt)
+    wp = K_.pack_weight(w, 2 if dual else 1)
+    kw = dict(packed_shape=(rows, K), status=status, **(dict(act="silu_mul", dual=True) if dual else {}))
+    finish = lambda z: torch.nn.functional.silu(z[:, :N]) * z[:, N:] if dual else z
+    z = x.float() @ w.float().t()
+    sums = torch.rand(5, M + 3, device="cuda") * 40 + 1.0                   # nothing to do with x
+    rstd = torch.rsqrt(sums[:, :M].sum(0) / 200 + 1e-5)
+    ref = finish(z * rstd[:, None])
+    _close(K_.gemm(x, wp, ss_in=sums, ss_dim=200, ss_eps=1e-5, **kw), ref, dt, scale=max(1.0, ref.abs().max().item()))
+    own = finish(z * torch.rsqrt(x.float().pow(2).sum(1, keepdim=True) / 200 + 1e-5))
+    if M <= 16:
+        _close(K_.gemm(x, wp, norm_x=True, ss_dim=200, ss_eps=1e-5, **kw), own, dt, scale=max(1.0, own.abs().max().item()))
+    else:
+        with pytest.raises(Exception, match="squares of its rows"):
+            K_.gemm(x, wp, norm_x=True, ss_dim=200, ss_eps=1e-5, **kw)
