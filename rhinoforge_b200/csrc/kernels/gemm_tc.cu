@@ -1493,25 +1493,39 @@ int launch_gemm_ps(const RfGemm* g, cudaStream_t stream);
 int widen_packed(const void* src, void* dst, int64_t blocks, int dtype, cudaStream_t stream);   // gemm_ps.cu
 }
 
-static int run_gemm(const RfGemm* g, cudaStream_t stream, bool w8) {
-  int rc = check_gemm(g);
-  if (rc) return rc;
+// Which kernel a checked GEMM runs on (RF_GEMM_*), and where that is one of the tcgen05 tile kernels its plan.
+static int route_gemm(const RfGemm* g, int* kernel, GemmPlan* pl) {
+  const bool w8 = g->w_int8 != 0;
   if (g->mul) RF_REQUIRE(!w8 && g->mul_row && rf::gemm_small_eligible(g), "GEMM %dx%dx%d has no gate-by-token epilogue (see rf_gemm_takes_mul)", g->M, g->N, g->K);
   const bool rows = rf::gemm_rows_takes(g);
   if (g->norm_x) {                    // no other kernel takes the squares of x
     RF_REQUIRE(rows, "GEMM %dx%dx%d does not take the squares of its rows itself (see rf_gemm_takes_norm)", g->M, g->N, g->K);
-    return rf::launch_gemm_rows(g, stream);
+    *kernel = RF_GEMM_ROWS;
+    return RF_OK;
   }
   // latency-bound shapes: gemm_small.cu, but for very few rows (fp16, us, gemm_rows.cu / gemm_small.cu: 1 x 4096 x 1024 3.1 / 7.8,
   // 8 x 1024 x 3072 4.4 / 7.0, 16 x 2048 x 2048 4.7 / 8.4)
-  if (!w8 && !rows && rf::gemm_small_eligible(g)) return rf::gemm_small_run(g, stream);
-  if (!w8 && rf::gemm_sk_eligible(g, nullptr)) return rf::launch_gemm_sk(g, stream);
-  if (rows) return rf::launch_gemm_rows(g, stream);
-  GemmPlan pl;
-  rc = plan_gemm(g, &pl);
+  if (!w8 && !rows && rf::gemm_small_eligible(g)) { *kernel = RF_GEMM_SMALL; return RF_OK; }
+  if (!w8 && rf::gemm_sk_eligible(g, nullptr)) { *kernel = RF_GEMM_STREAM_K; return RF_OK; }
+  if (rows) { *kernel = RF_GEMM_ROWS; return RF_OK; }
+  const int rc = plan_gemm(g, pl);
   if (rc) return rc;
-  if (!w8 && g->force_splits == 0 && g->force_bn == 0 && rf::gemm_ps_eligible(g, pl.swap != 0, pl.splits, pl.bn, pl.grid_x * pl.grid_y))
-    return rf::launch_gemm_ps(g, stream);
+  *kernel = !w8 && g->force_splits == 0 && g->force_bn == 0 && rf::gemm_ps_eligible(g, pl->swap != 0, pl->splits, pl->bn, pl->grid_x * pl->grid_y)
+                ? RF_GEMM_PERSISTENT : RF_GEMM_TILE;
+  return RF_OK;
+}
+
+static int run_gemm(const RfGemm* g, cudaStream_t stream, bool w8) {
+  int rc = check_gemm(g);
+  if (rc) return rc;
+  int kernel;
+  GemmPlan pl;
+  rc = route_gemm(g, &kernel, &pl);
+  if (rc) return rc;
+  if (kernel == RF_GEMM_SMALL) return rf::gemm_small_run(g, stream);
+  if (kernel == RF_GEMM_STREAM_K) return rf::launch_gemm_sk(g, stream);
+  if (kernel == RF_GEMM_ROWS) return rf::launch_gemm_rows(g, stream);
+  if (kernel == RF_GEMM_PERSISTENT) return rf::launch_gemm_ps(g, stream);
   if (w8 && g->w_bits != 4 && !pl.swap && g->M > 256 && g->w_packed && g->w_scratch && g->force_splits == 0 && g->force_bn == 0) {
     // Large token counts are compute-bound: widen the int8 weight image once into the caller's scratch (a pass
     // over the weights costs a few per cent of the GEMM) and run the 16-bit kernels, whose main loop has no
@@ -1550,6 +1564,15 @@ static int run_gemm(const RfGemm* g, cudaStream_t stream, bool w8) {
 extern "C" int rf_gemm_takes_mul(const RfGemm* g) { return g && check_gemm(g) == RF_OK && !g->w_int8 && rf::gemm_small_eligible(g); }
 
 extern "C" int rf_gemm_takes_norm(const RfGemm* g) { return g && check_gemm(g) == RF_OK && rf::gemm_rows_takes(g); }
+
+extern "C" int rf_gemm_kernel(const RfGemm* g) {
+  int rc = check_gemm(g);
+  if (rc) return rc;
+  int kernel;
+  GemmPlan pl;
+  rc = route_gemm(g, &kernel, &pl);
+  return rc ? rc : kernel;
+}
 
 extern "C" int rf_gemm_plan_info(const RfGemm* g, int32_t* out) {
   RF_REQUIRE(g && out, "rf_gemm_plan_info: null argument");

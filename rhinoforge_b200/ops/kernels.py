@@ -50,13 +50,15 @@ def _splitk_scratch(device: torch.device, ws_bytes: int, sems: int):
     return ws, sem
 
 
+GEMM_KERNELS = ("tile", "persistent", "stream_k", "rows", "small")        # RF_GEMM_* of rf_api.h
 GEMM_PLAN_KEYS = ("swap", "bn", "splits", "stages", "grid_x", "grid_y", "smem", "k_blocks", "persistent", "two_shot")
 
 
 def gemm_plan(M: int, N_out: int, K: int, *, dtype: torch.dtype = torch.float16, dual: bool = False, packed: bool = True,
               int8: bool = False, force_splits: int = 0) -> Optional[dict]:
     """The launch plan the library would pick for ``[M, K] x [N_out, K]^T`` - swap-AB, tile width, K splits, ring stages,
-    grid, shared memory, persistent / two-shot form.  A host-side query (no device, no launch); ``None`` when the native
+    grid, shared memory, persistent / two-shot form - and ``kernel``, the family that runs (of :data:`GEMM_KERNELS`; the other entries are the
+    plan of the tcgen05 tile kernels, which only ``tile`` and ``persistent`` launch).  A host-side query (no device, no launch); ``None`` when the native
     library is not built."""
     if not N.available():
         return None
@@ -72,7 +74,7 @@ def gemm_plan(M: int, N_out: int, K: int, *, dtype: torch.dtype = torch.float16,
     out = (C.c_int32 * len(GEMM_PLAN_KEYS))()
     if N.lib().rf_gemm_plan_info(C.byref(g), out) != 0:
         return None
-    return dict(zip(GEMM_PLAN_KEYS, (int(v) for v in out)))
+    return dict(zip(GEMM_PLAN_KEYS, (int(v) for v in out)), kernel=GEMM_KERNELS[N.lib().rf_gemm_kernel(C.byref(g))])
 
 
 def gemm(x: torch.Tensor, w: torch.Tensor, *, out: Optional[torch.Tensor] = None,
