@@ -9,7 +9,8 @@
 //    (int4), all neighbours along k.  mma.sync does not care which k a slot stands for as long as both operands agree, so the lane's
 //    words are the A fragments as they come, and the same k range of token g is the B fragment: no shuffles, and no meeting of warps.
 //    int8 and int4 are widened in registers on the way.
-//  * Four to eight blocks of weights per warp (64 KB a CTA, two CTAs an SM) are on their way in the warp's ring, over the ends of strips too; the
+//  * Four to eight blocks of weights per warp (two of a 16-bit and four of an int8 GLU pair; 64 KB a CTA, 40 of int4 and 70 to 80 of an
+//    int4 pair; two CTAs an SM) are on their way in the warp's ring, over the ends of strips too; the
 //    first ones are asked for ahead of the dependency wait.  cp.async, and not loads into registers: a warp waits for its loads on a handful of
 //    counters, and with weights and x on the same ones every block waited for the newest (12 x 151936 x 4096 int8 215 us in registers, 160 now;
 //    1 x 12288 x 4096 int8 SwiGLU 24.7 / 18.2).  Each lane copies what it will read; only int4 blocks, 512 bytes, are shared by the warp.
@@ -21,7 +22,7 @@
 // fp16, us, this kernel / gemm_tc.cu: 1 x 4096 x 1024 3.1 / 5.7, 1 x 1024 x 2048 3.0 / 5.5, 8 x 2048 x 2048 4.1 / 6.2, 1 x 6144 x 4096 10.5 / 12.9,
 // 1 x 4096 x 12288 17.0 / 19.5, 16 x 3072 x 2048 5.1 / 6.6, 16 x 4096 x 4096 9.2 / 10.5; SwiGLU 1 x 12288 x 4096 31.5 / 35.3 (30.3 at the copy
 // rate), 16 x 8192 x 2048 13.9 / 15.2.  int8: 1 x 4096 x 4096 6.3 / 11.9, 12 x 12288 x 4096 SwiGLU 24.0 / 44.4, 12 x 151936 x 4096 160 / 242; int4:
-// 12 x 12288 x 4096 SwiGLU 38.5 / 52.8, 12 x 4096 x 12288 18.7 / 29.4.  (Row tiles that start their k blocks at different places, as gemm_tc.cu has
+// 12 x 12288 x 4096 SwiGLU 31.7 / 52.8, 12 x 4096 x 12288 18.7 / 29.4.  (Row tiles that start their k blocks at different places, as gemm_tc.cu has
 // them: up to a quarter slower.  The strips of a row tile then still share its blocks, but the blocks read side by side are no longer neighbours.)
 #include "../common/dtype.cuh"
 #include "../common/host_util.h"
@@ -68,9 +69,11 @@ __device__ __forceinline__ uint16_t lds2(uint32_t a) {
 }
 
 // Ring of a warp: `depth` blocks of weights, each `bytes` (of every accumulator) long: 16 rows of 64 columns, behind int4 up to four scales a row.
-template <int BITS, bool DUAL> struct RowsRing {
+template <int BITS, bool DUAL, int NT> struct RowsRing {
   static constexpr int bytes = BITS == 16 ? 2048 : BITS == 8 ? 1024 : 512 + kRowsStrip * 8;
-  static constexpr int depth = (BITS == 16 ? 4 : 8) / (DUAL && BITS > 4 ? 2 : 1);
+  // an int4 pair of 9 to 16 rows, whose sums take 34 KB: seven, so that a second CTA fits (fp16, us, with eight / seven: 12 x 12288 x 4096
+  // SwiGLU, scales of 64 columns, 38.7 / 31.7, 16 x 9728 x 2560 23.3 / 17.4)
+  static constexpr int depth = DUAL ? (BITS == 16 ? 2 : BITS == 8 ? 4 : NT == 1 ? 8 : 7) : (BITS == 16 ? 4 : 8);
   static constexpr int warp_bytes = depth * bytes * (DUAL ? 2 : 1);
   static constexpr int total = warp_bytes * kRowsWarps;
 };
@@ -78,13 +81,14 @@ template <int BITS, bool DUAL> struct RowsRing {
 template <typename T, int BITS, bool DUAL, int NT>
 __global__ void __launch_bounds__(kRowsWarps * 32, 2)
 gemm_rows_kernel(const GemmRowsParams p) {
-  using Ring = RowsRing<BITS, DUAL>;
+  using Ring = RowsRing<BITS, DUAL, NT>;
   constexpr int kAcc = DUAL ? 2 : 1;
   constexpr int kPitch = kRowsStrip + 1;
   extern __shared__ __align__(128) uint8_t ring_mem[];
   __shared__ float sums[2][kRowsWarps][kAcc][NT * 8][kPitch];
   __shared__ float squares[kRowsWarps][NT * 8];
   __shared__ float rstd[NT * 8];
+  static_assert(2 * (Ring::total + sizeof(sums) + sizeof(squares) + sizeof(rstd) + 1024) <= 228 * 1024, "two CTAs have to fit an SM");
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
   const int KB = p.k_blocks, nk = (KB - warp + kRowsWarps - 1) / kRowsWarps;      // this warp's blocks of a strip: warp, warp + 8, ...
   const uint32_t ring = smem_u32(ring_mem) + warp * Ring::warp_bytes;
@@ -304,7 +308,7 @@ static int launch_rows(const RfGemm* g, cudaStream_t stream) {
   p.ss_in = g->ss_in; p.ss_tiles = g->ss_tiles; p.ss_ld = g->ss_ld;
   p.inv_dim = g->ss_dim > 0 ? 1.f / (float)g->ss_dim : 0.f;
   p.eps = g->ss_eps;
-  constexpr int smem = RowsRing<BITS, DUAL>::total;
+  constexpr int smem = RowsRing<BITS, DUAL, NT>::total;
   RF_ALLOW_SMEM_PER_DEVICE(kfn, smem);
   RF_CUDA_CHECK(::rf::launch_k(kfn, dim3(std::min(p.strips, 2 * sm_count())), dim3(kRowsWarps * 32), smem, stream, 1, p));
   ::rf::count_launch();
