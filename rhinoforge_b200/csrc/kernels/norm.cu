@@ -132,7 +132,7 @@ __global__ void layernorm_kernel(const T* __restrict__ x, const T* __restrict__ 
 
 // Many rows: a warp per row that holds it in registers, 16-byte pieces 256 values apart, all of them on their way at once; nothing but shuffles
 // between the two passes.  The kernels above keep the row in shared memory (eight-way bank conflicts) and meet at three to six block barriers,
-// which few rows hide no worse.  us, before / now: LayerNorm 3072 x 1152 9.0 / 6.8, 6000 x 2048 25.3 / 15.5; RMSNorm 5400 x 4096 31.5 / 21.6, 768 x 1152 4.4 / 3.3.
+// which a block per row hides as long as an SM has few rows (warp_pieces has the line).  us, block / warp: LayerNorm 3072 x 1152 9.0 / 6.8, 6000 x 2048 25.3 / 15.5; RMSNorm 5400 x 4096 31.5 / 21.6, 768 x 1152 4.4 / 3.3.
 template <typename T, int NC>
 __global__ void __launch_bounds__(128)
 rmsnorm_warp_kernel(const T* __restrict__ x, const T* __restrict__ residual, const T* __restrict__ w, T* __restrict__ y,
@@ -241,9 +241,16 @@ layernorm_warp_kernel(const T* __restrict__ x, const T* __restrict__ w, const T*
   }
 }
 
-// 256-value pieces of a row that the warp kernels hold (0: the row is too long, or the rows are too few to fill the GPU with a warp each)
-static int warp_pieces(int rows, int H) {
-  if (rows < 2 * sm_count() || H > 4096) return 0;
+// 256-value pieces of a row that the warp kernels hold, 0: a block per row.  A warp takes its row alone, so it needs several rows per SM to hide
+// its chain, and more of them the longer the row: above 1536 values the block kernels have twice the threads, and a second row (residual) or the
+// modulation (`extra`) leaves room for fewer warps.  LayerNorm's block form meets at twice the barriers.  fp16, us, block / warp: LayerNorm
+// 296 x 1024 2.6 / 2.9, 400 x 1152 3.6 / 3.3, 768 x 1152 5.6 / 4.0, 768 x 2048 5.9 / 6.2, 1500 x 4096 13.2 / 9.1; RMSNorm 296 x 4096 3.3 / 8.2,
+// 400 x 768 2.3 / 2.5, 768 x 1536 5.1 / 3.9, 768 x 4096 7.7 / 9.2, 1500 x 2560 8.2 / 7.1, 3072 x 3072 14.6 / 9.1; with a residual 768 x 1152
+// 5.7 / 4.4, 1500 x 2048 7.9 / 9.4, 3072 x 2048 14.0 / 11.2, 6000 x 4096 49.5 / 57.1; modulated 768 x 1152 4.9 / 3.7, 1500 x 2048 7.2 / 8.6,
+// 3072 x 2048 12.3 / 10.0.
+static int warp_pieces(int rows, int H, bool layer, bool extra, bool residual) {
+  const int per_two_sms = layer && H <= 1152 ? 5 : H <= 1536 ? 10 : extra ? 40 : 20;
+  if (2 * rows < per_two_sms * sm_count() || H > (residual ? 3072 : 4096)) return 0;
   const int nc = ceil_div(H, 256);
   return nc <= 4 ? 4 : nc <= 5 ? 5 : nc <= 8 ? 8 : nc <= 12 ? 12 : 16;
 }
@@ -316,7 +323,7 @@ extern "C" int rf_rmsnorm(const void* x, const void* residual, const void* w, vo
   const size_t smem = (size_t)(H + 32) * sizeof(float);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (rows_per_mod <= 0) rows_per_mod = 1;
-  if (const int nc = warp_pieces(rows, H)) {
+  if (const int nc = warp_pieces(rows, H, false, residual || mod, residual != nullptr)) {
     auto run = [&](auto kNC, auto zero) -> cudaError_t {
       using T = decltype(zero);
       return ::rf::launch_k(rmsnorm_warp_kernel<T, decltype(kNC)::value>, dim3(ceil_div(rows, 4)), dim3(128), 0, s, 1, (const T*)x, (const T*)residual, (const T*)w,
@@ -348,7 +355,7 @@ extern "C" int rf_layernorm(const void* x, const void* w, const void* b, void* y
   const int threads = H >= 2048 ? 256 : 128;
   const size_t smem = (size_t)(H + 32) * sizeof(float);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (const int nc = warp_pieces(rows, H)) {
+  if (const int nc = warp_pieces(rows, H, true, false, false)) {
     auto run = [&](auto kNC, auto zero) -> cudaError_t {
       using T = decltype(zero);
       return ::rf::launch_k(layernorm_warp_kernel<T, decltype(kNC)::value>, dim3(ceil_div(rows, 4)), dim3(128), 0, s, 1, (const T*)x, (const T*)w, (const T*)b,

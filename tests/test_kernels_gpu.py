@@ -1034,10 +1034,10 @@ def test_attn_prefill_two_tiles(dt, hd, Hq, Hkv, mode, status):
 
 @pytest.mark.parametrize("dt", DT)
 @pytest.mark.parametrize("H", [8, 264, 1024, 1152, 2040, 3072, 4096, 4104])
-@pytest.mark.parametrize("rows", [295, 1301])
+@pytest.mark.parametrize("rows", [295, 1301, 3001])
 def test_norms_of_many_rows(dt, H, rows):
-    """A warp per row (296 rows and more, up to 4096 values): rows that end inside a piece, a last block with idle warps, residual and modulation,
-    pitched rows, in place - and one size past each end of that range on the block kernels."""
+    """A warp per row (by rows per SM, length and operands, up to 4096 values): rows that end inside a piece, a last block with idle warps, residual
+    and modulation, pitched rows, in place - and sizes past each end of that range on the block kernels."""
     from rhinoforge_b200.ops import kernels as K_
     x = torch.randn(rows, H, device="cuda").to(dt)
     r = torch.randn(rows, H, device="cuda").to(dt)
