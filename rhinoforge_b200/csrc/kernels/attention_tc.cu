@@ -513,8 +513,10 @@ template <typename T, int HD, int VD = HD>
 static int launch_prefill_tc_t(const RfAttn* a, const AttnParams& p, cudaStream_t s) {
   if constexpr (HD <= 128) {
     // Two tiles to a CTA where that still makes about one CTA per SM and the tiles have more than a few blocks to share (12 x 256 rows and keys,
-    // 16 heads of 128: 47 us with two tiles, 42 with one)
-    if (a->max_q_len > 2 * kFaRows && 4l * ceil_div(a->max_q_len, 2 * kFaRows) * a->Hq * a->num_seqs >= 3l * sm_count())
+    // 16 heads of 128: 47 us with two tiles, 42 with one).  Not under masks by data, whose blocks are bound by the tests behind every score: there
+    // two CTAs of one tile hide each other's loads of the mask, and a sequence's odd last tile does not leave half an SM idle (12 x 300, 16 + 4
+    // heads of 64, boolean mask: 53.6 us with two tiles, 39.2 with one).
+    if (!a->mask && !a->seg_q && a->max_q_len > 2 * kFaRows && 4l * ceil_div(a->max_q_len, 2 * kFaRows) * a->Hq * a->num_seqs >= 3l * sm_count())
       return launch_prefill_tc_n<T, HD, VD, 2>(a, p, s);
   }
   return launch_prefill_tc_n<T, HD, VD, 1>(a, p, s);
