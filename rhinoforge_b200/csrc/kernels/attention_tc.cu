@@ -365,6 +365,24 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
           sv[i] = __float_as_uint(x);
           mx4[i & 3] = fmaxf(mx4[i & 3], x);
         }
+      } else if (mrow == nullptr && p.seg_q != nullptr) {
+        // segment ids alone: a lane fetches those of two keys and the warp hands them round (a load behind every key's range test: 1 x 1024 rows,
+        // 16 + 4 heads of 64, 153 us, 30.4 so)
+        int sk[KVB / 32];
+#pragma unroll
+        for (int c = 0; c < KVB / 32; ++c) {
+          const int tk = t0 + c * 32 + lane;
+          sk[c] = tk < kvlen ? p.seg_k[kv0 + tk] : 0;
+        }
+        const uint64_t bits = bits_from(lo_row - t0) & ~bits_from(hi_row - t0 + 1);
+        const uint32_t w32[2] = {(uint32_t)bits, (uint32_t)(bits >> 32)};
+#pragma unroll
+        for (int i = 0; i < KVB; ++i) {
+          const bool same = __shfl_sync(0xffffffffu, sk[i >> 5], i & 31) == sq;
+          const float x = same && (w32[i >> 5] & (1u << (i & 31))) ? __uint_as_float(sv[i]) * score_mul : -INFINITY;
+          sv[i] = __float_as_uint(x);
+          mx4[i & 3] = fmaxf(mx4[i & 3], x);
+        }
       } else {
 #pragma unroll
         for (int i = 0; i < KVB; ++i) {

@@ -1184,3 +1184,29 @@ def test_gemm_scaled_by_given_sums_or_by_its_own_squares(dt, M, dual, status):
     else:
         with pytest.raises(Exception, match="squares of its rows"):
             K_.gemm(x, wp, norm_x=True, ss_dim=200, ss_eps=1e-5, **kw)
+
+
+@pytest.mark.parametrize("dt", DT)
+@pytest.mark.parametrize("hd,Hq,Hkv", [(64, 4, 2), (128, 8, 2), (256, 2, 1)])
+@pytest.mark.parametrize("mode", ["full", "causal", "window"])
+def test_attn_prefill_scattered_segments(dt, hd, Hq, Hkv, mode, status):
+    """Segment ids in no order over sequences that end inside a block of keys, with keys ahead of the new rows, under causal and window masks too."""
+    from rhinoforge_b200.ops import kernels as K_
+    q_lens, kv_lens = [150, 1, 65, 290], [150, 70, 129, 300]
+    i32 = lambda l: torch.tensor(l, dtype=torch.int32, device="cuda")
+    starts = lambda lens: [sum(lens[:i]) for i in range(len(lens))]
+    q = torch.randn(sum(q_lens), Hq * hd, device="cuda").to(dt)
+    k, v = (torch.randn(sum(kv_lens), Hkv * hd, device="cuda").to(dt) for _ in range(2))
+    seg_k = torch.randint(0, 4, (sum(kv_lens),), dtype=torch.int32, device="cuda")
+    seg_q = torch.cat([seg_k[s + n - m:s + n] for s, n, m in zip(starts(kv_lens), kv_lens, q_lens)]).contiguous()      # a row sees itself
+    out = K_.attention_prefill(q, torch.zeros_like(q), Hq=Hq, Hkv=Hkv, hd=hd, q_start=i32(starts(q_lens)), q_len=i32(q_lens), kv_len=i32(kv_lens),
+                               max_q_len=max(q_lens), k=k, v=v, kv_start=i32(starts(kv_lens)), causal=mode != "full", window=70 if mode == "window" else 0,
+                               seg_q=seg_q, seg_k=seg_k, status=status)
+    for a, b, m, n in zip(starts(q_lens), starts(kv_lens), q_lens, kv_lens):
+        i, j = torch.arange(m, device="cuda")[:, None] + (n - m), torch.arange(n, device="cuda")[None]
+        mask = seg_q[a:a + m, None] == seg_k[None, b:b + n]
+        if mode != "full":
+            mask = mask & (j <= i) & ((j > i - 70) | torch.tensor(mode == "causal", device="cuda"))
+        heads = lambda t, r0, r1: t[r0:r1].view(r1 - r0, -1, hd).transpose(0, 1)
+        ref = _sdpa_ref(heads(q, a, a + m), heads(k, b, b + n), heads(v, b, b + n), mask).transpose(0, 1).reshape(m, Hq * hd)
+        _close(out[a:a + m], ref, dt)
