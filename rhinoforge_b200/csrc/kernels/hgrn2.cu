@@ -684,10 +684,17 @@ extern "C" int rf_hgrn2_chunked(const RfHgrn2* a, rf_stream_t stream) {
   // Value channels per CTA: 64 as long as all CTAs are resident at once (two to an SM, one with more than 128 key channels) and a head is shared
   // by at most eight, then 128.  What a CTA does for the gates and the in-block scores does not depend on its channels, and two CTAs hide each
   // other's barriers.  bf16, heads of 128 x 128, us with 32 / 64 / 128 channels: 16 x 1100 tokens 265 / 248 / 290, 64 x 1100 306 / 329 / 408,
-  // 96 x 1100 579 / 336 / 482, 144 x 1000 752 / 307 / 456, 192 x 500 426 / 266 / 244.
+  // 96 x 1100 579 / 336 / 482, 144 x 1000 752 / 307 / 456, 192 x 500 426 / 266 / 244.  Up to 64 key channels a CTA has less to hide, and from one
+  // wave on the form that holds a head of 128 by itself, with no sums to exchange, is ahead: 96 x 300, 64 x 128 channels 75 with 64, 70 with 128.
+  // 32 channels for few heads, whose CTAs have their SMs to themselves: 8 x 1000 211 / 227, 12 x 300 65 / 70, 16 x 1000 252 / 227 (32 / 64); heads of
+  // 256 values 4 x 1000 210 / 225, 8 x 1000 236 / 229; as long as there is an SM for each with more than 128 key channels: 32 x 1000, 256 x 128
+  // 299 / 353.  Not where 64 hold the whole head: 8 x 1000, 128 x 64 211 / 185.
   int vt = a->vdim <= 32 ? 32 : a->vdim <= 64 ? 64 : 128;
-  const int halves = ceil_div(a->vdim, 64);
-  if (vt == 128 && halves <= 8 && (long)a->rows.num_seqs * a->heads * halves <= (a->dim <= 128 ? 2l : 1l) * sm_count()) vt = 64;
+  const int halves = ceil_div(a->vdim, 64), quarters = ceil_div(a->vdim, 32);
+  const long pairs = (long)a->rows.num_seqs * a->heads, sms = sm_count();
+  const bool two_to_an_sm = a->dim <= 128 && (a->dim > 64 || a->vdim > 128);
+  if (vt == 128 && halves <= 8 && pairs * halves <= (two_to_an_sm ? 2 : 1) * sms) vt = 64;
+  if (vt == 64 && quarters <= 8 && pairs * quarters <= (a->dim > 128 ? sms : a->vdim > 64 ? sms / 3 : 0)) vt = 32;
   const int tiles = ceil_div(a->vdim, vt);
   if (vt == 32) return launch_chunked<2>(a, tiles, s);
   if (vt == 64) return launch_chunked<4>(a, tiles, s);

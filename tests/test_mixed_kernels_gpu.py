@@ -235,10 +235,11 @@ def test_hgrn2_against_the_recurrence(dtype, chunked, heads, D, VD, vdim):
     torch.testing.assert_close(state.double().cpu(), want_state, rtol=1e-4, atol=1e-4)
 
 
-@pytest.mark.parametrize("heads,D,VD", [(20, 16, 72), (26, 16, 72), (26, 40, 128), (26, 136, 72)])
+@pytest.mark.parametrize("heads,D,VD", [(20, 16, 72), (26, 16, 72), (26, 40, 128), (26, 136, 72), (10, 16, 72), (20, 72, 72), (26, 72, 72), (2, 16, 72), (3, 16, 72),
+                                        (8, 136, 72), (9, 136, 72)])
 def test_hgrn2_portions_of_many_heads(heads, D, VD):
-    """The block form on both sides of the line where its CTAs of 64 value channels are more than the GPU holds at once (128 to a CTA then), against
-    the token-by-token kernel."""
+    """The block form on both sides of the lines where its CTAs take 32, 64 and 128 value channels (by heads and sequences, key channels and value
+    channels), against the token-by-token kernel."""
     lens, pos0, slots = [1, 40, 2, 16, 17, 33], [4, 0, 33, 64, 0, 9], [5, 2, 0, 1, 4, 6]
     d, _, _ = pack(lens, pos0, slots)
     g = torch.Generator().manual_seed(heads + D)
