@@ -730,11 +730,16 @@ static int launch_decode(const RfAttn* a, AttnParams& p, cudaStream_t s) {
   int splits = pl.splits;
   p.pages_per_split = pl.pages_per_split;
   // Up to eight splits are one cluster and merged inside the launch: the second kernel cost 2.2 us (1 x 300 keys) to 3.5 us (50 rows, heads of
-  // 256) behind every layer's attention.  Where so many clusters would not all be resident, fewer splits, down to half, are tried before the
-  // second kernel is taken (12 x 517 keys, 8 K/V heads: 3 splits and the second kernel 14.0 us, 2 splits 11.4).
+  // 256) behind every layer's attention.  Where so many clusters would not all be resident with a place to spare (56 clusters of five, which is
+  // every place, were put down in two rounds: 7 x 1500 keys 15.2 us with the second kernel, 17.4), fewer splits, down to half, are tried before the
+  // second kernel is taken (12 x 517 keys, 8 K/V heads: 3 splits and the second kernel 14.0 us, 2 splits 11.4) - unless a CTA has many pages and
+  // the busiest SM would read more than a fifth more of them (12 x 2000 23.4 / 24.1, 12 x 8000 68.5 / 80.4; 6 x 6000, 6 splits and 5, 31.1 / 28.2),
+  // with heads of 256, whose second kernel costs more, a fourth (one K/V head, 24 x 3000, 6 splits and 5, 25.1 / 22.5; 36 x 3000, 4 and 3, 31.6 / 33.1).
+  auto busiest = [&](int n, int pages) { return (long)ceil_div(a->Hkv * p.g_tiles * a->num_seqs * n, sm_count()) * pages; };
   for (int n = splits; splits <= 8 && n > 1 && 2 * n >= splits; --n) {
     const int pages = n == splits ? pl.pages_per_split : round_up(ceil_div(pl.max_pages, n), 4), parts = ceil_div(pl.max_pages, pages);
-    if (parts > 1 && (long)a->Hkv * p.g_tiles * a->num_seqs <= clusters_resident<T, HD>(parts, smem)) {
+    if (n < splits && pages * HD > 48 * 128 && 15 * busiest(parts, pages) > (HD == 256 ? 19 : 18) * busiest(splits, pl.pages_per_split)) break;
+    if (parts > 1 && (long)a->Hkv * p.g_tiles * a->num_seqs < clusters_resident<T, HD>(parts, smem)) {
       p.cluster = 1;
       splits = parts;
       p.pages_per_split = pages;

@@ -1210,3 +1210,23 @@ def test_attn_prefill_scattered_segments(dt, hd, Hq, Hkv, mode, status):
         heads = lambda t, r0, r1: t[r0:r1].view(r1 - r0, -1, hd).transpose(0, 1)
         ref = _sdpa_ref(heads(q, a, a + m), heads(k, b, b + n), heads(v, b, b + n), mask).transpose(0, 1).reshape(m, Hq * hd)
         _close(out[a:a + m], ref, dt)
+
+
+@pytest.mark.parametrize("dt", DT)
+@pytest.mark.parametrize("n,kv,Hq,Hkv,hd", [(8, 500, 16, 8, 128), (12, 500, 16, 8, 128), (12, 3900, 16, 8, 128), (7, 1500, 16, 8, 128), (9, 2100, 8, 8, 64),
+                                            (24, 1400, 8, 1, 256), (3, 4100, 4, 1, 256), (40, 333, 40, 2, 128)])
+def test_attn_decode_split_plans(dt, n, kv, Hq, Hkv, hd, status):
+    """Batches whose splits fit as clusters, as fewer or smaller clusters, and not (second kernel), with ragged and nearly empty sequences: against the
+    unsplit kernel at every sequence and against fp32 at three."""
+    from rhinoforge_b200.ops import kernels as K_
+    lens = [max(1, kv - 37 * (i * i % 29)) if i % 5 else kv for i in range(n - 1)] + [3]
+    k_pool, v_pool, pt, ks, vs = _paged(Hkv, hd, lens, dt)
+    q = torch.randn(n, Hq * hd, device="cuda").to(dt)
+    kw = dict(Hq=Hq, Hkv=Hkv, hd=hd, kv_len=torch.tensor(lens, dtype=torch.int32, device="cuda"), max_kv_len=kv, k_pool=k_pool, v_pool=v_pool, page_table=pt,
+              status=status)
+    out = K_.attention_decode(q, torch.full_like(q, float("nan")), ws=K_.attn_decode_scratch(n, Hq, hd, "cuda"), **kw)
+    whole = K_.attention_decode(q, torch.full_like(q, float("nan")), **kw)
+    _close(out, whole.float(), dt)
+    for s in (0, n // 2, n - 1):
+        ref = _sdpa_ref(q[s].view(Hq, 1, hd), ks[s], vs[s], torch.ones(1, lens[s], dtype=torch.bool, device="cuda"))
+        _close(out[s], ref.reshape(Hq * hd), dt)
