@@ -279,8 +279,11 @@ extern "C" int rf_qk_norm_rope_kv(const RfRopeKv* a, rf_stream_t stream) {
   if (vec_on && aligned && a->rot_dim % 16 == 0 && (a->hd == 64 || a->hd == 128 || a->hd == 256)) {
     cudaError_t e;
     const int angle_vec = !a->axis_of_freq && ((reinterpret_cast<uintptr_t>(a->cos) | reinterpret_cast<uintptr_t>(a->sin)) & 15) == 0;
-    // few tokens: one pass over the heads, in blocks of two warps
-    const int per_warp = 256 / a->hd, threads = a->tokens < 512 ? 64 : 256;
+    // Few tokens: one pass over the heads, in blocks of two warps.  Many: eight warps, from more than four blocks an SM on only as many as have heads
+    // (idle ones ask for a row and the positions too).  10 + 2 x 2 heads of 64, us, eight warps / four: 512 tokens 2.9 / 3.4, 1000 4.6 / 3.6,
+    // 5400 17.5 / 10.6; 2 + 2 x 1, three position axes, 5400 tokens, eight / one 22.9 / 6.3.
+    const int per_warp = 256 / a->hd, warps_used = a->tokens <= 4 * sm_count() ? 8 : std::min(8, ceil_div(heads, per_warp));
+    const int threads = a->tokens < 512 ? 64 : 32 * warps_used;
     const dim3 grid(a->tokens, a->tokens < 512 ? ceil_div(heads, 2 * per_warp) : 1);
 #define RF_ROPE_VEC(T)                                                                                              \
     e = a->hd == 64 ? ::rf::launch_k(qk_norm_rope_kv_vec_kernel<T, 64>, grid, dim3(threads), 0, s, 1, *a, angle_vec)    \
