@@ -136,7 +136,7 @@ __global__ void __launch_bounds__(256) qk_norm_rope_kv_vec_kernel(const RfRopeKv
   // asked for before anything is waited for: the first head's row, the positions, the sequence
   const int h_first = first + lane / GROUP;
   uint4 ahead = *reinterpret_cast<const uint4*>(row + (size_t)(h_first < heads ? h_first : 0) * HD + o);
-  const int pos0 = a.pos ? a.pos[(size_t)tok * a.pos_stride] : 0;      // norms and insertion by cache_pos need no positions
+  const int pos0 = a.pos[(size_t)tok * a.pos_stride];
   const int seq = a.k_pool && a.seq_of_tok ? a.seq_of_tok[tok] : tok;
   const int cpos = a.k_pool && a.cache_pos ? a.cache_pos[tok] : pos0;
   int page = -1;
@@ -276,7 +276,9 @@ extern "C" int rf_qk_norm_rope_kv(const RfRopeKv* a, rf_stream_t stream) {
                        (!a->k_pool || ((reinterpret_cast<uintptr_t>(a->k_pool) | reinterpret_cast<uintptr_t>(a->v_pool)) & 15) == 0) &&
                        (!a->q_norm_w || (reinterpret_cast<uintptr_t>(a->q_norm_w) & 15) == 0) &&
                        (!a->k_norm_w || (reinterpret_cast<uintptr_t>(a->k_norm_w) & 15) == 0);
-  if (vec_on && aligned && a->rot_dim % 16 == 0 && (a->hd == 64 || a->hd == 128 || a->hd == 256)) {
+  RfRopeKv v = *a;
+  if (!v.pos) { v.pos = v.cache_pos; v.pos_stride = 1; }     // the 16-byte kernel reads one per token, used or not (a test for it: 2.40 -> 2.46 us for 16 tokens)
+  if (vec_on && aligned && v.pos && a->rot_dim % 16 == 0 && (a->hd == 64 || a->hd == 128 || a->hd == 256)) {
     cudaError_t e;
     const int angle_vec = !a->axis_of_freq && ((reinterpret_cast<uintptr_t>(a->cos) | reinterpret_cast<uintptr_t>(a->sin)) & 15) == 0;
     // Few tokens: one pass over the heads, in blocks of two warps.  Many: eight warps, from more than four blocks an SM on only as many as have heads
@@ -286,9 +288,9 @@ extern "C" int rf_qk_norm_rope_kv(const RfRopeKv* a, rf_stream_t stream) {
     const int threads = a->tokens < 512 ? 64 : 32 * warps_used;
     const dim3 grid(a->tokens, a->tokens < 512 ? ceil_div(heads, 2 * per_warp) : 1);
 #define RF_ROPE_VEC(T)                                                                                              \
-    e = a->hd == 64 ? ::rf::launch_k(qk_norm_rope_kv_vec_kernel<T, 64>, grid, dim3(threads), 0, s, 1, *a, angle_vec)    \
-      : a->hd == 128 ? ::rf::launch_k(qk_norm_rope_kv_vec_kernel<T, 128>, grid, dim3(threads), 0, s, 1, *a, angle_vec)  \
-                     : ::rf::launch_k(qk_norm_rope_kv_vec_kernel<T, 256>, grid, dim3(threads), 0, s, 1, *a, angle_vec);
+    e = a->hd == 64 ? ::rf::launch_k(qk_norm_rope_kv_vec_kernel<T, 64>, grid, dim3(threads), 0, s, 1, v, angle_vec)    \
+      : a->hd == 128 ? ::rf::launch_k(qk_norm_rope_kv_vec_kernel<T, 128>, grid, dim3(threads), 0, s, 1, v, angle_vec)  \
+                     : ::rf::launch_k(qk_norm_rope_kv_vec_kernel<T, 256>, grid, dim3(threads), 0, s, 1, v, angle_vec);
     if (a->dtype == 0) { RF_ROPE_VEC(__half) } else { RF_ROPE_VEC(__nv_bfloat16) }
 #undef RF_ROPE_VEC
     RF_CUDA_CHECK(e);

@@ -1152,10 +1152,16 @@ def test_rope_kv_without_positions(dt, hd, T):
         N.check(N.lib().rf_qk_norm_rope_kv(C.byref(a), C.c_void_p(torch.cuda.current_stream().cuda_stream)), "rf_qk_norm_rope_kv")
         got.append((rows, pools))
     assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
+    rows = qkv.clone()
+    a = N.RfRopeKv()                          # neither pool nor positions: norms in place
+    a.qkv, a.ld, a.tokens, a.Hq, a.Hkv, a.hd, a.pos_stride = rows.data_ptr(), rows.stride(0), T, Hq, Hkv, hd, 1
+    a.q_norm_w, a.k_norm_w, a.eps, a.dtype = w.data_ptr(), w.data_ptr(), 1e-6, K_.dtype_code(dt)
+    N.check(N.lib().rf_qk_norm_rope_kv(C.byref(a), C.c_void_p(torch.cuda.current_stream().cuda_stream)), "rf_qk_norm_rope_kv")
     x = qkv.view(T, -1, hd).float()
     ref = w.float() * (x[:, :Hq + Hkv] * torch.rsqrt(x[:, :Hq + Hkv].pow(2).mean(-1, keepdim=True) + 1e-6)).to(dt).float()
     at = lambda pool: pool[pt[0][(cpos // 16).long()].long(), :, (cpos % 16).long()]
     _close(got[0][0].view(T, -1, hd)[:, :Hq], ref[:, :Hq], dt, scale=3.0)
+    _close(rows.view(T, -1, hd)[:, :Hq + Hkv], ref, dt, scale=3.0)
     _close(at(got[0][1][0]), ref[:, Hq:], dt, scale=3.0)
     assert torch.equal(at(got[0][1][1]), qkv.view(T, -1, hd)[:, Hq + Hkv:])
 
