@@ -1263,13 +1263,13 @@ static int plan_gemm(const RfGemm* g, GemmPlan* pl) {
       for (int S = 8; S >= 2; S >>= 1) {
         if (S > max_by_k || tiles * S > cap) continue;
         int st, part;
-        const int b = tiles * S > sm_count() || S == 8 ? kTwoCtaSmem : 224 * 1024;
+        const int b = tiles * S > sm_count() || (swap && S == 8) ? kTwoCtaSmem : 224 * 1024;
         const size_t smem = layout(S, b, &st, &part);
         if (st < 2 || smem > 227 * 1024) continue;
         // A parked partial that takes more than half of shared memory leaves one CTA to an SM: then a grid of more CTAs than SMs runs
-        // in two rounds, and clusters of eight do not all find a place (fp16, us, with / without this line: 128 x 12288 x 4096 SwiGLU
+        // in two rounds, and clusters of eight do not all find a place (fp16, us, without / with this line: 128 x 12288 x 4096 SwiGLU
         // 81 / 46, 256 x 4096 x 12288 78 / 33, 256 x 2048 x 8192 35 / 24).
-        if (smem > kTwoCtaSmem && (tiles * S > sm_count() || S == 8)) continue;
+        if (smem > kTwoCtaSmem && (tiles * S > sm_count() || (swap && S == 8))) continue;
         splits = S;
         break;
       }
@@ -1278,8 +1278,9 @@ static int plan_gemm(const RfGemm* g, GemmPlan* pl) {
       int st, part;
       layout(splits, kTwoCtaSmem, &st, &part);
       // clusters of eight that own their SMs do not all find a place at once (16 of them: 20.9 us for 1 x 2048 x 8192, 16.0 with half as
-      // many CTAs in clusters of four, 11.2 with two CTAs to an SM)
-      budget = ((tiles * splits > sm_count() || splits == 8) && st >= 2) ? kTwoCtaSmem : 224 * 1024;
+      // many CTAs in clusters of four, 11.2 with two CTAs to an SM); the few tiles that split so with tokens on the rows do, and want the deeper
+      // ring (300 x 512 x 2048 10.7, 11.9 with two to an SM)
+      budget = ((tiles * splits > sm_count() || (swap && splits == 8)) && st >= 2) ? kTwoCtaSmem : 224 * 1024;
     }
   }
   if (env_smem_kb > 0) budget = std::min(224, std::max(48, env_smem_kb)) * 1024;
