@@ -565,7 +565,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         // 128 neighbouring bytes are one request between SMs (16-byte remote loads ran at a tenth of the rate)
         cluster_sync_all();
         if (!aborted && epi) {
-          // kS splits: 32 values of (token, split) in flight at a time (8 of the quantised kernels, which have fewer registers); a
+          // kS splits: 32 values of (token, split) in flight at a time (16 of the quantised kernels, which have fewer registers); a
           // round trip per token made this part of 64 x 12288 x 4096 (two splits) 5 us longer
           auto reduce = [&](auto kS_c) {
             constexpr int kS = decltype(kS_c)::value, kTok = (W8 ? 16 : 32) / kS;

@@ -174,6 +174,9 @@ static thread_local float* t_ss_out = nullptr;
 static thread_local const float* t_ss_in = nullptr;
 static thread_local bool t_norm_x = false;
 
+// RfGemm.streaming_only of the stack's linear layers
+static int streaming_only(const Stack& s) { return s.cfg.gemm_streaming_only == 0 ? 0 : s.cfg.gemm_streaming_only == 1 ? 2 : 1; }
+
 // Whether a linear layer of these sizes can take the squares of its input rows itself: then nobody has to write their sums for it, and it is
 // told so (t_norm_x), so that a GEMM which would need sums after all is refused and does not read those of an earlier call.
 static bool norms_itself(const Stack& s, const void* x, int M, int N, int K, int dual_offset) {
@@ -183,7 +186,7 @@ static bool norms_itself(const Stack& s, const void* x, int M, int N, int K, int
   g.M = M; g.N = N; g.K = K; g.dtype = s.cfg.dtype; g.dual_offset = dual_offset; g.act = dual_offset > 0 ? kActSiluMul : kActNone;
   g.w_packed = s.cfg.weights_packed;
   g.force_swap = -1;
-  g.streaming_only = s.cfg.gemm_streaming_only ? (s.cfg.tp_world > 1 ? 2 : 1) : 0;
+  g.streaming_only = streaming_only(s);
   return s.cfg.tp_world <= 1 && rf_gemm_takes_norm(&g);
 }
 
@@ -210,8 +213,7 @@ static int linear(const Stack& s, const void* x, int64_t ldx, const void* w, con
   }
   g.status = s.status();
   g.force_swap = -1;
-  // the ranks of a tensor-parallel group stay with one kernel family, whatever their shards' shapes
-  g.streaming_only = s.cfg.gemm_streaming_only ? (s.cfg.tp_world > 1 ? 2 : 1) : 0;
+  g.streaming_only = streaming_only(s);
   g.prefetch = t_pf_ptr; g.prefetch_bytes = t_pf_bytes;
   t_pf_ptr = nullptr; t_pf_bytes = 0;
   if (t_ss_out || t_ss_in || t_norm_x) {

@@ -63,9 +63,11 @@ typedef struct RfStackConfig {
   // tokens the residual GEMMs (o_proj, down_proj) emit per-token sums of squares and the next projection scales its
   // result by the reciprocal RMS, so no RMSNorm kernel runs between them; with more tokens a weight-free RMSNorm runs.
   int32_t norm_folded;
-  // 1: every GEMM of the stack runs on the tcgen05 kernels.  Decoder engines set it so that the tokens of a tensor-
-  // parallel run and of a one-GPU run come from one kernel family (the row-parallel GEMMs with a collective in them
-  // always do); the action heads leave it 0 and take the latency-bound kernel for their few-row shapes.
+  // 1: every GEMM of the stack runs on the tcgen05 kernels (the row-parallel GEMMs with a collective in them always do): the ranks of a
+  // tensor-parallel decoder.  2: GEMMs of at most 16 rows may run on gemm_rows.cu: decoders of one GPU.  The action heads leave it 0 and take the
+  // latency-bound kernel for their few-row shapes.  So a tensor-parallel run and a one-GPU run of at most 16 rows use different kernels and agree to
+  // rounding, as they do above 16 rows, where the number of K splits, and with it the order of a sum, follows the shard's size.  RF_GEMM_ROWS=0 keeps
+  // one GPU on the tcgen05 kernels too.
   int32_t gemm_streaming_only;
 } RfStackConfig;
 

@@ -14,6 +14,23 @@ from rhinoforge_b200.parallel.tp import CommBuffers, TPContext  # noqa: E402
 from rhinoforge_b200.runtime.engine import DecoderEngine  # noqa: E402
 
 
+LOGIT_BOUND = 3e-2      # largest difference of a logit between the two runs (checked below on the long prompts)
+
+
+def same_tokens(a, b, logits_behind) -> bool:
+    """Greedy tokens ``[B, n]`` of two runs whose logits agree to ``LOGIT_BOUND``: equal up to the first place where a sequence parts, and there the
+    first run's logits of the two tokens are at most twice the bound apart (either may be off by it; behind that the contexts differ).
+    ``logits_behind(s, tokens)`` gives the first run's logits behind sequence ``s`` and these tokens."""
+    for s in range(a.shape[0]):
+        differ = (a[s] != b[s]).nonzero().flatten()
+        if differ.numel():
+            i = int(differ[0])
+            lg = logits_behind(s, a[s, :i])
+            if float((lg[int(a[s, i])] - lg[int(b[s, i])]).abs()) > 2 * LOGIT_BOUND:
+                return False
+    return True
+
+
 def main() -> int:
     tp = TPContext.from_env()
     dev = tp.device
@@ -94,7 +111,7 @@ def main() -> int:
     prompts = [torch.randint(0, cfg.vocab_size, (L,), generator=gen) for L in (33, 70, 9)]
     e1 = DecoderEngine(cfg, get, device=dev, max_batch=3, max_seq_len=160)
     t1 = e1.generate(prompts, 16).cpu()
-    e1.close()
+    behind = lambda s, toks: e1.prefill([torch.cat((prompts[s], toks.to(prompts[s].dtype)))], return_logits=True)[1][0].float().cpu()
     eN = DecoderEngine(cfg, get, max_batch=3, max_seq_len=160, tp=tp, max_prefill_tokens=256)
     tN = eN.generate(prompts, 16).cpu()
     tN2 = eN.generate(prompts, 16).cpu()
@@ -102,8 +119,9 @@ def main() -> int:
     eN.close()
     toks = tp.all_gather_object(tN)
     ranks_agree = all(torch.equal(toks[0], t) for t in toks)
-    # all 16 tokens of every sequence must equal the single-GPU engine's
-    match = bool((t1 == tN).all())
+    # all 16 tokens of every sequence must equal the single-GPU engine's but for near ties: few-row GEMMs run on other kernels there
+    match = same_tokens(t1, tN, behind)
+    e1.close()
     report.update({"ranks_agree": ranks_agree, "tp_matches_single": match, "replay_stable": bool(torch.equal(tN, tN2)),
                    "t1": t1.tolist(), "tN": tN.tolist()})
     ok &= ranks_agree and match and torch.equal(tN, tN2)
@@ -115,7 +133,6 @@ def main() -> int:
     f1, l1 = e1.prefill(long_prompts, return_logits=True)
     l1 = l1.float().cpu()
     d1 = e1.decode(8).cpu()
-    e1.close()
     eN = DecoderEngine(cfg, get, max_batch=2, max_seq_len=5248, tp=tp, max_prefill_tokens=8192)
     fN, lN = eN.prefill(long_prompts, return_logits=True)
     lN_all = torch.cat(tp.all_gather_object(lN.float().cpu()), 1)        # vocab shards side by side
@@ -123,7 +140,9 @@ def main() -> int:
     eN.check_status()
     eN.close()
     logit_err = float((lN_all - l1).abs().max())
-    long_ok = logit_err < 3e-2 and bool((f1.cpu() == fN.cpu()).all()) and bool((d1 == dN).all())
+    behind = lambda s, toks: e1.prefill([torch.cat((long_prompts[s], toks.to(long_prompts[s].dtype)))], return_logits=True)[1][0].float().cpu()
+    long_ok = logit_err < LOGIT_BOUND and same_tokens(torch.cat((f1.cpu()[:, None], d1), 1), torch.cat((fN.cpu()[:, None], dN), 1), behind)
+    e1.close()
     report.update({"rows_allreduce_logit_err": logit_err, "rows_allreduce_ok": long_ok, "d1": d1.tolist(), "dN": dN.tolist()})
     ok &= long_ok
     report["ok"] = bool(ok)
