@@ -373,10 +373,12 @@ class Pi05Engine:
         self.b_qlen = torch.full((Bm,), n, **i32)
         self.b_kvlen = torch.zeros(Bm, **i32)
         self.b_seq = torch.arange(Bm, **i32).repeat_interleave(n).contiguous()
-        # RF_PI05_SUFFIX_ATTN: `decode` = split-KV decode kernel, 16 (row, head) pairs to a CTA (many small CTAs, best at one
-        # or two samples); `block` = one bidirectional query block of `horizon` rows per sample (tensor-core prefill kernel:
-        # one CTA per sample and head, reads the pages once per sample and head).  `auto` (default) takes `block` from four samples up: measured denoise loop
-        # 14.2 / 51.1 / 97.0 ms (decode) against 20.7 / 45.5 / 58.7 ms (block) at 1 / 8 / 32 samples.
+        # RF_PI05_SUFFIX_ATTN: `decode` = split-KV decode kernel, 16 (row, head) pairs to a CTA (many small CTAs, best for few
+        # samples); `block` = one bidirectional query block of `horizon` rows per sample (tensor-core prefill kernel: one CTA
+        # per sample and head, reads the pages once per sample and head).  `auto` (default) takes `block` from six samples up:
+        # denoise loop of ten steps over three views, ms, decode / block at 1, 2, 4, 5, 6, 8, 32 samples: 10.3 / 15.8,
+        # 15.9 / 19.9, 23.5 / 25.9, 23.9 / 25.9, 25.3 / 21.8, 26.7 / 23.2, 62.8 / 44.6; over one view at 4, 5, 6: 21.4 / 21.8,
+        # 21.6 / 21.9, 20.9 / 17.7.
         self.suffix_attn = os.environ.get("RF_PI05_SUFFIX_ATTN", "auto")
         self.prefix_hidden = torch.zeros(Bm * self.max_prefix, v.hidden, dtype=dtype, device=dev)
         # static inputs of the captured prefill: the valid cameras' pixels and the valid language token ids
@@ -493,7 +495,7 @@ class Pi05Engine:
         x, h, hn = self.x[:T], self.h[:T], self.hn[:T]
         for s in range(num_steps):
             K.gemm(x, self.in_w, bias=self.in_b, out=h)
-            if self.suffix_attn == "block" or (self.suffix_attn == "auto" and B >= 4):
+            if self.suffix_attn == "block" or (self.suffix_attn == "auto" and B >= 6):
                 self.expert_stack.forward(h, q_start=self.b_qstart[:B], q_len=self.b_qlen[:B], kv_len=self.b_kvlen[:B], max_q_len=n,
                                           max_kv_len=self.max_seq, pos=self.s_pos[:T], cos=self.cos, sin=self.sin,
                                           seq_of_tok=self.b_seq[:T], cache_pos=self.s_pos[:T], page_table=self.cache.page_table[:B],

@@ -182,3 +182,28 @@ def test_engine_over_an_interleaved_oversubscribed_page_table():
         eng.decode(40)                        # 6 + 8 + 6 pages would be needed, the pool has 18
     assert eng.cache.free_pages() <= free
     eng.close()
+
+
+@pytest.mark.parametrize("slots", [None, [4, 1, 5, 0, 3]])
+def test_prompts_that_end_beside_others_and_in_the_last_page(slots):
+    """Launches of 64 rows over prompts that span several of them, end in the middle of one and fill a sequence's last page (five pages to a sequence,
+    no whole number of the attention kernel's blocks of keys): the last logits of each against a prefill of its own."""
+    from rhinoforge_b200.models.decoder import random_state_dict, tiny_config
+    from rhinoforge_b200.runtime.engine import DecoderEngine
+    cfg = tiny_config()
+    sd = random_state_dict(cfg, seed=0, dtype=torch.float16, norm_jitter=0.05)
+    get = lambda n: sd[n] if n in sd else sd["model.embed_tokens.weight"]
+    gen = torch.Generator().manual_seed(3)
+    prompts = [torch.randint(0, cfg.vocab_size, (L,), generator=gen) for L in (79, 3, 66, 1, 40)]
+    eng = DecoderEngine(cfg, get, dtype=torch.float16, max_batch=6, max_seq_len=80, max_prefill_tokens=64)
+    first, logits = eng.extend(prompts, slots=slots, return_logits=True)
+    first, logits = first.clone(), logits.clone()
+    eng.check_status()
+    eng.close()
+    one = DecoderEngine(cfg, get, dtype=torch.float16, max_batch=1, max_seq_len=128)
+    for s, p in enumerate(prompts):
+        f, want = one.prefill([p], return_logits=True)
+        # the same kernels over other row counts: one rounding of fp16 logits of order one, as between the oracle and the engine
+        assert (logits[s].float() - want[0].float()).abs().max().item() < 6e-3
+        assert first[s] == f[0] or (want[0, f[0]] - want[0, first[s]]).item() < 6e-3
+    one.close()

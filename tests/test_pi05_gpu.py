@@ -24,7 +24,7 @@ def _inputs(cfg, B, seed=0):
 @pytest.mark.parametrize("form", ["decode", "block"])
 @pytest.mark.parametrize("B", [1, 5])
 def test_suffix_attention_forms(B, form):
-    """Both launch forms of the action rows' attention (one-token sequences on the decode kernel; one bidirectional
+    """Both launch forms of the action rows' attention (query rows of one sequence on the decode kernel; one bidirectional
     query block per sample on the prefill kernel) against the fp32 formulation; ``auto`` picks by sample count."""
     from rhinoforge_b200.models.pi05 import Pi05Engine, TorchPi05, random_pi05_state_dict, tiny_pi05_config
     cfg = tiny_pi05_config()
