@@ -665,8 +665,9 @@ static DecodeSplitPlan plan_decode_split(int num_seqs, int rows_per_seq, int Hq,
   int splits = 1;
   // RF_ATTN_DECODE_CTAS_PER_SM (default 2; 1 for heads of 256): CTAs per SM the split aims at; RF_ATTN_DECODE_MIN_PAGES (default 8): fewest
   // pages a split may cover
-  // (heads of 256 run one CTA per SM: measured on the Pi0.5 denoise loop, 50 rows x 1 KV head over ~870 keys, 12.5 ms at
-  // two per SM against 11.6 ms at one; heads of 128, Qwen3-8B decode at batch 1 / 8: 3.41 / 3.83 ms against 3.51 / 4.03)
+  // (a CTA with heads of 256 has its SM to itself: 24 sequences of 3000 keys, one K/V head, us, 22.7 at one per SM, 32.3 at two; the Pi0.5 denoise
+  // loop, 50 rows of a sequence, takes the same either way.  Heads of 128, 32 + 2 x 8, at one / two: 8 x 4000 43.5 / 25.5, 3 x 6000 23.7 / 20.1,
+  // 2 x 2000 9.2 / 11.2)
   static const int per_sm_env = [] { const char* e = getenv("RF_ATTN_DECODE_CTAS_PER_SM"); return e ? std::max(1, atoi(e)) : 0; }();
   const int per_sm = per_sm_env > 0 ? per_sm_env : (hd >= 256 ? 1 : 2);
   static const int min_pages = [] { const char* e = getenv("RF_ATTN_DECODE_MIN_PAGES"); return e ? std::max(4, atoi(e)) : 8; }();
