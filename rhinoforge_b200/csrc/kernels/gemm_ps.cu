@@ -538,12 +538,13 @@ static PsShape ps_shape(const RfGemm* g) {
     }
   }
   // 256 x 128 and 128 x 256 tiles move the same pieces, but a stage of the latter has one row piece to wait for and its MMAs are twice as wide: 9 %
-  // off a k block.  Its four epilogue warps have twice the columns each, which shows behind short rows if there is more to do than the activation
-  // (fp16, us, 256 x 128 / 128 x 256: 825 x 4096 x 12288 101 / 91, 3072 x 1152 x 4304 39.0 / 35.9, 1300 x 2048 x 2048 21.4 / 20.3; with bias and
-  // residual 825 x 4096 x 12288 105 / 95, 825 x 4096 x 4096 40.9 / 38.5, 1300 x 2560 x 2560 28.7 / 28.5, 1300 x 2048 x 2048 24.2 / 25.0).
+  // off a k block.  Its four epilogue warps have twice the columns each, which shows behind short rows, longer ones if there is more to do than the
+  // activation (fp16, us, 256 x 128 / 128 x 256: 825 x 4096 x 12288 101 / 91, 3072 x 1152 x 4304 39.0 / 35.9, 1300 x 2048 x 2048 21.4 / 20.3; bf16
+  // 6600 x 2048 x 1024 30.3 / 28.4, x 512 18.4 / 18.9, x 128 10.9 / 15.2; with bias and residual 825 x 4096 x 12288 105 / 95, 825 x 4096 x 4096
+  // 40.9 / 38.5, 1300 x 2560 x 2560 28.7 / 28.5, 1300 x 2048 x 2048 24.2 / 25.0).
   const bool extra = g->bias || g->scale || g->row_scale || g->residual;
   auto rounds = [&](int rows, int cols) { return ceil_div(ceil_div(g->M, rows) * ceil_div(g->N, cols), sms); };
-  if (forced == 0 && !dual && best.rows == 256 && best.bn == 128 && g->N > 128 && (!extra || k_blocks >= 48) && rounds(128, 256) <= rounds(256, 128))
+  if (forced == 0 && !dual && best.rows == 256 && best.bn == 128 && g->N > 128 && k_blocks >= (extra ? 48 : 16) && rounds(128, 256) <= rounds(256, 128))
     best = {256, 128, best.ns};
   return best;
 }
