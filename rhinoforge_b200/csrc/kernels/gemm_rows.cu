@@ -17,7 +17,7 @@
 //  * x comes from L2 or L1, one block ahead; what the epilogue adds and multiplies by ahead of a strip's products.
 //  * The warps' sums meet in shared memory once per strip; one thread finishes one value.
 //  * A folded RMSNorm needs no sums of squares from the kernel before (norm_x): every CTA reads all of x anyway and squares it on the way.
-//    Sums that the caller has (ss_in) are added up instead.
+//    GEMMs that are given sums (ss_in) run on gemm_tc.cu: adding them up here made the kernel slower without them (int8, 12 rows, 4 %).
 //
 // fp16, us, this kernel / gemm_tc.cu: 1 x 4096 x 1024 3.1 / 5.7, 1 x 1024 x 2048 3.0 / 5.5, 8 x 2048 x 2048 4.1 / 6.2, 1 x 6144 x 4096 10.5 / 12.9,
 // 1 x 4096 x 12288 17.0 / 19.5, 16 x 3072 x 2048 5.1 / 6.6, 16 x 4096 x 4096 9.2 / 10.5; SwiGLU 1 x 12288 x 4096 31.5 / 35.3 (30.3 at the copy
@@ -43,8 +43,7 @@ struct GemmRowsParams {
   int M, N, K, k_blocks, strips, act, dual_offset, dual_tiles, blk_bytes;
   ActArgs act_args;
   int ns, fp4;                  // int4: scales per row of a block, e2m1 codes
-  int norm;                     // scale every token by the reciprocal root mean square of its row: 1 the squares of x, 2 the caller's sums
-  const float* ss_in; int ss_tiles, ss_ld;
+  int norm;                     // scale every token by the reciprocal root mean square of its row of x
   float inv_dim, eps;
 };
 
@@ -170,7 +169,7 @@ gemm_rows_kernel(const GemmRowsParams p) {
       load_x(j + 1 < nk ? j + 1 : 0);            // x is the same for every strip
       asm volatile("cp.async.wait_group %0;" ::"n"(Ring::depth - 1) : "memory");
       if constexpr (BITS == 4) __syncwarp();     // its pieces were copied by other lanes
-      if (p.norm == 1 && first) {
+      if (p.norm && first) {
 #pragma unroll
         for (int n = 0; n < NT; ++n)
 #pragma unroll
@@ -229,7 +228,7 @@ gemm_rows_kernel(const GemmRowsParams p) {
       for (int n = 0; n < NT; ++n)
 #pragma unroll
         for (int i = 0; i < 4; ++i) sums[buf][warp][c][n * 8 + 2 * t + (i & 1)][g + 8 * (i >> 1)] = acc[c][n][i];
-    if (p.norm == 1 && first) {
+    if (p.norm && first) {
 #pragma unroll
       for (int n = 0; n < NT; ++n) {
         sq[n] += __shfl_xor_sync(0xffffffffu, sq[n], 1);
@@ -241,12 +240,8 @@ gemm_rows_kernel(const GemmRowsParams p) {
     if (p.norm && first) {
       if (tid < NT * 8) {
         float v = 0.f;
-        if (p.norm == 1) {
 #pragma unroll
-          for (int i = 0; i < kRowsWarps; ++i) v += squares[i][tid];
-        } else if (tid < p.M) {
-          for (int i = 0; i < p.ss_tiles; ++i) v += p.ss_in[(size_t)i * p.ss_ld + tid];
-        }
+        for (int i = 0; i < kRowsWarps; ++i) v += squares[i][tid];
         rstd[tid] = rsqrtf(v * p.inv_dim + p.eps);
       }
       __syncthreads();
@@ -283,7 +278,7 @@ static int rows_limit() {
 // products are twice as many, and long rows and an uneven last round of strips lose (16 x 4096 x 4096 9.2 / 10.5, 16 x 2560 x 4096 8.0 / 8.7;
 // 16 x 6144 x 4096 14.7 / 13.5, 16 x 6144 x 2560 10.5 / 9.8, 16 x 2048 x 8192 12.2 / 11.7).
 bool gemm_rows_takes(const RfGemm* g) {
-  if (g->M > rows_limit() || !g->w_packed || g->ar_world > 1 || g->streaming_only == 2 || g->ss_out || g->mul || g->force_splits || g->force_bn || g->force_swap >= 0)
+  if (g->M > rows_limit() || !g->w_packed || g->ar_world > 1 || g->streaming_only == 2 || g->ss_in || g->ss_out || g->mul || g->force_splits || g->force_bn || g->force_swap >= 0)
     return false;
   if ((reinterpret_cast<uintptr_t>(g->x) & 15) != 0) return false;
   if (g->w_int8) return true;
@@ -304,8 +299,7 @@ static int launch_rows(const RfGemm* g, cudaStream_t stream) {
   p.blk_bytes = BITS == 16 ? 16384 : BITS == 8 ? 8192 : rf_w4_block_bytes(g->w_group);
   p.ns = BITS == 4 && g->w_group > 0 ? kRowsBK / std::min(g->w_group, kRowsBK) : 0;
   p.fp4 = g->w_fp4;
-  p.norm = g->norm_x ? 1 : g->ss_in ? 2 : 0;
-  p.ss_in = g->ss_in; p.ss_tiles = g->ss_tiles; p.ss_ld = g->ss_ld;
+  p.norm = g->norm_x;
   p.inv_dim = g->ss_dim > 0 ? 1.f / (float)g->ss_dim : 0.f;
   p.eps = g->ss_eps;
   constexpr int smem = RowsRing<BITS, DUAL, NT>::total;
