@@ -952,7 +952,7 @@ def test_gemm_persistent_epilogue(dt, M, N, K, vec, status):
 def test_gemm_very_few_rows(dt, M, N, K, dual, status):
     """Up to 16 rows over 16-bit weights: strips of 16 features that end inside a weight block or past N, fewer k blocks than warps and
     partial ones, every epilogue option, strided and odd-pitched outputs, a CTA that takes several strips; the RMSNorm that the kernel
-    folds in itself."""
+    folds in itself, or takes from given sums."""
     from rhinoforge_b200.ops import kernels as K_
     rows = 2 * N if dual else N
     x = (torch.randn(M, K + 8, device="cuda") * 0.5).to(dt)[:, :K]
@@ -969,7 +969,11 @@ def test_gemm_very_few_rows(dt, M, N, K, dual, status):
     assert bool((out[:, N:] == 7.0).all())
     ss = torch.zeros((max(K // 128, 1), 256), device="cuda")
     ss[0, :M] = x.float().pow(2).sum(1)
-    _close(K_.gemm(x, wp, ss_in=ss, ss_dim=K, ss_eps=1e-6, **kw), finish(z * torch.rsqrt(x.float().pow(2).mean(1, keepdim=True) + 1e-6)), dt, scale=4.0)
+    normed = finish(z * torch.rsqrt(x.float().pow(2).mean(1, keepdim=True) + 1e-6))
+    _close(K_.gemm(x, wp, ss_in=ss, ss_dim=K, ss_eps=1e-6, **kw), normed, dt, scale=4.0)          # the sums are given: another kernel
+    # long rows of 8 rows, and large weights of more, are other kernels' (the dispatcher's rule)
+    if M * K <= 80 << 10 if M <= 8 and not dual else dual or N * K <= 8 << 20:
+        _close(K_.gemm(x, wp, norm_x=True, ss_eps=1e-6, **kw), normed, dt, scale=4.0)
 
 
 @pytest.mark.parametrize("dt", DT)
