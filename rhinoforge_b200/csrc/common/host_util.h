@@ -69,11 +69,11 @@ int device_ordinal();
 // Whether kernels are launched with programmatic stream serialization (RF_PDL=0 turns it off).
 bool pdl_enabled();
 
-// Launch with the library's standard attributes: programmatic dependent launch and,
-// when cluster_z > 1, a (1,1,cluster_z) thread-block cluster.
+// Launch with the library's standard attributes: programmatic dependent launch and a
+// thread-block cluster where `cluster` is more than one block.
 template <typename... KArgs, typename... Args>
-inline cudaError_t launch_k(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
-                            int cluster_z, Args&&... args) {
+inline cudaError_t launch_clusters(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
+                                   dim3 cluster, Args&&... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = block;
@@ -86,16 +86,23 @@ inline cudaError_t launch_k(void (*kernel)(KArgs...), dim3 grid, dim3 block, siz
     attr[n].val.programmaticStreamSerializationAllowed = 1;
     ++n;
   }
-  if (cluster_z > 1) {
+  if (cluster.x * cluster.y * cluster.z > 1) {
     attr[n].id = cudaLaunchAttributeClusterDimension;
-    attr[n].val.clusterDim.x = 1;
-    attr[n].val.clusterDim.y = 1;
-    attr[n].val.clusterDim.z = (unsigned)cluster_z;
+    attr[n].val.clusterDim.x = cluster.x;
+    attr[n].val.clusterDim.y = cluster.y;
+    attr[n].val.clusterDim.z = cluster.z;
     ++n;
   }
   cfg.attrs = attr;
   cfg.numAttrs = n;
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+}
+
+// The same with a (1,1,cluster_z) cluster.
+template <typename... KArgs, typename... Args>
+inline cudaError_t launch_k(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
+                            int cluster_z, Args&&... args) {
+  return launch_clusters(kernel, grid, block, smem, st, dim3(1, 1, (unsigned)std::max(1, cluster_z)), args...);
 }
 
 // Launch WITHOUT programmatic dependent launch: the kernel starts after everything before it in the stream has

@@ -21,6 +21,13 @@ __device__ __forceinline__ uint64_t global_timer_ns() {
   return t;
 }
 __device__ __forceinline__ int lane_id() { return threadIdx.x & 31; }
+// True in one lane of a fully converged warp.  A role whose whole warp runs the loop around it keeps its operands in uniform registers,
+// where the tcgen05 and bulk-copy instructions want them.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n .reg .pred q;\n elect.sync _|q, 0xffffffff;\n selp.b32 %0, 1, 0, q;\n}" : "=r"(p));
+  return p != 0;
+}
 
 // Wait limits.  Local waits (smem barriers) cover at most one tile of work;
 // peer waits cover a whole kernel on another GPU.
@@ -99,6 +106,16 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity,
       if (backoff_ns) __nanosleep(backoff_ns);
     }
     if (global_timer_ns() - t0 > limit_ns) return false;
+  }
+}
+
+// The same for roles that go on after a timeout (with whatever data there is, so that everything in flight drains by itself): the
+// first one reports `code` and leaves no patience for the waits behind it.
+__device__ __forceinline__ void mbar_wait_or_report(uint64_t* bar, uint32_t parity, uint64_t* limit_ns, uint32_t backoff_ns, int32_t* status,
+                                                    int32_t code, int32_t tag, int32_t detail) {
+  if (!mbar_wait(bar, parity, *limit_ns, backoff_ns)) {
+    if (*limit_ns) report_status(status, code, tag, detail);
+    *limit_ns = 0;
   }
 }
 
@@ -219,6 +236,14 @@ __device__ __forceinline__ void umma_f16(uint32_t tmem_d, uint64_t desc_a, uint6
       "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
       " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}" ::"r"(tmem_d),
       "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+// The same with A in tensor memory: lane r holds row r, a 32-bit column two neighbouring values of K.
+__device__ __forceinline__ void umma_f16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
+      " tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}" ::"r"(tmem_d),
+      "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
       : "memory");
 }
 // mbarrier arrives once every MMA issued so far by this thread has finished.
@@ -349,6 +374,42 @@ __device__ __forceinline__ float ld_dsmem_f32(uint32_t addr) {
   float v;
   asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
   return v;
+}
+
+// ---------------------------------------- CTA pairs (cta_group::2) ----
+// Two CTAs of a cluster whose ranks differ in the last bit work on one MMA: each holds half of the rows of A and of D and half of
+// the rows of B.  The even rank issues; barriers may lie in its shared memory for both.
+__device__ __forceinline__ void pair_tmem_alloc(uint32_t* smem_holder, uint32_t ncols) {      // one warp of each CTA
+  asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(smem_holder)), "r"(ncols) : "memory");
+}
+__device__ __forceinline__ void pair_tmem_relinquish() { asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory"); }
+__device__ __forceinline__ void pair_tmem_dealloc(uint32_t taddr, uint32_t ncols) {
+  asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
+}
+__device__ __forceinline__ void pair_umma_f16(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
+      " tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n}" ::"r"(tmem_d),
+      "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+// The barrier at this offset in BOTH CTAs' shared memory arrives once every MMA issued so far by this thread has finished.
+__device__ __forceinline__ void pair_umma_commit(uint64_t* bar) {
+  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(smem_u32(bar)),
+               "h"((uint16_t)3)
+               : "memory");
+}
+// Tiled load into this CTA's shared memory that completes on a barrier of either CTA of the pair (`bar`: a shared::cluster address).
+__device__ __forceinline__ void pair_tma_load_2d(void* smem_dst, const CUtensorMap* m, uint32_t bar, int32_t c0, int32_t c1) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes"
+      " [%0], [%1, {%3, %4}], [%2];" ::"r"(smem_u32(smem_dst)),
+      "l"(reinterpret_cast<uint64_t>(m)), "r"(bar), "r"(c0), "r"(c1)
+      : "memory");
+}
+// Arrival on a barrier of any CTA of the cluster (`bar`: a shared::cluster address).
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar) {
+  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
 }
 
 // ----------------------------------------------- system-scope flag I/O ----

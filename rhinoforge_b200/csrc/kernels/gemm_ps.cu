@@ -549,19 +549,23 @@ static PsShape ps_shape(const RfGemm* g) {
   return best;
 }
 
-// True when the persistent kernel takes this GEMM (called by rf_gemm after its argument checks): it is estimated to be no slower than
+long gemm_pair_ns(const RfGemm* g);                              // gemm_pair.cu: the form with two CTAs to a tile
+int launch_gemm_pair(const RfGemm* g, cudaStream_t stream);
+
+// True when a persistent kernel takes this GEMM (called by rf_gemm after its argument checks): it is estimated to be no slower than
 // the one-tile kernel with `splits` K splits, whose CTAs pay the same per k block (two of them share an SM's operand stream), about
 // 4.5 us around it and 6.5 us more for the reduction of a split (fp16, us, persistent / split kernel: 825 x 2560 x 2048 20 / 26,
 // 825 x 2048 x 2048 20 / 30; 768 x 1152 x 4304 34 / 23, 825 x 2048 x 16384 119 / 96).
 bool gemm_ps_eligible(const RfGemm* g, bool swap, int splits, int bn, int tiles) {
   static const bool enabled = [] { const char* e = getenv("RF_GEMM_PERSISTENT"); return !(e && e[0] == '0'); }();
   if (!enabled || swap || g->ar_world > 1 || !g->w_packed || g->w_int8) return false;
+  const long pair_ns = gemm_pair_ns(g);
   const PsShape s = ps_shape(g);
   if (s.bn == 0) return false;
   const long sms = sm_count(), ctas = (long)tiles * splits, kb = ceil_div(ceil_div(g->K, kPsBK), splits);
   const long kb_ns = (g->dual_offset > 0 || bn > 128) ? 595 : 450;
   const long load = splits == 1 ? (ctas + sms - 1) / sms * 100 : std::max(100l, ctas * 100 / sms);    // busiest SM's CTAs, per cent
-  return s.ns <= 4500 + (splits > 1 ? 6500 : 0) + kb * kb_ns * load / 100;
+  return (pair_ns ? std::min(pair_ns, s.ns) : s.ns) <= 4500 + (splits > 1 ? 6500 : 0) + kb * kb_ns * load / 100;
 }
 
 template <typename T, bool EXTRA>
@@ -570,7 +574,10 @@ static int launch_ps_t(const RfGemm* g, bool dual, int bn, int rows, cudaStream_
   return dual ? launch_ps<T, true, 1, EXTRA>(g, bn, stream) : launch_ps<T, false, 1, EXTRA>(g, bn, stream);
 }
 
+// CTA pairs wherever their bulk copies can write the result and read the residual (fp16, us, one CTA / two to a tile: 3072 x 4304 x 1152 32.3 / 25,
+// 4770 x 2048 x 2048 50.8 / 33.2, 825 x 2048 x 8192 50.8 / 28.6, 4770 x 16384 x 2048 SwiGLU 626 / 416); other row pitches stay with one.
 int launch_gemm_ps(const RfGemm* g, cudaStream_t stream) {
+  if (gemm_pair_ns(g)) return launch_gemm_pair(g, stream);
   const bool dual = g->dual_offset > 0;
   const PsShape s = ps_shape(g);
   const bool extra = g->bias || g->scale || g->row_scale || g->residual;

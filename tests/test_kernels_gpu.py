@@ -947,6 +947,32 @@ def test_gemm_persistent_epilogue(dt, M, N, K, vec, status):
 
 
 @pytest.mark.parametrize("dt", DT)
+@pytest.mark.parametrize("M,N,K", [(257, 1152, 1152), (511, 2568, 520), (769, 2048, 4104), (2100, 1096, 1160), (9000, 2048, 64), (4097, 8, 1032), (20000, 1032, 128)])
+@pytest.mark.parametrize("dual", [False, True])
+def test_gemm_cta_pairs(dt, M, N, K, dual, status):
+    """Tiles shared by two CTAs: last tiles whose second CTA has no rows or whose second half has no columns, a partial k block, fewer k blocks than
+    ring stages, one and several tiles to a pair, 128 and 256 columns, every epilogue option, the residual in the output's place."""
+    from rhinoforge_b200.ops import kernels as K_
+    assert K_.gemm_plan(M, N, K, dtype=dt, dual=dual)["kernel"] == "persistent"
+    rows = 2 * N if dual else N
+    x = (torch.randn(M, K + 8, device="cuda") * 0.5).to(dt)[:, :K]
+    w = (torch.randn(rows, K, device="cuda") / K ** 0.5).to(dt)
+    b, sc = torch.randn(rows, device="cuda").to(dt), (torch.rand(rows, device="cuda") + 0.5).to(dt)
+    rs, r = torch.rand(M, device="cuda") + 0.5, torch.randn(M, N + 8, device="cuda").to(dt)[:, :N]
+    out = torch.full((M + 1, N + 8), 7.0, device="cuda").to(dt)
+    kw = dict(packed_shape=(rows, K), status=status, **(dict(act="silu_mul", dual=True) if dual else {}))
+    finish = lambda z: torch.nn.functional.silu(z[:, :N]) * z[:, N:] if dual else z
+    wp, z = K_.pack_weight(w, 2 if dual else 1), x.float() @ w.float().t()
+    _close(K_.gemm(x, wp, out=out[:M, :N], **kw), finish(z), dt)
+    full = dict(bias=b, scale=sc, row_scale=rs)
+    ref = finish(z * rs[:, None] * sc.float() + b.float()) + r.float()
+    _close(K_.gemm(x, wp, residual=r, out=out[:M, :N], **full, **kw), ref, dt, scale=2.0)
+    assert bool((out[M:] == 7.0).all()) and bool((out[:, N:] == 7.0).all())
+    acc = r.clone()
+    _close(K_.gemm(x, wp, residual=acc, out=acc, **full, **kw), ref, dt, scale=2.0)
+
+
+@pytest.mark.parametrize("dt", DT)
 @pytest.mark.parametrize("M,N,K", [(1, 16, 64), (1, 1000, 72), (7, 264, 520), (8, 40, 8), (9, 1536, 1024), (16, 5000, 1160), (3, 24, 4096), (16, 7, 2048)])
 @pytest.mark.parametrize("dual", [False, True])
 def test_gemm_very_few_rows(dt, M, N, K, dual, status):
