@@ -3,22 +3,25 @@
 // One CTA owns one or two tiles of 128 query rows of one head.  Both GEMMs of attention run as tcgen05.mma with
 // accumulators in tensor memory:
 //   S = Q . K^T   A = Q tile  [128 x HD]  (K-major, smem)   B = K tile [KVB x HD] (K-major, smem)   D = S in TMEM
-//   O += P . V    A = P tile  [128 x KVB] (K-major, smem)   B = V tile [KVB x HD] (MN-major, smem)  D = O in TMEM
+//   O += P . V    A = P tile  [128 x KVB] (TMEM)            B = V tile [KVB x HD] (MN-major, smem)  D = O in TMEM
 // Warp roles: warp 0 = TMA producer (K/V pages or rows through a ring), warp 1 = MMA issuer (and
 // TMEM owner), then four softmax warps per tile: thread r owns query row r, which is TMEM lane r, so row max and
 // row sum need no shuffles.  S is double buffered in TMEM: Q.K^T of block j+1 runs on the tensor core
-// while the softmax warps work on block j.  The running maximum is only raised when a block exceeds
+// while the softmax warps work on block j, and P of block j lies in the columns that its S was read from.  The softmax warps
+// never wait for P.V unless they have to rescale O.  The running maximum is only raised when a block exceeds
 // it by more than 2^8 (the accumulator and the row sum share the stale maximum, so the final
 // O / l is exact); raising it rescales the O accumulator in TMEM (tcgen05.ld / tcgen05.st).
 //
 // What bounds it: a block of one tile is a chain - S from TMEM, maximum, 64 exponentials a thread (512 cycles of the special-function
-// unit for a warp), P to shared memory, P.V - of some 1100 cycles, so that an SM needs two tiles in different places of their chains, and K/V
+// unit for a warp), P back to TMEM - so that an SM needs two tiles in different places of their chains, and K/V
 // must be under way earlier than that.  Two tiles in ONE CTA share the K/V blocks (half the copies, and they come in 2 KB boxes) and leave room for
 // a ring of four; two CTAs of one tile each with two-block rings waited for their copies (2.1 us a block).  One tile to a CTA is for short
 // inputs, where the CTAs would not fill the GPU otherwise, and for heads above 128.
 // fp16, us (one tile with a two-block ring / now), heads of 128 unless said: 128 queries x 2048 keys 76 / 41 (the chain alone: one CTA per SM);
 // 8192 causal, 32 + 8 heads 1324 / 890; 8192 queries on 16384 keys 3317 / 2462; 8 x 1024 causal 382 / 209; 6 x 1100, window 1024 194 / 104;
 // 2 x 4096, heads of 64 588 / 417; 12 x 256 full 45 / 41 (one tile each); 93 causal, heads of 64 14.2 / 6.9.
+// Then, with P in shared memory, a wait for P.V in every block and one lane in the MMA loop / as it is: 8192 causal 889 / 612; 7808 queries on 16000
+// keys 2380 / 1593; 8 x 1024 causal 209 / 168; 2 x 4096, heads of 64 416 / 290; 6 x 1100, window 1024 104 / 83.
 // V needs no transpose: the [tokens x 64] slabs a TMA box leaves in shared memory are exactly the
 // MN-major 128-byte-swizzle operand layout.
 //
@@ -38,25 +41,24 @@ constexpr int kFaMaxStages = 8;
 constexpr float kFaRaise = 8.0f;      // raise the reference maximum only beyond 2^8
 
 struct alignas(8) FaCtl {
-  uint64_t q_full, kv_full[kFaMaxStages], kv_empty[kFaMaxStages], s_full[2][2], s_empty[2][2], p_full[2], p_empty[2], o_full[2];
+  uint64_t q_full, kv_full[kFaMaxStages], kv_empty[kFaMaxStages], s_full[2][2], p_full[2][2], pv_done[2], o_full[2];
   uint32_t tmem_base;
   int32_t abort_flag;
 };
 
 // HD: size of a query / key head, VD: of a value head, NQ: query tiles of a CTA
 template <int HD, int VD, int NQ> struct FaGeom {
-  static constexpr int J = HD / 64, JV = VD / 64;        // 64-column chunks of the heads
+  static constexpr int J = (HD + 63) / 64, JV = (VD + 63) / 64;      // 64-column chunks of the heads
   static constexpr int KVB = 64;                         // kv tokens per block
-  static constexpr int PC = KVB / 64;                    // 64-token chunks of P
   static constexpr int kQTile = J * kFaRows * 128;
   static constexpr int kKBytes = J * KVB * 128;          // K of one stage, V behind it
   static constexpr int kStageBytes = kKBytes + JV * KVB * 128;
-  static constexpr int kPTile = PC * kFaRows * 128;
-  static constexpr int kFixed = NQ * (kQTile + kPTile);  // the ring lies behind Q and P
+  static constexpr int kFixed = NQ * kQTile;             // the ring lies behind Q
   static constexpr int kSCols = NQ * 2 * KVB;            // S: two buffers per tile, then O per tile
-  static constexpr int kTmemCols = kSCols + NQ * VD > 256 ? 512 : 256;
+  static constexpr int kOCols = (VD + 31) / 32 * 32;
+  static constexpr int kTmemCols = kSCols + NQ * kOCols > 256 ? 512 : 256;
   static constexpr int kThreads = 64 + NQ * 128;
-  static_assert(kSCols + NQ * VD <= 512, "accumulators do not fit tensor memory");
+  static_assert(kSCols + NQ * kOCols <= 512, "accumulators do not fit tensor memory");
 };
 // bits a .. 63 set (all of them from a <= 0, none from a >= 64)
 __device__ __forceinline__ uint64_t bits_from(int a) { return a >= 64 ? 0ull : ~0ull << max(a, 0); }
@@ -83,7 +85,6 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
     return;
   }
   uint8_t* qsm = smem;
-  uint8_t* psm = smem + NQ * G::kQTile;
   uint8_t* kvsm = smem + G::kFixed;
   FaCtl* ctl = reinterpret_cast<FaCtl*>(kvsm + (size_t)stages * G::kStageBytes);
 
@@ -127,10 +128,9 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
     for (int t = 0; t < NQ; ++t) {
       for (int b = 0; b < 2; ++b) {
         mbar_init(&ctl->s_full[t][b], 1);
-        mbar_init(&ctl->s_empty[t][b], 4);
+        mbar_init(&ctl->p_full[t][b], 4);              // per buffer: a warp may be a block ahead of its tile's others
       }
-      mbar_init(&ctl->p_full[t], 4);
-      mbar_init(&ctl->p_empty[t], 1);
+      mbar_init(&ctl->pv_done[t], 1);
       mbar_init(&ctl->o_full[t], 1);
     }
     ctl->abort_flag = 0;
@@ -216,55 +216,64 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------- MMA issuer ----
-    if (lane == 0 && nblk > 0) {
+    if (nblk > 0) {
+      const bool lead = elect_one();
+      uint64_t limit = kLocalWaitNs;
       const uint32_t idesc_qk = umma_idesc_f16(kFaRows, KVB, Num<T>::kFmt, 0);
       const uint32_t idesc_pv = umma_idesc_f16(kFaRows, VD, Num<T>::kFmt, 1);
       // One lane issues every MMA, twelve per tile and block: the operand descriptors are made once and advance by constants (16-byte units)
-      const uint64_t q_desc = umma_desc_k128(smem_u32(qsm)), p_desc = umma_desc_k128(smem_u32(psm));
+      const uint64_t q_desc = umma_desc_k128(smem_u32(qsm));
       const uint64_t k_desc0 = umma_desc_k128(smem_u32(kvsm)), v_desc0 = umma_desc_mn128(smem_u32(kvsm) + G::kKBytes, (uint32_t)(KVB * 128));
-      bool ok = mbar_wait(&ctl->q_full, 0);
-      auto issue_qk = [&](int t, int j) -> bool {
-        const int s = j % stages, b = j & 1;
-        if (!mbar_wait(&ctl->kv_full[s], (uint32_t)(j / stages) & 1u)) return false;
-        if (!mbar_wait(&ctl->s_empty[t][b], ((uint32_t)(j >> 1) & 1u) ^ 1u)) return false;
+      auto wait = [&](uint64_t* bar, uint32_t parity) {
+        mbar_wait_or_report(bar, parity, &limit, 0, p.status, kStatusMmaTimeout, kTagAttnPrefill, 1000);
+      };
+      wait(&ctl->q_full, 0);
+      auto issue_qk = [&](int t, int j, int s, uint32_t ph) {
+        const int b = j & 1;
+        wait(&ctl->kv_full[s], ph);
+        // this S buffer holds P of block j - 2 until its product is done (the other tile's products are in the queue behind that one)
+        if (j >= 2) wait(&ctl->pv_done[t], (uint32_t)j & 1u);
         tc_fence_after_sync();
-        const uint64_t qd = q_desc + (uint32_t)(t * (G::kQTile >> 4)), kd = k_desc0 + (uint32_t)(s * (G::kStageBytes >> 4));
-        const uint32_t d = tmem_base + (uint32_t)((t * 2 + b) * KVB);
+        if (lead) {
+          const uint64_t qd = q_desc + (uint32_t)(t * (G::kQTile >> 4)), kd = k_desc0 + (uint32_t)(s * (G::kStageBytes >> 4));
+          const uint32_t d = tmem_base + (uint32_t)((t * 2 + b) * KVB);
 #pragma unroll
-        for (int c = 0; c < J; ++c)
+          for (int c = 0; c < J; ++c)
 #pragma unroll
-          for (int kk = 0; kk < 4; ++kk)
-            umma_f16(d, qd + (uint32_t)((c * kFaRows * 128 + kk * 32) >> 4), kd + (uint32_t)((c * KVB * 128 + kk * 32) >> 4), idesc_qk, (c | kk) ? 1u : 0u);
-        umma_commit(&ctl->s_full[t][b]);
-        return true;
+            for (int kk = 0; kk < 4 && c * 64 + kk * 16 < HD; ++kk)
+              umma_f16(d, qd + (uint32_t)((c * kFaRows * 128 + kk * 32) >> 4), kd + (uint32_t)((c * KVB * 128 + kk * 32) >> 4), idesc_qk, (c | kk) ? 1u : 0u);
+          umma_commit(&ctl->s_full[t][b]);
+        }
       };
 #pragma unroll
       for (int t = 0; t < NQ; ++t)
-        if (ok && nblk_t[t] > 0) ok = issue_qk(t, 0);
-      for (int j = 0; ok && j < nblk; ++j) {
+        if (nblk_t[t] > 0) issue_qk(t, 0, 0, 0);
+      int s = 0, s_next = 1;                                          // stages of blocks j and j + 1 (at least two), phase of the latter
+      uint32_t ph_next = 0;
+      for (int j = 0; j < nblk; ++j) {
 #pragma unroll
         for (int t = 0; t < NQ; ++t)
-          if (ok && j + 1 < nblk_t[t]) ok = issue_qk(t, j + 1);      // runs while the softmax warps work on block j
-        const int s = j % stages;
+          if (j + 1 < nblk_t[t]) issue_qk(t, j + 1, s_next, ph_next);      // runs while the softmax warps work on block j
         const uint64_t vd = v_desc0 + (uint32_t)(s * (G::kStageBytes >> 4));
 #pragma unroll
         for (int t = 0; t < NQ; ++t) {
-          if (!ok || j >= nblk_t[t]) continue;
-          if (!mbar_wait(&ctl->p_full[t], (uint32_t)j & 1u)) { ok = false; continue; }
+          if (j >= nblk_t[t]) continue;
+          wait(&ctl->p_full[t][j & 1], (uint32_t)(j >> 1) & 1u);
           tc_fence_after_sync();
+          if (lead) {
 #pragma unroll
-          for (int k = 0; k < KVB / 16; ++k)
-            umma_f16(tmem_base + (uint32_t)(G::kSCols + t * VD), p_desc + (uint32_t)((t * G::kPTile + (k >> 2) * (kFaRows * 128) + (k & 3) * 32) >> 4),
-                     vd + (uint32_t)((k * kFaBox) >> 4), idesc_pv, (j | k) ? 1u : 0u);
-          umma_commit(&ctl->p_empty[t]);
-          if (j + 1 == nblk_t[t]) umma_commit(&ctl->o_full[t]);
+            for (int k = 0; k < KVB / 16; ++k)
+              umma_f16_ts(tmem_base + (uint32_t)(G::kSCols + t * G::kOCols), tmem_base + (uint32_t)((t * 2 + (j & 1)) * KVB + k * 8),
+                          vd + (uint32_t)((k * kFaBox) >> 4), idesc_pv, (j | k) ? 1u : 0u);
+            umma_commit(&ctl->pv_done[t]);
+            if (j + 1 == nblk_t[t]) umma_commit(&ctl->o_full[t]);
+          }
         }
-        if (ok) umma_commit(&ctl->kv_empty[s]);                     // every tile's products with this block
+        if (lead) umma_commit(&ctl->kv_empty[s]);                     // every tile's products with this block
+        s = s_next;
+        if (++s_next == stages) { s_next = 0; ph_next ^= 1u; }
       }
-      if (!ok) {
-        if (!*abort_flag) report_status(p.status, kStatusMmaTimeout, kTagAttnPrefill, 1000);
-        ctl->abort_flag = 1;
-      }
+      if (limit == 0) ctl->abort_flag = 1;
     }
   } else {
     // ------------------------------------------------- softmax / correction / epilogue ----
@@ -273,14 +282,13 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
     const int quarter = warp & 3;                         // TMEM lanes this warp may touch
     const int r = quarter * 32 + lane;                    // query row of this thread inside the tile
     const int qi = (qt0 + t) * kFaRows + r;               // row index inside the sequence
-    const uint32_t o_col = (uint32_t)(G::kSCols + t * VD);
+    const uint32_t o_col = (uint32_t)(G::kSCols + t * G::kOCols);
     const uint32_t lane_base = tmem_base + ((uint32_t)(quarter * 32) << 16);
     const uint8_t* mrow = p.mask ? p.mask + (size_t)seq * p.mask_seq_stride + (size_t)min(qi, qlen - 1) * p.mask_ld : nullptr;
     const int sq = (p.seg_q && qi < qlen) ? p.seg_q[p.q_start[seq] + qi] : 0;
     const int kv0 = p.paged ? 0 : p.kv_start[seq];
     float m_ref = -INFINITY, l = 0.f;
     bool ok = true;
-    uint8_t* prow = psm + t * G::kPTile + r * 128;
     // bounds of the valid kv positions of this row that do not depend on data: [lo, hi]
     const int hi_row = min(kvlen - 1, p.causal ? qpos0 + qi : 0x7fffffff);
     int lo_row = p.window > 0 ? qpos0 + qi - p.window + 1 : 0;
@@ -299,10 +307,6 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
 #pragma unroll
       for (int c0 = 0; c0 < KVB; c0 += 32) tmem_ld32(s_addr + c0, *reinterpret_cast<uint32_t(*)[32]>(&sv[c0]));
       tmem_ld_wait();
-      // S[b] may now be overwritten by Q.K^T of block j+2
-      tc_fence_before_sync();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&ctl->s_empty[t][b]);
       // masking: interior blocks need none; edge blocks compare against the row's [lo, hi]; boolean
       // masks and segment ids (rare) take the per-element path
       const bool edge = __any_sync(0xffffffffu, (t0 < lo_row && t0 + KVB > p.keep_first) || t0 + KVB - 1 > hi_row) || data_mask;
@@ -398,14 +402,15 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
         }
       }
       const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
-      // P and O belong to the tensor core until P.V of the previous block has finished
-      if (j > 0 && !mbar_wait(&ctl->p_empty[t], (uint32_t)(j - 1) & 1u)) { ok = false; break; }
-      tc_fence_after_sync();
       const bool raise = mx > m_ref + kFaRaise || (m_ref == -INFINITY && mx > -INFINITY);
       if (__any_sync(0xffffffffu, raise)) {               // tcgen05.ld/st are warp-wide
         const float m_new = raise ? mx : m_ref;
         const float alpha = (m_ref == -INFINITY) ? 0.f : exp2f(m_ref - m_new);
         if (j > 0) {
+          // O belongs to the tensor core until P.V of the previous block has finished (that of the block before is: it was issued ahead of
+          // this block's Q.K^T, so the parity is not ambiguous)
+          if (!mbar_wait(&ctl->pv_done[t], (uint32_t)(j - 1) & 1u)) { ok = false; break; }
+          tc_fence_after_sync();
 #pragma unroll 1
           for (int c0 = 0; c0 < VD; c0 += 32) {
             uint32_t ov[32];
@@ -422,26 +427,26 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
           m_ref = m_new;
         }
       }
-      // probabilities against the reference maximum -> 16-bit P tile (K-major, 128-byte swizzle)
+      // probabilities against the reference maximum -> 16-bit P in place of the first half of S, two keys to a column
       const float mref = m_ref == -INFINITY ? 0.f : m_ref;
       float rs[4] = {0.f, 0.f, 0.f, 0.f};
+      uint32_t pk[KVB / 2];
 #pragma unroll
-      for (int u = 0; u < KVB / 8; ++u) {                 // 16-byte units of 8 values
-        float f8[8];
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          f8[i] = ex2(fmaf(__uint_as_float(sv[u * 8 + i]), mul, -mref));   // masked entries are -inf -> 0
-          rs[i & 3] += f8[i];
-        }
-        uint8_t* chunk_base = prow + (u >> 3) * (kFaRows * 128);
-        store8(reinterpret_cast<T*>(chunk_base + (((u & 7) ^ (r & 7)) << 4)), f8);
+      for (int i = 0; i < KVB / 2; ++i) {
+        const float e0 = ex2(fmaf(__uint_as_float(sv[2 * i]), mul, -mref));         // masked entries are -inf -> 0
+        const float e1 = ex2(fmaf(__uint_as_float(sv[2 * i + 1]), mul, -mref));
+        rs[(2 * i) & 3] += e0;
+        rs[(2 * i + 1) & 3] += e1;
+        const typename Num<T>::T2 v = Num<T>::from_f2(e0, e1);
+        pk[i] = *reinterpret_cast<const uint32_t*>(&v);
       }
+      tmem_st32(s_addr, pk);
       l += (rs[0] + rs[1]) + (rs[2] + rs[3]);
+      tmem_st_wait();
       // P (and a rescaled O) are ready for the tensor core
       tc_fence_before_sync();
-      fence_proxy_async();
       __syncwarp();
-      if (lane == 0) mbar_arrive(&ctl->p_full[t]);
+      if (lane == 0) mbar_arrive(&ctl->p_full[t][b]);
     }
     // epilogue: O / l
     if (ok && nblk > 0) ok = mbar_wait(&ctl->o_full[t], 0);
@@ -472,6 +477,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
         if (qi < qlen) {
 #pragma unroll
           for (int u = 0; u < 4; ++u) {
+            if (c0 + u * 8 >= VD) break;
             float f8[8];
 #pragma unroll
             for (int i = 0; i < 8; ++i) f8[i] = __uint_as_float(ov[u * 8 + i]) * inv;
