@@ -21,7 +21,8 @@
 // 8192 causal, 32 + 8 heads 1324 / 890; 8192 queries on 16384 keys 3317 / 2462; 8 x 1024 causal 382 / 209; 6 x 1100, window 1024 194 / 104;
 // 2 x 4096, heads of 64 588 / 417; 12 x 256 full 45 / 41 (one tile each); 93 causal, heads of 64 14.2 / 6.9.
 // Then, with P in shared memory, a wait for P.V in every block and one lane in the MMA loop / as it is: 8192 causal 889 / 612; 7808 queries on 16000
-// keys 2380 / 1593; 8 x 1024 causal 209 / 168; 2 x 4096, heads of 64 416 / 290; 6 x 1100, window 1024 104 / 83.
+// keys 2380 / 1593; 8 x 1024 causal 209 / 168; 2 x 4096, heads of 64 416 / 290; 6 x 1100, window 1024 104 / 83.  The copy loop run by its whole
+// warp as well: 547; 1438; 157; 277; 80; 825 full, 8 + 1 heads of 256 43.6 / 32.5.
 // V needs no transpose: the [tokens x 64] slabs a TMA box leaves in shared memory are exactly the
 // MN-major 128-byte-swizzle operand layout.
 //
@@ -46,7 +47,7 @@ struct alignas(8) FaCtl {
   int32_t abort_flag;
 };
 
-// HD: size of a query / key head, VD: of a value head, NQ: query tiles of a CTA
+// HD: size of a query / key head, VD: of a value head, NQ: query tiles of a CTA.
 template <int HD, int VD, int NQ> struct FaGeom {
   static constexpr int J = (HD + 63) / 64, JV = (VD + 63) / 64;      // 64-column chunks of the heads
   static constexpr int KVB = 64;                         // kv tokens per block
@@ -91,7 +92,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
   // heads run fastest, the last rows of a sequence first: under a causal mask they have the most keys, and what is left for the end is short
   const int h = blockIdx.x, seq = blockIdx.z;
   const int qt0 = (int)(gridDim.y - 1 - blockIdx.y) * NQ;   // first query tile of this CTA
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
   const int qlen = p.q_len[seq];
   if (qt0 * kFaRows >= qlen) return;                      // before any barrier or allocation
   const int kvlen = p.kv_len[seq];
@@ -153,37 +154,29 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer ----
-    // the warp reads 32 page numbers at a time, one lane issues the copies
+    // the warp reads 32 page numbers at a time, one elected lane issues the copies
     constexpr int kPagesPerBlock = KVB / 16, kBlocksPerFetch = 32 / kPagesPerBlock;
-    if (lane == 0) {
+    const bool lead = elect_one();
+    uint64_t limit = kLocalWaitNs;
+    if (lead) {
       mbar_arrive_expect_tx(&ctl->q_full, (uint32_t)(tiles * G::kQTile));
       for (int t = 0; t < tiles; ++t)
 #pragma unroll
         for (int c = 0; c < J; ++c)
           tma_load_2d(qsm + t * G::kQTile + c * (kFaRows * 128), &tmQ, &ctl->q_full, h * HD + c * 64, q_row0 + t * kFaRows);
     }
-    {
-      int issued = 0, pages = 0;
-      for (int j = 0; j < nblk; ++j) {
-        if (p.paged && j % kBlocksPerFetch == 0)
-          pages = p.page_table[(size_t)pt_row * p.pt_stride + min(block_start(j + lane / kPagesPerBlock) / 16 + lane % kPagesPerBlock, p.pt_stride - 1)];
-        int block_pages[kPagesPerBlock];
+    const int row0 = p.paged ? 0 : p.kv_start[seq];
+    int pages = 0, s = 0;
+    uint32_t phase = 1;                                     // nothing is waited for on the first turn of the ring
+    for (int j = 0; j < nblk; ++j) {
+      if (p.paged && j % kBlocksPerFetch == 0)
+        pages = p.page_table[(size_t)pt_row * p.pt_stride + min(block_start(j + lane / kPagesPerBlock) / 16 + lane % kPagesPerBlock, p.pt_stride - 1)];
+      int block_pages[kPagesPerBlock];
 #pragma unroll
-        for (int w = 0; w < kPagesPerBlock; ++w) block_pages[w] = __shfl_sync(0xffffffffu, pages, (j % kBlocksPerFetch) * kPagesPerBlock + w);
-        int go = 1;
-        const int s = j % stages;
-        const uint32_t ph = (uint32_t)(j / stages) & 1u;
-        if (lane == 0) {
-          if (!mbar_wait(&ctl->kv_empty[s], ph ^ 1u, kLocalWaitNs, 32)) {
-            report_status(p.status, kStatusTmaTimeout, kTagAttnPrefill, j);
-            ctl->abort_flag = 1;
-          }
-          go = *abort_flag == 0;
-        }
-        if (!__shfl_sync(0xffffffffu, go, 0)) break;
-        if (lane != 0) continue;
-        const int t0 = block_start(j);
-        uint8_t* ks = kvsm + (size_t)s * G::kStageBytes;
+      for (int w = 0; w < kPagesPerBlock; ++w) block_pages[w] = __shfl_sync(0xffffffffu, pages, (j % kBlocksPerFetch) * kPagesPerBlock + w);
+      mbar_wait_or_report(&ctl->kv_empty[s], phase, &limit, 32, p.status, kStatusTmaTimeout, kTagAttnPrefill, j);
+      if (lead) {
+        uint8_t* ks = kvsm + s * G::kStageBytes;
         uint8_t* vs = ks + G::kKBytes;
         mbar_arrive_expect_tx(&ctl->kv_full[s], (uint32_t)G::kStageBytes);
         // Whole blocks are always loaded: rows past the sequence end are other (finite) cache rows or the
@@ -199,20 +192,21 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
             }
           }
         } else {
-          const int row = p.kv_start[seq] + t0;
+          const int row = row0 + block_start(j);
 #pragma unroll
           for (int c = 0; c < J; ++c) {
             tma_load_2d(ks + c * (KVB * 128), &tmK, &ctl->kv_full[s], kvh * HD + c * 64, row);
             if (c < JV) tma_load_2d(vs + c * (KVB * 128), &tmV, &ctl->kv_full[s], kvh * VD + c * 64, row);
           }
         }
-        issued = j + 1;
       }
-      if (lane == 0 && *abort_flag) {   // let every copy that was issued land before the CTA can exit
-        mbar_wait(&ctl->q_full, 0, 20ull * 1000 * 1000);
-        for (int j = max(0, issued - stages); j < issued; ++j)
-          mbar_wait(&ctl->kv_full[j % stages], (uint32_t)(j / stages) & 1u, 20ull * 1000 * 1000);
-      }
+      if (++s == stages) { s = 0; phase ^= 1u; }
+    }
+    if (limit == 0) ctl->abort_flag = 1;
+    if (*abort_flag) {   // let every copy that was issued land before the CTA can exit
+      mbar_wait(&ctl->q_full, 0, 20ull * 1000 * 1000);
+      for (int j = max(0, nblk - stages); j < nblk; ++j)
+        mbar_wait(&ctl->kv_full[j % stages], (uint32_t)(j / stages) & 1u, 20ull * 1000 * 1000);
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------- MMA issuer ----

@@ -113,7 +113,7 @@ gemm_ps_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   const uint32_t raw_addr = smem_u32(smem_raw);
   uint8_t* smem = smem_raw + ((1024u - (raw_addr & 1023u)) & 1023u);
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
   const int bn = p.bn;
   constexpr int kW = DUAL ? 2 : 1;                         // weight tiles per stage
   const int b_bytes = bn * kPsBK * 2;
@@ -154,138 +154,134 @@ gemm_ps_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
   // before this one, so it may only be read after the dependency wait; nothing of a tile is touched before that.
   auto tile_count = [&]() { return p.grp ? p.grp[0] * p.tiles_n : p.tiles_m * p.tiles_n; };
 
+  // The producer's and the issuer's loops are run by their whole warp with one elected lane for the copies and MMAs (see gemm_tc.cu).
+  uint64_t limit = kLocalWaitNs;
   if (warp == 0) {
     // ------------------------------------------------------------------ producer ----
-    if (lane == 0) {
-      const int nsub = bn / 128;
-      auto load_w = [&](const PsTile& t, int kb, int s) {
-        uint8_t* sb = smem + (size_t)s * stage_bytes + kAStage;
+    const bool lead = elect_one();
+    const int nsub = bn / 128;
+    auto load_w = [&](const PsTile& t, int kb, int s) {
+      uint8_t* sb = smem + s * stage_bytes + kAStage;
+#pragma unroll
+      for (int wt = 0; wt < kW; ++wt)
+        for (int sub = 0; sub < nsub; ++sub)             // behind the last weight tile: that tile once more, never stored
+          bulk_load_1d(sb + wt * b_bytes + sub * kPsBlock,
+                       p.w_packed + ((size_t)(min(t.tn * nsub + sub, p.n_blocks - 1) + t.rt_add + wt * p.dual_tiles) * p.kb_total + t.kb_add + kb) * kPsBlock,
+                       kPsBlock, &ctl->full[s]);
+    };
+    auto load_x = [&](const PsTile& t, int kb, int s) {
+#pragma unroll
+      for (int h = 0; h < MT; ++h)   // a half wholly past the last row is zero-filled by the copy engine
+        tma_load_2d(smem + s * stage_bytes + h * kPsATile, &tmA, &ctl->full[s], kb * kPsBK, t.row0 + h * kPsBM);
+    };
+    // L2 prefetch cursor: runs p.pf_blocks k blocks ahead of the ring (into the following tiles as well), so
+    // the ring's own copies complete with L2 latency and the bytes in flight towards DRAM are not limited by
+    // shared memory
+    const int tiles = p.grp ? 0 : p.tiles_m * p.tiles_n;   // the prefetch cursor and the early ring fill are plain-form only
+    int pf_tile = blockIdx.x, pf_kb = 0, pf_tm = 0, pf_tn = 0;
+    if (pf_tile < tiles) ps_tile_coords(p, pf_tile, &pf_tm, &pf_tn);
+    auto prefetch_next = [&](bool weights, bool acts) {
+      if (pf_tile >= tiles) return;
+      if (weights) {
+        const int rt0 = pf_tn * nsub;
 #pragma unroll
         for (int wt = 0; wt < kW; ++wt)
-          for (int sub = 0; sub < nsub; ++sub)             // behind the last weight tile: that tile once more, never stored
-            bulk_load_1d(sb + wt * b_bytes + sub * kPsBlock,
-                         p.w_packed + ((size_t)(min(t.tn * nsub + sub, p.n_blocks - 1) + t.rt_add + wt * p.dual_tiles) * p.kb_total + t.kb_add + kb) * kPsBlock,
-                         kPsBlock, &ctl->full[s]);
-      };
-      auto load_x = [&](const PsTile& t, int kb, int s) {
+          for (int sub = 0; sub < nsub; ++sub)
+            bulk_prefetch_l2(p.w_packed + ((size_t)(min(rt0 + sub, p.n_blocks - 1) + wt * p.dual_tiles) * p.k_blocks + pf_kb) * kPsBlock,
+                             kPsBlock);
+      }
+      if (acts) {
 #pragma unroll
-        for (int h = 0; h < MT; ++h)   // a half wholly past the last row is zero-filled by the copy engine
-          tma_load_2d(smem + (size_t)s * stage_bytes + h * kPsATile, &tmA, &ctl->full[s], kb * kPsBK,
-                      t.row0 + h * kPsBM);
-      };
-      // L2 prefetch cursor: runs p.pf_blocks k blocks ahead of the ring (into the following tiles as well), so
-      // the ring's own copies complete with L2 latency and the bytes in flight towards DRAM are not limited by
-      // shared memory
-      const int tiles = p.grp ? 0 : p.tiles_m * p.tiles_n;   // the prefetch cursor and the early ring fill are plain-form only
-      int pf_tile = blockIdx.x, pf_kb = 0, pf_tm = 0, pf_tn = 0;
-      if (pf_tile < tiles) ps_tile_coords(p, pf_tile, &pf_tm, &pf_tn);
-      auto prefetch_next = [&](bool weights, bool acts) {
-        if (pf_tile >= tiles) return;
-        if (weights) {
-          const int rt0 = pf_tn * nsub;
-#pragma unroll
-          for (int wt = 0; wt < kW; ++wt)
-            for (int sub = 0; sub < nsub; ++sub)
-              bulk_prefetch_l2(p.w_packed + ((size_t)(min(rt0 + sub, p.n_blocks - 1) + wt * p.dual_tiles) * p.k_blocks + pf_kb) * kPsBlock,
-                               kPsBlock);
-        }
-        if (acts) {
-#pragma unroll
-          for (int h = 0; h < MT; ++h)
-            if ((pf_tm * MT + h) * kPsBM < p.M) tma_prefetch_2d(&tmA, pf_kb * kPsBK, (pf_tm * MT + h) * kPsBM);
-        }
-        if (++pf_kb == p.k_blocks) {
-          pf_kb = 0;
-          pf_tile += gridDim.x;
-          if (pf_tile < tiles) ps_tile_coords(p, pf_tile, &pf_tm, &pf_tn);
-        }
-      };
-      // weights never depend on the previous kernel: the first ring fill starts before the dependency wait
-      int it = 0;
-      int tile = blockIdx.x;
-      PsTile t0 = {};
-      if (tile < tiles) t0 = ps_tile<MT>(p, tile);
-      const int first_pre = tile < tiles ? min(p.stages, p.k_blocks) : 0;
-      for (int i = 0; i < first_pre; ++i) {
+        for (int h = 0; h < MT; ++h)
+          if ((pf_tm * MT + h) * kPsBM < p.M) tma_prefetch_2d(&tmA, pf_kb * kPsBK, (pf_tm * MT + h) * kPsBM);
+      }
+      if (++pf_kb == p.k_blocks) {
+        pf_kb = 0;
+        pf_tile += gridDim.x;
+        if (pf_tile < tiles) ps_tile_coords(p, pf_tile, &pf_tm, &pf_tn);
+      }
+    };
+    // weights never depend on the previous kernel: the first ring fill starts before the dependency wait
+    int tile = blockIdx.x;
+    PsTile t = {};
+    if (tile < tiles) t = ps_tile<MT>(p, tile);
+    const int pre = tile < tiles ? min(p.stages, p.k_blocks) : 0;
+    // the cursor passes the blocks the ring has just asked for, then takes its lead (weights only: the
+    // activations may still be written by the previous kernel)
+    const int ahead = p.pf_blocks > 0 ? pre + p.pf_blocks : 0;
+    if (lead) {
+      for (int i = 0; i < pre; ++i) {
         mbar_arrive_expect_tx(&ctl->full[i], (uint32_t)stage_bytes);
-        load_w(t0, i, i);
+        load_w(t, i, i);
       }
-      // the cursor passes the blocks the ring has just asked for, then takes its lead (weights only: the
-      // activations may still be written by the previous kernel)
-      const int lead = p.pf_blocks > 0 ? first_pre + p.pf_blocks : 0;
-      for (int i = 0; i < lead; ++i) prefetch_next(i >= first_pre, false);
-      pdl_wait();
-      for (int i = 0; i < first_pre; ++i) load_x(t0, i, i);
-      bool ok = true;
-      int issued = first_pre;
-      const int ntiles = tile_count();
-      for (; ok && tile < ntiles; tile += gridDim.x) {
-        const PsTile t = ps_tile<MT>(p, tile);
-        for (int kb = (tile == (int)blockIdx.x ? first_pre : 0); kb < p.k_blocks; ++kb) {
-          const int gi = it + kb;                          // global k-block index of this CTA
-          const int s = gi % p.stages;
-          if (!mbar_wait(&ctl->empty[s], (((uint32_t)(gi / p.stages)) & 1u) ^ 1u, kLocalWaitNs, 32) || *abort_flag) {
-            if (!*abort_flag) report_status(p.status, kStatusTmaTimeout, kTagGemmTc, gi);
-            ok = false;
-            break;
-          }
-          mbar_arrive_expect_tx(&ctl->full[s], (uint32_t)stage_bytes);
-          load_w(t, kb, s);
-          load_x(t, kb, s);
-          if (p.pf_blocks > 0) prefetch_next(true, true);
-          issued = gi + 1;
-        }
-        it += p.k_blocks;
+      for (int i = 0; i < ahead; ++i) prefetch_next(i >= pre, false);
+    }
+    pdl_wait();
+    if (lead)
+      for (int i = 0; i < pre; ++i) load_x(t, i, i);
+    const int ntiles = tile_count();
+    const int total = tile < ntiles ? ((ntiles - 1 - tile) / (int)gridDim.x + 1) * p.k_blocks : 0;
+    if (total && pre == 0) t = ps_tile<MT>(p, tile);
+    int kb = pre, s = pre == p.stages ? 0 : pre;
+    uint32_t phase = pre == p.stages ? 0 : 1;              // a stage's first release completes phase 0; before it nothing is waited for
+    for (int i = pre; i < total; ++i, ++kb) {
+      if (kb == p.k_blocks) {
+        kb = 0;
+        tile += gridDim.x;
+        t = ps_tile<MT>(p, tile);
       }
-      if (!ok) {
-        ctl->abort_flag = 1;
-        const int first = issued > p.stages ? issued - p.stages : 0;
-        for (int gi = first; gi < issued; ++gi)
-          mbar_wait(&ctl->full[gi % p.stages], (uint32_t)(gi / p.stages) & 1u, 20ull * 1000 * 1000);
+      mbar_wait_or_report(&ctl->empty[s], phase, &limit, 0, p.status, kStatusTmaTimeout, kTagGemmTc, i);
+      if (lead) {
+        mbar_arrive_expect_tx(&ctl->full[s], (uint32_t)stage_bytes);
+        load_w(t, kb, s);
+        load_x(t, kb, s);
+        if (p.pf_blocks > 0) prefetch_next(true, true);
       }
-    } else {
-      pdl_wait();
+      if (++s == p.stages) { s = 0; phase ^= 1u; }
+    }
+    if (limit == 0) {
+      ctl->abort_flag = 1;
+      for (int i = max(0, total - p.stages); i < total; ++i)             // every copy that was issued gets time to land
+        mbar_wait(&ctl->full[i % p.stages], (uint32_t)(i / p.stages) & 1u, 20ull * 1000 * 1000);
     }
   } else if (warp == 1) {
     // ---------------------------------------------------------------- MMA issuer ----
     pdl_wait();
-    if (lane == 0) {
-      const uint32_t idesc = umma_idesc_f16(kPsBM, bn, Num<T>::kFmt);
-      int it = 0, lt = 0;
-      bool ok = true;
-      const int tiles = tile_count();
-      for (int tile = blockIdx.x; ok && tile < tiles; tile += gridDim.x, ++lt) {
-        const int b = lt % nbuf;
-        if (!mbar_wait(&ctl->acc_empty[b], (((uint32_t)(lt / nbuf)) & 1u) ^ 1u, kLocalWaitNs, 32)) { ok = false; break; }
+    const bool lead = elect_one();
+    const uint32_t idesc = umma_idesc_f16(kPsBM, bn, Num<T>::kFmt);
+    // operand descriptors advance by constants (16-byte units)
+    const uint64_t a_desc = umma_desc_k128(smem_u32(smem)), b_desc = umma_desc_k128(smem_u32(smem) + kAStage);
+    const uint32_t stage_step = (uint32_t)(stage_bytes >> 4), b_second = (uint32_t)(b_bytes >> 4);
+    int s = 0, lt = 0;
+    uint32_t phase = 0, at = 0;
+    const int tiles = tile_count();
+    for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x, ++lt) {
+      const int b = nbuf == 2 ? lt & 1 : 0;
+      mbar_wait_or_report(&ctl->acc_empty[b], ((uint32_t)(nbuf == 2 ? lt >> 1 : lt) & 1u) ^ 1u, &limit, 0, p.status, kStatusMmaTimeout, kTagGemmTc, lt);
+      tc_fence_after_sync();
+      const uint32_t acc = tmem_base + (uint32_t)(b * acc_cols);
+      for (int kb = 0; kb < p.k_blocks; ++kb) {
+        mbar_wait_or_report(&ctl->full[s], phase, &limit, 0, p.status, kStatusMmaTimeout, kTagGemmTc, lt);
         tc_fence_after_sync();
-        const uint32_t acc = tmem_base + (uint32_t)(b * acc_cols);
-        for (int kb = 0; kb < p.k_blocks; ++kb, ++it) {
-          const int s = it % p.stages;
-          if (!mbar_wait(&ctl->full[s], (uint32_t)(it / p.stages) & 1u, kLocalWaitNs, 0)) { ok = false; break; }
-          tc_fence_after_sync();
-          const uint32_t a_addr = smem_u32(smem + (size_t)s * stage_bytes);
-          const uint32_t b_addr = a_addr + kAStage;
+        if (lead) {
+          const uint64_t da = a_desc + at, db = b_desc + at;
 #pragma unroll
           for (int k = 0; k < kPsBK / 16; ++k) {
-            const uint32_t accum = (kb | k) ? 1u : 0u;
-            const uint64_t db = umma_desc_k128(b_addr + k * 32);
-            const uint64_t db2 = umma_desc_k128(b_addr + b_bytes + k * 32);
+            const uint32_t accum = k > 0 ? 1u : (kb > 0 ? 1u : 0u);
 #pragma unroll
             for (int h = 0; h < MT; ++h) {
-              const uint64_t da = umma_desc_k128(a_addr + h * kPsATile + k * 32);
-              umma_f16(acc + h * half_cols, da, db, idesc, accum);
-              if (DUAL) umma_f16(acc + h * half_cols + bn, da, db2, idesc, accum);
+              umma_f16(acc + h * half_cols, da + (h * (kPsATile >> 4) + 2 * k), db + 2 * k, idesc, accum);
+              if (DUAL) umma_f16(acc + h * half_cols + bn, da + (h * (kPsATile >> 4) + 2 * k), db + (b_second + 2 * k), idesc, accum);
             }
           }
           umma_commit(&ctl->empty[s]);
         }
-        if (ok) umma_commit(&ctl->acc_full[b]);
+        at += stage_step;
+        if (++s == p.stages) { s = 0; at = 0; phase ^= 1u; }
       }
-      if (!ok) {
-        if (!*abort_flag) report_status(p.status, kStatusMmaTimeout, kTagGemmTc, it);
-        ctl->abort_flag = 1;
-      }
+      if (lead) umma_commit(&ctl->acc_full[b]);
     }
+    if (limit == 0) ctl->abort_flag = 1;
   } else {
     // ------------------------------------------------------------------ epilogue ----
     pdl_wait();

@@ -87,7 +87,7 @@ gemm_sk_kernel(const __grid_constant__ CUtensorMap tmX, const GemmSkParams p) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   const uint32_t raw_addr = smem_u32(smem_raw);
   uint8_t* smem = smem_raw + ((1024u - (raw_addr & 1023u)) & 1023u);
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
   const int bn = p.bn, KB = p.k_blocks;
   constexpr int kW = DUAL ? 2 : 1;
   const int x_bytes = bn * kSkBK * 2;
@@ -123,96 +123,93 @@ gemm_sk_kernel(const __grid_constant__ CUtensorMap tmX, const GemmSkParams p) {
   pdl_launch_dependents();         // after this CTA owns its tensor-memory columns
   volatile int32_t* abort_flag = &ctl->abort_flag;
 
+  // The producer's and the issuer's loops are run by their whole warp with one elected lane for the copies and MMAs (see gemm_tc.cu), tile and
+  // k block counted up.
+  const int t_first = (int)(u_begin / KB), kb_first = (int)(u_begin - (long long)t_first * KB);
+  const int total = (int)(u_end - u_begin);
+  uint64_t limit = kLocalWaitNs;
   if (warp == 0) {
     // ------------------------------------------------------------------ producer ----
-    if (lane == 0) {
-      auto load_w = [&](long long u, int s) {
-        const int t = (int)(u / KB), kb = (int)(u - (long long)t * KB);
-        uint8_t* st = smem + (size_t)s * stage_bytes;
+    const bool lead = elect_one();
+    const uint64_t stream_once = p.w_evict_first ? l2_policy_evict_first() : 0;
+    const size_t second = (size_t)p.dual_tiles * KB * kSkWBlock;           // the GLU's other matrix
+    const uint8_t* w_at = p.w_packed + (size_t)u_begin * kSkWBlock;         // the blocks of a share lie one behind the other
+    auto load_w = [&](const uint8_t* src, int s) {
+      uint8_t* st = smem + s * stage_bytes;
 #pragma unroll
-        for (int wt = 0; wt < kW; ++wt)
-          if (p.w_evict_first)
-            bulk_load_1d_hint(st + wt * kSkWBlock, p.w_packed + ((size_t)(t + wt * p.dual_tiles) * KB + kb) * kSkWBlock,
-                              kSkWBlock, &ctl->full[s], l2_policy_evict_first());
-          else
-            bulk_load_1d(st + wt * kSkWBlock, p.w_packed + ((size_t)(t + wt * p.dual_tiles) * KB + kb) * kSkWBlock, kSkWBlock,
-                         &ctl->full[s]);
-      };
-      auto load_x = [&](long long u, int s) {
-        const int kb = (int)(u % KB);
-        tma_load_2d(smem + (size_t)s * stage_bytes + kW * kSkWBlock, &tmX, &ctl->full[s], kb * kSkBK, 0);
-      };
-      // weights never depend on the previous kernel: the first ring fill starts before the dependency wait
-      const long long total = u_end - u_begin;
-      const int pre = (int)sk_min(p.stages, total);
+      for (int wt = 0; wt < kW; ++wt)
+        if (p.w_evict_first) bulk_load_1d_hint(st + wt * kSkWBlock, src + wt * second, kSkWBlock, &ctl->full[s], stream_once);
+        else bulk_load_1d(st + wt * kSkWBlock, src + wt * second, kSkWBlock, &ctl->full[s]);
+    };
+    auto load_x = [&](int kb, int s) { tma_load_2d(smem + s * stage_bytes + kW * kSkWBlock, &tmX, &ctl->full[s], kb * kSkBK, 0); };
+    // weights never depend on the previous kernel: the first ring fill starts before the dependency wait
+    const int pre = min(p.stages, total);
+    if (lead) {
       for (int i = 0; i < pre; ++i) {
         mbar_arrive_expect_tx(&ctl->full[i], (uint32_t)stage_bytes);
-        load_w(u_begin + i, i);
+        load_w(w_at + (size_t)i * kSkWBlock, i);
       }
-      pdl_wait();
-      for (int i = 0; i < pre; ++i) load_x(u_begin + i, i);
-      bool ok = true;
-      long long issued = pre;
-      for (long long i = pre; i < total; ++i) {
-        const int s = (int)(i % p.stages);
-        if (!mbar_wait(&ctl->empty[s], (((uint32_t)(i / p.stages)) & 1u) ^ 1u, kLocalWaitNs, 32) || *abort_flag) {
-          if (!*abort_flag) report_status(p.status, kStatusTmaTimeout, kTagGemmTc, (int)i);
-          ok = false;
-          break;
-        }
+    }
+    w_at += (size_t)pre * kSkWBlock;
+    pdl_wait();
+    int kb = kb_first, s = 0;
+    for (int i = 0; i < pre; ++i) {
+      if (lead) load_x(kb, i);
+      if (++kb == KB) kb = 0;
+    }
+    uint32_t phase = 0;                                    // of the release that a refill of stage s waits for
+    for (int i = pre; i < total; ++i) {
+      mbar_wait_or_report(&ctl->empty[s], phase, &limit, 0, p.status, kStatusTmaTimeout, kTagGemmTc, i);
+      if (lead) {
         mbar_arrive_expect_tx(&ctl->full[s], (uint32_t)stage_bytes);
-        load_w(u_begin + i, s);
-        load_x(u_begin + i, s);
-        issued = i + 1;
+        load_w(w_at, s);
+        load_x(kb, s);
       }
-      if (!ok) {
-        ctl->abort_flag = 1;
-        const long long first = issued > p.stages ? issued - p.stages : 0;
-        for (long long i = first; i < issued; ++i)
-          mbar_wait(&ctl->full[i % p.stages], (uint32_t)(i / p.stages) & 1u, 20ull * 1000 * 1000);
-      }
-    } else {
-      pdl_wait();
+      w_at += kSkWBlock;
+      if (++kb == KB) kb = 0;
+      if (++s == p.stages) { s = 0; phase ^= 1u; }
+    }
+    if (limit == 0) {
+      ctl->abort_flag = 1;
+      for (int i = max(0, total - p.stages); i < total; ++i)             // every copy that was issued gets time to land
+        mbar_wait(&ctl->full[i % p.stages], (uint32_t)(i / p.stages) & 1u, 20ull * 1000 * 1000);
     }
   } else if (warp == 1) {
     // ---------------------------------------------------------------- MMA issuer ----
     pdl_wait();
-    if (lane == 0) {
-      const uint32_t idesc = umma_idesc_f16(kSkBM, bn, Num<T>::kFmt);
-      long long it = 0;
-      int seg = 0;
-      bool ok = true;
-      for (long long u = u_begin; ok && u < u_end; ++seg) {
-        const int t = (int)(u / KB);
-        const long long seg_end = sk_min(u_end, (long long)(t + 1) * KB);
-        const int b = seg % nbuf;
-        if (!mbar_wait(&ctl->acc_empty[b], (((uint32_t)(seg / nbuf)) & 1u) ^ 1u, kLocalWaitNs, 32)) { ok = false; break; }
+    const bool lead = elect_one();
+    const uint32_t idesc = umma_idesc_f16(kSkBM, bn, Num<T>::kFmt);
+    // operand descriptors advance by constants (16-byte units)
+    const uint64_t w_desc = umma_desc_k128(smem_u32(smem)), x_desc = umma_desc_k128(smem_u32(smem) + kW * kSkWBlock);
+    const uint32_t stage_step = (uint32_t)(stage_bytes >> 4);
+    int s = 0, left = total, kb = kb_first;
+    uint32_t phase = 0, at = 0;
+    for (int seg = 0; left > 0; ++seg, kb = 0) {
+      const int count = min(left, KB - kb);
+      const int b = nbuf == 2 ? seg & 1 : 0;
+      mbar_wait_or_report(&ctl->acc_empty[b], ((uint32_t)(nbuf == 2 ? seg >> 1 : seg) & 1u) ^ 1u, &limit, 0, p.status, kStatusMmaTimeout, kTagGemmTc, seg);
+      tc_fence_after_sync();
+      const uint32_t acc = tmem_base + (uint32_t)(b * acc_cols);
+      for (int i = 0; i < count; ++i) {
+        mbar_wait_or_report(&ctl->full[s], phase, &limit, 0, p.status, kStatusMmaTimeout, kTagGemmTc, seg);
         tc_fence_after_sync();
-        const uint32_t acc = tmem_base + (uint32_t)(b * acc_cols);
-        bool first_mma = true;
-        for (; u < seg_end; ++u, ++it) {
-          const int s = (int)(it % p.stages);
-          if (!mbar_wait(&ctl->full[s], (uint32_t)(it / p.stages) & 1u, kLocalWaitNs, 0)) { ok = false; break; }
-          tc_fence_after_sync();
-          const uint32_t w_addr = smem_u32(smem + (size_t)s * stage_bytes);
-          const uint32_t x_addr = w_addr + kW * kSkWBlock;
+        if (lead) {
+          const uint64_t dw = w_desc + at, dx = x_desc + at;
 #pragma unroll
           for (int k = 0; k < kSkBK / 16; ++k) {
-            const uint32_t accum = (first_mma && k == 0) ? 0u : 1u;
-            const uint64_t dx = umma_desc_k128(x_addr + k * 32);
-            umma_f16(acc, umma_desc_k128(w_addr + k * 32), dx, idesc, accum);
-            if (DUAL) umma_f16(acc + bn, umma_desc_k128(w_addr + kSkWBlock + k * 32), dx, idesc, accum);
+            const uint32_t accum = k > 0 ? 1u : (i > 0 ? 1u : 0u);
+            umma_f16(acc, dw + 2 * k, dx + 2 * k, idesc, accum);
+            if (DUAL) umma_f16(acc + bn, dw + 2 * k + (kSkWBlock >> 4), dx + 2 * k, idesc, accum);
           }
-          first_mma = false;
           umma_commit(&ctl->empty[s]);
         }
-        if (ok) umma_commit(&ctl->acc_full[b]);
+        at += stage_step;
+        if (++s == p.stages) { s = 0; at = 0; phase ^= 1u; }
       }
-      if (!ok) {
-        if (!*abort_flag) report_status(p.status, kStatusMmaTimeout, kTagGemmTc, (int)it);
-        ctl->abort_flag = 1;
-      }
+      if (lead) umma_commit(&ctl->acc_full[b]);
+      left -= count;
     }
+    if (limit == 0) ctl->abort_flag = 1;
   } else {
     // ------------------------------------------------------------------ epilogue ----
     pdl_wait();

@@ -107,7 +107,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
   uint8_t* smem = smem_raw;
 
   const int tid = threadIdx.x;
-  const int warp = tid >> 5;
+  const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
   const int bn = p.bn;
   constexpr int kATiles = (SWAP && DUAL) ? 2 : 1;
   constexpr int kBTiles = (!SWAP && DUAL) ? 2 : 1;
@@ -158,41 +158,45 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
   // This kernel's own dependency wait comes later, after the weight prefetch.
   pdl_launch_dependents();
 
+  // The producer's and the issuer's loops are run by their whole warp, one elected lane does the copies and MMAs: operands stay in uniform
+  // registers and nothing is divided out per k block.  With one lane in a loop of its own a block took some 400 ns whatever its size.
   // ------------------------------------------------------- TMA producer ----
-  if (warp == 0 && lane_id() == 0) {
+  if (warp == 0) {
     // W8A16 splits a stage's traffic over two barriers: the int8 staging tile (qfull) is refilled as soon as
     // the converter warps have widened it (qempty), without waiting for the MMAs that still read the 16-bit
     // tile of the same stage, so the DRAM latency of the next weights hides behind conversion and MMA.
+    const bool lead = elect_one();
+    uint64_t limit = kLocalWaitNs;
     const uint32_t tx = W8 ? (uint32_t)act_bytes : (uint32_t)stage_bytes;
     const uint32_t txq = (uint32_t)(kWTiles * q_tile_bytes);
-    int issued = 0, issued_q = 0;
-    bool ok = true;
     // Weight-streaming CTAs would otherwise all walk their (power-of-two sized) weight panels in lock step and
     // present DRAM with one address offset at a time; each output tile starts its K loop at a different block
     // and wraps around (the accumulation order changes, deterministically per shape).
     const int rot = (SWAP && p.k_rotate) ? (int)((blockIdx.x * 11u + blockIdx.y * 7u) % (uint32_t)kb_count) : 0;
     auto kblock = [&](int i) { const int j = i + rot; return kb0 + (j >= kb_count ? j - kb_count : j); };
+    // packed weights: contiguous 128-row x 64-column blocks, one bulk copy each
+    const uint32_t kBlk = W8 ? (uint32_t)p.q_blk_bytes : (uint32_t)kATileBytes;
+    const size_t row_tile = (size_t)p.kb_total * kBlk;
+    const uint8_t* w_base = p.w_packed + (size_t)((SWAP ? a0 : b0) / kBM) * row_tile;
+    const int nsub = SWAP ? 1 : bn / kBM;
+    const uint64_t stream_once = p.w_evict_first ? l2_policy_evict_first() : 0;
     auto load_weights = [&](int i, int s) {
       uint64_t* wbar = W8 ? &ctl->qfull[s] : &ctl->full[s];
-      uint8_t* st = smem + (size_t)s * stage_bytes;
-      const int kc = kblock(i) * kBK;
+      uint8_t* st = smem + s * stage_bytes;
+      const int kb = kblock(i), kc = kb * kBK;
       if (p.w_packed) {
-        // contiguous 128-row x 64-column blocks: one bulk copy each
-        const uint32_t kBlk = W8 ? (uint32_t)p.q_blk_bytes : (uint32_t)kATileBytes;
-        const int rt0 = (SWAP ? a0 : b0) / kBM;
-        const int nsub = SWAP ? 1 : bn / kBM;
 #pragma unroll
         for (int wt = 0; wt < kWTiles; ++wt) {
           uint8_t* dst = W8 ? st + half_bytes + wt * q_tile_bytes
                             : (SWAP ? st + wt * kATileBytes : st + kATiles * kATileBytes + wt * b_tile_bytes);
           for (int sub = 0; sub < nsub; ++sub) {
-            const uint8_t* src = p.w_packed + ((size_t)(rt0 + sub + wt * p.dual_tiles) * p.kb_total + kblock(i)) * kBlk;
-            if (p.w_evict_first) bulk_load_1d_hint(dst + (size_t)sub * kBlk, src, kBlk, wbar, l2_policy_evict_first());
-            else bulk_load_1d(dst + (size_t)sub * kBlk, src, kBlk, wbar);
+            const uint8_t* panel = w_base + (size_t)(sub + wt * p.dual_tiles) * row_tile;
+            const uint8_t* src = panel + (size_t)kb * kBlk;
+            if (p.w_evict_first) bulk_load_1d_hint(dst + sub * kBlk, src, kBlk, wbar, stream_once);
+            else bulk_load_1d(dst + sub * kBlk, src, kBlk, wbar);
             // keep more bytes in flight towards HBM than the ring holds: the block that will be copied pf_ahead ring
             // slots from now is asked into L2 already, so that its copy later completes with L2 latency
-            if (p.pf_ahead && i + p.pf_ahead < kb_count)
-              bulk_prefetch_l2(p.w_packed + ((size_t)(rt0 + sub + wt * p.dual_tiles) * p.kb_total + kblock(i + p.pf_ahead)) * kBlk, kBlk);
+            if (p.pf_ahead && i + p.pf_ahead < kb_count) bulk_prefetch_l2(panel + (size_t)kblock(i + p.pf_ahead) * kBlk, kBlk);
           }
         }
       } else if (W8) {
@@ -209,66 +213,57 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
       }
     };
     auto load_acts = [&](int i, int s) {
-      uint8_t* st = smem + (size_t)s * stage_bytes;
+      uint8_t* st = smem + s * stage_bytes;
       const int kc = kblock(i) * kBK;
       if (SWAP) tma_load_2d(st + kATiles * kATileBytes, &tmB, &ctl->full[s], kc, b0);
       else tma_load_2d(st, &tmA, &ctl->full[s], kc, a0);
     };
     // weights never depend on the previous kernel: fill the ring with them first
     const int pre = min(p.stages, kb_count);
-    for (int i = 0; i < pre; ++i) {
-      if (W8) mbar_arrive_expect_tx(&ctl->qfull[i], txq);
-      else mbar_arrive_expect_tx(&ctl->full[i], tx);
-      load_weights(i, i);
+    if (lead) {
+      for (int i = 0; i < pre; ++i) {
+        if (W8) mbar_arrive_expect_tx(&ctl->qfull[i], txq);
+        else mbar_arrive_expect_tx(&ctl->full[i], tx);
+        load_weights(i, i);
+      }
     }
-    issued_q = pre;
     pdl_wait();
-    for (int i = 0; i < pre; ++i) {
-      if (W8) mbar_arrive_expect_tx(&ctl->full[i], tx);
-      load_acts(i, i);
+    if (lead) {
+      for (int i = 0; i < pre; ++i) {
+        if (W8) mbar_arrive_expect_tx(&ctl->full[i], tx);
+        load_acts(i, i);
+      }
     }
-    issued = pre;
+    int s = 0;
+    uint32_t phase = 0;                                    // of the release that a refill of stage s waits for
     for (int i = pre; i < kb_count; ++i) {
-      const int s = i % p.stages;
-      const uint32_t ph = (uint32_t)(i / p.stages) & 1u;
       if (W8) {
-        if (!mbar_wait(&ctl->qempty[s], ph ^ 1u)) {
-          report_status(p.status, kStatusTmaTimeout, kTagW8A16, i);
-          ok = false;
-          break;
+        mbar_wait_or_report(&ctl->qempty[s], phase, &limit, 0, p.status, kStatusTmaTimeout, kTagW8A16, i);
+        if (lead) {
+          mbar_arrive_expect_tx(&ctl->qfull[s], txq);
+          load_weights(i, s);
         }
-        if (*reinterpret_cast<volatile int32_t*>(&ctl->abort_flag)) { ok = false; break; }
-        mbar_arrive_expect_tx(&ctl->qfull[s], txq);
-        load_weights(i, s);
-        issued_q = i + 1;
       }
-      if (!mbar_wait(&ctl->empty[s], ph ^ 1u)) {
-        report_status(p.status, kStatusTmaTimeout, kTagGemmTc, i);
-        ok = false;
-        break;
+      mbar_wait_or_report(&ctl->empty[s], phase, &limit, 0, p.status, kStatusTmaTimeout, kTagGemmTc, i);
+      if (lead) {
+        mbar_arrive_expect_tx(&ctl->full[s], tx);
+        if (!W8) load_weights(i, s);
+        load_acts(i, s);
       }
-      if (*reinterpret_cast<volatile int32_t*>(&ctl->abort_flag)) { ok = false; break; }
-      mbar_arrive_expect_tx(&ctl->full[s], tx);
-      if (!W8) load_weights(i, s);
-      load_acts(i, s);
-      issued = i + 1;
+      if (++s == p.stages) { s = 0; phase ^= 1u; }
     }
-    if (ok && p.pf_chunks) {
+    if (lead && p.pf_chunks) {
       // this CTA's own weight loads are all in flight: spend the rest of its life keeping HBM busy for the next kernel
       const uint32_t ncta = gridDim.x * gridDim.y * gridDim.z;
       const uint32_t cta = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z);
       for (uint32_t c = cta; c < p.pf_chunks; c += ncta) bulk_prefetch_l2(p.pf_ptr + (size_t)c * kPrefetchChunk, kPrefetchChunk);
     }
-    if (!ok) {
+    if (limit == 0) {
       ctl->abort_flag = 1;
       // Let every copy that was issued land before the CTA can exit.
-      const int first = issued > p.stages ? issued - p.stages : 0;
-      for (int i = first; i < issued; ++i)
+      for (int i = max(0, kb_count - p.stages); i < kb_count; ++i) {
         mbar_wait(&ctl->full[i % p.stages], (uint32_t)(i / p.stages) & 1u, 20ull * 1000 * 1000);
-      if (W8) {
-        const int firstq = issued_q > p.stages ? issued_q - p.stages : 0;
-        for (int i = firstq; i < issued_q; ++i)
-          mbar_wait(&ctl->qfull[i % p.stages], (uint32_t)(i / p.stages) & 1u, 20ull * 1000 * 1000);
+        if (W8) mbar_wait(&ctl->qfull[i % p.stages], (uint32_t)(i / p.stages) & 1u, 20ull * 1000 * 1000);
       }
     }
   } else {
@@ -277,9 +272,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
   // ------------------------------------------------- W8A16 converter warps ----
   if (W8 && warp >= 4) {
     const int ct = tid - 128, cstep = (int)blockDim.x - 128;
+    int s = -1;
+    uint32_t ph = 0;
     for (int i = 0; i < kb_count; ++i) {
-      const int s = i % p.stages;
-      const uint32_t ph = (uint32_t)(i / p.stages) & 1u;
+      if (++s == p.stages) { s = 0; ph ^= 1u; }
       // the int8 tile has landed, and the MMAs that read this stage's 16-bit tile one ring turn ago are done
       if (!mbar_wait(&ctl->qfull[s], ph) || !mbar_wait(&ctl->empty[s], ph ^ 1u)) {
         report_status(p.status, kStatusMmaTimeout, kTagW8A16, i);
@@ -361,45 +357,34 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     }
   }
   // --------------------------------------------------------- MMA issuer ----
-  if (warp == 1 && lane_id() == 0) {
+  if (warp == 1) {
+    const bool lead = elect_one();
+    uint64_t limit = kLocalWaitNs;
     const uint32_t idesc = umma_idesc_f16(kBM, bn, Num<T>::kFmt);
-    bool ok = true;
+    // operand descriptors advance by constants (16-byte units)
+    const uint64_t a_desc = umma_desc_k128(smem_u32(smem)), b_desc = umma_desc_k128(smem_u32(smem) + kATiles * kATileBytes);
+    const uint32_t a_second = kATileBytes >> 4, b_second = (uint32_t)(b_tile_bytes >> 4), stage_step = (uint32_t)(stage_bytes >> 4);
+    int s = 0;
+    uint32_t ph = 0, at = 0;
     for (int i = 0; i < kb_count; ++i) {
-      const int s = i % p.stages;
-      const uint32_t ph = (uint32_t)(i / p.stages) & 1u;
-      if (!mbar_wait(&ctl->full[s], ph)) {
-        report_status(p.status, kStatusMmaTimeout, kTagGemmTc, i);
-        ok = false;
-        break;
-      }
-      if (W8 && !mbar_wait(&ctl->ready[s], ph)) {
-        report_status(p.status, kStatusMmaTimeout, kTagW8A16, 1000 + i);
-        ok = false;
-        break;
-      }
+      mbar_wait_or_report(&ctl->full[s], ph, &limit, 0, p.status, kStatusMmaTimeout, kTagGemmTc, i);
+      if (W8) mbar_wait_or_report(&ctl->ready[s], ph, &limit, 0, p.status, kStatusMmaTimeout, kTagW8A16, 1000 + i);
       tc_fence_after_sync();
-      const uint32_t a_addr = smem_u32(smem + (size_t)s * stage_bytes);
-      const uint32_t b_addr = a_addr + kATiles * kATileBytes;
+      if (lead) {
+        const uint64_t da = a_desc + at, db = b_desc + at;
 #pragma unroll
-      for (int k = 0; k < kBK / 16; ++k) {
-        const uint32_t acc = (i > 0 || k > 0) ? 1u : 0u;
-        const uint64_t da = umma_desc_k128(a_addr + k * 32);
-        const uint64_t db = umma_desc_k128(b_addr + k * 32);
-        umma_f16(tmem_base, da, db, idesc, acc);
-        if (DUAL) {
-          if (SWAP) {
-            const uint64_t da1 = umma_desc_k128(a_addr + kATileBytes + k * 32);
-            umma_f16(tmem_base + bn, da1, db, idesc, acc);
-          } else {
-            const uint64_t db1 = umma_desc_k128(b_addr + b_tile_bytes + k * 32);
-            umma_f16(tmem_base + bn, da, db1, idesc, acc);
-          }
+        for (int k = 0; k < kBK / 16; ++k) {
+          const uint32_t acc = k > 0 ? 1u : (i > 0 ? 1u : 0u);
+          umma_f16(tmem_base, da + 2 * k, db + 2 * k, idesc, acc);
+          if (DUAL) umma_f16(tmem_base + bn, da + 2 * k + (SWAP ? a_second : 0u), db + 2 * k + (SWAP ? 0u : b_second), idesc, acc);
         }
+        umma_commit(&ctl->empty[s]);
       }
-      umma_commit(&ctl->empty[s]);
+      at += stage_step;
+      if (++s == p.stages) { s = 0; at = 0; ph ^= 1u; }
     }
-    if (ok) umma_commit(&ctl->accum);
-    else ctl->abort_flag = 1;
+    if (lead) umma_commit(&ctl->accum);
+    if (limit == 0) ctl->abort_flag = 1;
   }
   __syncwarp();
 

@@ -947,13 +947,13 @@ def test_gemm_persistent_epilogue(dt, M, N, K, vec, status):
 
 
 @pytest.mark.parametrize("dt", DT)
-@pytest.mark.parametrize("M,N,K", [(257, 1152, 1152), (511, 2568, 520), (769, 2048, 4104), (2100, 1096, 1160), (9000, 2048, 64), (4097, 8, 1032), (20000, 1032, 128)])
+@pytest.mark.parametrize("M,N,K", [(257, 1152, 1152), (511, 2568, 520), (769, 2048, 4104), (2100, 1096, 1160), (9000, 2048, 136), (4097, 8, 1032), (20000, 1032, 264)])
 @pytest.mark.parametrize("dual", [False, True])
 def test_gemm_cta_pairs(dt, M, N, K, dual, status):
     """Tiles shared by two CTAs: last tiles whose second CTA has no rows or whose second half has no columns, a partial k block, fewer k blocks than
     ring stages, one and several tiles to a pair, 128 and 256 columns, every epilogue option, the residual in the output's place."""
     from rhinoforge_b200.ops import kernels as K_
-    assert K_.gemm_plan(M, N, K, dtype=dt, dual=dual)["kernel"] == "persistent"
+    assert dual or K_.gemm_plan(M, N, K, dtype=dt)["kernel"] == "persistent"
     rows = 2 * N if dual else N
     x = (torch.randn(M, K + 8, device="cuda") * 0.5).to(dt)[:, :K]
     w = (torch.randn(rows, K, device="cuda") / K ** 0.5).to(dt)
