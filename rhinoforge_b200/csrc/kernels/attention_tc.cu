@@ -47,7 +47,8 @@ struct alignas(8) FaCtl {
   int32_t abort_flag;
 };
 
-// HD: size of a query / key head, VD: of a value head, NQ: query tiles of a CTA.
+// HD: size of a query / key head, VD: of a value head, NQ: query tiles of a CTA.  Heads of 80 (vision towers' 72) arrive as two 64-column boxes
+// whose second one runs into the next head or past the row's end (zeros); the products stop at 80.
 template <int HD, int VD, int NQ> struct FaGeom {
   static constexpr int J = (HD + 63) / 64, JV = (VD + 63) / 64;      // 64-column chunks of the heads
   static constexpr int KVB = 64;                         // kv tokens per block
@@ -546,11 +547,13 @@ int launch_prefill_tc(const RfAttn* a, const AttnParams& p, cudaStream_t s) {
              "prefill attention needs q_start, q_len, max_q_len, q_rows_total");
   if (a->dtype == 0) {
     if (a->hd == 64) return launch_prefill_tc_t<__half, 64>(a, p, s);
+    if (a->hd == 80) return launch_prefill_tc_t<__half, 80>(a, p, s);
     if (a->hd == 128) return launch_prefill_tc_t<__half, 128>(a, p, s);
     if (a->hd == 192) return launch_prefill_tc_t<__half, 192, 128>(a, p, s);
     return launch_prefill_tc_t<__half, 256>(a, p, s);
   }
   if (a->hd == 64) return launch_prefill_tc_t<__nv_bfloat16, 64>(a, p, s);
+  if (a->hd == 80) return launch_prefill_tc_t<__nv_bfloat16, 80>(a, p, s);
   if (a->hd == 128) return launch_prefill_tc_t<__nv_bfloat16, 128>(a, p, s);
   if (a->hd == 192) return launch_prefill_tc_t<__nv_bfloat16, 192, 128>(a, p, s);
   return launch_prefill_tc_t<__nv_bfloat16, 256>(a, p, s);

@@ -670,7 +670,8 @@ using namespace rf;
 extern "C" int64_t rf_stack_create(const RfStackConfig* cfg) {
   if (!cfg) { fail(RF_ERR_BAD_ARG, "null config"); return -1; }
   if (cfg->layers <= 0 || cfg->hidden <= 0 || cfg->hidden % 8 || cfg->Hq <= 0 || cfg->Hkv <= 0 ||
-      cfg->Hq % cfg->Hkv || (cfg->hd != 64 && cfg->hd != 128 && cfg->hd != 256) || cfg->inter <= 0 ||
+      cfg->Hq % cfg->Hkv ||
+      (cfg->hd != 64 && cfg->hd != 128 && cfg->hd != 256 && !(cfg->hd == 80 && !cfg->paged_kv && !cfg->qk_norm && cfg->rot_dim == 0)) || cfg->inter <= 0 ||
       cfg->inter % 8 || cfg->max_tokens <= 0 || cfg->max_seqs <= 0 || (cfg->dtype != 0 && cfg->dtype != 1) ||
       cfg->tp_world < 1 || cfg->tp_world > 8 || cfg->tp_rank < 0 || cfg->tp_rank >= cfg->tp_world) {
     fail(RF_ERR_BAD_ARG, "invalid stack config (layers=%d hidden=%d Hq=%d Hkv=%d hd=%d inter=%d)", cfg->layers,

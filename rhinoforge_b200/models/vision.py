@@ -33,6 +33,12 @@ def padded_head_dim(hd: int) -> int:
     raise RPUBackendError(f"head_dim {hd} is larger than the attention kernels support (256)")
 
 
+def tower_head_dim(hd: int) -> int:
+    """Padded head size of a tower without rotary embedding: heads of 65 to 80 values run as 80 (of 128, three eighths of the QKV
+    projection, the attention products and the output projection would be work on zeros)."""
+    return 80 if 64 < hd <= 80 else padded_head_dim(hd)
+
+
 def fuse_qkv(wq, wk, wv, bq, bk, bv, heads: int, hd: int, hd_pad: int):
     """Fused, head-padded QKV weight ``[3*heads*hd_pad, hidden]`` and bias (missing biases are zero)."""
     ws, bs = [], []
@@ -77,9 +83,9 @@ class VisionTower:
     (or frames) and their per-sequence lengths; attention never crosses a sequence boundary."""
 
     def __init__(self, geo: TowerGeometry, layer_weights: List[Dict[str, torch.Tensor]], *, max_tokens: int,
-                 max_seqs: int = 64, rotary: bool = False, device="cuda", dtype=torch.float16):
+                 max_seqs: int = 64, rotary: bool = False, device="cuda", dtype=torch.float16, hd_pad: Optional[int] = None):
         self.geo, self.device, self.dtype = geo, torch.device(device), dtype
-        self.hd_pad = padded_head_dim(geo.head_dim)
+        self.hd_pad = hd_pad or padded_head_dim(geo.head_dim)         # of the weights given
         spec = StackSpec(layers=geo.layers, hidden=geo.hidden, heads=geo.heads, kv_heads=geo.heads,
                          head_dim=self.hd_pad, inter=geo.inter, norm=geo.norm, mlp=geo.mlp, eps=geo.eps,
                          rot_dim=(geo.head_dim if rotary else 0), paged_kv=False, causal=False,
@@ -285,7 +291,7 @@ class SiglipVisionEncoder:
     """SigLIP vision transformer: ``forward(pixel_values [B,3,H,W])`` -> ``[B, N, hidden]`` after the
     post-LayerNorm, or ``[B, N, proj_dim]`` when a projector (PaliGemma's ``multi_modal_projector``)
     is attached.  All images of a call run as one packed varlen batch.  Heads of 72 are zero-padded
-    to 128 so that the attention kernels apply; the softmax scale stays 1/sqrt(72)."""
+    to 80 so that the attention kernels apply; the softmax scale stays 1/sqrt(72)."""
 
     def __init__(self, cfg: SiglipConfig, sd: Dict[str, torch.Tensor], *, prefix: str = "vision_model.", device="cuda",
                  dtype=torch.float16, max_images: int = 8, projector: Optional[Tuple[torch.Tensor, torch.Tensor]] = None,
@@ -293,7 +299,7 @@ class SiglipVisionEncoder:
         self.cfg, self.device, self.dtype = cfg, torch.device(device), dtype
         H, heads = cfg.hidden_size, cfg.num_attention_heads
         hd = H // heads
-        hd_pad = padded_head_dim(hd)
+        hd_pad = tower_head_dim(hd)
         g = lambda n: sd[prefix + n]
         self.patch_w = _conv_as_linear(g("embeddings.patch_embedding.weight"), self.device, dtype)
         self.patch_b = g("embeddings.patch_embedding.bias").to(self.device, dtype).contiguous()
@@ -315,7 +321,7 @@ class SiglipVisionEncoder:
             raise RPUBackendError(f"unsupported SigLIP activation {cfg.hidden_act}")
         geo = TowerGeometry(H, cfg.num_hidden_layers, heads, hd, cfg.intermediate_size, cfg.layer_norm_eps, act)
         self.tower = VisionTower(geo, layers, max_tokens=max_images * self.tokens_per_image, max_seqs=max_images,
-                                 device=device, dtype=dtype)
+                                 device=device, dtype=dtype, hd_pad=hd_pad)
         self.post_norm = post_norm       # HYViT2 feeds the last block's output straight to its projector
         if post_norm:
             self.post_w = g("post_layernorm.weight").to(self.device, dtype).contiguous()

@@ -28,7 +28,7 @@ class StackSpec:
     hidden: int
     heads: int                 # local query heads
     kv_heads: int              # local kv heads
-    head_dim: int              # padded head dim (64 / 128 / 256)
+    head_dim: int              # padded head dim (64 / 128 / 256; 80 without rotary embedding, head norms and pages)
     inter: int                 # local intermediate size
     norm: str = "rms"
     mlp: str = "swiglu"
@@ -70,7 +70,7 @@ LAYER_FIELDS = ("norm1_w", "norm1_b", "wqkv", "bqkv", "sqkv", "q_norm_w", "k_nor
 def pad_heads(w: torch.Tensor, heads: int, hd: int, hd_pad: int, dim: int) -> torch.Tensor:
     """Zero-pad every head of a projection from ``hd`` to ``hd_pad`` along ``dim`` (0: output rows of
     q/k/v or a bias vector, 1: input columns of the output projection).  Zero rows/columns leave
-    the attention result unchanged, so odd head sizes (72, 80) run on the 128-wide kernels."""
+    the attention result unchanged, so odd head sizes (72, 80) run on the kernels of the next size up."""
     if hd == hd_pad:
         return w
     if w.dim() == 1:

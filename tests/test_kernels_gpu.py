@@ -1062,6 +1062,34 @@ def test_attn_prefill_two_tiles(dt, hd, Hq, Hkv, mode, status):
 
 
 @pytest.mark.parametrize("dt", DT)
+@pytest.mark.parametrize("heads,lens", [(2, [16, 1, 65]), (16, [256, 256, 256]), (32, [300, 513, 129, 64])])
+@pytest.mark.parametrize("mode", ["full", "causal", "mask"])
+def test_attn_prefill_heads_of_80(dt, heads, lens, mode, status):
+    """Heads of 80 over rows of one QKV buffer: the second box of a head runs into the next one, of the last head past the row's end."""
+    from rhinoforge_b200.ops import kernels as K_
+    T, n, hd = sum(lens), heads * 80, 80
+    i32 = lambda l: torch.tensor(l, dtype=torch.int32, device="cuda")
+    starts = [sum(lens[:i]) for i in range(len(lens))]
+    qkv = torch.randn(T, 3 * n, device="cuda").to(dt)
+    kw = dict(Hq=heads, Hkv=heads, hd=hd, q_start=i32(starts), q_len=i32(lens), kv_len=i32(lens), kv_start=i32(starts), max_q_len=max(lens),
+              causal=mode == "causal", status=status)
+    given = torch.rand(len(lens), max(lens), (max(lens) + 15) // 16 * 16, device="cuda") > 0.4
+    given[:, :, 0] = True
+    if mode == "mask":
+        kw["mask"] = given
+    out = K_.attention_prefill(qkv, torch.zeros(T, n, device="cuda", dtype=dt), k=qkv[:, n:2 * n], v=qkv[:, 2 * n:], **kw)
+    for s, L in enumerate(lens):
+        q, k, v = (qkv[starts[s]:starts[s] + L, i * n:(i + 1) * n].view(L, heads, hd).transpose(0, 1) for i in range(3))
+        mask = torch.ones(L, L, dtype=torch.bool, device="cuda")
+        mask = mask.tril() if mode == "causal" else given[s, :L, :L] if mode == "mask" else mask
+        _close(out[starts[s]:starts[s] + L], _sdpa_ref(q, k, v, mask).transpose(0, 1).reshape(L, n), dt)
+    with pytest.raises(Exception, match="80"):
+        K_.attention_decode(qkv[:, :n], out, Hq=heads, Hkv=heads, hd=hd, kv_len=i32([1] * T), max_kv_len=16,
+                            k_pool=torch.zeros(1, heads, 16, hd, device="cuda", dtype=dt), v_pool=torch.zeros(1, heads, 16, hd, device="cuda", dtype=dt),
+                            page_table=i32([[0]] * T), ws=K_.attn_decode_scratch(T, heads, hd, "cuda"))
+
+
+@pytest.mark.parametrize("dt", DT)
 @pytest.mark.parametrize("H", [8, 264, 1024, 1152, 2040, 3072, 4096, 4104])
 @pytest.mark.parametrize("rows", [295, 1301, 3001])
 def test_norms_of_many_rows(dt, H, rows):
