@@ -205,8 +205,16 @@ __global__ void __launch_bounds__(kRtTokens * 32) moe_choose_kernel(const RfMoeR
     for (int s = 0; s < S; ++s) {
       const int e = s * 32 + lane;
       sc[s] = 0.f;
-      if (e < E)
-        for (int z = 0; z < splits; ++z) sc[s] += p.logits[((size_t)z * p.rows + first + t) * columns + e];
+      if (e < E) {
+        const float* part = p.logits + (size_t)(first + t) * columns + e;
+        const size_t step = (size_t)p.rows * columns;
+        int z = 0;
+        for (; z + 4 <= splits; z += 4) {                   // four on their way together, added in order
+          const float v0 = part[z * step], v1 = part[(z + 1) * step], v2 = part[(z + 2) * step], v3 = part[(z + 3) * step];
+          sc[s] = (((sc[s] + v0) + v1) + v2) + v3;
+        }
+        for (; z < splits; ++z) sc[s] += part[z * step];
+      }
     }
     if (p.shared_gate && lane == 0) {
       float v = 0.f;
@@ -375,20 +383,33 @@ __global__ void __launch_bounds__(256) moe_gather_kernel(const RfMoeRouter p, T*
 }
 
 // --------------------------------------------------------------------------------- expert GEMMs, few rows ----
-__device__ __forceinline__ uint4 ld_weight(const uint8_t* p) {       // read once: no allocation in L1
+// weights are read once: around L1
+__device__ __forceinline__ void copy_weight(uint32_t dst, const uint8_t* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ uint4 lds_weight(uint32_t a) {
   uint4 v;
-  asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+  asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a) : "memory");
   return v;
 }
 
+// Ring of a warp: steps of 32 columns by all of its features, 512 bytes for each eight of them.  With loads into registers a step was asked for
+// when the one before was done, at 64 KB on their way an SM; three steps of two CTAs (six of one) are 192 KB.
+template <int MT, bool DUAL, int KW, int NT> struct MoeRing {
+  static constexpr int step = (DUAL ? 2 : 1) * NT * 512, depth = (MT == 1 ? 3 : 6), warp_bytes = depth * step, total = 8 * warp_bytes;
+  static constexpr int sums = KW * (DUAL ? 2 : 1) * 16 * MT * (8 / KW * NT * 8 + 4) * (int)sizeof(float);
+  static constexpr int smem = total > sums ? total : sums;
+};
+
 // One CTA: up to 16 * MT sorted rows of one expert times FW * NT * 8 of its features.  KW warps split the contraction, FW the
-// features.  Weights come from the tile-major image (128 rows x 64 columns, 16-byte pieces swizzled inside a row) straight into
-// the fragments: no staging, no barriers until the warps add up.
+// features.  Weights come from the tile-major image (128 rows x 64 columns, 16-byte pieces swizzled inside a row) through a cp.async ring of
+// each warp, a lane's pieces into the fragments that it holds: no meeting of lanes or warps until the warps add up.
 template <typename T, int MT, bool DUAL, int KW, int NT>
 __global__ void __launch_bounds__(256, MT == 1 ? 2 : 1) moe_small_kernel(const RfMoeExperts p) {
   pdl_prologue();
   constexpr int FW = 8 / KW, FEAT = FW * NT * 8, D = DUAL ? 2 : 1;
-  extern __shared__ __align__(16) float red[];                       // [KW][D][16 * MT][FEAT + 4]
+  using Ring = MoeRing<MT, DUAL, KW, NT>;
+  extern __shared__ __align__(16) float red[];                       // the warps' rings, then [KW][D][16 * MT][FEAT + 4]
   constexpr int LD = FEAT + 4;
   if ((int)blockIdx.y >= p.tiles[0]) return;
   const int4 tile = reinterpret_cast<const int4*>(p.tiles)[1 + blockIdx.y];
@@ -427,31 +448,55 @@ __global__ void __launch_bounds__(256, MT == 1 ? 2 : 1) moe_small_kernel(const R
         for (int i = 0; i < 4; ++i) acc[d][m][n][i] = 0.f;
   const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
   const int kn = (K + 31) / 32;
-#pragma unroll 2
-  for (int kb = kw; kb < kn; kb += KW) {
-    const size_t off = (size_t)(kb >> 1) * 16384 + (((((kb & 1) << 2) | q) ^ g) << 4);     // f & 7 == g
-    uint4 b[D][NT], a[MT][2];
+  const uint32_t ring = smem_u32(red) + warp * Ring::warp_bytes + lane * 16;
+  int ask_kb = kw, ask_slot = 0;
+  auto ask = [&] {                                                    // one group per call, also behind the last step
+    if (ask_kb < kn) {
+      const size_t off = (size_t)(ask_kb >> 1) * 16384 + (((((ask_kb & 1) << 2) | q) ^ g) << 4);     // f & 7 == g
 #pragma unroll
-    for (int d = 0; d < D; ++d)
+      for (int d = 0; d < D; ++d)
 #pragma unroll
-      for (int n = 0; n < NT; ++n) b[d][n] = ld_weight(wrow[d] + off + n * 1024);
+        for (int n = 0; n < NT; ++n) copy_weight(ring + ask_slot * Ring::step + (d * NT + n) * 512, wrow[d] + off + n * 1024);
+      ask_kb += KW;
+      if (++ask_slot == Ring::depth) ask_slot = 0;
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+#pragma unroll
+  for (int u = 0; u < Ring::depth; ++u) ask();
+  uint4 next[MT][2];
+  auto load_x = [&](int kb) {
     const int k = kb * 32 + q * 8;
 #pragma unroll
     for (int m = 0; m < MT; ++m)
 #pragma unroll
-      for (int h = 0; h < 2; ++h) a[m][h] = xrow[m][h] && k < K ? *reinterpret_cast<const uint4*>(xrow[m][h] + k) : zero;
+      for (int h = 0; h < 2; ++h) next[m][h] = xrow[m][h] && k < K ? *reinterpret_cast<const uint4*>(xrow[m][h] + k) : zero;
+  };
+  load_x(kw);
+  int slot = 0;
+  for (int kb = kw; kb < kn; kb += KW) {
+    uint4 a[MT][2];
 #pragma unroll
-    for (int m = 0; m < MT; ++m) {
-      const uint32_t a0[4] = {a[m][0].x, a[m][1].x, a[m][0].y, a[m][1].y}, a1[4] = {a[m][0].z, a[m][1].z, a[m][0].w, a[m][1].w};
+    for (int m = 0; m < MT; ++m) { a[m][0] = next[m][0]; a[m][1] = next[m][1]; }
+    load_x(kb + KW);                                                  // zeros behind the last column
+    asm volatile("cp.async.wait_group %0;" ::"n"(Ring::depth - 1) : "memory");
 #pragma unroll
-      for (int d = 0; d < D; ++d)
+    for (int d = 0; d < D; ++d)
 #pragma unroll
-        for (int n = 0; n < NT; ++n) {
-          MmaOp<T>::mma(acc[d][m][n], a0, b[d][n].x, b[d][n].y);
-          MmaOp<T>::mma(acc[d][m][n], a1, b[d][n].z, b[d][n].w);
+      for (int n = 0; n < NT; ++n) {
+        const uint4 b = lds_weight(ring + slot * Ring::step + (d * NT + n) * 512);
+#pragma unroll
+        for (int m = 0; m < MT; ++m) {
+          const uint32_t a0[4] = {a[m][0].x, a[m][1].x, a[m][0].y, a[m][1].y}, a1[4] = {a[m][0].z, a[m][1].z, a[m][0].w, a[m][1].w};
+          MmaOp<T>::mma(acc[d][m][n], a0, b.x, b.y);
+          MmaOp<T>::mma(acc[d][m][n], a1, b.z, b.w);
         }
-    }
+      }
+    ask();                                                            // into the slot just read
+    if (++slot == Ring::depth) slot = 0;
   }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  __syncthreads();                                                    // every ring is empty: the sums take its place
 #pragma unroll
   for (int d = 0; d < D; ++d)
 #pragma unroll
@@ -587,8 +632,9 @@ static int launch_choose(const RfMoeRouter* a, int splits, cudaStream_t s) {
 template <typename T, int MT, bool DUAL, int KW, int NT>
 static int launch_small(const RfMoeExperts* a, cudaStream_t s) {
   constexpr int FEAT = 8 / KW * NT * 8;
-  const size_t smem = (size_t)KW * (DUAL ? 2 : 1) * 16 * MT * (FEAT + 4) * sizeof(float);
-  RF_ALLOW_SMEM_PER_DEVICE((moe_small_kernel<T, MT, DUAL, KW, NT>), 160 * 1024);
+  constexpr size_t smem = MoeRing<MT, DUAL, KW, NT>::smem;
+  static_assert((MT == 1 ? 2 : 1) * (smem + 1024) <= 228 * 1024, "the CTAs of an SM have to fit");
+  RF_ALLOW_SMEM_PER_DEVICE((moe_small_kernel<T, MT, DUAL, KW, NT>), smem);
   const dim3 grid(ceil_div(std::max(a->n, a->shared_n), FEAT), a->max_tiles);
   RF_CUDA_CHECK(::rf::launch_k(moe_small_kernel<T, MT, DUAL, KW, NT>, grid, dim3(256), smem, s, 1, *a));
   ::rf::count_launch();
