@@ -50,8 +50,8 @@ __device__ __forceinline__ void pair_tile_coords(const GemmPairParams& p, int ti
 // EXTRA: scale, bias or row scale (the residual is handled either way)
 template <typename T, bool DUAL, bool EXTRA>
 __global__ void __launch_bounds__(64 + 32 * kPrEpiWarps, 1)
-gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmO,
-                 const __grid_constant__ CUtensorMap tmR, const GemmPairParams p) {
+gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmW32,
+                 const __grid_constant__ CUtensorMap tmO, const __grid_constant__ CUtensorMap tmR, const GemmPairParams p) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
   const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
@@ -96,21 +96,35 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     const int total = first < tiles ? ((tiles - 1 - first) / step + 1) * p.k_blocks : 0;     // k blocks of this pair
     const uint32_t full0 = dsmem_addr(smem_u32(&ctl->full[0]), 0);                           // the even CTA's barriers
     const uint32_t tx = 2u * (uint32_t)stage_bytes;
-    // Weight rows of a tile in the image seen as one column of 64-value rows; a tile may end behind the last block: that block once
+    // Weight rows n .. of a tile in the image seen as one column of 64-value rows; a tile may end behind the last block: that block once
     // more, never stored.
-    auto w_row = [&](int tn) {
+    auto image_row = [&](int n) { return (min(n >> 7, p.n_blocks - 1) + (DUAL ? (int)rank * p.n_blocks : 0)) * p.k_blocks * 128 + (n & 127); };
+    // 96 rows begin at a multiple of 32 and lie in one block or two: a box of 64 and one of 32, whichever comes first
+    const bool split = !DUAL && p.bn == 192;
+    int tm = 0, tn = 0, xr = 0, wr = 0, wr32 = 0, at64 = 0, at32 = 0;
+    auto enter_tile = [&](int tile) {
+      pair_tile_coords(p, tile, &tm, &tn);
+      xr = (tm * 2 + (int)rank) * kPrBM;
       const int n = DUAL ? tn * 128 : tn * p.bn + (int)rank * w_rows;
-      return (min(n >> 7, p.n_blocks - 1) + (DUAL ? (int)rank * p.n_blocks : 0)) * p.k_blocks * 128 + (n & 127);
+      if (split) {
+        at64 = n & 32;
+        at32 = 64 - 2 * (n & 32);
+        wr32 = image_row(n + at32);
+      }
+      wr = image_row(n + at64);
     };
-    int tm = 0, tn = 0;
-    if (total) pair_tile_coords(p, first, &tm, &tn);
-    int wr = w_row(tn), xr = (tm * 2 + (int)rank) * kPrBM;
+    auto load_w = [&](int kb, int s) {
+      uint8_t* dst = smem + s * stage_bytes + kPrPiece;
+      pair_tma_load_2d(dst + at64 * 128, &tmW, full0 + s * 8, 0, wr + kb * 128);
+      if (split) pair_tma_load_2d(dst + at32 * 128, &tmW32, full0 + s * 8, 0, wr32 + kb * 128);
+    };
+    if (total) enter_tile(first);
     // weights never depend on the kernel before this one: the first ring fill starts ahead of the dependency wait
     const int pre = min(min(p.stages, p.k_blocks), total);
     if (lead) {
       for (int i = 0; i < pre; ++i) {
         if (rank == 0) mbar_arrive_expect_tx(&ctl->full[i], tx);
-        pair_tma_load_2d(smem + i * stage_bytes + kPrPiece, &tmW, full0 + i * 8, 0, wr + i * 128);
+        load_w(i, i);
       }
     }
     pdl_wait();
@@ -122,14 +136,12 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       if (kb == p.k_blocks) {
         kb = 0;
         tile += step;
-        pair_tile_coords(p, tile, &tm, &tn);
-        wr = w_row(tn);
-        xr = (tm * 2 + (int)rank) * kPrBM;
+        enter_tile(tile);
       }
       mbar_wait_or_report(&ctl->empty[s], phase, &limit, 0, p.status, kStatusTmaTimeout, kTagGemmTc, i);
       if (lead) {
         if (rank == 0) mbar_arrive_expect_tx(&ctl->full[s], tx);
-        pair_tma_load_2d(smem + s * stage_bytes + kPrPiece, &tmW, full0 + s * 8, 0, wr + kb * 128);
+        load_w(kb, s);
         pair_tma_load_2d(smem + s * stage_bytes, &tmA, full0 + s * 8, kb * kPrBK, xr);
       }
       if (++s == p.stages) { s = 0; phase ^= 1u; }
@@ -179,13 +191,14 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     const int ew = warp - 2, quarter = warp & 3, group = ew >> 2;      // a warp reads the tensor-memory lanes of its quarter
     const T* bias = EXTRA ? reinterpret_cast<const T*>(p.bias) : nullptr;
     const T* scale = EXTRA ? reinterpret_cast<const T*>(p.scale) : nullptr;
-    const int out_cols = DUAL ? 128 : p.bn, chunks = out_cols / 64;      // two or four: a warp has every other one
+    const int out_cols = DUAL ? 128 : p.bn, chunks = out_cols / 64;
     uint8_t* stg = epi_stage + (size_t)ew * 2 * kPrChunk;
     const uint32_t acc_empty0 = dsmem_addr(smem_u32(&ctl->acc_empty[0]), 0);
 
-    // The warp's chunks, tile after tile.  `cur` is being finished, the residual and the column vectors of the one behind it are on
-    // their way.
+    // The warp's chunks, tile after tile: every other one of a tile, the first of the pair's lt-th tile being group lt & 1's where a tile has
+    // three.  `cur` is being finished, the residual and the column vectors of the one behind it are on their way.
     struct Chunk { int tile, c, col, row; };
+    auto first_chunk = [&](int lt) { return chunks == 3 ? (group + lt) & 1 : group; };
     auto locate = [&](Chunk& k) {
       if (k.tile >= tiles) return;
       int tm, tn;
@@ -240,7 +253,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       while (cur.tile == tile) {
         Chunk next = cur;
         next.c += 2;
-        if (next.c >= chunks) { next.c = group; next.tile += step; }
+        if (next.c >= chunks) { next.c = first_chunk(lt + 1); next.tile += step; }
         locate(next);
         Vecs vnext;
         const bool now = live(cur);
@@ -349,12 +362,18 @@ static int launch_pair(const RfGemm* g, int bn, cudaStream_t stream) {
   p.tiles_m = ceil_div(g->M, 2 * kPrBM); p.tiles_n = ceil_div(g->N, bn);
   p.residual = g->residual != nullptr;
   const int w_rows = DUAL ? 128 : bn / 2;
-  CUtensorMap tmA, tmW, tmO, tmR;
+  CUtensorMap tmA, tmW, tmW32, tmO, tmR;
   int rc = make_tmap_2d(&tmA, g->x, g->dtype, 2, g->K, g->M, g->ldx, kPrBK, kPrBM, true);
   if (rc) return rc;
   // the weight image as one column of 64-value rows, already in the order that shared memory wants
-  rc = make_tmap_2d(&tmW, g->w, g->dtype, 2, kPrBK, (uint64_t)(DUAL ? 2 : 1) * p.n_blocks * p.k_blocks * 128, kPrBK, kPrBK, w_rows, false);
+  const uint64_t image_rows = (uint64_t)(DUAL ? 2 : 1) * p.n_blocks * p.k_blocks * 128;
+  rc = make_tmap_2d(&tmW, g->w, g->dtype, 2, kPrBK, image_rows, kPrBK, kPrBK, w_rows == 96 ? 64 : w_rows, false);
   if (rc) return rc;
+  tmW32 = tmW;
+  if (w_rows == 96) {
+    rc = make_tmap_2d(&tmW32, g->w, g->dtype, 2, kPrBK, image_rows, kPrBK, kPrBK, 32, false);
+    if (rc) return rc;
+  }
   rc = make_tmap_2d(&tmO, g->out, g->dtype, 2, g->N, g->M, g->ldo, 64, 32, true);
   if (rc) return rc;
   tmR = tmO;
@@ -369,7 +388,7 @@ static int launch_pair(const RfGemm* g, int bn, cudaStream_t stream) {
   p.stages = std::min(kPrMaxStages, (227 * 1024 - other) / stage_bytes);
   const size_t smem = (size_t)p.stages * stage_bytes + other;
   const int pairs = std::min(p.tiles_m * p.tiles_n, sm_count() / 2);
-  RF_CUDA_CHECK(::rf::launch_clusters(kfn, dim3(2 * pairs), dim3(64 + 32 * kPrEpiWarps), smem, stream, dim3(2), tmA, tmW, tmO, tmR, p));
+  RF_CUDA_CHECK(::rf::launch_clusters(kfn, dim3(2 * pairs), dim3(64 + 32 * kPrEpiWarps), smem, stream, dim3(2), tmA, tmW, tmW32, tmO, tmR, p));
   ::rf::count_launch();
   return RF_OK;
 }
@@ -382,11 +401,12 @@ static bool pair_can(const RfGemm* g) {
   return (reinterpret_cast<uintptr_t>(g->x) & 15) == 0;
 }
 
-// Tile width and estimated time.  A k block of a tile takes 205 ns at 128 columns and 345 ns at 256 with all SMs busy; tiles of few k
-// blocks take what their epilogue does, longer with a residual and vectors to add.  The 128-wide tiles have less to fill and drain.
-// Measured, fp16, us, 128 / 256 columns (model): 825 x 2048 x 16384 55.5 / 80.1 (56 / 94), 1536 x 8192 x 2048 42.4 / 38.0 (43 / 38),
-// 4770 x 2048 x 2048 33.2 / 34.9 (37 / 38), 4770 x 2560 x 2048 39.8 / 37.0 (43 / 38), 300 x 6144 x 4096 27.9 / 26.2 (30 / 27),
-// 825 x 1152 x 1152 7.3 / 10.6 (7.4 / 11.5).
+// Tile width and estimated time.  A k block of a tile takes 205 ns at 128 columns, 270 at 192 and 345 at 256 with all SMs busy; tiles of few k
+// blocks take what their epilogue does, longer with a residual and vectors to add.  Narrow tiles have less to fill and drain; 192 columns are for
+// the sizes whose tiles otherwise leave SMs idle in the last round.  The constants are the best fit to 396 sizes (300 to 8192 rows, 18 weights, with
+// and without a residual): the width taken is 0.5 % off the best one in the mean, 2.2 % without 192.  Measured, fp16, us, 128 / 192 / 256 columns
+// (model): 825 x 2048 x 16384 56 / 67 / 81 (56 / 75 / 94), 1536 x 2048 x 16384 103 / 77 / 87 (109 / 75 / 94), 3072 x 1152 x 4304 29.7 / 24.1 / 28.4
+// (32 / 24 / 29), 1536 x 8192 x 2048 42 / - / 38 (43 / 32 / 38), 825 x 1152 x 1152 7.3 / - / 10.6 (7.4 / 10 / 12).
 struct PairShape { int bn; long ns; };
 static PairShape pair_shape(const RfGemm* g) {
   const bool extra = g->bias || g->scale || g->row_scale || g->residual;
@@ -396,8 +416,13 @@ static PairShape pair_shape(const RfGemm* g) {
     return around + (tiles + pairs - 1) / pairs * std::max(k_blocks * kb_ns, drain);
   };
   if (g->dual_offset > 0) return {128, estimate(128, 345, extra ? 8300 : 5300, 2000)};
-  const long narrow = estimate(128, 205, extra ? 5200 : 3700, extra ? 3100 : 1650), wide = estimate(256, 345, extra ? 8300 : 5300, extra ? 5000 : 2000);
-  return narrow <= wide ? PairShape{128, narrow} : PairShape{256, wide};
+  const PairShape shapes[3] = {{128, estimate(128, 205, extra ? 5200 : 3700, extra ? 3100 : 1650)},
+                               {192, estimate(192, 270, extra ? 8000 : 5500, extra ? 3800 : 1900)},
+                               {256, estimate(256, 345, extra ? 8300 : 5300, extra ? 5000 : 2000)}};
+  PairShape best = shapes[0];
+  for (const PairShape& s : shapes)
+    if (s.ns < best.ns) best = s;
+  return best;
 }
 
 // Estimated time in ns where the kernel takes this GEMM, 0 where it cannot.

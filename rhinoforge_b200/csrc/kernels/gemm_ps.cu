@@ -555,7 +555,8 @@ int launch_gemm_pair(const RfGemm* g, cudaStream_t stream);
 bool gemm_ps_eligible(const RfGemm* g, bool swap, int splits, int bn, int tiles) {
   static const bool enabled = [] { const char* e = getenv("RF_GEMM_PERSISTENT"); return !(e && e[0] == '0'); }();
   if (!enabled || swap || g->ar_world > 1 || !g->w_packed || g->w_int8) return false;
-  const long pair_ns = gemm_pair_ns(g);
+  // up to 255 columns that the tile kernel can split along K: no faster on pairs, few of which have a tile (4770 x 128 x 2048 17 / 18 us)
+  const long pair_ns = splits > 1 && g->N < 256 ? 0 : gemm_pair_ns(g);
   const PsShape s = ps_shape(g);
   if (s.bn == 0) return false;
   const long sms = sm_count(), ctas = (long)tiles * splits, kb = ceil_div(ceil_div(g->K, kPsBK), splits);

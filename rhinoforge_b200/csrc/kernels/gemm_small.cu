@@ -342,6 +342,26 @@ bool gemm_small_eligible(const RfGemm* g) {
   return (long)g->N * g->K * (dual ? 2 : 1) <= max_elems;
 }
 
+long gemm_pair_ns(const RfGemm* g);        // gemm_pair.cu
+
+// Whether it should, where a tcgen05 kernel can as well (no gate by token, packed weights).  The tcgen05 kernels' loops have got shorter since the
+// bounds above were measured.  fp16, us, here / there:
+//   * up to 64 rows what is gained back to back (50 x 1024 x 4096 8.7 / 7.2) is not there behind other kernels, where this one's weights are on their way
+//     earlier (Pi0.5 denoise loop, QKV and down projection of 50 rows, 8.1 / 8.2);
+//   * 65 to 256 rows: 93 x 1024 x 4096 16.8 / 8.3, 256 x 3072 x 2048 31.4 / 13.4, GLU 93 x 4096 x 1024 19.0 / 13.1; 128 x 2 Mi elements 8.3 / 8.3,
+//     128 x 2560 x 1024 9.4 / 11.0, 256 x 1024 x 2048 9.5 / 12.2, x 2560 x 1024 20.8 / 11.5;
+//   * above that by the estimate of the CTA-pair kernel against 6 us and 16 ns a million products: 300 x 64 x 64 7.5 / 3.5, 600 x 1024 x 1024
+//     20.6 / 6.7, 300 x 1024 x 384 GLU 14.2 / 7.1, but 300 x 128 x 2048 6.3 / 8.9, 600 x 128 x 2048 7.8 / 8.9.
+bool gemm_small_takes(const RfGemm* g) {
+  if (!gemm_small_eligible(g)) return false;
+  if (g->mul || !g->w_packed || g->M <= 64) return true;
+  const bool dual = g->dual_offset > 0;
+  const long elems = (long)g->N * g->K * (dual ? 2 : 1);
+  if (g->M <= 256) return elems <= (g->M <= 128 ? 3L << 20 : 2L << 20);
+  const long pair_ns = gemm_pair_ns(g);
+  return pair_ns == 0 || pair_ns > 6000 + (long)g->M * elems / 1000000 * 16;
+}
+
 template <typename T, int BM, bool DUAL, int STAGES>
 static int launch_small_st(const SmallParams& p, dim3 grid, cudaStream_t s) {
   constexpr size_t smem = small_smem<BM, DUAL, STAGES>();

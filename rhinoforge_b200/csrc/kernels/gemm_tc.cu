@@ -1469,12 +1469,14 @@ extern "C" int rf_gemm_plan_info(const RfGemm* g, int32_t* out);
 namespace rf {
 bool gemm_sk_eligible(const RfGemm* g, int* ctas);               // gemm_sk.cu: persistent stream-K kernel for small M
 bool gemm_small_eligible(const RfGemm* g);                         // gemm_small.cu: latency-bound shapes (few rows, small weight)
+bool gemm_small_takes(const RfGemm* g);                            // ... where it is the better one
 int gemm_small_run(const RfGemm* g, cudaStream_t stream);
 bool gemm_rows_takes(const RfGemm* g);                             // gemm_rows.cu: very few rows, weights straight into MMA fragments
 int launch_gemm_rows(const RfGemm* g, cudaStream_t stream);
 void gemm_sk_scratch(const RfGemm* g, uint64_t* ws_bytes, int32_t* flags);
 int launch_gemm_sk(const RfGemm* g, cudaStream_t stream);
 bool gemm_ps_eligible(const RfGemm* g, bool swap, int splits, int bn, int tiles);   // gemm_ps.cu: persistent kernel for large M
+long gemm_pair_ns(const RfGemm* g);                                // gemm_pair.cu: its form with two CTAs to a tile
 int launch_gemm_ps(const RfGemm* g, cudaStream_t stream);
 int widen_packed(const void* src, void* dst, int64_t blocks, int dtype, cudaStream_t stream);   // gemm_ps.cu
 }
@@ -1491,11 +1493,17 @@ static int route_gemm(const RfGemm* g, int* kernel, GemmPlan* pl) {
   }
   // latency-bound shapes: gemm_small.cu, but for very few rows (fp16, us, gemm_rows.cu / gemm_small.cu: 1 x 4096 x 1024 3.1 / 7.8,
   // 8 x 1024 x 3072 4.4 / 7.0, 16 x 2048 x 2048 4.7 / 8.4)
-  if (!w8 && !rows && rf::gemm_small_eligible(g)) { *kernel = RF_GEMM_SMALL; return RF_OK; }
+  if (!w8 && !rows && rf::gemm_small_takes(g)) { *kernel = RF_GEMM_SMALL; return RF_OK; }
   if (!w8 && rf::gemm_sk_eligible(g, nullptr)) { *kernel = RF_GEMM_STREAM_K; return RF_OK; }
   if (rows) { *kernel = RF_GEMM_ROWS; return RF_OK; }
   const int rc = plan_gemm(g, pl);
   if (rc) return rc;
+  // 129 to 256 rows of short K: one row tile of the CTA pairs does without the tile kernel's reduction over splits.  fp16, us, tile / pairs: 200 x 2048 x 2048
+  // 13.7 / 9.3, 200 x 8192 x 2048 GLU 34.3 / 21.8; 200 x 4096 x 4096 18.3 / 20.8, 200 x 1152 x 4304 16.2 / 16.6, 200 x 2048 x 8192 21.3 / 28.1.
+  if (!w8 && g->M > 128 && g->M <= 256 && g->K <= 2048 && pl->swap && g->force_swap < 0 && g->force_splits == 0 && g->force_bn == 0 && rf::gemm_pair_ns(g)) {
+    *kernel = RF_GEMM_PERSISTENT;
+    return RF_OK;
+  }
   *kernel = !w8 && g->force_splits == 0 && g->force_bn == 0 && rf::gemm_ps_eligible(g, pl->swap != 0, pl->splits, pl->bn, pl->grid_x * pl->grid_y)
                 ? RF_GEMM_PERSISTENT : RF_GEMM_TILE;
   return RF_OK;
