@@ -469,8 +469,8 @@ class Pi05Engine:
                 flat = flat[im.flatten().nonzero().flatten().to(flat.device)]
             self.img_in[:m["n_valid"]].copy_(flat, non_blocking=True)
         if m["n_ids"]:
-            ids = tokens.cpu()[tm].to(torch.int32)
-            self.ids_in[:m["n_ids"]].copy_(ids)
+            ids = tokens.cpu()[tm].to(torch.int32).pin_memory()
+            self.ids_in[:m["n_ids"]].copy_(ids, non_blocking=True)
         if not use_graph:
             self._prefill_run(m)
             return m["lens"]
@@ -512,9 +512,10 @@ class Pi05Engine:
         cfg, dev = self.cfg, self.device
         B, n = noise.shape[0], cfg.horizon
         T = B * n
+        # through pinned memory: a copy from pageable memory waits for the prefix, and the launch of the loop's 1400 kernels then lies open behind it
         pl = torch.tensor(list(prefix_lens), dtype=torch.int32)
-        self.b_kvlen[:B].copy_((pl + n).to(dev), non_blocking=True)
-        self.s_pos[:T].copy_((pl[:, None] + torch.arange(n, dtype=torch.int32)[None]).flatten().to(dev), non_blocking=True)
+        self.b_kvlen[:B].copy_((pl + n).pin_memory(), non_blocking=True)
+        self.s_pos[:T].copy_((pl[:, None] + torch.arange(n, dtype=torch.int32)[None]).flatten().pin_memory(), non_blocking=True)
         self.x[:T].copy_(noise.reshape(T, -1).to(dev, self.dtype))
         if not use_graph:
             self._denoise_loop(B, num_steps)
