@@ -324,12 +324,12 @@ static int launch_decode(const RfHgrn2* a, cudaStream_t s) {
 // warps - 16 value channels x a share of the key channels each - where the product with it reads it as an operand.
 // A CTA owns VG * 16 value channels of one head of one sequence; the CTAs of a head form a cluster that exchanges the sums of
 // squares of the head norm one step behind the computation.
-constexpr int kHcTok = 16, kHcThreads = 256, kHcWarps = 8, kHcRing = 4;
+constexpr int kHcTok = 16, kHcRing = 4;
 
-// Shared memory of a CTA with DP (padded) key channels and VT value channels, in bytes from the base.
-template <int DP, int VT> struct Hgrn2Geom {
+// Shared memory of a CTA of W warps with DP (padded) key channels and VT value channels, in bytes from the base.
+template <int DP, int VT, int W> struct Hgrn2Geom {
   static constexpr int kRawLd = 2 * DP + VT + 8, kQLd = DP + 4, kBLd = DP + 8, kPLd = 24, kOLd = VT + 4;
-  static constexpr int kDG = kHcWarps / (VT / 16);
+  static constexpr int kDG = W / (VT / 16);
   static constexpr int raw = 0;                                   // [ring][16] rows q | f | v as they come
   static constexpr int sq = raw + kHcRing * kHcTok * kRawLd * 2;  // [16][DP] silu(q), gates
   static constexpr int sf = sq + kHcTok * kQLd * 4;
@@ -361,13 +361,16 @@ __device__ __forceinline__ void hc_split2(float a, float b, uint32_t& hi, uint32
   lo = *reinterpret_cast<uint32_t*>(&l);
 }
 
-// VG: groups of 16 value channels per CTA; the 8 / VG warps of a group share its key channels, DT 16-channel tiles each.
-template <int VG, int DP>
-__global__ void __launch_bounds__(kHcThreads, DP == 256 ? 1 : 2) hgrn2_chunked_kernel(const RfHgrn2 p, int col_tiles) {
+// VG: groups of 16 value channels per CTA; the W / VG warps of a group share its key channels, DT 16-channel tiles each.  Sixteen warps are for CTAs
+// that have an SM to themselves: half of them take the in-block scores, two source tokens each, the others the running products.
+template <int VG, int DP, int W>
+__global__ void __launch_bounds__(W * 32, DP == 256 || W == 16 ? 1 : 2) hgrn2_chunked_kernel(const RfHgrn2 p, int col_tiles) {
   pdl_prologue();
   using T = __nv_bfloat16;
-  constexpr int VT = VG * 16, DG = kHcWarps / VG, NV = VT / 16, DT = DP / 16 / DG;
-  using L = Hgrn2Geom<DP, VT>;
+  constexpr int kHcThreads = W * 32, TPT = W * 2;         // threads of the CTA, of a token in the epilogue
+  constexpr int VT = VG * 16, DG = W / VG, NV = VT / TPT, DT = DP / 16 / DG;
+  constexpr int PW = W / 2, PS = kHcTok / PW;             // warps of the in-block scores, source tokens of each
+  using L = Hgrn2Geom<DP, VT, W>;
   extern __shared__ __align__(16) uint8_t csm[];
   T* raw = reinterpret_cast<T*>(csm + L::raw);
   float* sq = reinterpret_cast<float*>(csm + L::sq);
@@ -429,7 +432,7 @@ __global__ void __launch_bounds__(kHcThreads, DP == 256 ? 1 : 2) hgrn2_chunked_k
   // output of the step before, still to be normalised: token row `orow`, values ov of channels ocol ..
   float ov[NV];
   int orow = -1;
-  const int otok = tid >> 4, ocol = (tid & 15) * NV;
+  const int otok = tid / TPT, ocol = (tid % TPT) * NV;
   float nw[NV];
 #pragma unroll
   for (int i = 0; i < NV; ++i) nw[i] = (p.norm_w && v0 + ocol + i < p.vdim) ? p.norm_w[v0 + ocol + i] : 1.f;
@@ -470,49 +473,76 @@ __global__ void __launch_bounds__(kHcThreads, DP == 256 ? 1 : 2) hgrn2_chunked_k
       *reinterpret_cast<float2*>(sf + t * L::kQLd + gc) = f;
     }
     __syncthreads();
-    if (warp < 4) {
-      // ---- P: source tokens warp, warp + 4, .. of this warp, the lanes over the key channels
-      float acc[4 * kHcTok];
+    if (warp < PW) {
+      // ---- P: source tokens warp, warp + PW, .. of this warp, the lanes over the key channels
+      float acc[PS * kHcTok];
 #pragma unroll
-      for (int i = 0; i < 4 * kHcTok; ++i) acc[i] = 0.f;
+      for (int i = 0; i < PS * kHcTok; ++i) acc[i] = 0.f;
       for (int c = lane * 4; c < DP; c += 128) {
-        float4 w[4];
+        float4 w[PS];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const float4 f0 = *reinterpret_cast<const float4*>(sf + (warp + 4 * i) * L::kQLd + c);
+        for (int i = 0; i < PS; ++i) {
+          const float4 f0 = *reinterpret_cast<const float4*>(sf + (warp + PW * i) * L::kQLd + c);
           w[i] = make_float4(1.f - f0.x, 1.f - f0.y, 1.f - f0.z, 1.f - f0.w);
         }
 #pragma unroll
         for (int t = 0; t < kHcTok; ++t) {
           const float4 f = *reinterpret_cast<const float4*>(sf + t * L::kQLd + c), q = *reinterpret_cast<const float4*>(sq + t * L::kQLd + c);
 #pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            if (t >= 4 * i) {                    // source token s = warp + 4 i cannot be later than t otherwise
-              const int s = warp + 4 * i;
+          for (int i = 0; i < PS; ++i) {
+            if (t >= PW * i) {                   // source token s = warp + PW i cannot be later than t otherwise
+              const int s = warp + PW * i;
               if (t > s) { w[i].x *= f.x; w[i].y *= f.y; w[i].z *= f.z; w[i].w *= f.w; }
               if (t >= s) acc[i * kHcTok + t] += fmaf(q.x, w[i].x, fmaf(q.y, w[i].y, fmaf(q.z, w[i].z, q.w * w[i].w)));
             }
           }
         }
       }
-      // sum over the lanes: halves of the 64 sums change sides until a lane holds two of them, index lane * 2 (+ 1)
+      // sum over the lanes: halves of the 16 PS sums change sides until a lane holds PL of them, from index lane * PL on
+      constexpr int PL = PS / 2;
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) {
         const bool up = (lane & o) != 0;
 #pragma unroll
-        for (int i = 0; i < 2 * kHcTok; ++i) {
-          if (i < 2 * o) {
-            const float send = up ? acc[i] : acc[i + 2 * o], keep = up ? acc[i + 2 * o] : acc[i];
+        for (int i = 0; i < PL * kHcTok; ++i) {
+          if (i < PL * o) {
+            const float send = up ? acc[i] : acc[i + PL * o], keep = up ? acc[i + PL * o] : acc[i];
             acc[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
           }
         }
       }
-      const int s = warp + 4 * (lane >> 3), t = (lane & 7) * 2;
-      hc_split(acc[0], ph[t * L::kPLd + s], pl[t * L::kPLd + s]);
-      hc_split(acc[1], ph[(t + 1) * L::kPLd + s], pl[(t + 1) * L::kPLd + s]);
+#pragma unroll
+      for (int i = 0; i < PL; ++i) {
+        const int at = lane * PL + i, s = warp + PW * (at / kHcTok), t = at % kHcTok;
+        hc_split(acc[i], ph[t * L::kPLd + s], pl[t * L::kPLd + s]);
+      }
+    } else if constexpr (W == 16) {
+      // ---- running products per key channel: from the block's start by the first DP threads, from its end by the next DP
+      for (int i = tid - PW * 32; i < 2 * DP; i += PW * 32) {
+        const int c = i % DP;
+        float f[kHcTok];
+#pragma unroll
+        for (int t = 0; t < kHcTok; ++t) f[t] = sf[t * L::kQLd + c];
+        if (i < DP) {
+          float G = 1.f;
+#pragma unroll
+          for (int t = 0; t < kHcTok; ++t) {
+            G *= f[t];
+            hc_split(sq[t * L::kQLd + c] * G, qh[t * L::kBLd + c], ql[t * L::kBLd + c]);
+          }
+          gt[c] = G;
+        } else {
+          float E = 1.f;
+#pragma unroll
+          for (int r = kHcTok - 1; r >= 0; --r) {
+            hc_split((1.f - f[r]) * E, kh[r * L::kBLd + c], kl[r * L::kBLd + c]);
+            E *= f[r];
+          }
+        }
+      }
     } else {
       // ---- running products per key channel
-      for (int c = tid - 128; c < DP; c += 128) {
+      for (int c = tid - PW * 32; c < DP; c += PW * 32) {
         float f[kHcTok], q[kHcTok];
 #pragma unroll
         for (int t = 0; t < kHcTok; ++t) { f[t] = sf[t * L::kQLd + c]; q[t] = sq[t * L::kQLd + c]; }
@@ -588,7 +618,7 @@ __global__ void __launch_bounds__(kHcThreads, DP == 256 ? 1 : 2) hgrn2_chunked_k
         for (int e = 0; e < 4; ++e) dst[(nt * 8 + q4 * 2 + (e & 1)) * L::kOLd + (e >> 1) * 8] = o[nt][e] + (o1[nt][e] + o2[nt][e]);
     }
     __syncthreads();
-    // ---- this step's outputs: sixteen threads per token
+    // ---- this step's outputs: TPT threads per token
     {
       float ss = 0.f;
 #pragma unroll
@@ -600,12 +630,12 @@ __global__ void __launch_bounds__(kHcThreads, DP == 256 ? 1 : 2) hgrn2_chunked_k
         ss += v * v;
       }
 #pragma unroll
-      for (int o = 8; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+      for (int o = TPT / 2; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
       orow = otok < valid ? q0 + b * kHcTok + otok : -1;
       if (col_tiles > 1) {
-        // lane c of a token's sixteen threads stores the sum into CTA c of the cluster
-        if ((tid & 15) < col_tiles)
-          st_dsmem_u32(dsmem_addr(smem_u32(csum + ((b & 1) * 8 + (int)cluster_ctarank()) * kHcTok + otok), (uint32_t)(tid & 15)), __float_as_uint(ss));
+        // thread c of a token's stores the sum into CTA c of the cluster
+        if (tid % TPT < col_tiles)
+          st_dsmem_u32(dsmem_addr(smem_u32(csum + ((b & 1) * 8 + (int)cluster_ctarank()) * kHcTok + otok), (uint32_t)(tid % TPT)), __float_as_uint(ss));
         __syncwarp();
         asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
       } else {
@@ -626,20 +656,20 @@ __global__ void __launch_bounds__(kHcThreads, DP == 256 ? 1 : 2) hgrn2_chunked_k
     }
 }
 
-template <int VG, int DP>
+template <int VG, int DP, int W>
 static int launch_chunked_t(const RfHgrn2* a, int tiles, cudaStream_t s) {
-  constexpr int smem = Hgrn2Geom<DP, VG * 16>::total;
-  RF_ALLOW_SMEM_PER_DEVICE((hgrn2_chunked_kernel<VG, DP>), smem);
-  RF_CUDA_CHECK(::rf::launch_k(hgrn2_chunked_kernel<VG, DP>, dim3(a->rows.num_seqs, a->heads, tiles), dim3(kHcThreads), smem, s, tiles, *a, tiles));
+  constexpr int smem = Hgrn2Geom<DP, VG * 16, W>::total;
+  RF_ALLOW_SMEM_PER_DEVICE((hgrn2_chunked_kernel<VG, DP, W>), smem);
+  RF_CUDA_CHECK(::rf::launch_k(hgrn2_chunked_kernel<VG, DP, W>, dim3(a->rows.num_seqs, a->heads, tiles), dim3(W * 32), smem, s, tiles, *a, tiles));
   ::rf::count_launch();
   return RF_OK;
 }
 
 template <int VG>
 static int launch_chunked(const RfHgrn2* a, int tiles, cudaStream_t s) {
-  if (a->dim <= 64) return launch_chunked_t<VG, 64>(a, tiles, s);
-  if (a->dim <= 128) return launch_chunked_t<VG, 128>(a, tiles, s);
-  return launch_chunked_t<VG, 256>(a, tiles, s);
+  if (a->dim <= 64) return launch_chunked_t<VG, 64, 8>(a, tiles, s);
+  if (a->dim <= 128) return launch_chunked_t<VG, 128, 8>(a, tiles, s);
+  return launch_chunked_t<VG, 256, 8>(a, tiles, s);
 }
 
 }  // namespace rf
@@ -688,13 +718,24 @@ extern "C" int rf_hgrn2_chunked(const RfHgrn2* a, rf_stream_t stream) {
   // wave on the form that holds a head of 128 by itself, with no sums to exchange, is ahead: 96 x 300, 64 x 128 channels 75 with 64, 70 with 128.
   // 32 channels for few heads, whose CTAs have their SMs to themselves: 8 x 1000 211 / 227, 12 x 300 65 / 70, 16 x 1000 252 / 227 (32 / 64); heads of
   // 256 values 4 x 1000 210 / 225, 8 x 1000 236 / 229; as long as there is an SM for each with more than 128 key channels: 32 x 1000, 256 x 128
-  // 299 / 353.  Not where 64 hold the whole head: 8 x 1000, 128 x 64 211 / 185.
+  // 299 / 353 (heads of 256 x 256 would be clusters of eight: 16 x 1000 599 / 354).  Not where 64 hold the whole head: 8 x 1000, 128 x 64 211 / 185.
   int vt = a->vdim <= 32 ? 32 : a->vdim <= 64 ? 64 : 128;
   const int halves = ceil_div(a->vdim, 64), quarters = ceil_div(a->vdim, 32);
   const long pairs = (long)a->rows.num_seqs * a->heads, sms = sm_count();
   const bool two_to_an_sm = a->dim <= 128 && (a->dim > 64 || a->vdim > 128);
   if (vt == 128 && halves <= 8 && pairs * halves <= (two_to_an_sm ? 2 : 1) * sms) vt = 64;
-  if (vt == 64 && quarters <= 8 && pairs * quarters <= (a->dim > 128 ? sms : a->vdim > 64 ? sms / 3 : 0)) vt = 32;
+  if (vt == 64 && quarters <= (a->dim > 128 ? 4 : 8) && pairs * quarters <= (a->dim > 128 ? sms : a->vdim > 64 ? sms / 3 : 0)) vt = 32;
+  // Heads of 65 to 128 key channels on sixteen warps, one CTA to an SM, from two fifths of the SMs up to all of them: a CTA holds a head of 128 values by
+  // itself, with no sums to exchange and nothing done twice, of larger ones 64.  us, two CTAs of eight warps to an SM / this: 4 x 1100 tokens, 16 heads of
+  // 128 x 128 294 / 259, 6 x 1100 337 / 262, 9 x 1000 308 / 238, 3 x 1000, 24 heads 269 / 237; 8 heads of 128 x 256 4 x 1000 286 / 245.  Fewer heads gain
+  // from having more CTAs: 2 x 1100, 16 heads 250 / 259.
+  if (a->dim > 64 && a->dim <= 128 && a->vdim > 64) {
+    const long ctas = a->vdim <= 128 ? pairs : pairs * halves;
+    if (5 * ctas >= 2 * sms && ctas <= sms && (a->vdim <= 128 || halves <= 8)) {
+      if (a->vdim <= 128) return launch_chunked_t<8, 128, 16>(a, 1, s);
+      return launch_chunked_t<4, 128, 16>(a, halves, s);
+    }
+  }
   const int tiles = ceil_div(a->vdim, vt);
   if (vt == 32) return launch_chunked<2>(a, tiles, s);
   if (vt == 64) return launch_chunked<4>(a, tiles, s);

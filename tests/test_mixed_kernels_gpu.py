@@ -253,6 +253,23 @@ def test_hgrn2_portions_of_many_heads(heads, D, VD):
     torch.testing.assert_close(a, b, rtol=1e-4, atol=1e-4)
 
 
+@pytest.mark.parametrize("heads,D,VD", [(9, 72, 72), (10, 72, 72), (12, 128, 128), (24, 96, 120), (25, 72, 72), (3, 72, 200), (6, 128, 136), (9, 128, 192), (4, 128, 520)])
+def test_hgrn2_on_sixteen_warps(heads, D, VD):
+    """The block form at both ends of the range where a CTA of sixteen warps has an SM to itself: whole heads of up to 128 values, 64 values of larger
+    ones, key and value channels that end inside a tile, against the token-by-token kernel."""
+    lens, pos0, slots = [1, 40, 2, 16, 17, 133], [4, 0, 33, 64, 0, 9], [5, 2, 0, 1, 4, 6]
+    d, _, _ = pack(lens, pos0, slots)
+    g = torch.Generator().manual_seed(heads + D + VD)
+    x = torch.randn(sum(lens), heads * (2 * D + VD), generator=g).to("cuda", torch.bfloat16)
+    fb, lower, nw = torch.randn(heads * D, generator=g).cuda(), torch.rand(heads * D, generator=g).cuda() ** 3, torch.randn(VD, generator=g).cuda()
+    a = torch.randn(7, heads, D, VD, generator=g).cuda()
+    b = a.clone()
+    got = K().hgrn2(x, fb, lower, nw, a, K().rows(**d), eps=1e-5, chunked=True)
+    want = K().hgrn2(x, fb, lower, nw, b, K().rows(**d), eps=1e-5)
+    close(got, want.double().cpu(), torch.bfloat16, 4)
+    torch.testing.assert_close(a, b, rtol=1e-4, atol=1e-4)
+
+
 def test_hgrn2_keeps_a_value_written_long_ago():
     """A channel whose gate stays open carries one token's value over hundreds of others."""
     D = VD = 64
