@@ -4,7 +4,7 @@
 // barriers, tensor-memory allocation, a ring whose stages are handed from warp to warp, and a cluster rendezvous on both sides of the split-K
 // reduction.  Here every warp has a ring of its own and feeds its own MMAs.
 //
-//  * A CTA of eight warps takes strips of 16 output features; its warps share a strip's 64-column k blocks.  Inside a block a lane
+//  * A CTA of eight warps takes strips of 16 output features (int8 also 32); its warps share a strip's 64-column k blocks.  Inside a block a lane
 //    (g = lane / 4, t = lane % 4) holds 16 bytes of rows g and g + 8: eight values (16-bit), sixteen (int8) or, with 8 bytes, sixteen
 //    (int4), all neighbours along k.  mma.sync does not care which k a slot stands for as long as both operands agree, so the lane's
 //    words are the A fragments as they come, and the same k range of token g is the B fragment: no shuffles, and no meeting of warps.
@@ -68,23 +68,24 @@ __device__ __forceinline__ uint16_t lds2(uint32_t a) {
 }
 
 // Ring of a warp: `depth` blocks of weights, each `bytes` (of every accumulator) long: 16 rows of 64 columns, behind int4 up to four scales a row.
-template <int BITS, bool DUAL, int NT> struct RowsRing {
+template <int BITS, bool DUAL, int NT, int SF> struct RowsRing {
   static constexpr int bytes = BITS == 16 ? 2048 : BITS == 8 ? 1024 : 512 + kRowsStrip * 8;
   // an int4 pair of 9 to 16 rows, whose sums take 34 KB: seven, so that a second CTA fits (fp16, us, with eight / seven: 12 x 12288 x 4096
   // SwiGLU, scales of 64 columns, 38.7 / 31.7, 16 x 9728 x 2560 23.3 / 17.4)
-  static constexpr int depth = DUAL ? (BITS == 16 ? 2 : BITS == 8 ? 4 : NT == 1 ? 8 : 7) : (BITS == 16 ? 4 : 8);
-  static constexpr int warp_bytes = depth * bytes * (DUAL ? 2 : 1);
+  static constexpr int depth = (DUAL ? (BITS == 16 ? 2 : BITS == 8 ? 4 : NT == 1 ? 8 : 7) : (BITS == 16 ? 4 : 8)) / SF;
+  static constexpr int slot_bytes = bytes * SF * (DUAL ? 2 : 1), warp_bytes = depth * slot_bytes;
   static constexpr int total = warp_bytes * kRowsWarps;
 };
 
-template <typename T, int BITS, bool DUAL, int NT>
+// SF: groups of 16 features in a strip
+template <typename T, int BITS, bool DUAL, int NT, int SF>
 __global__ void __launch_bounds__(kRowsWarps * 32, 2)
 gemm_rows_kernel(const GemmRowsParams p) {
-  using Ring = RowsRing<BITS, DUAL, NT>;
-  constexpr int kAcc = DUAL ? 2 : 1;
-  constexpr int kPitch = kRowsStrip + 1;
+  using Ring = RowsRing<BITS, DUAL, NT, SF>;
+  constexpr int kAcc = DUAL ? 2 : 1, kStrip = kRowsStrip * SF;
+  constexpr int kPitch = kStrip + 1, kSumBufs = SF == 1 ? 2 : 1;
   extern __shared__ __align__(128) uint8_t ring_mem[];
-  __shared__ float sums[2][kRowsWarps][kAcc][NT * 8][kPitch];
+  __shared__ float sums[kSumBufs][kRowsWarps][kAcc][NT * 8][kPitch];
   __shared__ float squares[kRowsWarps][NT * 8];
   __shared__ float rstd[NT * 8];
   static_assert(2 * (Ring::total + sizeof(sums) + sizeof(squares) + sizeof(rstd) + 1024) <= 228 * 1024, "two CTAs have to fit an SM");
@@ -97,11 +98,12 @@ gemm_rows_kernel(const GemmRowsParams p) {
   int as = blockIdx.x, aj = 0, aslot = 0;
   auto ask = [&] {
     if (nk > 0 && as < p.strips) {
-      const int rt = as >> 3, r0 = (as & 7) * kRowsStrip;           // 128-row tile, first row inside it
+      const int rt = as / (8 / SF), strip0 = (as % (8 / SF)) * kStrip;      // 128-row tile, first row inside it
 #pragma unroll
-      for (int c = 0; c < kAcc; ++c) {
+      for (int cf = 0; cf < kAcc * SF; ++cf) {
+        const int c = cf / SF, r0 = strip0 + cf % SF * kRowsStrip;
         const uint8_t* blk = p.w + ((size_t)(rt + c * p.dual_tiles) * KB + warp + aj * kRowsWarps) * p.blk_bytes;
-        const uint32_t dst = ring + (uint32_t)((aslot * kAcc + c) * Ring::bytes + lane * 16);
+        const uint32_t dst = ring + (uint32_t)(aslot * Ring::slot_bytes + cf * Ring::bytes + lane * 16);
         if constexpr (BITS == 16) {                                 // a lane copies what it will read: 16-byte pieces t and 4 + t of rows g and g + 8
 #pragma unroll
           for (int h = 0; h < 2; ++h) {
@@ -142,7 +144,7 @@ gemm_rows_kernel(const GemmRowsParams p) {
     }
   };
   if (nk > 0) load_x(0);
-  const int tok = tid >> 4, r = tid & 15;        // the value that this thread finishes in every strip
+  const int tok = tid >> 4, r = tid & 15;        // the value that this thread finishes in every group of 16 features
   const T* bias = reinterpret_cast<const T*>(p.bias);
   const T* scale = reinterpret_cast<const T*>(p.scale);
   const T* resid = reinterpret_cast<const T*>(p.residual);
@@ -152,16 +154,19 @@ gemm_rows_kernel(const GemmRowsParams p) {
   for (int strip = blockIdx.x; strip < p.strips; strip += gridDim.x, buf ^= 1) {
     const bool first = strip == (int)blockIdx.x;
     // what the epilogue adds and multiplies by is asked for ahead of the products
-    const int n_out = strip * kRowsStrip + r;
-    const bool mine = tok < p.M && n_out < p.N;
     const T one = Num<T>::from_f(1.f), zero = Num<T>::from_f(0.f);
-    T sc[2] = {one, one}, bi[2] = {zero, zero}, re = zero;
-    if (mine) {
-      if (scale) { sc[0] = scale[n_out]; if (DUAL) sc[1] = scale[p.dual_offset + n_out]; }
-      if (bias) { bi[0] = bias[n_out]; if (DUAL) bi[1] = bias[p.dual_offset + n_out]; }
-      if (resid) re = resid[(size_t)tok * p.ldr + n_out];
+    T sc[SF][2], bi[SF][2], re[SF];
+#pragma unroll
+    for (int f = 0; f < SF; ++f) {
+      const int n_out = strip * kStrip + f * kRowsStrip + r;
+      sc[f][0] = sc[f][1] = one;
+      bi[f][0] = bi[f][1] = re[f] = zero;
+      if (tok >= p.M || n_out >= p.N) continue;
+      if (scale) { sc[f][0] = scale[n_out]; if (DUAL) sc[f][1] = scale[p.dual_offset + n_out]; }
+      if (bias) { bi[f][0] = bias[n_out]; if (DUAL) bi[f][1] = bias[p.dual_offset + n_out]; }
+      if (resid) re[f] = resid[(size_t)tok * p.ldr + n_out];
     }
-    float acc[kAcc][NT][4] = {};
+    float acc[kAcc * SF][NT][4] = {};
     for (int j = 0; j < nk; ++j) {
       uint4 b[NT][2];
 #pragma unroll
@@ -181,8 +186,8 @@ gemm_rows_kernel(const GemmRowsParams p) {
           }
       }
 #pragma unroll
-      for (int c = 0; c < kAcc; ++c) {
-        const uint32_t src = ring + (uint32_t)((slot * kAcc + c) * Ring::bytes);
+      for (int c = 0; c < kAcc * SF; ++c) {
+        const uint32_t src = ring + (uint32_t)(slot * Ring::slot_bytes + c * Ring::bytes);
         uint4 q[2];
         uint2 q4[2];
         if constexpr (BITS == 8) { q[0] = lds16(src + lane * 16); q[1] = lds16(src + 512 + lane * 16); }
@@ -222,12 +227,16 @@ gemm_rows_kernel(const GemmRowsParams p) {
       if (++slot == Ring::depth) slot = 0;
     }
     // ---- the warps' sums: token rows of 16 features; two buffers, so one rendezvous per strip is enough
+    if constexpr (SF > 1) {
+      if (!first) __syncthreads();               // one buffer: the strip before has been read
+    }
 #pragma unroll
-    for (int c = 0; c < kAcc; ++c)
+    for (int c = 0; c < kAcc * SF; ++c)
 #pragma unroll
       for (int n = 0; n < NT; ++n)
 #pragma unroll
-        for (int i = 0; i < 4; ++i) sums[buf][warp][c][n * 8 + 2 * t + (i & 1)][g + 8 * (i >> 1)] = acc[c][n][i];
+        for (int i = 0; i < 4; ++i)
+          sums[kSumBufs == 2 ? buf : 0][warp][c / SF][n * 8 + 2 * t + (i & 1)][c % SF * kRowsStrip + g + 8 * (i >> 1)] = acc[c][n][i];
     if (p.norm && first) {
 #pragma unroll
       for (int n = 0; n < NT; ++n) {
@@ -246,20 +255,23 @@ gemm_rows_kernel(const GemmRowsParams p) {
       }
       __syncthreads();
     }
-    if (mine) {
+#pragma unroll
+    for (int f = 0; f < SF; ++f) {
+      const int n_out = strip * kStrip + f * kRowsStrip + r;
+      if (tok >= p.M || n_out >= p.N) continue;
       float gate = 0.f, up = 0.f;
 #pragma unroll
       for (int w = 0; w < kRowsWarps; ++w) {
-        gate += sums[buf][w][0][tok][r];
-        if (DUAL) up += sums[buf][w][kAcc - 1][tok][r];
+        gate += sums[kSumBufs == 2 ? buf : 0][w][0][tok][f * kRowsStrip + r];
+        if (DUAL) up += sums[kSumBufs == 2 ? buf : 0][w][kAcc - 1][tok][f * kRowsStrip + r];
       }
       const float rs = p.norm ? rstd[tok] * row_scale : row_scale;
       gate *= rs;
       up *= rs;
-      if (scale) { gate *= Num<T>::to_f(sc[0]); up *= Num<T>::to_f(sc[1]); }
-      if (bias) { gate += Num<T>::to_f(bi[0]); up += Num<T>::to_f(bi[1]); }
+      if (scale) { gate *= Num<T>::to_f(sc[f][0]); up *= Num<T>::to_f(sc[f][1]); }
+      if (bias) { gate += Num<T>::to_f(bi[f][0]); up += Num<T>::to_f(bi[f][1]); }
       float v = apply_act(p.act, gate, up, p.act_args);
-      if (resid) v += Num<T>::to_f(re);
+      if (resid) v += Num<T>::to_f(re[f]);
       reinterpret_cast<T*>(p.out)[(size_t)tok * p.ldo + n_out] = Num<T>::from_f(v);
     }
   }
@@ -287,14 +299,14 @@ bool gemm_rows_takes(const RfGemm* g) {
   return (int64_t)g->N * g->K <= (8 << 20) || (g->K <= 4096 && g->N <= 2 * kRowsStrip * sm_count());
 }
 
-template <typename T, int BITS, bool DUAL, int NT>
-static int launch_rows(const RfGemm* g, cudaStream_t stream) {
-  auto kfn = gemm_rows_kernel<T, BITS, DUAL, NT>;
+template <typename T, int BITS, bool DUAL, int NT, int SF>
+static int launch_rows_sf(const RfGemm* g, cudaStream_t stream) {
+  auto kfn = gemm_rows_kernel<T, BITS, DUAL, NT, SF>;
   GemmRowsParams p = {};
   p.x = g->x; p.ldx = g->ldx; p.out = g->out; p.ldo = g->ldo; p.residual = g->residual; p.ldr = g->ldr;
   p.bias = g->bias; p.scale = g->scale; p.row_scale = g->row_scale;
   p.w = reinterpret_cast<const uint8_t*>(g->w);
-  p.M = g->M; p.N = g->N; p.K = g->K; p.k_blocks = ceil_div(g->K, kRowsBK); p.strips = ceil_div(g->N, kRowsStrip);
+  p.M = g->M; p.N = g->N; p.K = g->K; p.k_blocks = ceil_div(g->K, kRowsBK); p.strips = ceil_div(g->N, kRowsStrip * SF);
   p.act = g->act; p.act_args = {g->act_limit, g->act_alpha}; p.dual_offset = g->dual_offset; p.dual_tiles = ceil_div(g->N, 128);
   p.blk_bytes = BITS == 16 ? 16384 : BITS == 8 ? 8192 : rf_w4_block_bytes(g->w_group);
   p.ns = BITS == 4 && g->w_group > 0 ? kRowsBK / std::min(g->w_group, kRowsBK) : 0;
@@ -302,11 +314,23 @@ static int launch_rows(const RfGemm* g, cudaStream_t stream) {
   p.norm = g->norm_x;
   p.inv_dim = g->ss_dim > 0 ? 1.f / (float)g->ss_dim : 0.f;
   p.eps = g->ss_eps;
-  constexpr int smem = RowsRing<BITS, DUAL, NT>::total;
+  constexpr int smem = RowsRing<BITS, DUAL, NT, SF>::total;
   RF_ALLOW_SMEM_PER_DEVICE(kfn, smem);
   RF_CUDA_CHECK(::rf::launch_k(kfn, dim3(std::min(p.strips, 2 * sm_count())), dim3(kRowsWarps * 32), smem, stream, 1, p));
   ::rf::count_launch();
   return RF_OK;
+}
+
+template <typename T, int BITS, bool DUAL, int NT>
+static int launch_rows(const RfGemm* g, cudaStream_t stream) {
+  // Strips of 32 features read x half as often, which with int8 weights is as many bytes as the weights themselves, as long as there is one for every SM.
+  // int8, fp16, us, 16 / 32: 1 x 151936 x 4096 118 / 94 (the copy rate), 12 rows 167 / 126, 1 x 6144 x 4096 9.9 / 7.8, 12 rows 12.2 / 9.5, 8 x 9728 x 2048
+  // 9.5 / 7.5; 1 x 4096 x 4096 6.2 / 6.9, 12 x 4096 x 12288 17.0 / 21.5.  Not GLU pairs, whose ring gets too short (12 x 12288 x 4096 24.5 / 27.4), nor
+  // 16-bit weights (1 x 9728 x 2048 9.5 / 10.7).
+  if constexpr (BITS == 8 && !DUAL) {
+    if (ceil_div(g->N, 2 * kRowsStrip) > sm_count()) return launch_rows_sf<T, BITS, DUAL, NT, 2>(g, stream);
+  }
+  return launch_rows_sf<T, BITS, DUAL, NT, 1>(g, stream);
 }
 
 template <typename T, int BITS, int NT>

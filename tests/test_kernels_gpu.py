@@ -1090,6 +1090,23 @@ def test_attn_prefill_heads_of_80(dt, heads, lens, mode, status):
 
 
 @pytest.mark.parametrize("dt", DT)
+@pytest.mark.parametrize("M,N,K", [(1, 4744, 64), (3, 5000, 1040), (8, 4768, 2048), (9, 9999, 528), (16, 20001, 1024)])
+def test_gemm_very_few_rows_int8_wide(dt, M, N, K, status):
+    """int8 weights in strips of 32 features: a last strip with one group of 16 or part of it, fewer k blocks than warps, several strips to a CTA, scale,
+    bias, residual and an odd output pitch."""
+    from rhinoforge_b200.ops import kernels as K_
+    x = (torch.randn(M, K, device="cuda") * 0.5).to(dt)
+    q = torch.randint(-127, 128, (N, K), device="cuda", dtype=torch.int8)
+    sc, b = (torch.rand(N, device="cuda") * 0.02 + 0.002).to(dt), torch.randn(N, device="cuda").to(dt)
+    r, out = torch.randn(M, N, device="cuda").to(dt), torch.full((M, N + 3), 7.0, device="cuda").to(dt)
+    assert K_.gemm_plan(M, N, K, dtype=dt, int8=True)["kernel"] == "rows"
+    y = K_.gemm(x, K_.pack_weight(q), packed_shape=(N, K), scale=sc, bias=b, residual=r, out=out[:, :N], status=status)
+    ref = x.float() @ q.float().t() * sc.float() + b.float() + r.float()
+    _close(y, ref, dt, scale=max(1.0, ref.abs().max().item()))
+    assert bool((out[:, N:] == 7.0).all())
+
+
+@pytest.mark.parametrize("dt", DT)
 @pytest.mark.parametrize("H", [8, 264, 1024, 1152, 2040, 3072, 4096, 4104])
 @pytest.mark.parametrize("rows", [295, 1301, 3001])
 def test_norms_of_many_rows(dt, H, rows):
