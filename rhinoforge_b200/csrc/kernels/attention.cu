@@ -96,11 +96,47 @@ __device__ __forceinline__ void pv_page(float (&o)[HD / 8][4], const uint32_t (&
   }
 }
 
-// ------------------------------------------------------------------ decode --
+// One head of a token, eight values to a lane: RMSNorm by `w` (null: none) and rotation, with the roundings of qk_norm_rope_kv_vec_kernel
+// (rope_kv.cu).  All lanes of the warp take part.
 template <typename T, int HD>
+__device__ __forceinline__ void norm_rotate_head(float (&x)[8], const T* w, const AttnInsert& a, int lane, const float (&cs)[8], const float (&sn)[8]) {
+  constexpr int GROUP = HD / 8;
+  const int o = (lane % GROUP) * 8, half = a.rot_dim >> 1, hl = half >> 3;
+  const int region = o < half ? 0 : (o < a.rot_dim ? 1 : 2);
+  const int partner = lane + (region == 0 ? hl : (region == 1 ? -hl : 0));
+  auto norm = [&]() {
+    float s2 = 0.f;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) s2 += x[j] * x[j];
+#pragma unroll
+    for (int d = GROUP / 2; d >= 1; d >>= 1) s2 += __shfl_xor_sync(0xffffffffu, s2, d);
+    if (w) {
+      const float rstd = rsqrtf(s2 / (float)HD + a.eps);
+      float wv[8];
+      load8(w + o, wv);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) x[j] = (a.norm_mode & 1) ? x[j] * rstd * (1.f + wv[j]) : wv[j] * Num<T>::to_f(Num<T>::from_f(x[j] * rstd));
+    }
+  };
+  auto rope = [&]() {
+    if (!a.cos || a.rot_dim <= 0) return;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const float own = Num<T>::to_f(Num<T>::from_f(x[j]));
+      const float oth = __shfl_sync(0xffffffffu, own, partner);
+      if (region < 2) x[j] = region == 0 ? own * cs[j] - oth * sn[j] : own * cs[j] + oth * sn[j];
+    }
+  };
+  if (a.rope_before_norm) { rope(); norm(); } else { norm(); rope(); }
+}
+
+// ------------------------------------------------------------------ decode --
+// INSERT: the query heads, and the key head whose page the CTA has, are normalised and rotated here, and that key and value go to their page:
+// a launch less per layer (step-by-step decode of 28 small layers: the insertion kernel's 2.8 us each).
+template <typename T, int HD, bool INSERT>
 __global__ void __launch_bounds__(160)
 attn_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
-                   const AttnParams p) {
+                   const AttnParams p, const AttnInsert ins) {
   pdl_prologue();
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw_addr = smem_u32(smem_raw);
@@ -193,10 +229,52 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
       if ((lane >> 2) < R) rate0 = p.rates[head_of(lane >> 2)];
       if ((lane >> 2) + 8 < R) rate1 = p.rates[head_of((lane >> 2) + 8)];
     }
+    constexpr int kNewLd = HD + 8;
+    static_assert(sizeof(AttnCtl) % 16 == 0, "16-byte rows behind it");
+    T* fresh = reinterpret_cast<T*>(ctl + 1);               // INSERT: [R] query heads, then the new key, then its value
+    int new_page = -1, new_slot = 0;                        // the new token's page among this CTA's, or -1; its row of it
+    if constexpr (INSERT) {
+      constexpr int GROUP = HD / 8, HPW = 32 / GROUP;
+      const int gl = lane % GROUP, o = gl * 8, half = ins.rot_dim >> 1;
+      const T* row = reinterpret_cast<const T*>(p.q) + (size_t)seq * p.ldq;
+      const int pos0 = ins.pos[(size_t)seq * ins.pos_stride], cpos = ins.cache_pos ? ins.cache_pos[seq] : pos0;
+      float cs[8], sn[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) { cs[j] = 1.f; sn[j] = 0.f; }
+      if (ins.cos && o < ins.rot_dim) {
+        const size_t at = (size_t)pos0 * half + (o < half ? o : o - half);
+        const float4 c0 = *reinterpret_cast<const float4*>(ins.cos + at), c1 = *reinterpret_cast<const float4*>(ins.cos + at + 4);
+        const float4 s0 = *reinterpret_cast<const float4*>(ins.sin + at), s1 = *reinterpret_cast<const float4*>(ins.sin + at + 4);
+        cs[0] = c0.x; cs[1] = c0.y; cs[2] = c0.z; cs[3] = c0.w; cs[4] = c1.x; cs[5] = c1.y; cs[6] = c1.z; cs[7] = c1.w;
+        sn[0] = s0.x; sn[1] = s0.y; sn[2] = s0.z; sn[3] = s0.w; sn[4] = s1.x; sn[5] = s1.y; sn[6] = s1.z; sn[7] = s1.w;
+      }
+      new_slot = cpos & 15;
+      if (cpos >= 0 && (cpos >> 4) >= pg_begin && (cpos >> 4) < pg_end) new_page = (cpos >> 4) - pg_begin;
+      // a token beyond the keys that are read is still put away, by the first split
+      const bool writes = new_page >= 0 || (split == 0 && cpos >= 0 && (cpos >> 4) >= total_pages);
+      for (int h0 = warp * HPW; h0 < R + 2; h0 += 4 * HPW) {
+        const int h = h0 + lane / GROUP;                    // query heads, key, value
+        const int col = h < R ? head_of(h) : h == R ? p.Hq + kvh : p.Hq + p.Hkv + kvh;
+        const uint4 raw = h < R + 2 ? *reinterpret_cast<const uint4*>(row + (size_t)col * HD + o) : make_uint4(0u, 0u, 0u, 0u);
+        float x[8];
+        unpack8<T>(raw, x);
+        norm_rotate_head<T, HD>(x, reinterpret_cast<const T*>(h < R ? ins.q_norm_w : ins.k_norm_w), ins, lane, cs, sn);
+        if (h <= R) store8(fresh + h * kNewLd + o, x);
+        else if (h == R + 1) *reinterpret_cast<uint4*>(fresh + h * kNewLd + o) = raw;
+        if (writes && h >= R && h < R + 2) {
+          const size_t at = ((size_t)p.page_table[(size_t)pt_row * p.pt_stride + (cpos >> 4)] * p.Hkv + kvh) * 16 + new_slot;
+          if (h == R) store8(reinterpret_cast<T*>(ins.k_pool) + at * HD + o, x);
+          else *reinterpret_cast<uint4*>(reinterpret_cast<T*>(ins.v_pool) + at * HD + o) = raw;
+        }
+      }
+      asm volatile("bar.sync 1, 128;" ::: "memory");        // the four consumer warps
+    }
     {
       const int g0 = lane >> 2, g1 = g0 + 8;
-      const T* q0 = reinterpret_cast<const T*>(p.q) + (size_t)row_of(g0 < R ? g0 : 0) * p.ldq + (size_t)head_of(g0 < R ? g0 : 0) * HD;
-      const T* q1 = reinterpret_cast<const T*>(p.q) + (size_t)row_of(g1 < R ? g1 : 0) * p.ldq + (size_t)head_of(g1 < R ? g1 : 0) * HD;
+      const T* q0 = INSERT ? fresh + (g0 < R ? g0 : 0) * kNewLd
+                           : reinterpret_cast<const T*>(p.q) + (size_t)row_of(g0 < R ? g0 : 0) * p.ldq + (size_t)head_of(g0 < R ? g0 : 0) * HD;
+      const T* q1 = INSERT ? fresh + (g1 < R ? g1 : 0) * kNewLd
+                           : reinterpret_cast<const T*>(p.q) + (size_t)row_of(g1 < R ? g1 : 0) * p.ldq + (size_t)head_of(g1 < R ? g1 : 0) * HD;
 #pragma unroll
       for (int ks = 0; ks < HD / 16; ++ks) {
         const int col = ks * 16 + (lane & 3) * 2;
@@ -218,6 +296,17 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
       if (pgl < npg) {
         const uint32_t kbase = smem_u32(smem + (size_t)s * kStageBytes + warp * kPageBytes);
         const uint32_t vbase = kbase + (HD / 64) * kBoxBytes;
+        if (INSERT && pgl == new_page) {
+          // the page as it came may be without the new token, or with part of it
+          for (int i = lane; i < HD / 4; i += 32) {
+            const int c = i % (HD / 8), v = i / (HD / 8);
+            const uint4 w = *reinterpret_cast<const uint4*>(fresh + (R + v) * kNewLd + c * 8);
+            asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(swz128((v ? vbase : kbase) + (c >> 3) * kBoxBytes, new_slot, c & 7)), "r"(w.x), "r"(w.y),
+                         "r"(w.z), "r"(w.w) : "memory");
+          }
+          fence_proxy_async();                              // ahead of the copy that may follow into this stage
+          __syncwarp();
+        }
         float s0[4] = {0.f, 0.f, 0.f, 0.f}, s1[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
         for (int ks = 0; ks < HD / 16; ++ks) qk_step<T>(s0, s1, qf[ks], kbase, ks, lane);
@@ -685,10 +774,10 @@ static DecodeSplitPlan plan_decode_split(int num_seqs, int rows_per_seq, int Hq,
 }
 
 // Clusters of `size` CTAs of the kernel that the current device holds at once (asked once per kernel, device and size)
-template <typename T, int HD>
+template <typename T, int HD, bool INSERT>
 static long clusters_resident(int size, size_t smem) {
   static std::atomic<int> known[64][9];
-  auto kfn = attn_decode_kernel<T, HD>;
+  auto kfn = attn_decode_kernel<T, HD, INSERT>;
   const int dev = device_ordinal();
   const bool track = dev >= 0 && dev < 64;
   if (track) {
@@ -710,8 +799,8 @@ static long clusters_resident(int size, size_t smem) {
   return n;
 }
 
-template <typename T, int HD>
-static int launch_decode(const RfAttn* a, AttnParams& p, cudaStream_t s) {
+template <typename T, int HD, bool INSERT>
+static int launch_decode_as(const RfAttn* a, AttnParams& p, const AttnInsert& ins, cudaStream_t s) {
   CUtensorMap tmK, tmV;
   int rc = kv_tmaps(a, &tmK, &tmV);
   if (rc) return rc;
@@ -720,8 +809,8 @@ static int launch_decode(const RfAttn* a, AttnParams& p, cudaStream_t s) {
   int stages = HD == 256 ? 2 : (HD == 128 ? 3 : 4);
   while (stages * kStageBytes < merge_bytes) ++stages;
   p.stages = stages;
-  const size_t smem = (size_t)stages * kStageBytes + sizeof(AttnCtl) + 1024 + 64;
-  auto kfn = attn_decode_kernel<T, HD>;
+  const size_t smem = (size_t)stages * kStageBytes + sizeof(AttnCtl) + 1024 + 64 + (INSERT ? (std::min(p.G, 16) + 2) * (HD + 8) * 2 : 0);
+  auto kfn = attn_decode_kernel<T, HD, INSERT>;
   RF_ALLOW_SMEM_PER_DEVICE(kfn, 200 * 1024);
   // split the KV range so that small batches still fill the machine
   // a chunk or window may begin anywhere in a page: one page more than its own size; the kept first positions end anywhere
@@ -741,7 +830,7 @@ static int launch_decode(const RfAttn* a, AttnParams& p, cudaStream_t s) {
   for (int n = splits; splits <= 8 && n > 1 && 2 * n >= splits; --n) {
     const int pages = n == splits ? pl.pages_per_split : round_up(ceil_div(pl.max_pages, n), 4), parts = ceil_div(pl.max_pages, pages);
     if (n < splits && pages * HD > 48 * 128 && 15 * busiest(parts, pages) > (HD == 256 ? 19 : 18) * busiest(splits, pl.pages_per_split)) break;
-    if (parts > 1 && (long)a->Hkv * p.g_tiles * a->num_seqs < clusters_resident<T, HD>(parts, smem)) {
+    if (parts > 1 && (long)a->Hkv * p.g_tiles * a->num_seqs < clusters_resident<T, HD, INSERT>(parts, smem)) {
       p.cluster = 1;
       splits = parts;
       p.pages_per_split = pages;
@@ -760,7 +849,7 @@ static int launch_decode(const RfAttn* a, AttnParams& p, cudaStream_t s) {
     p.kv_stream = ef && p.g_tiles == 1;      // pages that several CTAs of the launch read stay
   }
   const dim3 grid(a->Hkv * p.g_tiles, a->num_seqs, splits);
-  RF_CUDA_CHECK(::rf::launch_k(kfn, grid, dim3(160), smem, s, p.cluster ? splits : 1, tmK, tmV, p));
+  RF_CUDA_CHECK(::rf::launch_k(kfn, grid, dim3(160), smem, s, p.cluster ? splits : 1, tmK, tmV, p, ins));
   ::rf::count_launch();
   if (splits > 1 && !p.cluster) {
     const dim3 g2(a->Hq, a->num_seqs * p.rows_per_seq);
@@ -768,6 +857,11 @@ static int launch_decode(const RfAttn* a, AttnParams& p, cudaStream_t s) {
     ::rf::count_launch();
   }
   return RF_OK;
+}
+
+template <typename T, int HD>
+static int launch_decode(const RfAttn* a, AttnParams& p, cudaStream_t s) {
+  return launch_decode_as<T, HD, false>(a, p, AttnInsert{}, s);
 }
 
 template <typename T, int HD>
@@ -831,6 +925,40 @@ extern "C" int rf_attn_decode(const RfAttn* a, rf_stream_t stream) {
   RF_REQUIRE(a->max_kv_len > 0, "decode attention needs max_kv_len");
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   RF_ATTN_DISPATCH(launch_decode)
+}
+
+// Whether rf_attn_decode_insert takes the pair: one row per sequence that sees its whole cache, heads and operands that the 16-byte form of
+// rf_qk_norm_rope_kv takes with one position axis, at most 16 query heads to a K/V head, and nothing that wants the rotated rows themselves.
+extern "C" int rf_attn_decode_inserts(const RfAttn* a, const RfRopeKv* r) {
+  if (!a || !r || !a->k_pool || a->num_seqs <= 0 || a->rows_per_seq > 1 || a->pos || a->slot || a->window > 0 || a->chunk > 0 || a->keep_first > 0) return 0;
+  if ((a->hd != 64 && a->hd != 128 && a->hd != 256) || a->Hkv <= 0 || a->Hq % a->Hkv || a->Hq / a->Hkv > 16) return 0;
+  if (r->qkv != a->q || r->ld != a->ldq || r->tokens != a->num_seqs || r->Hq != a->Hq || r->Hkv != a->Hkv || r->hd != a->hd || r->dtype != a->dtype) return 0;
+  if (r->k_pool != a->k_pool || r->v_pool != a->v_pool || r->page_table != a->page_table || r->pt_stride != a->pt_stride) return 0;
+  if (r->seq_of_tok || r->axis_of_freq || r->q_out || r->write_k_inplace || r->v_norm || !r->pos || r->pos_stride < 1) return 0;
+  if (r->rot_dim % 16 || r->rot_dim < 0 || r->rot_dim > r->hd || r->ld % 8) return 0;
+  const auto at = [](const void* x) { return reinterpret_cast<uintptr_t>(x); };
+  return ((at(r->qkv) | at(r->k_pool) | at(r->v_pool) | at(r->q_norm_w) | at(r->k_norm_w) | at(r->cos) | at(r->sin)) & 15) == 0;
+}
+
+// rf_qk_norm_rope_kv followed by rf_attn_decode in one launch; the rows of the QKV buffer stay as they are.
+extern "C" int rf_attn_decode_insert(const RfAttn* a, const RfRopeKv* r, rf_stream_t stream) {
+  RF_SKIP_IF_REPLAYING();
+  RF_REQUIRE(rf_attn_decode_inserts(a, r), "decode attention does not insert for these operands (see rf_attn_decode_inserts)");
+  AttnParams p;
+  int rc = fill_params(a, &p);
+  if (rc) return rc;
+  RF_REQUIRE(a->num_seqs <= 65535, "decode attention: %d rows in one launch", a->num_seqs);
+  RF_REQUIRE(a->max_kv_len > 0, "decode attention needs max_kv_len");
+  const AttnInsert ins = {const_cast<void*>(r->k_pool), const_cast<void*>(r->v_pool), r->q_norm_w, r->k_norm_w, r->rot_dim > 0 ? r->cos : nullptr, r->sin,
+                          r->pos, r->pos_stride, r->cache_pos, r->eps, r->norm_mode, r->rope_before_norm, r->rot_dim};
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+#define RF_INSERT(T)                                                            \
+  if (a->hd == 64) return launch_decode_as<T, 64, true>(a, p, ins, s);           \
+  if (a->hd == 128) return launch_decode_as<T, 128, true>(a, p, ins, s);         \
+  return launch_decode_as<T, 256, true>(a, p, ins, s);
+  if (a->dtype == 0) { RF_INSERT(__half) }
+  RF_INSERT(__nv_bfloat16)
+#undef RF_INSERT
 }
 
 namespace rf {

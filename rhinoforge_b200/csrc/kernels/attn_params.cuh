@@ -34,6 +34,17 @@ struct AttnParams {
   int32_t cluster;        // decode: the splits of a (sequence, K/V head) are one thread-block cluster
 };
 
+// What a decode launch that inserts needs of RfRopeKv (`q` is the QKV buffer as its GEMM left it, one row per sequence).
+struct AttnInsert {
+  void* k_pool; void* v_pool;
+  const void* q_norm_w; const void* k_norm_w;
+  const float* cos; const float* sin;
+  const int32_t* pos; int32_t pos_stride;
+  const int32_t* cache_pos;
+  float eps;
+  int32_t norm_mode, rope_before_norm, rot_dim;
+};
+
 constexpr float kLog2e = 1.4426950408889634f;
 // log2(1 + rate * distance); distances in front of a row (masked by the caller) may give anything
 __device__ __forceinline__ float log2_distance(float rate, float distance) {

@@ -455,6 +455,8 @@ static int forward(Stack& s, const RfStackForward& f, cudaStream_t st) {
                   false, st);
     if (rc) return rc;
     // twin q/k norm weights that differ from the layer's own: the per-head norm + rope + KV insert runs per row range
+    RfRopeKv insert = {};                  // a decode step's norm, rotation and insertion, when its attention launch may do them
+    bool one_insert = false;
     const bool twin_qk = twin && c.qk_norm && tw->q_norm_w && (tw->q_norm_w != w.q_norm_w || tw->k_norm_w != w.k_norm_w);
     for (int part = 0; part < (twin_qk ? 2 : 1); ++part) {
       const int r0 = part == 0 ? 0 : split, rn = twin_qk ? (part == 0 ? split : T - split) : T;
@@ -479,6 +481,11 @@ static int forward(Stack& s, const RfStackForward& f, cudaStream_t st) {
       const bool needed = a.q_norm_w || a.rot_dim > 0 || c.paged_kv;
       if (needed) {
         RF_REQUIRE(f.pos != nullptr, "forward: positions are required");
+        if (f.decode && !twin_qk) {
+          insert = a;
+          one_insert = true;
+          continue;
+        }
         rc = rf_qk_norm_rope_kv(&a, st);
         if (rc) return rc;
       }
@@ -504,7 +511,15 @@ static int forward(Stack& s, const RfStackForward& f, cudaStream_t st) {
         RF_REQUIRE(c.window <= 0, "decode attention has no sliding-window form: a stack with window=%d would prefill "
                    "with the window and decode over the whole context", c.window);
         a.ws = s.at<float>(s.off_attn_ws); a.ws_bytes = s.attn_ws_bytes; a.rows_per_seq = f.rows_per_seq;
-        rc = rf_attn_decode(&a, st);
+        if (one_insert && rf_attn_decode_inserts(&a, &insert)) {
+          rc = rf_attn_decode_insert(&a, &insert, st);
+        } else {
+          if (one_insert) {
+            rc = rf_qk_norm_rope_kv(&insert, st);
+            if (rc) return rc;
+          }
+          rc = rf_attn_decode(&a, st);
+        }
       } else {
         a.q_start = f.q_start; a.q_len = f.q_len;
         a.causal = c.causal; a.window = c.window;

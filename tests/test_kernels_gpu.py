@@ -1107,6 +1107,61 @@ def test_gemm_very_few_rows_int8_wide(dt, M, N, K, status):
 
 
 @pytest.mark.parametrize("dt", DT)
+@pytest.mark.parametrize("hd,Hq,Hkv,rot", [(64, 8, 8, 64), (64, 32, 2, 32), (128, 16, 8, 128), (128, 14, 1, 0), (256, 8, 1, 64)])
+@pytest.mark.parametrize("lens", [[300], [1, 16, 17, 33, 160], [700] * 40, [1500, 15, 16, 3000, 2, 999, 64]])
+@pytest.mark.parametrize("mode", [(True, 0, 0), (True, 1, 1), (False, 0, 0)])
+def test_attn_decode_inserts(dt, hd, Hq, Hkv, rot, lens, mode, status):
+    """Decode attention that normalises, rotates and inserts itself against the two launches, bit for bit, pool included: new tokens in the first and
+    last row of a page and in a page of their own, one and several splits, a row whose token goes nowhere, one that lies behind the keys read."""
+    import ctypes as C
+    from rhinoforge_b200 import _native as N
+    from rhinoforge_b200.ops import kernels as K_
+    norms, gemma, rope_first = mode
+    n, maxp = len(lens), (max(lens) + 15) // 16 + 2
+    g = torch.Generator(device="cuda").manual_seed(hd + n)
+    qkv = torch.randn(n, (Hq + 2 * Hkv) * hd + 8, device="cuda", generator=g).to(dt)
+    pools = torch.randn(2, n * maxp, Hkv, 16, hd, device="cuda", generator=g).to(dt)
+    pt = torch.randperm(n * maxp, device="cuda", generator=g).to(torch.int32).view(n, maxp)
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")
+    kv_len, pos = i32(lens), i32([l - 1 for l in lens])
+    cache_pos = pos.clone()
+    if n > 2:
+        cache_pos[1], cache_pos[2] = -1, cache_pos[2] + 16
+    cos, sin = torch.randn(max(lens), max(rot, 2) // 2, device="cuda"), torch.randn(max(lens), max(rot, 2) // 2, device="cuda")
+    qn, kn = (1 + 0.1 * torch.randn(2, hd, device="cuda")).to(dt)
+    ws = K_.attn_decode_scratch(n, Hq, hd, "cuda")
+
+    def run(fused):
+        rows, kp, vp = qkv.clone(), pools[0].clone(), pools[1].clone()
+        out = torch.zeros(n, Hq * hd, device="cuda", dtype=dt)
+        r, a = N.RfRopeKv(), N.RfAttn()
+        r.qkv, r.ld, r.tokens, r.Hq, r.Hkv, r.hd, r.rot_dim = rows.data_ptr(), rows.stride(0), n, Hq, Hkv, hd, rot
+        if norms:
+            r.q_norm_w, r.k_norm_w = qn.data_ptr(), kn.data_ptr()
+        r.eps, r.norm_mode, r.rope_before_norm, r.dtype = 1e-6, gemma, rope_first, 0 if dt == torch.float16 else 1
+        r.cos, r.sin, r.pos, r.pos_stride, r.cache_pos = cos.data_ptr(), sin.data_ptr(), pos.data_ptr(), 1, cache_pos.data_ptr()
+        r.k_pool, r.v_pool, r.page_table, r.pt_stride = kp.data_ptr(), vp.data_ptr(), pt.data_ptr(), maxp
+        a.q, a.ldq, a.out, a.ldo, a.q_rows_total = rows.data_ptr(), rows.stride(0), out.data_ptr(), out.stride(0), n
+        a.k_pool, a.v_pool, a.pool_pages, a.page_table, a.pt_stride = kp.data_ptr(), vp.data_ptr(), n * maxp, pt.data_ptr(), maxp
+        a.num_seqs, a.Hq, a.Hkv, a.hd, a.kv_len, a.max_kv_len, a.dtype = n, Hq, Hkv, hd, kv_len.data_ptr(), max(lens), r.dtype
+        a.ws, a.ws_bytes, a.status, a.rows_per_seq = ws.data_ptr(), ws.numel() * 4, status.data_ptr(), 1
+        L, st = N.lib(), C.c_void_p(torch.cuda.current_stream().cuda_stream)
+        if fused:
+            assert L.rf_attn_decode_inserts(C.byref(a), C.byref(r)) == 1
+            N.check(L.rf_attn_decode_insert(C.byref(a), C.byref(r), st), "insert")
+            assert torch.equal(rows, qkv)
+            r.seq_of_tok = pos.data_ptr()                       # a token that may belong elsewhere: two launches, refused here
+            assert L.rf_attn_decode_inserts(C.byref(a), C.byref(r)) == 0 and L.rf_attn_decode_insert(C.byref(a), C.byref(r), st) != 0
+        else:
+            N.check(L.rf_qk_norm_rope_kv(C.byref(r), st), "rope")
+            N.check(L.rf_attn_decode(C.byref(a), st), "decode")
+        return out, kp, vp
+
+    for x, y in zip(run(True), run(False)):
+        assert torch.equal(x, y)
+
+
+@pytest.mark.parametrize("dt", DT)
 @pytest.mark.parametrize("H", [8, 264, 1024, 1152, 2040, 3072, 4096, 4104])
 @pytest.mark.parametrize("rows", [295, 1301, 3001])
 def test_norms_of_many_rows(dt, H, rows):
