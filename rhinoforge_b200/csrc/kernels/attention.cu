@@ -137,7 +137,7 @@ template <typename T, int HD, bool INSERT>
 __global__ void __launch_bounds__(160)
 attn_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
                    const AttnParams p, const AttnInsert ins) {
-  pdl_prologue();
+  pdl_launch_dependents();
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw_addr = smem_u32(smem_raw);
   uint8_t* smem = smem_raw + ((1024u - (raw_addr & 1023u)) & 1023u);
@@ -147,10 +147,25 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
 
   const int split = blockIdx.z, kvh = (int)blockIdx.x / p.g_tiles, r_first = ((int)blockIdx.x % p.g_tiles) * 16, seq = blockIdx.y;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  if (tid == 0) {
+    for (int s = 0; s < p.stages; ++s) {
+      mbar_init(&ctl->full[s], 1);
+      mbar_init(&ctl->empty[s], 4);
+    }
+    ctl->abort_flag = 0;
+    fence_barrier_init();
+    tma_prefetch_desc(&tmK);
+    tma_prefetch_desc(&tmV);
+  }
+  pdl_wait();
   // by row: the row's own position bounds its keys and its sequence's slot owns the pages
   const int owner = p.pos && p.seq_of_row ? p.seq_of_row[seq] : seq;
   const int pt_row = p.slot ? p.slot[owner] : owner;
+  // the first stage's page numbers are asked for beside the length, not behind it, where pages are read in order
+  int early_page = -1;
   const int kvlen = p.pos ? p.pos[seq] + 1 : p.kv_len[seq];
+  if (warp == 4 && lane < 4 && p.paged && p.window <= 0 && p.chunk <= 0 && split * p.pages_per_split + lane < p.pt_stride)
+    early_page = p.page_table[(size_t)pt_row * p.pt_stride + split * p.pages_per_split + lane];
   int kvlo = p.chunk > 0 && kvlen > 0 ? (kvlen - 1) / p.chunk * p.chunk : 0;
   if (p.window > 0) kvlo = max(kvlo, kvlen - p.window);
   // pages in the order they are read: the ones of the kept first positions, then from the first visible position on
@@ -165,16 +180,6 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
   auto head_of = [&](int r) { return kvh * p.G + (p.rows_per_seq == 1 ? r_first + r : (r_first + r) % p.G); };
   auto row_of = [&](int r) { return p.rows_per_seq == 1 ? seq : seq * p.rows_per_seq + (r_first + r) / p.G; };
 
-  if (tid == 0) {
-    for (int s = 0; s < p.stages; ++s) {
-      mbar_init(&ctl->full[s], 1);
-      mbar_init(&ctl->empty[s], 4);
-    }
-    ctl->abort_flag = 0;
-    fence_barrier_init();
-    tma_prefetch_desc(&tmK);
-    tma_prefetch_desc(&tmV);
-  }
   __syncthreads();
 
   float m0 = -INFINITY, m1 = -INFINITY, l0 = 0.f, l1 = 0.f;
@@ -192,7 +197,7 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
         return p.paged ? (p.page_table[(size_t)pt_row * p.pt_stride + pg] * p.Hkv + kvh) * 16 : p.kv_start[seq] + pg * 16;
       };
       const int col0 = p.paged ? 0 : kvh * HD;
-      int row = row_of_page(lane);
+      int row = early_page >= 0 ? (early_page * p.Hkv + kvh) * 16 : row_of_page(lane);
       for (int it = 0; it < iters; ++it) {
         const int s = it % p.stages, next = row_of_page((it + 1) * 4 + lane);
         const uint32_t ph = (uint32_t)(it / p.stages) & 1u;
