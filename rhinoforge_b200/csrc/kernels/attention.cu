@@ -17,8 +17,8 @@
 //    thread-block cluster that they form (up to eight) or, beyond that, by a second kernel.
 //
 // Decode, fp16, us, with one lane that copies page by page, merges in rows of bank conflicts and a second kernel / now: 1 x 300 keys, 16 + 2 x 8
-// heads of 128 9.4 / 7.2; 64 x 1024, 32 + 2 x 8 54.8 / 49.6 (K/V at the copy rate: 40.4); 8 x 8000 53.3 / 45.9 (39.4); 32 x 260, 16 + 2 x 4
-// 12.3 / 9.4; 50 rows on 880 keys, 8 + 2 x 1 heads of 256 22.0 as 50 sequences / 13.8 as one.
+// heads of 128 9.4 / 6.6; 64 x 1024, 32 + 2 x 8 54.8 / 49.6 (K/V at the copy rate: 40.4); 8 x 8000 53.3 / 45.9 (39.4); 32 x 260, 16 + 2 x 4
+// 12.3 / 9.4; 50 rows on 880 keys, 8 + 2 x 1 heads of 256 22.0 as 50 sequences / 11.7 as one.
 //
 // Replaces llm_fp16_32b_prefill_flash_attn_univ_* and its vctxlen / minibatch
 // variants (src/ops/rpu_sdpa.cpp:30-37,202-203, src/ops/rpu_sdpa_vctxlen.cpp,
@@ -45,6 +45,8 @@ struct alignas(8) AttnCtl {
   int32_t abort_flag;
   // decode, per MMA row: the warps' maxima and (scaled) sums of weights, this split's own
   float warp_max[4][16], warp_sum[4][16], row_max[16], row_sum[16];
+  // decode in a cluster: the splits' weights of a row, and what its weighted sum is divided by
+  float split_w[8][16], row_den[16];
 };
 
 // STREAM: the page is read once in this launch (decode): it takes the L2 evict-first policy, so that a step's KV
@@ -404,9 +406,10 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
     // The splits of a (sequence, K/V head) are one cluster: every CTA leaves its sums in its own shared memory and finishes a share of them.
     // A CTA that gave up counts as empty (maximum -inf): its sums are not used.
     if (!aborted) {
-      for (int idx = tid; idx < R * HD; idx += blockDim.x) {
-        float* at = mo + idx / HD * LDO + idx % HD;        // read and written by this thread alone
-        *at = (at[0] + at[16 * LDO]) + (at[32 * LDO] + at[48 * LDO]);
+      for (int idx = tid * 4; idx < R * HD; idx += blockDim.x * 4) {
+        float4* at = reinterpret_cast<float4*>(mo + idx / HD * LDO + idx % HD);        // read and written by this thread alone
+        const float4 a = at[0], b = at[4 * LDO], c = at[8 * LDO], d = at[12 * LDO];
+        *at = make_float4((a.x + b.x) + (c.x + d.x), (a.y + b.y) + (c.y + d.y), (a.z + b.z) + (c.z + d.z), (a.w + b.w) + (c.w + d.w));
       }
     }
     if (tid < R) {
@@ -416,32 +419,87 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
     cluster_sync_all();
     const int share = (R * HD / 32 + p.splits - 1) / p.splits * 32, lo = split * share, hi = min(lo + share, R * HD);   // whole warps: one row to a warp
     const uint32_t a_o = smem_u32(mo), a_m = smem_u32(ctl->row_max), a_s = smem_u32(ctl->row_sum);
-    for (int idx = lo + tid; idx < hi; idx += blockDim.x) {
-      const int g = idx / HD;
-      const uint32_t at = a_o + (uint32_t)(g * LDO + idx % HD) * 4u;
-      float m[8], l[8], part[8];
+    if (share <= (int)blockDim.x) {
+      // one value to a thread, which works out its row's weights itself
+      const int idx = lo + tid, g = idx / HD;
+      if (idx < hi) {
+        const uint32_t at = a_o + (uint32_t)(g * LDO + idx % HD) * 4u;
+        float m[8], l[8], part[8];
 #pragma unroll
-      for (int k = 0; k < 8; ++k) {              // all on their way before the first is used
-        m[k] = -INFINITY; l[k] = 0.f; part[k] = 0.f;
-        if (k < p.splits) {
-          m[k] = ld_dsmem_f32(dsmem_addr(a_m + g * 4u, k));
-          l[k] = ld_dsmem_f32(dsmem_addr(a_s + g * 4u, k));
-          part[k] = ld_dsmem_f32(dsmem_addr(at, k));
+        for (int k = 0; k < 8; ++k) {              // all on their way before the first is used
+          m[k] = -INFINITY; l[k] = 0.f; part[k] = 0.f;
+          if (k < p.splits) {
+            m[k] = ld_dsmem_f32(dsmem_addr(a_m + g * 4u, k));
+            l[k] = ld_dsmem_f32(dsmem_addr(a_s + g * 4u, k));
+            part[k] = ld_dsmem_f32(dsmem_addr(at, k));
+          }
         }
+        float M = -INFINITY, num = 0.f, den = 0.f;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) M = fmaxf(M, m[k]);
+        if (M != -INFINITY) {
+#pragma unroll
+          for (int k = 0; k < 8; ++k) {
+            const float f = exp2f(m[k] - M);
+            num += m[k] == -INFINITY ? 0.f : f * part[k];
+            den += m[k] == -INFINITY ? 0.f : f * l[k];
+          }
+          if (p.sink) den += exp2f(p.sink[head_of(g)] * kLog2e - M);
+        }
+        store(g, idx % HD, den > 0.f ? num / den : 0.f);
       }
-      float M = -INFINITY, num = 0.f, den = 0.f;
+      cluster_sync_relaxed();                      // peers may still be reading this CTA's sums
+      return;
+    }
+    // More of them: several values of every split are on their way before the first is used, and the weights of a row are worked out once, beside
+    // them.  50 rows on 880 keys, 8 + 2 x 1 heads of 256, us: value by value as above 13.5, so 11.6; one value to a thread (1 x 300 keys, 16 + 2 x 8
+    // heads of 128): 6.8, with the table of weights 7.2.
+    constexpr int kAtOnce = HD >= 128 ? 4 : 2;
+    float part[kAtOnce][8];
+    auto fetch = [&](int first) {
+#pragma unroll
+      for (int i = 0; i < kAtOnce; ++i) {
+        const int idx = first + i * (int)blockDim.x;
+        const uint32_t at = a_o + (uint32_t)(idx / HD * LDO + idx % HD) * 4u;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) part[i][k] = k < p.splits && idx < hi ? ld_dsmem_f32(dsmem_addr(at, k)) : 0.f;
+      }
+    };
+    fetch(lo + tid);
+    if (tid < R) {
+      float m[8], l[8], M = -INFINITY, den = 0.f;
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        m[k] = k < p.splits ? ld_dsmem_f32(dsmem_addr(a_m + tid * 4u, k)) : -INFINITY;
+        l[k] = k < p.splits ? ld_dsmem_f32(dsmem_addr(a_s + tid * 4u, k)) : 0.f;
+      }
 #pragma unroll
       for (int k = 0; k < 8; ++k) M = fmaxf(M, m[k]);
-      if (M != -INFINITY) {
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        const float f = m[k] == -INFINITY ? -1.f : exp2f(m[k] - M);   // -1: an empty split, whose sums are not used
+        ctl->split_w[k][tid] = f;
+        den += f < 0.f ? 0.f : f * l[k];
+      }
+      if (M != -INFINITY && p.sink) den += exp2f(p.sink[head_of(tid)] * kLog2e - M);
+      ctl->row_den[tid] = den;
+    }
+    __syncthreads();
+    for (int first = lo + tid; first < hi; first += kAtOnce * blockDim.x) {
+      if (first != lo + tid) fetch(first);
+#pragma unroll
+      for (int i = 0; i < kAtOnce; ++i) {
+        const int idx = first + i * (int)blockDim.x, g = idx / HD;
+        if (idx >= hi) break;
+        float num = 0.f;
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
-          const float f = exp2f(m[k] - M);
-          num += m[k] == -INFINITY ? 0.f : f * part[k];
-          den += m[k] == -INFINITY ? 0.f : f * l[k];
+          const float f = ctl->split_w[k][g];
+          num += f < 0.f ? 0.f : f * part[i][k];
         }
-        if (p.sink) den += exp2f(p.sink[head_of(g)] * kLog2e - M);
+        const float den = ctl->row_den[g];
+        store(g, idx % HD, den > 0.f ? num / den : 0.f);
       }
-      store(g, idx % HD, den > 0.f ? num / den : 0.f);
     }
     cluster_sync_relaxed();                      // peers may still be reading this CTA's sums
     return;
