@@ -59,6 +59,13 @@ __device__ __forceinline__ void load8(const T* p, float (&f)[8]) {
     f[2 * i + 1] = t.y;
   }
 }
+// Eight 16-bit values as they are in memory, in one piece if the caller knows that they lie on a 16-byte boundary.
+template <typename T>
+__device__ __forceinline__ uint4 load_raw8(const T* p, bool whole) {
+  if (whole) return *reinterpret_cast<const uint4*>(p);
+  const uint32_t* w = reinterpret_cast<const uint32_t*>(p);
+  return make_uint4(w[0], w[1], w[2], w[3]);
+}
 // The 8 values of a 16-byte register quad that was loaded earlier.
 template <typename T>
 __device__ __forceinline__ void unpack8(const uint4& q, float (&f)[8]) {
@@ -81,19 +88,43 @@ __device__ __forceinline__ uint4 vec8_upto(const T* row, int n, int N, bool vec)
     if (n + j < N) v[j] = row[n + j];
   return q;
 }
+// 16-bit values leave as one 16-byte store where the address allows it: the pair types copy by pairs, so that a Vec8 is four 4-byte stores, each over
+// every sector (in shared memory: bank) of the warp's row.
 template <typename T>
 __device__ __forceinline__ void store8(T* p, const float (&f)[8]) {
-  Vec8<T> x;
+  if constexpr (sizeof(T) == 2) {
+    uint32_t w[4];
 #pragma unroll
-  for (int i = 0; i < 4; ++i) x.v[i] = Num<T>::from_f2(f[2 * i], f[2 * i + 1]);
-  *reinterpret_cast<Vec8<T>*>(p) = x;
+    for (int i = 0; i < 4; ++i) {
+      const typename Num<T>::T2 v = Num<T>::from_f2(f[2 * i], f[2 * i + 1]);
+      w[i] = *reinterpret_cast<const uint32_t*>(&v);
+    }
+    if ((reinterpret_cast<uintptr_t>(p) & 15) == 0) {
+      *reinterpret_cast<uint4*>(p) = make_uint4(w[0], w[1], w[2], w[3]);
+    } else {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) reinterpret_cast<uint32_t*>(p)[i] = w[i];
+    }
+  } else {
+    Vec8<T> x;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) x.v[i] = Num<T>::from_f2(f[2 * i], f[2 * i + 1]);
+    *reinterpret_cast<Vec8<T>*>(p) = x;
+  }
 }
 
 // Activations run inside GEMM epilogues whose instruction count is on the critical path (the epilogue warps
 // share schedulers with the MMA-issuing lane), so they use the approximate special-function units: results are
 // rounded to 16 bits afterwards and the approximation error (2^-11 relative for tanh, 2 ulp for the division)
 // is below that rounding.
-__device__ __forceinline__ float silu_f(float x) { return __fdividef(x, 1.0f + __expf(-x)); }
+// x / (1 + e^-x) without the steps that exponential and quotient take for results below 2^-126: one is added to the former, and the latter is
+// zero there in any case.
+__device__ __forceinline__ float silu_f(float x) {
+  float e, r;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(x * -1.4426950408889634f));
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(1.0f + e));
+  return x * r;
+}
 __device__ __forceinline__ float tanh_approx_f(float x) {
   float y;
   asm("tanh.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
