@@ -1365,3 +1365,22 @@ def test_attn_decode_split_plans(dt, n, kv, Hq, Hkv, hd, status):
     for s in (0, n // 2, n - 1):
         ref = _sdpa_ref(q[s].view(Hq, 1, hd), ks[s], vs[s], torch.ones(1, lens[s], dtype=torch.bool, device="cuda"))
         _close(out[s], ref.reshape(Hq * hd), dt)
+
+
+@pytest.mark.parametrize("dt", DT)
+@pytest.mark.parametrize("H", [8, 248, 256, 1000, 4096, 8192, 8200])
+def test_rmsnorm_rows_of_any_width(dt, H):
+    """A row of at most 8192 values in the registers of its block, and the first width beyond: whole and ragged warps, every form, in place."""
+    from rhinoforge_b200.ops import kernels as K_
+    x, r = (torch.randn(5, H, device="cuda").to(dt) for _ in range(2))
+    w, mod = (1 + 0.1 * torch.randn(H, device="cuda")).to(dt), (0.3 * torch.randn(5, 3 * H, device="cuda")).to(dt)
+    norm = lambda t: t.float() * torch.rsqrt(t.float().pow(2).mean(-1, keepdim=True) + 1e-6)
+    total = torch.empty_like(x)
+    y = K_.rmsnorm(x, w, 1e-6, residual=r, residual_out=total)
+    assert torch.equal(total, (x.float() + r.float()).to(dt))
+    _close(y, norm(total) * w.float(), dt, scale=2.0)
+    _close(K_.rmsnorm(x, w, 1e-6, gemma=True), norm(x) * (1 + w.float()), dt, scale=2.0)
+    _close(K_.rmsnorm(x, None, 1e-6, mod=mod), norm(x) * (1 + mod[:, :H].float()) + mod[:, H:2 * H].float(), dt, scale=2.0)
+    z = x.clone()
+    K_.rmsnorm(z, None, 1e-6, out=z)
+    _close(z, norm(x), dt)
