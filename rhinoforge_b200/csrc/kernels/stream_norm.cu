@@ -18,9 +18,18 @@ __device__ __forceinline__ float stream_block_sum(float v, float* red) {
   return t;
 }
 
+// Four values: a struct of four 16-bit ones is copied value by value, so they move as one 8-byte piece where the address allows it.
 template <typename T> struct alignas(sizeof(T) * 4) Quad { T v[4]; };
 template <typename T>
+__device__ __forceinline__ float4 widen4(const uint2& q) {
+  const T* v = reinterpret_cast<const T*>(&q);
+  return make_float4(Num<T>::to_f(v[0]), Num<T>::to_f(v[1]), Num<T>::to_f(v[2]), Num<T>::to_f(v[3]));
+}
+template <typename T>
 __device__ __forceinline__ float4 load4(const T* p) {
+  if constexpr (sizeof(T) == 2) {
+    if ((reinterpret_cast<uintptr_t>(p) & 7) == 0) return widen4<T>(*reinterpret_cast<const uint2*>(p));
+  }
   const Quad<T> q = *reinterpret_cast<const Quad<T>*>(p);
   return make_float4(Num<T>::to_f(q.v[0]), Num<T>::to_f(q.v[1]), Num<T>::to_f(q.v[2]), Num<T>::to_f(q.v[3]));
 }
@@ -28,6 +37,12 @@ template <typename T>
 __device__ __forceinline__ void store4(T* p, float4 f) {
   Quad<T> q;
   q.v[0] = Num<T>::from_f(f.x); q.v[1] = Num<T>::from_f(f.y); q.v[2] = Num<T>::from_f(f.z); q.v[3] = Num<T>::from_f(f.w);
+  if constexpr (sizeof(T) == 2) {
+    if ((reinterpret_cast<uintptr_t>(p) & 7) == 0) {
+      *reinterpret_cast<uint2*>(p) = *reinterpret_cast<const uint2*>(&q);
+      return;
+    }
+  }
   *reinterpret_cast<Quad<T>*>(p) = q;
 }
 // four columns of the outstanding output of row `src`: one row, or the sum of the picked ones
@@ -198,8 +213,23 @@ __global__ void __launch_bounds__(VPT == 4 ? 512 : 1024) stream_norm_reg_kernel(
     return t;
   };
   float4 v[VPT], a[VPT];
+  const bool whole = sizeof(T) == 2 && (reinterpret_cast<uintptr_t>(y) & 7) == 0;
   auto load = [&](int r) {
     const int src = p.row_idx ? p.row_idx[r] : r;
+    if (p.x && y && p.y_picks <= 0 && whole && !p.table2) {       // the usual row: everything on its way before anything is widened
+      uint2 raw[VPT];
+#pragma unroll
+      for (int k = 0; k < VPT; ++k) {
+        const bool in = col(k) < H;
+        v[k] = in ? *reinterpret_cast<const float4*>(p.x + (size_t)src * H + col(k)) : zero;
+        raw[k] = in ? *reinterpret_cast<const uint2*>(y + (size_t)src * H + col(k)) : make_uint2(0u, 0u);
+      }
+      if constexpr (sizeof(T) == 2) {
+#pragma unroll
+        for (int k = 0; k < VPT; ++k) a[k] = widen4<T>(raw[k]);
+      }
+      return;
+    }
     const T* second = p.table2 ? reinterpret_cast<const T*>(p.table2) + (size_t)pair_row(p, src) * H : nullptr;
     if (second) carry_token(p, src);
 #pragma unroll
@@ -237,6 +267,12 @@ __global__ void __launch_bounds__(VPT == 4 ? 512 : 1024) stream_norm_reg_kernel(
   for (int r = r0; r < r1; ++r) {
     float* state = nullptr;
     bool state_here = false, fresh = false;
+    // the CTA's next row is on its way to L2 while this one is summed
+    if (threadIdx.x == 0 && r + 1 < r1 && p.x && !p.row_idx) {
+      bulk_prefetch_l2(p.x + (size_t)(r + 1) * H, (uint32_t)H * 4u);
+      if (y && p.y_picks <= 0 && sizeof(T) * H % 16 == 0 && reinterpret_cast<uintptr_t>(y) % 16 == 0)
+        bulk_prefetch_l2(y + (size_t)(r + 1) * H, (uint32_t)(H * sizeof(T)));
+    }
     if (p.shift) {
       const int seq = p.rows.seq_of_row ? p.rows.seq_of_row[r] : r;
       const int q0 = p.rows.q_start ? p.rows.q_start[seq] : r;
@@ -543,8 +579,6 @@ extern "C" int rf_stream_norm(const RfStreamNorm* args, rf_stream_t stream) {
   if (a->conv_w) RF_REQUIRE(a->conv_taps >= 1 && (a->conv_taps == 1 || a->conv_state) && a->norm_w && a->rows.pos && !a->rows.q_start && !a->shift &&
                                 !a->row_idx && a->dtype != kF32 && a->H / 8 <= 1024, "stream_norm: the input convolution takes decode rows in 16 bits");
   if (a->n_rows == 0) return RF_OK;
-  // halo of one row per CTA with the shift: walk several rows per CTA once that still fills the GPU
-  const int rpc = (a->shift && a->rows.q_start) ? std::max(1, std::min(8, a->n_rows / (2 * sm_count()))) : 1;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const int groups = a->H / 8;
   if (!a->shift && a->dtype != kF32 && groups <= 1024) {
@@ -566,6 +600,10 @@ extern "C" int rf_stream_norm(const RfStreamNorm* args, rf_stream_t stream) {
     // decode rows: as many threads as there are quads (one round trip); many rows: smaller CTAs, several per SM
     const int vpt = a->n_rows > 4 * sm_count() ? (quads > 512 ? 4 : quads > 256 ? 2 : 1) : (quads > 1024 ? 2 : 1);
     const int threads = std::max(32, round_up(ceil_div(quads, vpt), 32));
+    // Halo of one row per CTA with the shift: a CTA walks several rows, at most twelve, and as many as make whole rounds of CTAs (64 registers a thread,
+    // 128 with four quads).  4770 rows of 2048, us: eight rows, five CTAs more than a round 54, nine rows 40, with the next row on its way 39, and in whole pieces 35.
+    const int resident = sm_count() * std::max(1, (vpt == 4 ? 512 : 1024) / threads), rounds = ceil_div(a->n_rows, 12 * resident);
+    const int rpc = a->shift && a->rows.q_start ? ceil_div(a->n_rows, rounds * resident) : 1;
     const dim3 grid(ceil_div(a->n_rows, rpc));
 #define RF_SN(V) RF_DISPATCH3(a->dtype, RF_CUDA_CHECK(::rf::launch_k(stream_norm_reg_kernel<T, V>, grid, dim3(threads), 0, s, 1, *a, rpc)))
     if (vpt == 1) { RF_SN(1); } else if (vpt == 2) { RF_SN(2); } else { RF_SN(4); }
@@ -573,7 +611,7 @@ extern "C" int rf_stream_norm(const RfStreamNorm* args, rf_stream_t stream) {
     ::rf::count_launch();
     return RF_OK;
   }
-  const int threads = 512;
+  const int threads = 512, rpc = a->shift && a->rows.q_start ? std::max(1, std::min(8, a->n_rows / (2 * sm_count()))) : 1;
   const size_t smem = ((size_t)a->H * (a->shift ? 2 : 1) + 32) * sizeof(float);
   RF_REQUIRE(smem <= 200 * 1024, "stream_norm: rows of %d values do not fit in shared memory", a->H);
   RF_DISPATCH3(a->dtype, {

@@ -328,3 +328,27 @@ def test_gemm_epilogue_gates_by_token(M, N, Kd):
     ids = torch.randint(0, 9, (M,), generator=g).to("cuda", torch.int32)
     got = K().gemm(x, K().pack_weight(w), packed_shape=(N, Kd), act="gelu_tanh", mul=table[:, 8:], mul_row=ids)
     close(got, oracle.gelu_tanh(x.double() @ w.double().T) * table.double()[ids.long(), 8:8 + N], torch.bfloat16)
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("lens", [[1183, 1], [700, 3, 482], [2369]])
+def test_stream_norm_of_many_rows(dtype, lens):
+    """One, two and three rows to a CTA (1184 CTAs of 512 values are resident), sequences that begin and end inside a CTA's rows, the halo row."""
+    H, n = 512, sum(lens)
+    d, pos, seq = pack(lens, [4] * len(lens), list(range(len(lens))))
+    g = torch.Generator().manual_seed(3)
+    rnd = lambda *s: torch.randn(*s, generator=g, dtype=torch.float64)
+    f32 = lambda t: t.to("cuda", torch.float32)
+    x, y, w, mu, state = f32(rnd(n, H)), rnd(n, H).to("cuda", dtype), f32(rnd(H)), f32(torch.rand(H, generator=g, dtype=torch.float64)), f32(rnd(len(lens), H))
+    st = state.clone()
+    xo, h, _ = K().stream_norm(x, K().rows(**d), dtype=dtype, eps=1e-3, norm_w=w, y=y, shift=mu, shift_state=st, dim=H, cast=True)
+    D = lambda t: t.double().cpu()
+    X = D(x) + D(y)
+    N_ = oracle.rms(X, 1e-3, D(w))
+    want, o = torch.empty_like(N_), 0
+    for s, L in enumerate(lens):
+        want[o:o + L] = oracle.token_shift(N_[o:o + L], D(mu), D(state)[s])
+        close(st[s], N_[o + L - 1], torch.float32, 4)
+        o += L
+    close(xo, X, torch.float32, 4)
+    close(h, want, dtype, 4)
