@@ -23,12 +23,14 @@ namespace rf {
 
 // ------------------------------------------------------------------ conv1d ----
 // y[t, c] = silu( sum_j w[c, j] * xin[t - (K-1) + j, c] ), xin = [state | x] per sequence.
-// One thread owns 8 adjacent channels of one token.
+// One thread owns 8 adjacent channels and walks the block's tokens, the next four on their way while four are worked on.  3762 tokens of 6144 channels,
+// us: one token at a time and the weights value by value 45, so 38.5 (14 at the copy rate).  About 20 instructions a value on nine to twelve warps per SM
+// bound it: with 16 tokens to a block, whose weights and carried rows then weigh more, it takes 50.
 template <typename T, int KW>
-__global__ void conv1d_kernel(const T* __restrict__ x, int64_t ldx, T* __restrict__ y, int64_t ldy,
+__global__ void __launch_bounds__(128) conv1d_kernel(const T* __restrict__ x, int64_t ldx, T* __restrict__ y, int64_t ldy,
                               const T* __restrict__ w, const T* __restrict__ state,
                               const int32_t* __restrict__ q_start, const int32_t* __restrict__ q_len,
-                              const int32_t* __restrict__ slot, int C, int tokens_per_block, int silu) {
+                              const int32_t* __restrict__ slot, int C, int tokens_per_block, int silu, int whole) {
   pdl_prologue();
   const int seq = blockIdx.z;
   const int s0 = q_start ? q_start[seq] : seq;
@@ -38,10 +40,18 @@ __global__ void conv1d_kernel(const T* __restrict__ x, int64_t ldx, T* __restric
   const int sl = slot ? slot[seq] : seq;
   const T* st = state + (size_t)sl * (KW - 1) * C;
   float wk[KW][8];
+  const T* wc = w + (size_t)c * KW;             // 8 * KW values in a row
+  if ((reinterpret_cast<uintptr_t>(w) & 15) == 0) {
 #pragma unroll
-  for (int ch = 0; ch < 8; ++ch) {
+    for (int i = 0; i < KW; ++i) {
+      float v[8];
+      unpack8<T>(*reinterpret_cast<const uint4*>(wc + i * 8), v);
 #pragma unroll
-    for (int j = 0; j < KW; ++j) wk[j][ch] = Num<T>::to_f(w[(size_t)(c + ch) * KW + j]);
+      for (int j = 0; j < 8; ++j) wk[(i * 8 + j) % KW][(i * 8 + j) / KW] = v[j];
+    }
+  } else {
+#pragma unroll
+    for (int i = 0; i < KW * 8; ++i) wk[i % KW][i / KW] = Num<T>::to_f(wc[i]);
   }
   const int t0 = blockIdx.y * tokens_per_block;
   const int t1 = min(n, t0 + tokens_per_block);
@@ -54,23 +64,40 @@ __global__ void conv1d_kernel(const T* __restrict__ x, int64_t ldx, T* __restric
     if (ti >= 0) load8(x + (size_t)(s0 + ti) * ldx + c, win[j]);
     else load8(st + (size_t)(KW - 1 + ti) * C + c, win[j]);
   }
-  for (int t = t0; t < t1; ++t) {
-    float cur[8], acc[8];
-    load8(x + (size_t)(s0 + t) * ldx + c, cur);
+  constexpr int U = 4;
+  uint4 ahead[U];
+  auto fetch = [&](int tb) {
 #pragma unroll
-    for (int ch = 0; ch < 8; ++ch) {
-      float a = wk[KW - 1][ch] * cur[ch];
+    for (int u = 0; u < U; ++u)
+      if (tb + u < t1) ahead[u] = load_raw8(x + (size_t)(s0 + tb + u) * ldx + c, whole);
+  };
+  fetch(t0);
+  for (int tb = t0; tb < t1; tb += U) {
+    uint4 raw[U];
 #pragma unroll
-      for (int j = 0; j < KW - 1; ++j) a += wk[j][ch] * win[j][ch];
-      acc[ch] = silu ? silu_f(a) : a;
+    for (int u = 0; u < U; ++u) raw[u] = ahead[u];
+    fetch(tb + U);
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int t = tb + u;
+      if (t >= t1) break;
+      float cur[8], acc[8];
+      unpack8<T>(raw[u], cur);
+#pragma unroll
+      for (int ch = 0; ch < 8; ++ch) {
+        float a = wk[KW - 1][ch] * cur[ch];
+#pragma unroll
+        for (int j = 0; j < KW - 1; ++j) a += wk[j][ch] * win[j][ch];
+        acc[ch] = silu ? silu_f(a) : a;
+      }
+      store8(y + (size_t)(s0 + t) * ldy + c, acc);
+#pragma unroll
+      for (int j = 0; j < KW - 2; ++j)
+#pragma unroll
+        for (int ch = 0; ch < 8; ++ch) win[j][ch] = win[j + 1][ch];
+#pragma unroll
+      for (int ch = 0; ch < 8; ++ch) win[KW - 2][ch] = cur[ch];
     }
-    store8(y + (size_t)(s0 + t) * ldy + c, acc);
-#pragma unroll
-    for (int j = 0; j < KW - 2; ++j)
-#pragma unroll
-      for (int ch = 0; ch < 8; ++ch) win[j][ch] = win[j + 1][ch];
-#pragma unroll
-    for (int ch = 0; ch < 8; ++ch) win[KW - 2][ch] = cur[ch];
   }
 }
 
@@ -621,7 +648,43 @@ gdn_chunked_kernel(const RfGdn p) {
 }
 
 // ------------------------------------------------- gated RMSNorm over Dv ----
-// y = (w * rmsnorm(x)) * silu(z); one warp per (token, head) row of D <= 256 values.
+// y = (w * rmsnorm(x)) * silu(z); one warp per (token, head) row of D <= 256 values.  VEC: a lane's D / 32 values (2, 4 or 8) lie in one aligned piece of
+// every row (3762 tokens, 16 heads of 128, us: value by value 24, so 15.5).
+template <int BYTES> struct RowPiece;
+template <> struct RowPiece<4> { using type = uint32_t; };
+template <> struct RowPiece<8> { using type = uint2; };
+template <> struct RowPiece<16> { using type = uint4; };
+
+template <typename T, int PER>
+__global__ void rmsnorm_gated_vec_kernel(const T* __restrict__ x, int64_t ldx, const T* __restrict__ z, int64_t ldz, const T* __restrict__ w,
+                                         T* __restrict__ y, int64_t ldy, int rows, int heads, float eps) {
+  pdl_prologue();
+  using Piece = typename RowPiece<PER * 2>::type;
+  const int r = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  if (r >= rows) return;
+  const int lane = threadIdx.x & 31, t = r / heads, h = r % heads, at = h * PER * 32 + lane * PER;
+  const Piece px = *reinterpret_cast<const Piece*>(x + (size_t)t * ldx + at), pz = *reinterpret_cast<const Piece*>(z + (size_t)t * ldz + at),
+              pw = *reinterpret_cast<const Piece*>(w + lane * PER);
+  const T *vx = reinterpret_cast<const T*>(&px), *vz = reinterpret_cast<const T*>(&pz), *vw = reinterpret_cast<const T*>(&pw);
+  float v[PER], ss = 0.f;
+#pragma unroll
+  for (int i = 0; i < PER; ++i) {
+    v[i] = Num<T>::to_f(vx[i]);
+    ss += v[i] * v[i];
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+  const float inv = rsqrtf(ss / (float)(PER * 32) + eps);
+  Piece out;
+  T* vo = reinterpret_cast<T*>(&out);
+#pragma unroll
+  for (int i = 0; i < PER; ++i) {
+    const float nx = Num<T>::to_f(Num<T>::from_f(v[i] * inv));   // rounded like the unfused form
+    vo[i] = Num<T>::from_f(Num<T>::to_f(vw[i]) * nx * silu_f(Num<T>::to_f(vz[i])));
+  }
+  *reinterpret_cast<Piece*>(y + (size_t)t * ldy + at) = out;
+}
+
 template <typename T>
 __global__ void rmsnorm_gated_kernel(const T* __restrict__ x, int64_t ldx, const T* __restrict__ z, int64_t ldz,
                                      const T* __restrict__ w, T* __restrict__ y, int64_t ldy, int rows, int heads,
@@ -732,12 +795,13 @@ extern "C" int rf_causal_conv1d(const RfConv1d* a, rf_stream_t stream) {
   const int threads = 128;
   const int cblocks = (a->C / 8 + threads - 1) / threads;
   const int max_len = a->q_len ? (a->max_q_len > 0 ? a->max_q_len : 1) : 1;
-  const int tpb = 32;
+  // 64 tokens to a block where that still makes a few blocks an SM (32 tokens 40.5 us, see the kernel)
+  const int tpb = (long)cblocks * ceil_div(max_len, 64) * a->num_seqs >= 3L * sm_count() ? 64 : 32;
   const int tblocks = (max_len + tpb - 1) / tpb;
   RF_DISPATCH_T(a->dtype, {
     RF_CUDA_CHECK(::rf::launch_k(conv1d_kernel<T, 4>, dim3(cblocks, tblocks, a->num_seqs), dim3(threads), 0, s, 1,
                                  (const T*)a->x, a->ldx, (T*)a->y, a->ldy, (const T*)a->w, (const T*)a->state,
-                                 a->q_start, a->q_len, a->slot, a->C, tpb, a->silu));
+                                 a->q_start, a->q_len, a->slot, a->C, tpb, a->silu, reinterpret_cast<uintptr_t>(a->x) % 16 == 0));
     ::rf::count_launch();
     RF_CUDA_CHECK(::rf::launch_k(conv1d_state_kernel<T, 4>, dim3(cblocks, a->num_seqs), dim3(threads), 0, s, 1,
                                  (const T*)a->x, a->ldx, (T*)a->state, a->q_start, a->q_len, a->slot, a->C));
@@ -795,7 +859,16 @@ extern "C" int rf_rmsnorm_gated(const void* x, int64_t ldx, const void* z, int64
   RF_REQUIRE(D % 32 == 0 && D <= 256, "rmsnorm_gated: width %d must be a multiple of 32, at most 256", D);
   if (tokens == 0) return RF_OK;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  const int rows = tokens * heads, wpb = 8;
+  const int rows = tokens * heads, wpb = 8, per = D / 32;
+  const auto whole = [&](const void* p, int64_t ld) { return reinterpret_cast<uintptr_t>(p) % (per * 2) == 0 && ld % per == 0; };
+  if ((per == 2 || per == 4 || per == 8) && D % 64 == 0 && whole(x, ldx) && whole(z, ldz) && whole(y, ldy) && whole(w, 0)) {
+#define RF_GATED(PER) RF_DISPATCH_T(dtype, RF_CUDA_CHECK(::rf::launch_k(rmsnorm_gated_vec_kernel<T, PER>, dim3((rows + wpb - 1) / wpb), dim3(wpb * 32), 0, s, 1, \
+                                                         (const T*)x, ldx, (const T*)z, ldz, (const T*)w, (T*)y, ldy, rows, heads, eps)))
+    if (per == 2) { RF_GATED(2); } else if (per == 4) { RF_GATED(4); } else { RF_GATED(8); }
+#undef RF_GATED
+    ::rf::count_launch();
+    return RF_OK;
+  }
   RF_DISPATCH_T(dtype, RF_CUDA_CHECK(::rf::launch_k(rmsnorm_gated_kernel<T>, dim3((rows + wpb - 1) / wpb), dim3(wpb * 32), 0,
                                                     s, 1, (const T*)x, ldx, (const T*)z, ldz, (const T*)w, (T*)y, ldy,
                                                     rows, heads, D, eps)));

@@ -378,3 +378,35 @@ def test_qwen3_5_vision_path_matches_hf():
     finally:
         os.environ.pop("RPU_QWEN3_5_ALLOW_ANY_PROFILE", None)
         live_handle._reset_for_tests()
+
+
+@pytest.mark.parametrize("dt", DT)
+@pytest.mark.parametrize("D", [32, 64, 96, 128, 256])
+@pytest.mark.parametrize("off", [0, 1, 4])
+def test_gated_norm_in_pieces_and_by_value(dt, D, off):
+    """Rows a lane reads in one piece (heads of 64, 128 and 256 on its alignment) and value by value (anything else) against fp32."""
+    from rhinoforge_b200.ops import kernels as K
+    T, heads = 9, 3
+    x, z = (torch.randn(T, heads * D + 8, device="cuda").to(dt)[:, off:off + heads * D] for _ in range(2))
+    w = (1 + 0.1 * torch.randn(D, device="cuda")).to(dt)
+    xf, zf = (t.float().reshape(T, heads, D) for t in (x, z))
+    n = (xf * torch.rsqrt(xf.pow(2).mean(-1, keepdim=True) + 1e-6)).to(dt).float()
+    ref = (w.float() * n * F.silu(zf)).reshape(T, heads * D)
+    assert _rel(K.rmsnorm_gated(x, z, w, heads, 1e-6), ref) < (2e-3 if dt == torch.float16 else 1.6e-2)
+
+
+@pytest.mark.parametrize("dt", DT)
+@pytest.mark.parametrize("off", [0, 1])
+@pytest.mark.parametrize("L", [1, 8, 9, 31, 32, 41])
+def test_conv1d_of_a_few_tokens(dt, off, L):
+    """Around the eight tokens that are asked for together and a block's 32; weights on and off their 16-byte boundary."""
+    from rhinoforge_b200.ops import kernels as K
+    Cc = 1032
+    x, st = torch.randn(L, Cc, device="cuda").to(dt), torch.randn(1, 3, Cc, device="cuda").to(dt)
+    w = (torch.randn(Cc * 4 + 8, device="cuda") * 0.5).to(dt)[off:off + Cc * 4].view(Cc, 4)
+    ql, z = torch.tensor([L], dtype=torch.int32, device="cuda"), torch.zeros(1, dtype=torch.int32, device="cuda")
+    full = torch.cat((st[0].float(), x.float()), 0)
+    ref = F.silu(F.conv1d(full.t()[None], w.float()[:, None], groups=Cc)[0].t())
+    y = K.causal_conv1d(x, w, st, q_start=z, q_len=ql, max_q_len=L, slot=z)
+    assert _rel(y, ref) < (4e-3 if dt == torch.float16 else 2e-2)
+    assert torch.equal(st[0].float(), full[-3:].to(dt).float())
