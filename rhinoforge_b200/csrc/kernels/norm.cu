@@ -186,13 +186,12 @@ __global__ void layernorm_kernel(const T* __restrict__ x, const T* __restrict__ 
 }
 
 // Many rows: a warp per row that holds it in registers, 16-byte pieces 256 values apart, all of them on their way at once; nothing but shuffles
-// between the two passes.  The kernels above keep the row in shared memory (eight-way bank conflicts) and meet at three to six block barriers,
-// which a block per row hides as long as an SM has few rows (warp_pieces has the line).  us, block / warp: LayerNorm 3072 x 1152 9.0 / 6.8, 6000 x 2048 25.3 / 15.5; RMSNorm 5400 x 4096 31.5 / 21.6, 768 x 1152 4.4 / 3.3.
+// between the two passes.  A block per row has a barrier in its chain (LayerNorm's four), which it hides as long as an SM has few rows: layernorm_by_warp and
+// rmsnorm_by_warp have the lines.  us, block / warp: LayerNorm 3072 x 1152 9.0 / 4.4, 6000 x 2048 25.3 / 15.5; RMSNorm 6000 x 4096 37 / 23.
 template <typename T, int NC>
 __global__ void __launch_bounds__(128)
-rmsnorm_warp_kernel(const T* __restrict__ x, const T* __restrict__ residual, const T* __restrict__ w, T* __restrict__ y,
-                    T* __restrict__ residual_out, const T* __restrict__ mod, int rows_per_mod, int rows, int H, int64_t ldx, int64_t ldy, float eps,
-                    int mode) {
+rmsnorm_warp_kernel(const T* __restrict__ x, const T* __restrict__ w, T* __restrict__ y, const T* __restrict__ mod, int rows_per_mod, int rows, int H,
+                    int64_t ldx, int64_t ldy, float eps, int mode) {
   pdl_prologue();
   const int row = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (row >= rows) return;
@@ -206,18 +205,8 @@ rmsnorm_warp_kernel(const T* __restrict__ x, const T* __restrict__ residual, con
   float ss = 0.f;
 #pragma unroll
   for (int c = 0; c < NC; ++c) {
-    const int i = c * 256 + lane * 8;
     float f[8];
     unpack8<T>(v[c], f);
-    if (residual && i < H) {
-      float r[8];
-      load8(residual + (size_t)row * ldx + i, r);
-#pragma unroll
-      for (int j = 0; j < 8; ++j) f[j] += r[j];
-      store8(reinterpret_cast<T*>(&v[c]), f);
-      unpack8<T>(v[c], f);                       // the sum as it is stored
-      if (residual_out) *reinterpret_cast<uint4*>(residual_out + (size_t)row * ldx + i) = v[c];
-    }
 #pragma unroll
     for (int j = 0; j < 8; ++j) ss += f[j] * f[j];
   }
@@ -313,23 +302,25 @@ layernorm_warp_kernel(const T* __restrict__ x, const T* __restrict__ w, const T*
   }
 }
 
-// 256-value pieces of a row that the warp kernels hold, 0: a block per row.  A warp takes its row alone, so it needs several rows per SM to hide
-// its chain, and more of them the longer the row: above 1536 values the block kernels have twice the threads, and a second row (residual) or the
-// modulation (`extra`) leaves room for fewer warps.  LayerNorm's block form meets at twice the barriers.  fp16, us, block / warp: LayerNorm
-// 296 x 1024 2.6 / 2.9, 400 x 1152 3.6 / 3.3, 768 x 1152 5.6 / 4.0, 768 x 2048 5.9 / 6.2, 1500 x 4096 13.2 / 9.1; RMSNorm 296 x 4096 3.3 / 8.2,
-// 400 x 768 2.3 / 2.5, 768 x 1536 5.1 / 3.9, 768 x 4096 7.7 / 9.2, 1500 x 2560 8.2 / 7.1, 3072 x 3072 14.6 / 9.1; with a residual 768 x 1152
-// 5.7 / 4.4, 1500 x 2048 7.9 / 9.4, 3072 x 2048 14.0 / 11.2, 6000 x 4096 49.5 / 57.1; modulated 768 x 1152 4.9 / 3.7, 1500 x 2048 7.2 / 8.6,
-// 3072 x 2048 12.3 / 10.0.
-// Rows of 16-byte pieces: every operand on its boundary (the kernels that go through shared memory take 4-byte ones)
-template <typename... P>
-static bool whole_pieces(P... p) { return (((reinterpret_cast<uintptr_t>(p) % 16) == 0) && ...); }
-
-static int warp_pieces(int rows, int H, bool layer, bool extra, bool residual) {
-  const int per_two_sms = layer && H <= 1152 ? 5 : H <= 1536 ? 10 : extra ? 40 : 20;
-  if (2 * rows < per_two_sms * sm_count() || H > (residual ? 3072 : 4096)) return 0;
+// 256-value pieces of a row that the warp kernels hold
+static int warp_pieces(int H) {
   const int nc = ceil_div(H, 256);
   return nc <= 4 ? 4 : nc <= 5 ? 5 : nc <= 8 ? 8 : nc <= 12 ? 12 : 16;
 }
+// A warp takes its row alone, so it needs several rows per SM to hide its chain, and more of them the longer the row.  LayerNorm, whose block form
+// meets at four barriers, fp16, us, block / warp: 296 x 1024 2.6 / 2.9, 400 x 1152 3.6 / 3.3, 768 x 1152 5.6 / 4.0, 768 x 2048 5.9 / 6.2, 1500 x 4096
+// 13.2 / 9.1.
+static bool layernorm_by_warp(int rows, int H) { return H <= 4096 && 2 * rows >= (H <= 1152 ? 5 : H <= 1536 ? 10 : 20) * sm_count(); }
+// RMSNorm's block form has one barrier, and is overtaken where an SM has some 20 thousand values (34 of rows above 1536 values), later with a modulation's two rows.  fp16, us, block / warp: 3072 x 1024 5.2 / 5.6, 4770 x 1024 7.0 / 6.5, 2200 x
+// 2048 6.7 / 7.6, 3072 x 2048 8.6 / 8.1, 1100 x 4096 8.4 / 9.8, 1500 x 4096 10.9 / 10.1; modulated 3072 x 1152 6.6 / 7.4, 4770 x 1152 8.8 / 8.0, 3072 x
+// 2048 9.4 / 10.1, 3072 x 2560 11.8 / 10.8.  With a residual never: 768 x 1152 3.1 / 6.0, 3072 x 2048 11.2 / 14.0, 9000 x 1536 22.3 / 22.4.
+static bool rmsnorm_by_warp(int rows, int H, bool mod, bool residual) {
+  const long per_sm = mod ? (H <= 1536 ? 24300 : 48600) : H <= 1536 ? 21600 : 34000;
+  return !residual && H <= 4096 && (long)rows * H >= per_sm * sm_count();
+}
+// Rows of 16-byte pieces: every operand on its boundary (the kernels that go through shared memory take 4-byte ones)
+template <typename... P>
+static bool whole_pieces(P... p) { return (((reinterpret_cast<uintptr_t>(p) % 16) == 0) && ...); }
 
 // Calls `run` with the piece count and the element type as types.
 template <typename Run>
@@ -400,13 +391,13 @@ extern "C" int rf_rmsnorm(const void* x, const void* residual, const void* w, vo
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (rows_per_mod <= 0) rows_per_mod = 1;
   const bool whole = whole_pieces(x, residual, w, y, residual_out, mod);
-  if (const int nc = whole ? warp_pieces(rows, H, false, residual || mod, residual != nullptr) : 0) {
+  if (whole && rmsnorm_by_warp(rows, H, mod != nullptr, residual != nullptr)) {
     auto run = [&](auto kNC, auto zero) -> cudaError_t {
       using T = decltype(zero);
-      return ::rf::launch_k(rmsnorm_warp_kernel<T, decltype(kNC)::value>, dim3(ceil_div(rows, 4)), dim3(128), 0, s, 1, (const T*)x, (const T*)residual, (const T*)w,
-                            (T*)y, (T*)residual_out, (const T*)mod, rows_per_mod, rows, H, ldx, ldy, eps, mode);
+      return ::rf::launch_k(rmsnorm_warp_kernel<T, decltype(kNC)::value>, dim3(ceil_div(rows, 4)), dim3(128), 0, s, 1, (const T*)x, (const T*)w, (T*)y,
+                            (const T*)mod, rows_per_mod, rows, H, ldx, ldy, eps, mode);
     };
-    RF_CUDA_CHECK(with_pieces(nc, dtype, run));
+    RF_CUDA_CHECK(with_pieces(warp_pieces(H), dtype, run));
     ::rf::count_launch();
     return RF_OK;
   }
@@ -442,13 +433,13 @@ extern "C" int rf_layernorm(const void* x, const void* w, const void* b, void* y
   const int threads = H >= 2048 ? 256 : 128;
   const size_t smem = (size_t)(H + 32) * sizeof(float);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (const int nc = whole_pieces(x, w, b, y) ? warp_pieces(rows, H, true, false, false) : 0) {
+  if (whole_pieces(x, w, b, y) && layernorm_by_warp(rows, H)) {
     auto run = [&](auto kNC, auto zero) -> cudaError_t {
       using T = decltype(zero);
       return ::rf::launch_k(layernorm_warp_kernel<T, decltype(kNC)::value>, dim3(ceil_div(rows, 4)), dim3(128), 0, s, 1, (const T*)x, (const T*)w, (const T*)b,
                             (T*)y, rows, H, ldx, ldy, eps);
     };
-    RF_CUDA_CHECK(with_pieces(nc, dtype, run));
+    RF_CUDA_CHECK(with_pieces(warp_pieces(H), dtype, run));
     ::rf::count_launch();
     return RF_OK;
   }

@@ -1384,3 +1384,20 @@ def test_rmsnorm_rows_of_any_width(dt, H):
     z = x.clone()
     K_.rmsnorm(z, None, 1e-6, out=z)
     _close(z, norm(x), dt)
+
+
+@pytest.mark.parametrize("dt", DT)
+@pytest.mark.parametrize("H,mod", [(1000, False), (2040, False), (1000, True), (2040, True)])
+def test_rmsnorm_around_the_line_between_block_and_warp(dt, H, mod):
+    """The last number of rows that a block each takes and the first that a warp each does."""
+    from rhinoforge_b200.ops import kernels as K_
+    per_sm = {(1000, False): 21600, (2040, False): 34000, (1000, True): 24300, (2040, True): 48600}[H, mod]
+    line = -(-per_sm * torch.cuda.get_device_properties(0).multi_processor_count // H)
+    x, w = torch.randn(line, H, device="cuda").to(dt), (1 + 0.1 * torch.randn(H, device="cuda")).to(dt)
+    m = (0.3 * torch.randn(line, 3 * H, device="cuda")).to(dt)
+    n = x.float() * torch.rsqrt(x.float().pow(2).mean(-1, keepdim=True) + 1e-6)
+    for rows in (line - 1, line):
+        if mod:
+            _close(K_.rmsnorm(x[:rows], None, 1e-6, mod=m), (n * (1 + m[:, :H].float()) + m[:, H:2 * H].float())[:rows], dt, scale=2.0)
+        else:
+            _close(K_.rmsnorm(x[:rows], w, 1e-6), (n * w.float())[:rows], dt, scale=2.0)
