@@ -23,6 +23,7 @@
 // Then, with P in shared memory, a wait for P.V in every block and one lane in the MMA loop / as it is: 8192 causal 889 / 612; 7808 queries on 16000
 // keys 2380 / 1593; 8 x 1024 causal 209 / 168; 2 x 4096, heads of 64 416 / 290; 6 x 1100, window 1024 104 / 83.  The copy loop run by its whole
 // warp as well: 547; 1438; 157; 277; 80; 825 full, 8 + 1 heads of 256 43.6 / 32.5.
+// A row's results stored 16 bytes at a time: 503; 1448; 114.5; 257; 67; 28.4; 12 x 256 full, heads of 80, behind a GEMM 26.9 / 20.2.
 // V needs no transpose: the [tokens x 64] slabs a TMA box leaves in shared memory are exactly the
 // MN-major 128-byte-swizzle operand layout.
 //
