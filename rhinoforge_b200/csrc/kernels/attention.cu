@@ -17,8 +17,8 @@
 //    thread-block cluster that they form (up to eight) or, beyond that, by a second kernel.
 //
 // Decode, fp16, us, with one lane that copies page by page, merges in rows of bank conflicts and a second kernel / now: 1 x 300 keys, 16 + 2 x 8
-// heads of 128 9.4 / 6.6; 64 x 1024, 32 + 2 x 8 54.8 / 49.6 (K/V at the copy rate: 40.4); 8 x 8000 53.3 / 45.9 (39.4); 32 x 260, 16 + 2 x 4
-// 12.3 / 9.4; 50 rows on 880 keys, 8 + 2 x 1 heads of 256 22.0 as 50 sequences / 11.7 as one.
+// heads of 128 9.4 / 6.6; 64 x 1024, 32 + 2 x 8 54.8 / 48.3 (K/V at the copy rate: 40.4); 8 x 8000 53.3 / 43.7 (39.4); 32 x 260, 16 + 2 x 4
+// 12.3 / 8.6; 50 rows on 880 keys, 8 + 2 x 1 heads of 256 22.0 as 50 sequences / 11.7 as one.
 //
 // Replaces llm_fp16_32b_prefill_flash_attn_univ_* and its vctxlen / minibatch
 // variants (src/ops/rpu_sdpa.cpp:30-37,202-203, src/ops/rpu_sdpa_vctxlen.cpp,

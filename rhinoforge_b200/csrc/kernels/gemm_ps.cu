@@ -15,7 +15,8 @@
 // on compute-bound shapes.  Tiles are numbered with the M index fastest, so the CTAs that run side by side
 // share one weight panel and the activation matrix stays in L2.
 // Scope: tokens on the MMA M axis, tile-major 16-bit weights, no split-K, no fused all-reduce (those shapes
-// stay with gemm_tc.cu).
+// stay with gemm_tc.cu).  Results and residuals that bulk copies can move go to the form with two CTAs to a tile
+// (gemm_pair.cu, see launch_gemm_ps): this one has the others and the grouped form.
 //
 // Grouped form (mixture of experts, rf_moe_grouped_gemm): the rows are (token, pick) pairs sorted by expert and
 // the tile list comes from device memory - one entry {expert, first row, end row} per 128-row block of one

@@ -114,7 +114,8 @@ int rf_gemm(const RfGemm* g, rf_stream_t stream);
 int rf_gemm_takes_mul(const RfGemm* g);   // host-only: can this GEMM apply RfGemm.mul in its epilogue?
 int rf_gemm_takes_norm(const RfGemm* g);  // host-only: can this GEMM take the squares of its rows of x itself (RfGemm.norm_x)?
 // The kernel family rf_gemm / rf_gemm_w8a16 / rf_gemm_w4a16 launch for these arguments (its scratch pointers among them), or a negative
-// RfError.  Host-only.  (int8 weights that are widened into scratch first count as RF_GEMM_TILE, whichever kernel multiplies them then.)
+// RfError.  Host-only.  (int8 weights that are widened into scratch first count as RF_GEMM_TILE, whichever kernel multiplies them then;
+// RF_GEMM_PERSISTENT is either form, one CTA to a tile or two.)
 enum { RF_GEMM_TILE = 0, RF_GEMM_PERSISTENT = 1, RF_GEMM_STREAM_K = 2, RF_GEMM_ROWS = 3, RF_GEMM_SMALL = 4 };
 int rf_gemm_kernel(const RfGemm* g);
 // Launch plan of a shape on the tcgen05 tile kernels without launching (rf_gemm_kernel says whether one of them takes it): out[10] = {swap, bn, splits, stages, grid_x, grid_y, smem bytes, k_blocks,
