@@ -93,8 +93,8 @@ __global__ void rmsnorm_kernel(const T* __restrict__ x, const T* __restrict__ re
   }
 }
 
-// The same for rows of at most 8192 values, eight to a thread that holds them: everything a row needs is asked for at once (its weights ahead of the
-// previous kernel's end, which they do not depend on) and the sum takes one barrier.  A row is one chain of trips to memory, and the kernel above has
+// The same for rows of at most 8192 values, eight to a thread that holds them: everything a row needs, its weights too, is asked for at once and the
+// sum takes one barrier.  A row is one chain of trips to memory, and the kernel above has
 // two of them, four barriers and eight-way bank conflicts in it.  Behind a GEMM, fp16, us, that one / this: 50 x 1024
 // 2.4 / 2.05, 12 x 4096 3.7 / 2.3.  The kernel above takes longer rows, and operands off their 16-byte boundary.
 template <typename T>
@@ -106,8 +106,8 @@ rmsnorm_row_kernel(const T* __restrict__ x, const T* __restrict__ residual, cons
   const int row = blockIdx.x, i = threadIdx.x * 8, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
   const bool in = i < H, weighted = w && !mod;
   const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+  pdl_wait();                                     // the weights may be the previous kernel's as well
   const uint4 wq = weighted && in ? *reinterpret_cast<const uint4*>(w + i) : zero;
-  pdl_wait();
   const T* mrow = mod ? mod + (size_t)(row / rows_per_mod) * 3 * H : nullptr;
   const uint4 xq = in ? *reinterpret_cast<const uint4*>(x + (size_t)row * ldx + i) : zero;
   const uint4 rq = residual && in ? *reinterpret_cast<const uint4*>(residual + (size_t)row * ldx + i) : zero;
@@ -239,14 +239,15 @@ rmsnorm_warp_kernel(const T* __restrict__ x, const T* __restrict__ w, T* __restr
   }
 }
 
-// Weights and biases do not depend on the previous kernel: short rows' are in registers before its results are there (behind a GEMM, us: 3072 x 1152
-// 7.6, so 5.2; 768 x 1152 6.1 / 3.0).
+// Short rows' weights and biases are asked for beside the row (behind its two sums, they were another trip to memory; behind a GEMM, us: 3072 x 1152
+// 7.6, so 5.3; 768 x 1152 6.1 / 3.1).
 template <typename T, int NC>
 __global__ void __launch_bounds__(128)
 layernorm_warp_kernel(const T* __restrict__ x, const T* __restrict__ w, const T* __restrict__ b, T* __restrict__ y, int rows, int H, int64_t ldx,
                       int64_t ldy, float eps) {
   constexpr int kEarly = NC <= 5 ? NC : 0;
   pdl_launch_dependents();
+  pdl_wait();
   const int row = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
   uint4 we[kEarly ? kEarly : 1], be[kEarly ? kEarly : 1];
@@ -256,7 +257,6 @@ layernorm_warp_kernel(const T* __restrict__ x, const T* __restrict__ w, const T*
     we[c] = i < H ? *reinterpret_cast<const uint4*>(w + i) : zero;
     be[c] = b && i < H ? *reinterpret_cast<const uint4*>(b + i) : zero;
   }
-  pdl_wait();
   if (row >= rows) return;
   const T* xr = x + (size_t)row * ldx;
   uint4 v[NC];
