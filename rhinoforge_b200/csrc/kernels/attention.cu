@@ -256,25 +256,29 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
         sn[0] = s0.x; sn[1] = s0.y; sn[2] = s0.z; sn[3] = s0.w; sn[4] = s1.x; sn[5] = s1.y; sn[6] = s1.z; sn[7] = s1.w;
       }
       new_slot = cpos & 15;
-      if (cpos >= 0 && (cpos >> 4) >= pg_begin && (cpos >> 4) < pg_end) new_page = (cpos >> 4) - pg_begin;
-      // a token beyond the keys that are read is still put away, by the first split
-      const bool writes = new_page >= 0 || (split == 0 && cpos >= 0 && (cpos >> 4) >= total_pages);
-      for (int h0 = warp * HPW; h0 < R + 2; h0 += 4 * HPW) {
+      // a token beyond the keys that are read is still put away, by the first split; one whose page nobody owns (a negative number) nowhere, and
+      // it is read as such a page reads: as zeros
+      int page = -1;
+      for (int h0 = warp * HPW; h0 == warp * HPW || h0 < R + 2; h0 += 4 * HPW) {
         const int h = h0 + lane / GROUP;                    // query heads, key, value
         const int col = h < R ? head_of(h) : h == R ? p.Hq + kvh : p.Hq + p.Hkv + kvh;
         const uint4 raw = h < R + 2 ? *reinterpret_cast<const uint4*>(row + (size_t)col * HD + o) : make_uint4(0u, 0u, 0u, 0u);
+        // behind the row's load, which does not wait for the position
+        if (h0 == warp * HPW && cpos >= 0 && (((cpos >> 4) >= pg_begin && (cpos >> 4) < pg_end) || (split == 0 && (cpos >> 4) >= total_pages)))
+          page = p.page_table[(size_t)pt_row * p.pt_stride + (cpos >> 4)];
         float x[8];
         unpack8<T>(raw, x);
         norm_rotate_head<T, HD>(x, reinterpret_cast<const T*>(h < R ? ins.q_norm_w : ins.k_norm_w), ins, lane, cs, sn);
         if (h <= R) store8(fresh + h * kNewLd + o, x);
         else if (h == R + 1) *reinterpret_cast<uint4*>(fresh + h * kNewLd + o) = raw;
-        if (writes && h >= R && h < R + 2) {
-          const size_t at = ((size_t)p.page_table[(size_t)pt_row * p.pt_stride + (cpos >> 4)] * p.Hkv + kvh) * 16 + new_slot;
+        if (h >= R && h < R + 2 && page >= 0) {
+          const size_t at = ((size_t)page * p.Hkv + kvh) * 16 + new_slot;
           if (h == R) store8(reinterpret_cast<T*>(ins.k_pool) + at * HD + o, x);
           else *reinterpret_cast<uint4*>(reinterpret_cast<T*>(ins.v_pool) + at * HD + o) = raw;
         }
       }
       asm volatile("bar.sync 1, 128;" ::: "memory");        // the four consumer warps
+      if (page >= 0 && (cpos >> 4) < pg_end) new_page = (cpos >> 4) - pg_begin;
     }
     {
       const int g0 = lane >> 2, g1 = g0 + 8;

@@ -1162,6 +1162,53 @@ def test_attn_decode_inserts(dt, hd, Hq, Hkv, rot, lens, mode, status):
 
 
 @pytest.mark.parametrize("dt", DT)
+@pytest.mark.parametrize("hd,Hq,Hkv", [(64, 8, 2), (128, 16, 8), (256, 8, 1)])
+@pytest.mark.parametrize("lens", [[33, 16, 7], [1500, 700, 15]])
+def test_attn_decode_inserts_nothing_into_a_page_of_nobody(dt, hd, Hq, Hkv, lens, status):
+    """A new token whose page number is negative, among the keys read and behind them: nothing is written, not in front of the pool either, and the
+    page reads as zeros, bit for bit as with the two launches."""
+    import ctypes as C
+    from rhinoforge_b200 import _native as N
+    from rhinoforge_b200.ops import kernels as K_
+    n, maxp = len(lens), (max(lens) + 15) // 16 + 2
+    g = torch.Generator(device="cuda").manual_seed(hd)
+    qkv = torch.randn(n, (Hq + 2 * Hkv) * hd, device="cuda", generator=g).to(dt)
+    room = torch.randn(2, n * maxp + 2, Hkv, 16, hd, device="cuda", generator=g).to(dt)           # a page in front of each pool and one behind
+    pt = torch.randperm(n * maxp, device="cuda", generator=g).to(torch.int32).view(n, maxp)
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")
+    kv_len, pos = i32(lens), i32([l - 1 for l in lens])
+    pt[0, (lens[0] - 1) // 16] = -1
+    pos[1] += 16
+    pt[1, (lens[1] + 15) // 16] = -1
+    cos, sin = torch.randn(2, max(lens) + 16, hd // 2, device="cuda", generator=g)
+    ws = K_.attn_decode_scratch(n, Hq, hd, "cuda")
+
+    def run(fused):
+        rows, buf, out = qkv.clone(), room.clone(), torch.zeros(n, Hq * hd, device="cuda", dtype=dt)
+        r, a = N.RfRopeKv(), N.RfAttn()
+        r.qkv, r.ld, r.tokens, r.Hq, r.Hkv, r.hd, r.rot_dim, r.dtype = rows.data_ptr(), rows.stride(0), n, Hq, Hkv, hd, hd, 0 if dt == torch.float16 else 1
+        r.cos, r.sin, r.pos, r.pos_stride, r.cache_pos = cos.data_ptr(), sin.data_ptr(), pos.data_ptr(), 1, pos.data_ptr()
+        r.k_pool, r.v_pool, r.page_table, r.pt_stride = buf[0, 1:].data_ptr(), buf[1, 1:].data_ptr(), pt.data_ptr(), maxp
+        a.q, a.ldq, a.out, a.ldo, a.q_rows_total = rows.data_ptr(), rows.stride(0), out.data_ptr(), out.stride(0), n
+        a.k_pool, a.v_pool, a.pool_pages, a.page_table, a.pt_stride = r.k_pool, r.v_pool, n * maxp, pt.data_ptr(), maxp
+        a.num_seqs, a.Hq, a.Hkv, a.hd, a.kv_len, a.max_kv_len, a.dtype = n, Hq, Hkv, hd, kv_len.data_ptr(), max(lens), r.dtype
+        a.ws, a.ws_bytes, a.status, a.rows_per_seq = ws.data_ptr(), ws.numel() * 4, status.data_ptr(), 1
+        L, st = N.lib(), C.c_void_p(torch.cuda.current_stream().cuda_stream)
+        if fused:
+            assert L.rf_attn_decode_inserts(C.byref(a), C.byref(r)) == 1
+            N.check(L.rf_attn_decode_insert(C.byref(a), C.byref(r), st), "insert")
+        else:
+            N.check(L.rf_qk_norm_rope_kv(C.byref(r), st), "rope")
+            N.check(L.rf_attn_decode(C.byref(a), st), "decode")
+        return out, buf
+
+    got, buf = run(True)
+    want, ref = run(False)
+    assert torch.equal(got, want) and torch.equal(buf, ref)
+    assert torch.equal(buf[:, :1], room[:, :1]) and torch.equal(buf[:, -1:], room[:, -1:])
+
+
+@pytest.mark.parametrize("dt", DT)
 @pytest.mark.parametrize("H", [8, 264, 1024, 1152, 2040, 3072, 4096, 4104])
 @pytest.mark.parametrize("rows", [295, 1301, 3001])
 def test_norms_of_many_rows(dt, H, rows):
