@@ -98,6 +98,7 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity,
                                           uint64_t limit_ns = kLocalWaitNs, uint32_t backoff_ns = 0) {
   if (mbar_try_wait(bar, parity)) return true;
+  if (limit_ns == 0) return false;
   const uint64_t t0 = global_timer_ns();
   while (true) {
 #pragma unroll 1
@@ -109,14 +110,37 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity,
   }
 }
 
-// The same for roles that go on after a timeout (with whatever data there is, so that everything in flight drains by itself): the
-// first one reports `code` and leaves no patience for the waits behind it.
-__device__ __forceinline__ void mbar_wait_or_report(uint64_t* bar, uint32_t parity, uint64_t* limit_ns, uint32_t backoff_ns, int32_t* status,
-                                                    int32_t code, int32_t tag, int32_t detail) {
-  if (!mbar_wait(bar, parity, *limit_ns, backoff_ns)) {
-    if (*limit_ns) report_status(status, code, tag, detail);
-    *limit_ns = 0;
-  }
+// What happens once in a launch's life or never stands out of line: inside the kernels it cost a GEMM of 93 rows half a microsecond of instruction
+// fetches (prompt of 93 tokens, 16 layers, us: 1236, so 1192).
+static __device__ __noinline__ void role_gives_up(int32_t* gave_up, int32_t* status, int32_t code, int32_t tag, int32_t detail, uint32_t peer) {
+  volatile int32_t* flag = gave_up;
+  if (!*flag) report_status(status, code, tag, detail);
+  *flag = 1;
+  if (peer) asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(peer), "r"(1u) : "memory");
+  asm volatile("fence.acq_rel.cluster;" ::: "memory");
+}
+// A wait of a role that its whole warp runs; the answer is the lane's own.  When it runs out, `code` is reported (by the first role of the CTA to give
+// up), `gave_up` is set, ahead of anything that the role does next, and its later waits have no patience.  Behind that
+//   * a role that writes what others may still use (copies into a ring, a new accumulator, stores, arrivals) starts nothing more;
+//   * the MMA role alone goes on through the k blocks of an accumulator whose operands did not come: it writes nothing but that accumulator, and
+//     whoever is told that it is complete looks at `gave_up` before taking it.  A test or a vote between barrier and MMA would cost every launch
+//     (prefill attention, a chain of such waits, 2 to 10 per cent);
+//   * the teardown waits for what was started (settle_copies, settle_mmas).
+// `peer`: the flag of the pair's other CTA (a shared::cluster address), 0 for none.
+__device__ __forceinline__ bool role_wait(uint64_t* bar, uint32_t parity, uint64_t* limit_ns, int32_t* gave_up, int32_t* status, int32_t code,
+                                          int32_t tag, int32_t detail, uint32_t backoff_ns = 0, uint32_t peer = 0) {
+  if (mbar_wait(bar, parity, *limit_ns, backoff_ns)) return true;
+  role_gives_up(gave_up, status, code, tag, detail, peer);
+  *limit_ns = 0;
+  return false;
+}
+// Whether a wait came true in every lane: the warp leaves a loop together.
+__device__ __forceinline__ bool agreed(bool ok) { return __all_sync(0xffffffffu, ok); }
+// Teardown after a role gave up, when every role has stopped: what was started has to end before the CTA's memory goes.  Copies: the last `stages`
+// of `issued` fills of a ring, each of which completes a phase of its stage's barrier.
+constexpr uint64_t kSettleNs = 20ull * 1000 * 1000;
+static __device__ __noinline__ void settle_copies(uint64_t* full, int stages, int issued) {
+  for (int i = issued > stages ? issued - stages : 0; i < issued; ++i) mbar_wait(&full[i % stages], (uint32_t)(i / stages) & 1u, kSettleNs);
 }
 
 // ----------------------------------------------------------------- TMA ----
@@ -251,6 +275,13 @@ __device__ __forceinline__ void umma_commit(uint64_t* bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
                    smem_u32(bar))
                : "memory");
+}
+// Teardown after a role gave up, by the warp whose elected lane issued (elect_one names the same one again): its MMAs end before tensor memory is
+// handed back.
+static __device__ __noinline__ void settle_mmas(uint64_t* bar) {
+  if (elect_one()) umma_commit(bar);
+  __syncwarp();
+  mbar_wait(bar, 0, kSettleNs);
 }
 __device__ __forceinline__ void tmem_ld_wait() {
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
@@ -393,10 +424,10 @@ __device__ __forceinline__ void pair_umma_f16(uint32_t tmem_d, uint64_t desc_a, 
       "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
       : "memory");
 }
-// The barrier at this offset in BOTH CTAs' shared memory arrives once every MMA issued so far by this thread has finished.
-__device__ __forceinline__ void pair_umma_commit(uint64_t* bar) {
+// The barrier at this offset in BOTH CTAs' shared memory (or those of `ctas`) arrives once every MMA issued so far by this thread has finished.
+__device__ __forceinline__ void pair_umma_commit(uint64_t* bar, uint16_t ctas = 3) {
   asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(smem_u32(bar)),
-               "h"((uint16_t)3)
+               "h"(ctas)
                : "memory");
 }
 // Tiled load into this CTA's shared memory that completes on a barrier of either CTA of the pair (`bar`: a shared::cluster address).

@@ -43,9 +43,9 @@ constexpr int kFaMaxStages = 8;
 constexpr float kFaRaise = 8.0f;      // raise the reference maximum only beyond 2^8
 
 struct alignas(8) FaCtl {
-  uint64_t q_full, kv_full[kFaMaxStages], kv_empty[kFaMaxStages], s_full[2][2], p_full[2][2], pv_done[2], o_full[2];
+  uint64_t q_full, kv_full[kFaMaxStages], kv_empty[kFaMaxStages], s_full[2][2], p_full[2][2], pv_done[2], o_full[2], settled;
   uint32_t tmem_base;
-  int32_t abort_flag;
+  int32_t abort_flag, issued;            // issued: K/V blocks that the producer has asked for
 };
 
 // HD: size of a query / key head, VD: of a value head, NQ: query tiles of a CTA.  Heads of 80 (vision towers' 72) arrive as two 64-column boxes
@@ -136,6 +136,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
       mbar_init(&ctl->pv_done[t], 1);
       mbar_init(&ctl->o_full[t], 1);
     }
+    mbar_init(&ctl->settled, 1);
     ctl->abort_flag = 0;
     fence_barrier_init();
     tma_prefetch_desc(&tmQ);
@@ -153,13 +154,13 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
   pdl_launch_dependents();     // only after this CTA owns its TMEM columns
   pdl_wait();                  // q, k, v come from the previous kernel
   volatile int32_t* abort_flag = &ctl->abort_flag;
+  uint64_t limit = kLocalWaitNs;
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer ----
     // the warp reads 32 page numbers at a time, one elected lane issues the copies
     constexpr int kPagesPerBlock = KVB / 16, kBlocksPerFetch = 32 / kPagesPerBlock;
     const bool lead = elect_one();
-    uint64_t limit = kLocalWaitNs;
     if (lead) {
       mbar_arrive_expect_tx(&ctl->q_full, (uint32_t)(tiles * G::kQTile));
       for (int t = 0; t < tiles; ++t)
@@ -170,14 +171,15 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
     const int row0 = p.paged ? 0 : p.kv_start[seq];
     int pages = 0, s = 0;
     uint32_t phase = 1;                                     // nothing is waited for on the first turn of the ring
-    for (int j = 0; j < nblk; ++j) {
+    int j = 0;
+    for (; j < nblk; ++j) {
       if (p.paged && j % kBlocksPerFetch == 0)
         pages = p.page_table[(size_t)pt_row * p.pt_stride + min(block_start(j + lane / kPagesPerBlock) / 16 + lane % kPagesPerBlock, p.pt_stride - 1)];
       int block_pages[kPagesPerBlock];
 #pragma unroll
       for (int w = 0; w < kPagesPerBlock; ++w) block_pages[w] = __shfl_sync(0xffffffffu, pages, (j % kBlocksPerFetch) * kPagesPerBlock + w);
-      mbar_wait_or_report(&ctl->kv_empty[s], phase, &limit, 32, p.status, kStatusTmaTimeout, kTagAttnPrefill, j);
-      if (lead) {
+      const bool free = role_wait(&ctl->kv_empty[s], phase, &limit, &ctl->abort_flag, p.status, kStatusTmaTimeout, kTagAttnPrefill, j, 32);
+      if (free && lead) {
         uint8_t* ks = kvsm + s * G::kStageBytes;
         uint8_t* vs = ks + G::kKBytes;
         mbar_arrive_expect_tx(&ctl->kv_full[s], (uint32_t)G::kStageBytes);
@@ -202,26 +204,21 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
           }
         }
       }
+      if (!agreed(free)) break;
       if (++s == stages) { s = 0; phase ^= 1u; }
     }
-    if (limit == 0) ctl->abort_flag = 1;
-    if (*abort_flag) {   // let every copy that was issued land before the CTA can exit
-      mbar_wait(&ctl->q_full, 0, 20ull * 1000 * 1000);
-      for (int j = max(0, nblk - stages); j < nblk; ++j)
-        mbar_wait(&ctl->kv_full[j % stages], (uint32_t)(j / stages) & 1u, 20ull * 1000 * 1000);
-    }
+    if (lead) ctl->issued = j;
   } else if (warp == 1) {
     // ------------------------------------------------------------- MMA issuer ----
     if (nblk > 0) {
       const bool lead = elect_one();
-      uint64_t limit = kLocalWaitNs;
       const uint32_t idesc_qk = umma_idesc_f16(kFaRows, KVB, Num<T>::kFmt, 0);
       const uint32_t idesc_pv = umma_idesc_f16(kFaRows, VD, Num<T>::kFmt, 1);
       // One lane issues every MMA, twelve per tile and block: the operand descriptors are made once and advance by constants (16-byte units)
       const uint64_t q_desc = umma_desc_k128(smem_u32(qsm));
       const uint64_t k_desc0 = umma_desc_k128(smem_u32(kvsm)), v_desc0 = umma_desc_mn128(smem_u32(kvsm) + G::kKBytes, (uint32_t)(KVB * 128));
       auto wait = [&](uint64_t* bar, uint32_t parity) {
-        mbar_wait_or_report(bar, parity, &limit, 0, p.status, kStatusMmaTimeout, kTagAttnPrefill, 1000);
+        role_wait(bar, parity, &limit, &ctl->abort_flag, p.status, kStatusMmaTimeout, kTagAttnPrefill, 1000);
       };
       wait(&ctl->q_full, 0);
       auto issue_qk = [&](int t, int j, int s, uint32_t ph) {
@@ -269,7 +266,6 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
         s = s_next;
         if (++s_next == stages) { s_next = 0; ph_next ^= 1u; }
       }
-      if (limit == 0) ctl->abort_flag = 1;
     }
   } else {
     // ------------------------------------------------- softmax / correction / epilogue ----
@@ -294,7 +290,8 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
     const float score_mul = p.slopes ? 1.f : p.scale_log2;
     for (int j = 0; j < nblk; ++j) {
       const int b = j & 1;
-      if (!mbar_wait(&ctl->s_full[t][b], (uint32_t)(j >> 1) & 1u) || *abort_flag) { ok = false; break; }
+      const bool have = role_wait(&ctl->s_full[t][b], (uint32_t)(j >> 1) & 1u, &limit, &ctl->abort_flag, p.status, kStatusEpilogueTimeout, kTagAttnPrefill, r);
+      if (!have || *abort_flag) { ok = false; break; }
       tc_fence_after_sync();
       const int t0 = block_start(j);
       const uint32_t s_addr = lane_base + (uint32_t)((t * 2 + b) * KVB);
@@ -405,7 +402,8 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
         if (j > 0) {
           // O belongs to the tensor core until P.V of the previous block has finished (that of the block before is: it was issued ahead of
           // this block's Q.K^T, so the parity is not ambiguous)
-          if (!mbar_wait(&ctl->pv_done[t], (uint32_t)(j - 1) & 1u)) { ok = false; break; }
+          ok = role_wait(&ctl->pv_done[t], (uint32_t)(j - 1) & 1u, &limit, &ctl->abort_flag, p.status, kStatusEpilogueTimeout, kTagAttnPrefill, r);
+          if (!ok) break;
           tc_fence_after_sync();
 #pragma unroll 1
           for (int c0 = 0; c0 < VD; c0 += 32) {
@@ -445,11 +443,8 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
       if (lane == 0) mbar_arrive(&ctl->p_full[t][b]);
     }
     // epilogue: O / l
-    if (ok && nblk > 0) ok = mbar_wait(&ctl->o_full[t], 0);
-    if (!ok) {
-      if (!*abort_flag) report_status(p.status, kStatusEpilogueTimeout, kTagAttnPrefill, r);
-      ctl->abort_flag = 1;
-    }
+    if (nblk > 0) ok &= role_wait(&ctl->o_full[t], 0, &limit, &ctl->abort_flag, p.status, kStatusEpilogueTimeout, kTagAttnPrefill, r);
+    ok = agreed(ok && !*abort_flag);
     tc_fence_after_sync();
     if (ok) {
       if (p.sink && l > 0.f) l += exp2f(p.sink[h] * kLog2e - m_ref);
@@ -492,6 +487,13 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
   // ----------------------------------------------------------------- teardown ----
   tc_fence_before_sync();
   __syncthreads();
+  if (*abort_flag) {           // a role gave up: what the others had started ends first
+    if (warp == 0) {
+      mbar_wait(&ctl->q_full, 0, kSettleNs);
+      settle_copies(ctl->kv_full, stages, ctl->issued);
+    }
+    if (warp == 1) settle_mmas(&ctl->settled);
+  }
   if (warp == 1) tmem_dealloc(tmem_base, (uint32_t)G::kTmemCols);
 }
 

@@ -34,8 +34,9 @@ struct GemmPairParams {
 };
 
 struct alignas(8) GemmPairCtl {
-  uint64_t full[kPrMaxStages], empty[kPrMaxStages], acc_full[2], acc_empty[2], res[kPrEpiWarps][2];
+  uint64_t full[kPrMaxStages], empty[kPrMaxStages], acc_full[2], acc_empty[2], res[kPrEpiWarps][2], settled;
   uint32_t tmem_base;
+  int32_t gave_up;                                         // a role of either CTA did (see role_wait)
 };
 
 // Bands of row tiles, row index fastest inside a band (see gemm_ps.cu): the pairs that run side by side share a few weight panels.
@@ -45,6 +46,21 @@ __device__ __forceinline__ void pair_tile_coords(const GemmPairParams& p, int ti
   const int rows_here = min(p.band, p.tiles_m - b * p.band);
   *tn = r / rows_here;
   *tm = b * p.band + r % rows_here;
+}
+
+// A role of one CTA gave up and all of both have stopped: what they had started ends first.  A copy completes on the even CTA's barrier, in a phase
+// that lacks an arrival where only one of the two had asked for its stage, so copies (residuals among them) get their time by the clock.
+static __device__ __noinline__ void settle_pair(uint64_t* settled, uint32_t rank, int warp) {
+  if (warp == 0) {
+    const uint64_t t0 = global_timer_ns();
+    while (global_timer_ns() - t0 < kSettleNs) __nanosleep(1000);
+  } else if (warp == 1 && rank == 0) {
+    if (elect_one()) pair_umma_commit(settled, 1);
+    __syncwarp();
+    mbar_wait(settled, 0, kSettleNs);
+  }
+  __syncwarp();
+  cluster_sync_all();
 }
 
 // EXTRA: scale, bias or row scale (the residual is handled either way)
@@ -72,6 +88,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       mbar_init(&ctl->acc_empty[b], 2 * kPrEpiWarps);
       for (int w = 0; w < kPrEpiWarps; ++w) mbar_init(&ctl->res[w][b], 1);
     }
+    mbar_init(&ctl->settled, 1);
+    ctl->gave_up = 0;
     fence_barrier_init();
     tma_prefetch_desc(&tmA);
     tma_prefetch_desc(&tmW);
@@ -89,6 +107,11 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   pdl_launch_dependents();
   const int tiles = p.tiles_m * p.tiles_n, first = blockIdx.x >> 1, step = gridDim.x >> 1;
   uint64_t limit = kLocalWaitNs;
+  volatile int32_t* gave_up = &ctl->gave_up;
+  const uint32_t peer_gave_up = dsmem_addr(smem_u32(&ctl->gave_up), rank ^ 1u);
+  auto wait = [&](uint64_t* bar, uint32_t parity, int32_t code, int32_t detail) {
+    return role_wait(bar, parity, &limit, &ctl->gave_up, p.status, code, kTagGemmTc, detail, 0, peer_gave_up);
+  };
 
   if (warp == 0) {
     // ------------------------------------------------------------------ producer ----
@@ -132,26 +155,25 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       for (int i = 0; i < pre; ++i) pair_tma_load_2d(smem + i * stage_bytes, &tmA, full0 + i * 8, i * kPrBK, xr);
     int tile = first, kb = pre, s = pre == p.stages ? 0 : pre;
     uint32_t phase = pre == p.stages ? 0 : 1;              // a stage's first release completes phase 0; before it nothing is waited for
+    bool go = true;
     for (int i = pre; i < total; ++i, ++kb) {
       if (kb == p.k_blocks) {
         kb = 0;
         tile += step;
         enter_tile(tile);
       }
-      mbar_wait_or_report(&ctl->empty[s], phase, &limit, 0, p.status, kStatusTmaTimeout, kTagGemmTc, i);
-      if (lead) {
+      const bool free = wait(&ctl->empty[s], phase, kStatusTmaTimeout, i);
+      if (free && lead) {
         if (rank == 0) mbar_arrive_expect_tx(&ctl->full[s], tx);
         load_w(kb, s);
         pair_tma_load_2d(smem + s * stage_bytes, &tmA, full0 + s * 8, kb * kPrBK, xr);
       }
+      go = agreed(free);
+      if (!go) break;
       if (++s == p.stages) { s = 0; phase ^= 1u; }
     }
     // The last stages' releases come from the even CTA's commits: neither CTA may leave before they are in.
-    for (int i = max(0, total - p.stages); i < total; ++i) {
-      const uint32_t parity = (uint32_t)(i / p.stages) & 1u;
-      mbar_wait_or_report(&ctl->empty[i % p.stages], parity, &limit, 0, p.status, kStatusTmaTimeout, kTagGemmTc, i);
-      if (limit == 0 && rank == 0) mbar_wait(&ctl->full[i % p.stages], parity, 20ull * 1000 * 1000);     // copies in flight get time to land
-    }
+    for (int i = max(0, total - p.stages); go && i < total; ++i) go = agreed(wait(&ctl->empty[i % p.stages], (uint32_t)(i / p.stages) & 1u, kStatusTmaTimeout, i));
   } else if (warp == 1) {
     // ------------------------------------------------- MMA issuer (even CTA) ----
     pdl_wait();
@@ -166,11 +188,11 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       uint32_t phase = 0, at = 0;
       for (int tile = first; tile < tiles; tile += step, ++lt) {
         const int b = lt & 1;
-        mbar_wait_or_report(&ctl->acc_empty[b], (((uint32_t)(lt >> 1)) & 1u) ^ 1u, &limit, 0, p.status, kStatusMmaTimeout, kTagGemmTc, lt);
+        if (!agreed(wait(&ctl->acc_empty[b], (((uint32_t)(lt >> 1)) & 1u) ^ 1u, kStatusMmaTimeout, lt) && limit)) break;
         tc_fence_after_sync();
         const uint32_t acc = tmem_base + (uint32_t)(b * 256);
         for (int kb = 0; kb < p.k_blocks; ++kb) {
-          mbar_wait_or_report(&ctl->full[s], phase, &limit, 0, p.status, kStatusMmaTimeout, kTagGemmTc, lt);
+          wait(&ctl->full[s], phase, kStatusMmaTimeout, lt);
           tc_fence_after_sync();
           if (lead) {
             const uint64_t ad = a_desc + at, bd = b_desc + at;
@@ -207,6 +229,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       k.row = (tm * 2 + (int)rank) * kPrBM + quarter * 32;
     };
     auto live = [&](const Chunk& k) { return k.tile < tiles && k.row < p.M && k.col < p.N; };
+    // Once a wait of this warp has run out, or another role has given up (limit == 0), the warp goes through its chunks without asking for a
+    // residual, handing an accumulator back or storing.
     // Two columns to a lane, put together when they are used: an instruction on them here would wait for the trip to memory.
     struct Cols {
       uint16_t lo = 0, hi = 0;
@@ -231,7 +255,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         if (DUAL && scale) v.su = pair_of(scale + p.dual_offset, n);
         if (p.row_scale && k.row + lane < p.M) v.rs = p.row_scale[k.row + lane];
       }
-      if (p.residual && lane == 0) {
+      if (p.residual && lane == 0 && limit) {
         bulk_wait_read_all();                              // this buffer's last result has left
         mbar_arrive_expect_tx(&ctl->res[ew][buf], kPrChunk);
         tma_load_2d(stg + buf * kPrChunk, &tmR, &ctl->res[ew][buf], k.col, k.row);
@@ -245,7 +269,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     ask(cur, 0, vec);
     for (int tile = first; tile < tiles; tile += step, ++lt) {
       const int b = lt & 1;
-      mbar_wait_or_report(&ctl->acc_full[b], (uint32_t)(lt >> 1) & 1u, &limit, 0, p.status, kStatusEpilogueTimeout, kTagGemmTc, tile);
+      wait(&ctl->acc_full[b], (uint32_t)(lt >> 1) & 1u, kStatusEpilogueTimeout, tile);
+      if (*gave_up) limit = 0;
       tc_fence_after_sync();
       // The accumulator may be overwritten by the pair's tile after next once this warp's last values are in registers: the arrival is
       // remote for the odd CTA and its release would wait for the stores below.
@@ -253,7 +278,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       auto release = [&]() {
         tc_fence_before_sync();
         __syncwarp();
-        if (lane == 0) mbar_arrive_cluster(acc_empty0 + b * 8);
+        if (lane == 0 && limit) mbar_arrive_cluster(acc_empty0 + b * 8);
         released = true;
       };
       while (cur.tile == tile) {
@@ -267,7 +292,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         if (now) {
           uint8_t* tile_out = stg + buf * kPrChunk;
           if (p.residual) {
-            mbar_wait_or_report(&ctl->res[ew][buf], (res_phase >> buf) & 1u, &limit, 0, p.status, kStatusTmaTimeout, kTagGemmTc, tile);
+            wait(&ctl->res[ew][buf], (res_phase >> buf) & 1u, kStatusTmaTimeout, tile);
             res_phase ^= 1u << buf;
           } else if (lane == 0) {
             bulk_wait_read_1();
@@ -343,7 +368,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
           }
           fence_proxy_async();
           __syncwarp();
-          if (lane == 0) {
+          if (lane == 0 && limit) {
             tma_store_2d(&tmO, tile_out, cur.col, cur.row);
             bulk_commit_group();
           }
@@ -359,6 +384,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   __syncwarp();
   tc_fence_before_sync();
   cluster_sync_all();                                      // the even CTA's MMAs read the odd one's shared memory to the end
+  if (*gave_up) settle_pair(&ctl->settled, rank, warp);
   if (warp == 1) pair_tmem_dealloc(tmem_base, 512u);
 }
 

@@ -96,9 +96,9 @@ __device__ __forceinline__ PsTile ps_tile(const GemmPsParams& p, int tile) {
 }
 
 struct alignas(8) GemmPsCtl {
-  uint64_t full[kPsMaxStages], empty[kPsMaxStages], acc_full[2], acc_empty[2];
+  uint64_t full[kPsMaxStages], empty[kPsMaxStages], acc_full[2], acc_empty[2], settled;
   uint32_t tmem_base;
-  int32_t abort_flag;
+  int32_t abort_flag, issued;                              // issued: k blocks that the producer has asked for
 };
 
 __device__ __forceinline__ uint4 shfl_u4(const uint4& q, int lane) {
@@ -136,6 +136,7 @@ gemm_ps_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
       mbar_init(&ctl->acc_full[b], 1);
       mbar_init(&ctl->acc_empty[b], 4 * MT);
     }
+    mbar_init(&ctl->settled, 1);
     ctl->abort_flag = 0;
     fence_barrier_init();
     tma_prefetch_desc(&tmA);
@@ -225,26 +226,24 @@ gemm_ps_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     if (total && pre == 0) t = ps_tile<MT>(p, tile);
     int kb = pre, s = pre == p.stages ? 0 : pre;
     uint32_t phase = pre == p.stages ? 0 : 1;              // a stage's first release completes phase 0; before it nothing is waited for
-    for (int i = pre; i < total; ++i, ++kb) {
+    int i = pre;
+    for (; i < total; ++i, ++kb) {
       if (kb == p.k_blocks) {
         kb = 0;
         tile += gridDim.x;
         t = ps_tile<MT>(p, tile);
       }
-      mbar_wait_or_report(&ctl->empty[s], phase, &limit, 0, p.status, kStatusTmaTimeout, kTagGemmTc, i);
-      if (lead) {
+      const bool free = role_wait(&ctl->empty[s], phase, &limit, &ctl->abort_flag, p.status, kStatusTmaTimeout, kTagGemmTc, i);
+      if (free && lead) {
         mbar_arrive_expect_tx(&ctl->full[s], (uint32_t)stage_bytes);
         load_w(t, kb, s);
         load_x(t, kb, s);
         if (p.pf_blocks > 0) prefetch_next(true, true);
       }
+      if (!agreed(free)) break;
       if (++s == p.stages) { s = 0; phase ^= 1u; }
     }
-    if (limit == 0) {
-      ctl->abort_flag = 1;
-      for (int i = max(0, total - p.stages); i < total; ++i)             // every copy that was issued gets time to land
-        mbar_wait(&ctl->full[i % p.stages], (uint32_t)(i / p.stages) & 1u, 20ull * 1000 * 1000);
-    }
+    if (lead) ctl->issued = i;
   } else if (warp == 1) {
     // ---------------------------------------------------------------- MMA issuer ----
     pdl_wait();
@@ -258,11 +257,11 @@ gemm_ps_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     const int tiles = tile_count();
     for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x, ++lt) {
       const int b = nbuf == 2 ? lt & 1 : 0;
-      mbar_wait_or_report(&ctl->acc_empty[b], ((uint32_t)(nbuf == 2 ? lt >> 1 : lt) & 1u) ^ 1u, &limit, 0, p.status, kStatusMmaTimeout, kTagGemmTc, lt);
+      if (!agreed(role_wait(&ctl->acc_empty[b], ((uint32_t)(nbuf == 2 ? lt >> 1 : lt) & 1u) ^ 1u, &limit, &ctl->abort_flag, p.status, kStatusMmaTimeout, kTagGemmTc, lt) && limit)) break;
       tc_fence_after_sync();
       const uint32_t acc = tmem_base + (uint32_t)(b * acc_cols);
       for (int kb = 0; kb < p.k_blocks; ++kb) {
-        mbar_wait_or_report(&ctl->full[s], phase, &limit, 0, p.status, kStatusMmaTimeout, kTagGemmTc, lt);
+        role_wait(&ctl->full[s], phase, &limit, &ctl->abort_flag, p.status, kStatusMmaTimeout, kTagGemmTc, lt);
         tc_fence_after_sync();
         if (lead) {
           const uint64_t da = a_desc + at, db = b_desc + at;
@@ -282,7 +281,6 @@ gemm_ps_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
       }
       if (lead) umma_commit(&ctl->acc_full[b]);
     }
-    if (limit == 0) ctl->abort_flag = 1;
   } else {
     // ------------------------------------------------------------------ epilogue ----
     pdl_wait();
@@ -323,11 +321,8 @@ gemm_ps_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
           for (int q = 0; q < (DUAL ? 4 : 2); ++q) rv[q >> 1][q & 1] = vec8_upto(resid + (size_t)row * p.ldr, n_base + q * 8, N, res_vec);
         }
       }
-      if (!mbar_wait(&ctl->acc_full[b], (uint32_t)(lt / nbuf) & 1u) || *abort_flag) {
-        if (!*abort_flag) report_status(p.status, kStatusEpilogueTimeout, kTagGemmTc, tile);
-        ctl->abort_flag = 1;
-        break;
-      }
+      const bool have = role_wait(&ctl->acc_full[b], (uint32_t)(lt / nbuf) & 1u, &limit, &ctl->abort_flag, p.status, kStatusEpilogueTimeout, kTagGemmTc, tile);
+      if (!agreed(have && !*abort_flag)) break;
       tc_fence_after_sync();
       const uint32_t acc = lane_base + (uint32_t)(b * acc_cols + half * half_cols);
       const float rs = (EXTRA && p.row_scale && row < M) ? p.row_scale[row] : 1.f;
@@ -460,6 +455,10 @@ gemm_ps_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
   }
   tc_fence_before_sync();
   __syncthreads();
+  if (*abort_flag) {                                       // a role gave up: what the others had started ends first
+    if (warp == 0) settle_copies(ctl->full, p.stages, ctl->issued);
+    if (warp == 1) settle_mmas(&ctl->settled);
+  }
   if (warp == 1) tmem_dealloc(tmem_base, 512u);
 }
 

@@ -61,9 +61,9 @@ struct GemmSkParams {
 };
 
 struct alignas(8) GemmSkCtl {
-  uint64_t full[kSkMaxStages], empty[kSkMaxStages], acc_full[2], acc_empty[2];
+  uint64_t full[kSkMaxStages], empty[kSkMaxStages], acc_full[2], acc_empty[2], settled;
   uint32_t tmem_base;
-  int32_t abort_flag;
+  int32_t abort_flag, issued;  // issued: k blocks that the producer has asked for
   int32_t partner_bad;
   int32_t partner_count;
 };
@@ -73,6 +73,13 @@ __device__ __forceinline__ void st_release_gpu(uint32_t* p, uint32_t v) {
 }
 __device__ __forceinline__ void epi_bar_sync() {   // the four epilogue warps only (named barrier 1)
   asm volatile("bar.sync 1, 128;" ::: "memory");
+}
+// The same, and whether any of their threads said so: one answer for all of them.
+__device__ __forceinline__ bool epi_bar_any(bool mine) {
+  uint32_t any;
+  asm volatile("{\n .reg .pred p, q;\n setp.ne.b32 p, %1, 0;\n barrier.cta.red.or.pred q, 1, 128, p;\n selp.b32 %0, 1, 0, q;\n}"
+               : "=r"(any) : "r"((uint32_t)mine) : "memory");
+  return any != 0;
 }
 
 // The share of CTA c: units [c * U / P, (c + 1) * U / P)
@@ -107,6 +114,7 @@ gemm_sk_kernel(const __grid_constant__ CUtensorMap tmX, const GemmSkParams p) {
       mbar_init(&ctl->acc_full[b], 1);
       mbar_init(&ctl->acc_empty[b], 4);
     }
+    mbar_init(&ctl->settled, 1);
     ctl->abort_flag = 0;
     ctl->partner_bad = 0;
     fence_barrier_init();
@@ -158,22 +166,20 @@ gemm_sk_kernel(const __grid_constant__ CUtensorMap tmX, const GemmSkParams p) {
       if (++kb == KB) kb = 0;
     }
     uint32_t phase = 0;                                    // of the release that a refill of stage s waits for
-    for (int i = pre; i < total; ++i) {
-      mbar_wait_or_report(&ctl->empty[s], phase, &limit, 0, p.status, kStatusTmaTimeout, kTagGemmTc, i);
-      if (lead) {
+    int i = pre;
+    for (; i < total; ++i) {
+      const bool free = role_wait(&ctl->empty[s], phase, &limit, &ctl->abort_flag, p.status, kStatusTmaTimeout, kTagGemmTc, i);
+      if (free && lead) {
         mbar_arrive_expect_tx(&ctl->full[s], (uint32_t)stage_bytes);
         load_w(w_at, s);
         load_x(kb, s);
       }
+      if (!agreed(free)) break;
       w_at += kSkWBlock;
       if (++kb == KB) kb = 0;
       if (++s == p.stages) { s = 0; phase ^= 1u; }
     }
-    if (limit == 0) {
-      ctl->abort_flag = 1;
-      for (int i = max(0, total - p.stages); i < total; ++i)             // every copy that was issued gets time to land
-        mbar_wait(&ctl->full[i % p.stages], (uint32_t)(i / p.stages) & 1u, 20ull * 1000 * 1000);
-    }
+    if (lead) ctl->issued = i;
   } else if (warp == 1) {
     // ---------------------------------------------------------------- MMA issuer ----
     pdl_wait();
@@ -187,11 +193,11 @@ gemm_sk_kernel(const __grid_constant__ CUtensorMap tmX, const GemmSkParams p) {
     for (int seg = 0; left > 0; ++seg, kb = 0) {
       const int count = min(left, KB - kb);
       const int b = nbuf == 2 ? seg & 1 : 0;
-      mbar_wait_or_report(&ctl->acc_empty[b], ((uint32_t)(nbuf == 2 ? seg >> 1 : seg) & 1u) ^ 1u, &limit, 0, p.status, kStatusMmaTimeout, kTagGemmTc, seg);
+      if (!agreed(role_wait(&ctl->acc_empty[b], ((uint32_t)(nbuf == 2 ? seg >> 1 : seg) & 1u) ^ 1u, &limit, &ctl->abort_flag, p.status, kStatusMmaTimeout, kTagGemmTc, seg) && limit)) break;
       tc_fence_after_sync();
       const uint32_t acc = tmem_base + (uint32_t)(b * acc_cols);
       for (int i = 0; i < count; ++i) {
-        mbar_wait_or_report(&ctl->full[s], phase, &limit, 0, p.status, kStatusMmaTimeout, kTagGemmTc, seg);
+        role_wait(&ctl->full[s], phase, &limit, &ctl->abort_flag, p.status, kStatusMmaTimeout, kTagGemmTc, seg);
         tc_fence_after_sync();
         if (lead) {
           const uint64_t dw = w_desc + at, dx = x_desc + at;
@@ -209,7 +215,6 @@ gemm_sk_kernel(const __grid_constant__ CUtensorMap tmX, const GemmSkParams p) {
       if (lead) umma_commit(&ctl->acc_full[b]);
       left -= count;
     }
-    if (limit == 0) ctl->abort_flag = 1;
   } else {
     // ------------------------------------------------------------------ epilogue ----
     pdl_wait();
@@ -245,16 +250,10 @@ gemm_sk_kernel(const __grid_constant__ CUtensorMap tmX, const GemmSkParams p) {
       const int k1 = (int)(seg_end - (long long)t * KB);
       u = seg_end;
       const int b = seg % nbuf;
-      if (!mbar_wait(&ctl->acc_full[b], (uint32_t)(seg / nbuf) & 1u)) {
-        if (!*abort_flag) report_status(p.status, kStatusEpilogueTimeout, kTagGemmTc, t);
-        ctl->abort_flag = 1;
-      }
+      const bool have = role_wait(&ctl->acc_full[b], (uint32_t)(seg / nbuf) & 1u, &limit, &ctl->abort_flag, p.status, kStatusEpilogueTimeout, kTagGemmTc, t);
       // one decision for all four warps: the named barriers below need every epilogue thread or none
-      epi_bar_sync();
-      if (*abort_flag) {
-        dead = true;
-        break;
-      }
+      dead = epi_bar_any(!have || *abort_flag);
+      if (dead) break;
       tc_fence_after_sync();
       const uint32_t acc = lane_base + (uint32_t)(b * acc_cols);
       if (k0 != 0) {
@@ -384,6 +383,10 @@ gemm_sk_kernel(const __grid_constant__ CUtensorMap tmX, const GemmSkParams p) {
   }
   tc_fence_before_sync();
   __syncthreads();
+  if (*abort_flag) {                                       // a role gave up: what the others had started ends first
+    if (warp == 0) settle_copies(ctl->full, p.stages, ctl->issued);
+    if (warp == 1) settle_mmas(&ctl->settled);
+  }
   if (warp == 1) tmem_dealloc(tmem_base, (uint32_t)p.tmem_cols);
 }
 

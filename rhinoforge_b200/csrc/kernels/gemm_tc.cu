@@ -78,9 +78,9 @@ struct alignas(8) GemmSmemCtl {
   uint64_t ready[kMaxStages];  // W8A16: the converter warps have written the 16-bit weight tile
   uint64_t qfull[kMaxStages];  // W8A16: the int8 staging tile has landed
   uint64_t qempty[kMaxStages]; // W8A16: the converter warps have read the int8 staging tile
-  uint64_t accum;
+  uint64_t accum, settled;
   uint32_t tmem_base;
-  int32_t abort_flag;
+  int32_t abort_flag, issued;  // issued: k blocks that the producer has asked for (W8A16: or at least for their int8 tile)
 };
 // Scratch behind the control block, present only in launches with a folded RMSNorm (ss_in): rs[256] = reciprocal RMS of this tile's
 // token columns.
@@ -138,6 +138,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
       mbar_init(&ctl->qempty[s], (blockDim.x - 128) >> 5);
     }
     mbar_init(&ctl->accum, 1);
+    mbar_init(&ctl->settled, 1);
     ctl->abort_flag = 0;
     fence_barrier_init();
     tma_prefetch_desc(&tmA);
@@ -236,35 +237,31 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     }
     int s = 0;
     uint32_t phase = 0;                                    // of the release that a refill of stage s waits for
-    for (int i = pre; i < kb_count; ++i) {
+    int i = pre;
+    for (; i < kb_count; ++i) {
       if (W8) {
-        mbar_wait_or_report(&ctl->qempty[s], phase, &limit, 0, p.status, kStatusTmaTimeout, kTagW8A16, i);
-        if (lead) {
+        const bool free = role_wait(&ctl->qempty[s], phase, &limit, &ctl->abort_flag, p.status, kStatusTmaTimeout, kTagW8A16, i);
+        if (free && lead) {
           mbar_arrive_expect_tx(&ctl->qfull[s], txq);
           load_weights(i, s);
         }
+        if (!agreed(free)) break;
       }
-      mbar_wait_or_report(&ctl->empty[s], phase, &limit, 0, p.status, kStatusTmaTimeout, kTagGemmTc, i);
-      if (lead) {
+      const bool free = role_wait(&ctl->empty[s], phase, &limit, &ctl->abort_flag, p.status, kStatusTmaTimeout, kTagGemmTc, i);
+      if (free && lead) {
         mbar_arrive_expect_tx(&ctl->full[s], tx);
         if (!W8) load_weights(i, s);
         load_acts(i, s);
       }
+      if (!agreed(free)) break;
       if (++s == p.stages) { s = 0; phase ^= 1u; }
     }
-    if (lead && p.pf_chunks) {
+    if (lead) ctl->issued = W8 ? min(i + 1, kb_count) : i;
+    if (lead && p.pf_chunks && i == kb_count) {
       // this CTA's own weight loads are all in flight: spend the rest of its life keeping HBM busy for the next kernel
       const uint32_t ncta = gridDim.x * gridDim.y * gridDim.z;
       const uint32_t cta = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z);
       for (uint32_t c = cta; c < p.pf_chunks; c += ncta) bulk_prefetch_l2(p.pf_ptr + (size_t)c * kPrefetchChunk, kPrefetchChunk);
-    }
-    if (limit == 0) {
-      ctl->abort_flag = 1;
-      // Let every copy that was issued land before the CTA can exit.
-      for (int i = max(0, kb_count - p.stages); i < kb_count; ++i) {
-        mbar_wait(&ctl->full[i % p.stages], (uint32_t)(i / p.stages) & 1u, 20ull * 1000 * 1000);
-        if (W8) mbar_wait(&ctl->qfull[i % p.stages], (uint32_t)(i / p.stages) & 1u, 20ull * 1000 * 1000);
-      }
     }
   } else {
     pdl_wait();
@@ -274,15 +271,12 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     const int ct = tid - 128, cstep = (int)blockDim.x - 128;
     int s = -1;
     uint32_t ph = 0;
+    uint64_t limit = kLocalWaitNs;
     for (int i = 0; i < kb_count; ++i) {
       if (++s == p.stages) { s = 0; ph ^= 1u; }
       // the int8 tile has landed, and the MMAs that read this stage's 16-bit tile one ring turn ago are done
-      if (!mbar_wait(&ctl->qfull[s], ph) || !mbar_wait(&ctl->empty[s], ph ^ 1u)) {
-        report_status(p.status, kStatusMmaTimeout, kTagW8A16, i);
-        ctl->abort_flag = 1;
-        break;
-      }
-      if (*reinterpret_cast<volatile int32_t*>(&ctl->abort_flag)) break;
+      const bool landed = role_wait(&ctl->qfull[s], ph, &limit, &ctl->abort_flag, p.status, kStatusMmaTimeout, kTagW8A16, i);
+      if (!agreed(role_wait(&ctl->empty[s], ph ^ 1u, &limit, &ctl->abort_flag, p.status, kStatusMmaTimeout, kTagW8A16, i) && landed)) break;
       uint8_t* st = smem + (size_t)s * stage_bytes;
 #pragma unroll
       for (int wt = 0; wt < kWTiles; ++wt) {
@@ -367,8 +361,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     int s = 0;
     uint32_t ph = 0, at = 0;
     for (int i = 0; i < kb_count; ++i) {
-      mbar_wait_or_report(&ctl->full[s], ph, &limit, 0, p.status, kStatusMmaTimeout, kTagGemmTc, i);
-      if (W8) mbar_wait_or_report(&ctl->ready[s], ph, &limit, 0, p.status, kStatusMmaTimeout, kTagW8A16, 1000 + i);
+      role_wait(&ctl->full[s], ph, &limit, &ctl->abort_flag, p.status, kStatusMmaTimeout, kTagGemmTc, i);
+      if (W8) role_wait(&ctl->ready[s], ph, &limit, &ctl->abort_flag, p.status, kStatusMmaTimeout, kTagW8A16, 1000 + i);
       tc_fence_after_sync();
       if (lead) {
         const uint64_t da = a_desc + at, db = b_desc + at;
@@ -384,7 +378,6 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
       if (++s == p.stages) { s = 0; at = 0; ph ^= 1u; }
     }
     if (lead) umma_commit(&ctl->accum);
-    if (limit == 0) ctl->abort_flag = 1;
   }
   __syncwarp();
 
@@ -1150,6 +1143,13 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
   // ----------------------------------------------------------- teardown ----
   tc_fence_before_sync();
   __syncthreads();
+  if (*reinterpret_cast<volatile int32_t*>(&ctl->abort_flag)) {      // a role gave up: what the others had started ends first
+    if (warp == 0) {                               // (a block may have its int8 tile only: the other barrier then takes its time)
+      settle_copies(ctl->full, p.stages, ctl->issued);
+      if (W8) settle_copies(ctl->qfull, p.stages, ctl->issued);
+    }
+    if (warp == 1) settle_mmas(&ctl->settled);
+  }
   if (warp == 1) tmem_dealloc(tmem_base, (uint32_t)p.tmem_cols);
 }
 
