@@ -59,7 +59,7 @@ __device__ __forceinline__ void load8(const T* p, float (&f)[8]) {
     f[2 * i + 1] = t.y;
   }
 }
-// Eight 16-bit values as they are in memory, in one piece if the caller knows that they lie on a 16-byte boundary.
+// Eight 16-bit values as they are in memory, in one piece if the caller knows that they lie on a 16-byte boundary (a 4-byte one is enough otherwise).
 template <typename T>
 __device__ __forceinline__ uint4 load_raw8(const T* p, bool whole) {
   if (whole) return *reinterpret_cast<const uint4*>(p);

@@ -28,6 +28,12 @@ __device__ __forceinline__ float block_sum(float v, float* red) {
   return red[0];
 }
 
+// Eight values of a row off its 16-byte boundary, or of one that may be.
+template <typename T>
+__device__ __forceinline__ void load8_at(const T* p, int whole, float (&f)[8]) {
+  unpack8<T>(load_raw8(p, whole != 0), f);
+}
+
 // y = norm(x [+ residual]) ; if residual_out: residual_out = x + residual.
 // mode bit0: gemma style weight (1 + w), product rounded once
 // mod (optional, adaRMS): per-token [rows / rows_per_mod, 3H] = [scale | shift | gate];
@@ -37,7 +43,7 @@ __global__ void rmsnorm_kernel(const T* __restrict__ x, const T* __restrict__ re
                                const T* __restrict__ w, T* __restrict__ y,
                                T* __restrict__ residual_out, const T* __restrict__ mod,
                                int rows_per_mod, int H, int64_t ldx, int64_t ldy, float eps,
-                               int mode) {
+                               int mode, int whole) {
   pdl_prologue();
   extern __shared__ float srow[];  // H floats + 32
   float* red = srow + H;
@@ -47,10 +53,10 @@ __global__ void rmsnorm_kernel(const T* __restrict__ x, const T* __restrict__ re
   float ss = 0.f;
   for (int i = threadIdx.x * 8; i < H; i += blockDim.x * 8) {
     float f[8];
-    load8(xr + i, f);
+    load8_at(xr + i, whole, f);
     if (rr) {
       float r[8];
-      load8(rr + i, r);
+      load8_at(rr + i, whole, r);
 #pragma unroll
       for (int j = 0; j < 8; ++j) f[j] = Num<T>::to_f(Num<T>::from_f(f[j] + r[j]));
       if (residual_out) store8(residual_out + (size_t)row * ldx + i, f);
@@ -68,14 +74,14 @@ __global__ void rmsnorm_kernel(const T* __restrict__ x, const T* __restrict__ re
     float o[8];
     if (mrow) {
       float sc[8], sh[8];
-      load8(mrow + i, sc);
-      load8(mrow + H + i, sh);
+      load8_at(mrow + i, whole, sc);
+      load8_at(mrow + H + i, whole, sh);
 #pragma unroll
       for (int j = 0; j < 8; ++j) o[j] = srow[i + j] * rstd * (1.f + sc[j]) + sh[j];
     } else {
       float wf[8];
       if (w) {
-        load8(w + i, wf);
+        load8_at(w + i, whole, wf);
       } else {   // no weight: plain x * rstd in either form
 #pragma unroll
         for (int j = 0; j < 8; ++j) wf[j] = (mode & 1) ? 0.f : 1.f;
@@ -151,7 +157,7 @@ rmsnorm_row_kernel(const T* __restrict__ x, const T* __restrict__ residual, cons
 template <typename T>
 __global__ void layernorm_kernel(const T* __restrict__ x, const T* __restrict__ w,
                                  const T* __restrict__ b, T* __restrict__ y, int H, int64_t ldx,
-                                 int64_t ldy, float eps) {
+                                 int64_t ldy, float eps, int whole) {
   pdl_prologue();
   extern __shared__ float srow[];
   float* red = srow + H;
@@ -160,7 +166,7 @@ __global__ void layernorm_kernel(const T* __restrict__ x, const T* __restrict__ 
   float s = 0.f;
   for (int i = threadIdx.x * 8; i < H; i += blockDim.x * 8) {
     float f[8];
-    load8(xr + i, f);
+    load8_at(xr + i, whole, f);
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
       srow[i + j] = f[j];
@@ -177,8 +183,8 @@ __global__ void layernorm_kernel(const T* __restrict__ x, const T* __restrict__ 
   const float rstd = rsqrtf(var + eps);
   for (int i = threadIdx.x * 8; i < H; i += blockDim.x * 8) {
     float wf[8], bf[8], o[8];
-    load8(w + i, wf);
-    if (b) load8(b + i, bf);
+    load8_at(w + i, whole, wf);
+    if (b) load8_at(b + i, whole, bf);
 #pragma unroll
     for (int j = 0; j < 8; ++j) o[j] = (srow[i + j] - mean) * rstd * wf[j] + (b ? bf[j] : 0.f);
     store8(y + (size_t)row * ldy + i, o);
@@ -321,6 +327,8 @@ static bool rmsnorm_by_warp(int rows, int H, bool mod, bool residual) {
 // Rows of 16-byte pieces: every operand on its boundary (the kernels that go through shared memory take 4-byte ones)
 template <typename... P>
 static bool whole_pieces(P... p) { return (((reinterpret_cast<uintptr_t>(p) % 16) == 0) && ...); }
+template <typename... P>
+static bool whole_words(P... p) { return (((reinterpret_cast<uintptr_t>(p) % 4) == 0) && ...); }
 
 // Calls `run` with the piece count and the element type as types.
 template <typename Run>
@@ -385,6 +393,7 @@ extern "C" int rf_rmsnorm(const void* x, const void* residual, const void* w, vo
   RF_SKIP_IF_REPLAYING();
   RF_REQUIRE(rows >= 0 && H > 0 && H % 8 == 0, "rmsnorm H=%d must be a multiple of 8", H);
   RF_REQUIRE(ldx % 8 == 0 && ldy % 8 == 0, "rmsnorm pitches must be multiples of 8");
+  RF_REQUIRE(whole_words(x, residual, w, y, residual_out, mod), "rmsnorm operands must lie on even elements");
   if (rows == 0) return RF_OK;
   const int threads = H >= 2048 ? 256 : 128;
   const size_t smem = (size_t)(H + 32) * sizeof(float);
@@ -414,12 +423,12 @@ extern "C" int rf_rmsnorm(const void* x, const void* residual, const void* w, vo
   if (dtype == 0)
     RF_CUDA_CHECK(::rf::launch_k(rmsnorm_kernel<__half>, dim3(rows), dim3(threads), smem, s, 1, 
         (const __half*)x, (const __half*)residual, (const __half*)w, (__half*)y,
-        (__half*)residual_out, (const __half*)mod, rows_per_mod, H, ldx, ldy, eps, mode));
+        (__half*)residual_out, (const __half*)mod, rows_per_mod, H, ldx, ldy, eps, mode, (int)whole));
   else
     RF_CUDA_CHECK(::rf::launch_k(rmsnorm_kernel<__nv_bfloat16>, dim3(rows), dim3(threads), smem, s, 1, 
         (const __nv_bfloat16*)x, (const __nv_bfloat16*)residual, (const __nv_bfloat16*)w,
         (__nv_bfloat16*)y, (__nv_bfloat16*)residual_out, (const __nv_bfloat16*)mod, rows_per_mod,
-        H, ldx, ldy, eps, mode));
+        H, ldx, ldy, eps, mode, (int)whole));
   RF_CUDA_CHECK(cudaGetLastError());
   ::rf::count_launch();
   return RF_OK;
@@ -429,11 +438,14 @@ extern "C" int rf_layernorm(const void* x, const void* w, const void* b, void* y
                             int64_t ldx, int64_t ldy, float eps, int dtype, rf_stream_t stream) {
   RF_SKIP_IF_REPLAYING();
   RF_REQUIRE(rows >= 0 && H > 0 && H % 8 == 0, "layernorm H=%d must be a multiple of 8", H);
+  RF_REQUIRE(ldx % 2 == 0 && ldy % 2 == 0, "layernorm pitches must be even (%lld, %lld)", (long long)ldx, (long long)ldy);
+  RF_REQUIRE(whole_words(x, w, b, y), "layernorm operands must lie on even elements");
   if (rows == 0) return RF_OK;
   const int threads = H >= 2048 ? 256 : 128;
   const size_t smem = (size_t)(H + 32) * sizeof(float);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (whole_pieces(x, w, b, y) && layernorm_by_warp(rows, H)) {
+  const bool whole = whole_pieces(x, w, b, y) && ldx % 8 == 0 && ldy % 8 == 0;       // every row on its boundary, not the first alone
+  if (whole && layernorm_by_warp(rows, H)) {
     auto run = [&](auto kNC, auto zero) -> cudaError_t {
       using T = decltype(zero);
       return ::rf::launch_k(layernorm_warp_kernel<T, decltype(kNC)::value>, dim3(ceil_div(rows, 4)), dim3(128), 0, s, 1, (const T*)x, (const T*)w, (const T*)b,
@@ -446,11 +458,11 @@ extern "C" int rf_layernorm(const void* x, const void* w, const void* b, void* y
   if (dtype == 0)
     RF_CUDA_CHECK(::rf::launch_k(layernorm_kernel<__half>, dim3(rows), dim3(threads), smem, s, 1, (const __half*)x, (const __half*)w,
                                                         (const __half*)b, (__half*)y, H, ldx, ldy,
-                                                        eps));
+                                                        eps, (int)whole));
   else
     RF_CUDA_CHECK(::rf::launch_k(layernorm_kernel<__nv_bfloat16>, dim3(rows), dim3(threads), smem, s, 1, 
         (const __nv_bfloat16*)x, (const __nv_bfloat16*)w, (const __nv_bfloat16*)b,
-        (__nv_bfloat16*)y, H, ldx, ldy, eps));
+        (__nv_bfloat16*)y, H, ldx, ldy, eps, (int)whole));
   RF_CUDA_CHECK(cudaGetLastError());
   ::rf::count_launch();
   return RF_OK;

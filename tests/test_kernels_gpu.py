@@ -1415,6 +1415,26 @@ def test_attn_decode_split_plans(dt, n, kv, Hq, Hkv, hd, status):
 
 
 @pytest.mark.parametrize("dt", DT)
+@pytest.mark.parametrize("H", [64, 1152, 2048])
+@pytest.mark.parametrize("pad,off", [(2, 0), (4, 0), (6, 0), (8, 2), (8, 0)])
+def test_layernorm_of_rows_off_their_boundary(dt, H, pad, off):
+    """Even pitches that are no multiple of eight values, and rows that begin off a 16-byte boundary, below and above the number of rows from which
+    a warp takes each (it reads 16 bytes at a time); odd pitches and offsets are refused."""
+    from rhinoforge_b200.ops import kernels as K_
+    w, b = (1 + 0.1 * torch.randn(H, device="cuda")).to(dt), torch.randn(H, device="cuda").to(dt)
+    for rows in (5, 2000):
+        x = torch.randn(rows, H + pad, device="cuda").to(dt)[:, off:off + H]
+        out = torch.full((rows, H + pad), 7.0, device="cuda").to(dt)
+        _close(K_.layernorm(x, w, b, 1e-6, out=out[:, off:off + H]), torch.nn.functional.layer_norm(x.float(), (H,), w.float(), b.float(), 1e-6), dt, scale=2.0)
+        assert bool((out[:, off + H:] == 7.0).all()) and bool((out[:, :off] == 7.0).all())
+    odd = torch.zeros(4, H + 1, device="cuda", dtype=dt)[:, :H]
+    with pytest.raises(Exception, match="even"):
+        K_.layernorm(odd, w, b, 1e-6)
+    with pytest.raises(Exception, match="even"):
+        K_.layernorm(torch.zeros(4, H + 8, device="cuda", dtype=dt)[:, 1:1 + H], w, b, 1e-6)
+
+
+@pytest.mark.parametrize("dt", DT)
 @pytest.mark.parametrize("H", [8, 248, 256, 1000, 4096, 8192, 8200])
 def test_rmsnorm_rows_of_any_width(dt, H):
     """A row of at most 8192 values in the registers of its block, and the first width beyond: whole and ragged warps, every form, in place."""
