@@ -388,6 +388,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   if (warp == 1) pair_tmem_dealloc(tmem_base, 512u);
 }
 
+int ps_forced_band();                                            // gemm_ps.cu
+
 template <typename T, bool DUAL, bool EXTRA>
 static int launch_pair(const RfGemm* g, int bn, cudaStream_t stream) {
   auto kfn = gemm_pair_kernel<T, DUAL, EXTRA>;
@@ -421,6 +423,7 @@ static int launch_pair(const RfGemm* g, int bn, cudaStream_t stream) {
   }
   // a band of activation rows of about 16 MB: it and a weight matrix of a few tens of MB stay in L2 together
   p.band = (int)std::max<int64_t>(1, std::min<int64_t>(p.tiles_m, (16ll << 20) / std::max<int64_t>(1, (int64_t)2 * kPrBM * g->K * 2)));
+  if (ps_forced_band() > 0) p.band = std::min(p.tiles_m, ps_forced_band());
   const int stage_bytes = kPrPiece + w_rows * kPrBK * 2;
   const int other = (int)sizeof(GemmPairCtl) + 1024 /*alignment slack*/ + kPrEpiWarps * 2 * kPrChunk;
   p.stages = std::min(kPrMaxStages, (227 * 1024 - other) / stage_bytes);
@@ -463,8 +466,12 @@ static PairShape pair_shape(const RfGemm* g) {
   return best;
 }
 
-// Estimated time in ns where the kernel takes this GEMM, 0 where it cannot.
-long gemm_pair_ns(const RfGemm* g) { return pair_can(g) ? pair_shape(g).ns : 0; }
+bool gemm_pairs_on();                                            // gemm_ps.cu
+
+// Estimated time in ns where the kernel takes this GEMM, 0 where it cannot or may not.
+long gemm_pair_ns(const RfGemm* g) { return gemm_pairs_on() && pair_can(g) ? pair_shape(g).ns : 0; }
+// Columns of a tile (of a GLU pair: of its result)
+int gemm_pair_cols(const RfGemm* g) { return pair_shape(g).bn; }
 
 int launch_gemm_pair(const RfGemm* g, cudaStream_t stream) {
   const int bn = pair_shape(g).bn;

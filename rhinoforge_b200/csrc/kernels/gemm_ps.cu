@@ -16,7 +16,7 @@
 // share one weight panel and the activation matrix stays in L2.
 // Scope: tokens on the MMA M axis, tile-major 16-bit weights, no split-K, no fused all-reduce (those shapes
 // stay with gemm_tc.cu).  Results and residuals that bulk copies can move go to the form with two CTAs to a tile
-// (gemm_pair.cu, see launch_gemm_ps): this one has the others and the grouped form.
+// (gemm_pair.cu, see gemm_ps_form): this one has the others and the grouped form.
 //
 // Grouped form (mixture of experts, rf_moe_grouped_gemm): the rows are (token, pick) pairs sorted by expert and
 // the tile list comes from device memory - one entry {expert, first row, end row} per 128-row block of one
@@ -462,6 +462,11 @@ gemm_ps_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
   if (warp == 1) tmem_dealloc(tmem_base, 512u);
 }
 
+int ps_forced_band() {
+  static const int band = [] { const char* e = getenv("RF_GEMM_PS_BAND"); return e ? atoi(e) : 0; }();
+  return band;
+}
+
 template <typename T, bool DUAL, int MT, bool EXTRA>
 static int launch_ps(const RfGemm* g, int bn, cudaStream_t stream) {
   auto kfn = gemm_ps_kernel<T, DUAL, MT, EXTRA>;
@@ -493,8 +498,7 @@ static int launch_ps(const RfGemm* g, int bn, cudaStream_t stream) {
     // a band of activation rows of about 16 MB: it and a weight matrix of a few tens of MB stay in L2 together
     const int64_t row_tile_bytes = (int64_t)kPsBM * MT * g->K * 2;
     p.band = (int)std::max<int64_t>(1, std::min<int64_t>(p.tiles_m, (16ll << 20) / std::max<int64_t>(1, row_tile_bytes)));
-    static const int band_env = [] { const char* e = getenv("RF_GEMM_PS_BAND"); return e ? atoi(e) : 0; }();
-    if (band_env > 0) p.band = std::min(p.tiles_m, band_env);
+    if (ps_forced_band() > 0) p.band = std::min(p.tiles_m, ps_forced_band());
     static const int pf_kb = [] { const char* e = getenv("RF_GEMM_L2_PREFETCH_KB"); return e ? atoi(e) : 0; }();
     p.pf_blocks = std::min(16, pf_kb * 1024 / stage_bytes);
   }
@@ -517,10 +521,13 @@ struct PsShape { int bn, rows; long ns; };
 // the busiest SM has tiles.  Tiles that take all of tensor memory (512 columns) also wait for their epilogue, about 3.5 us, each;
 // the others only for the last one.  fp16, us, 128-row / 256-row tiles 128 wide (model in brackets): 3072 x 1152 x 4304 60.4 / 39.9
 // (65 / 44), 768 x 4304 x 1152 19.7 / 15.0 (21 / 15); 3072 x 6144 x 1152 with 256 x 256 tiles 37.3 (39).
+static int ps_forced_rows() {
+  static const int rows = [] { const char* e = getenv("RF_GEMM_PS_ROWS"); return e ? atoi(e) : 0; }();
+  return rows;
+}
 static PsShape ps_shape(const RfGemm* g) {
   const bool dual = g->dual_offset > 0;
-  const int k_blocks = ceil_div(g->K, kPsBK), sms = sm_count();
-  static const int forced = [] { const char* e = getenv("RF_GEMM_PS_ROWS"); return e ? atoi(e) : 0; }();
+  const int k_blocks = ceil_div(g->K, kPsBK), sms = sm_count(), forced = ps_forced_rows();
   PsShape best = {0, 0, 0};
   for (int mt = 2; mt >= 1; --mt) {
     if ((forced == 128 || forced == 256) && forced != mt * kPsBM) continue;
@@ -548,21 +555,37 @@ static PsShape ps_shape(const RfGemm* g) {
 long gemm_pair_ns(const RfGemm* g);                              // gemm_pair.cu: the form with two CTAs to a tile
 int launch_gemm_pair(const RfGemm* g, cudaStream_t stream);
 
-// True when a persistent kernel takes this GEMM (called by rf_gemm after its argument checks): it is estimated to be no slower than
+// Whether the form with two CTAs to a tile may be chosen: not where the environment turns the persistent kernels off or sets the rows of a tile.
+bool gemm_pairs_on() {
+  static const bool on = [] { const char* e = getenv("RF_GEMM_PERSISTENT"); return !(e && e[0] == '0'); }();
+  return on && ps_forced_rows() != 128 && ps_forced_rows() != 256;
+}
+
+// Which persistent kernel takes this GEMM (called by rf_gemm after its argument checks, with the tile kernel's plan): 0 neither, 1 the one with a
+// CTA to a tile, 2 CTA pairs, wherever their bulk copies can write the result and read the residual (fp16, us, one CTA / two to a tile:
+// 3072 x 4304 x 1152 32.3 / 25, 4770 x 2048 x 2048 50.8 / 33.2, 825 x 2048 x 8192 50.8 / 28.6, 4770 x 16384 x 2048 SwiGLU 626 / 416).
+// Weights on the rows (at most 256 tokens): 129 to 256 tokens of short K, where one row tile of the CTA pairs does without the tile kernel's reduction over
+// splits.  fp16, us, tile / pairs: 200 x 2048 x 2048 13.7 / 9.3, 200 x 8192 x 2048 GLU 34.3 / 21.8; 200 x 4096 x 4096 18.3 / 20.8, 200 x 1152 x 4304
+// 16.2 / 16.6, 200 x 2048 x 8192 21.3 / 28.1.
+// Tokens on the rows: where it is estimated to be no slower than
 // the one-tile kernel with `splits` K splits, whose CTAs pay the same per k block (two of them share an SM's operand stream), about
 // 4.5 us around it and 6.5 us more for the reduction of a split (fp16, us, persistent / split kernel: 825 x 2560 x 2048 20 / 26,
 // 825 x 2048 x 2048 20 / 30; 768 x 1152 x 4304 34 / 23, 825 x 2048 x 16384 119 / 96).
-bool gemm_ps_eligible(const RfGemm* g, bool swap, int splits, int bn, int tiles) {
+int gemm_ps_form(const RfGemm* g, bool swap, int splits, int bn, int tiles) {
   static const bool enabled = [] { const char* e = getenv("RF_GEMM_PERSISTENT"); return !(e && e[0] == '0'); }();
-  if (!enabled || swap || g->ar_world > 1 || !g->w_packed || g->w_int8) return false;
-  // up to 255 columns that the tile kernel can split along K: no faster on pairs, few of which have a tile (4770 x 128 x 2048 17 / 18 us)
-  const long pair_ns = splits > 1 && g->N < 256 ? 0 : gemm_pair_ns(g);
+  if (!enabled || g->ar_world > 1 || !g->w_packed || g->w_int8 || g->force_splits || g->force_bn) return 0;
+  const long pairs_ns = gemm_pair_ns(g);
+  if (swap) return g->M > 128 && g->M <= 256 && g->K <= 2048 && g->force_swap < 0 && pairs_ns ? 2 : 0;
+  // Up to 255 columns that the tile kernel can split along K are left to it by the other form's estimate: few pairs have a tile.  That rests on
+  // one size, 4770 x 128 x 2048, tile / pairs 17 / 18 us, and on results staying what they were for routers of few experts.
+  const long pair_ns = splits > 1 && g->N < 256 ? 0 : pairs_ns;
   const PsShape s = ps_shape(g);
-  if (s.bn == 0) return false;
+  if (s.bn == 0) return 0;
   const long sms = sm_count(), ctas = (long)tiles * splits, kb = ceil_div(ceil_div(g->K, kPsBK), splits);
   const long kb_ns = (g->dual_offset > 0 || bn > 128) ? 595 : 450;
   const long load = splits == 1 ? (ctas + sms - 1) / sms * 100 : std::max(100l, ctas * 100 / sms);    // busiest SM's CTAs, per cent
-  return (pair_ns ? std::min(pair_ns, s.ns) : s.ns) <= 4500 + (splits > 1 ? 6500 : 0) + kb * kb_ns * load / 100;
+  if ((pair_ns ? std::min(pair_ns, s.ns) : s.ns) > 4500 + (splits > 1 ? 6500 : 0) + kb * kb_ns * load / 100) return 0;
+  return pairs_ns ? 2 : 1;
 }
 
 template <typename T, bool EXTRA>
@@ -571,10 +594,9 @@ static int launch_ps_t(const RfGemm* g, bool dual, int bn, int rows, cudaStream_
   return dual ? launch_ps<T, true, 1, EXTRA>(g, bn, stream) : launch_ps<T, false, 1, EXTRA>(g, bn, stream);
 }
 
-// CTA pairs wherever their bulk copies can write the result and read the residual (fp16, us, one CTA / two to a tile: 3072 x 4304 x 1152 32.3 / 25,
-// 4770 x 2048 x 2048 50.8 / 33.2, 825 x 2048 x 8192 50.8 / 28.6, 4770 x 16384 x 2048 SwiGLU 626 / 416); other row pitches stay with one.
-int launch_gemm_ps(const RfGemm* g, cudaStream_t stream) {
-  if (gemm_pair_ns(g)) return launch_gemm_pair(g, stream);
+// `form`: what gemm_ps_form said.
+int launch_gemm_ps(const RfGemm* g, int form, cudaStream_t stream) {
+  if (form == 2) return launch_gemm_pair(g, stream);
   const bool dual = g->dual_offset > 0;
   const PsShape s = ps_shape(g);
   const bool extra = g->bias || g->scale || g->row_scale || g->residual;

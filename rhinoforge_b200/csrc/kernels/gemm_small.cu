@@ -328,8 +328,7 @@ bool gemm_small_eligible(const RfGemm* g) {
   if (dual && !g->w_packed && g->dual_offset % 8) return false;
   // up to 64 rows the two kernels are close once K is long (41 x 1536 x 6144: 12.0 us on the streaming kernel, 11.6 us
   // here; 50 x 1024 x 2048: 8.5 against 5.7; inside the Pi0.5 denoise loop, K = 2048 / 4096 at 50 rows: 24.8 ms per chunk with
-  // this bound at 2048, 23.9 ms at 8192); above 64 rows this kernel wins everywhere that was measured
-  // (128 x 1536 x 384: 5.6 us against 19.6 us)
+  // this bound at 2048, 23.9 ms at 8192); above 64 rows gemm_small_takes draws the line
   static const int max_k64 = [] { const char* e = getenv("RF_GEMM_SMALL_MAX_K"); return e ? atoi(e) : 8192; }();
   if (g->M <= 64 && g->K > max_k64) return false;
   // up to 32 rows the streaming kernel runs 32-column tiles; it won on all but the smallest weights before the split-K

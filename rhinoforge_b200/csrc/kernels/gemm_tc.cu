@@ -1475,14 +1475,15 @@ bool gemm_rows_takes(const RfGemm* g);                             // gemm_rows.
 int launch_gemm_rows(const RfGemm* g, cudaStream_t stream);
 void gemm_sk_scratch(const RfGemm* g, uint64_t* ws_bytes, int32_t* flags);
 int launch_gemm_sk(const RfGemm* g, cudaStream_t stream);
-bool gemm_ps_eligible(const RfGemm* g, bool swap, int splits, int bn, int tiles);   // gemm_ps.cu: persistent kernel for large M
-long gemm_pair_ns(const RfGemm* g);                                // gemm_pair.cu: its form with two CTAs to a tile
-int launch_gemm_ps(const RfGemm* g, cudaStream_t stream);
+int gemm_ps_form(const RfGemm* g, bool swap, int splits, int bn, int tiles);        // gemm_ps.cu: persistent kernels for large M
+int gemm_pair_cols(const RfGemm* g);                               // gemm_pair.cu: the form with two CTAs to a tile
+int launch_gemm_ps(const RfGemm* g, int form, cudaStream_t stream);
 int widen_packed(const void* src, void* dst, int64_t blocks, int dtype, cudaStream_t stream);   // gemm_ps.cu
 }
 
-// Which kernel a checked GEMM runs on (RF_GEMM_*), and where that is one of the tcgen05 tile kernels its plan.
-static int route_gemm(const RfGemm* g, int* kernel, GemmPlan* pl) {
+// Which kernel a checked GEMM runs on (RF_GEMM_*), and where that is one of the tcgen05 tile kernels its plan and the persistent kernel's form.
+static int route_gemm(const RfGemm* g, int* kernel, GemmPlan* pl, int* form) {
+  *form = 0;
   const bool w8 = g->w_int8 != 0;
   if (g->mul) RF_REQUIRE(!w8 && g->mul_row && rf::gemm_small_eligible(g), "GEMM %dx%dx%d has no gate-by-token epilogue (see rf_gemm_takes_mul)", g->M, g->N, g->K);
   const bool rows = rf::gemm_rows_takes(g);
@@ -1498,28 +1499,22 @@ static int route_gemm(const RfGemm* g, int* kernel, GemmPlan* pl) {
   if (rows) { *kernel = RF_GEMM_ROWS; return RF_OK; }
   const int rc = plan_gemm(g, pl);
   if (rc) return rc;
-  // 129 to 256 rows of short K: one row tile of the CTA pairs does without the tile kernel's reduction over splits.  fp16, us, tile / pairs: 200 x 2048 x 2048
-  // 13.7 / 9.3, 200 x 8192 x 2048 GLU 34.3 / 21.8; 200 x 4096 x 4096 18.3 / 20.8, 200 x 1152 x 4304 16.2 / 16.6, 200 x 2048 x 8192 21.3 / 28.1.
-  if (!w8 && g->M > 128 && g->M <= 256 && g->K <= 2048 && pl->swap && g->force_swap < 0 && g->force_splits == 0 && g->force_bn == 0 && rf::gemm_pair_ns(g)) {
-    *kernel = RF_GEMM_PERSISTENT;
-    return RF_OK;
-  }
-  *kernel = !w8 && g->force_splits == 0 && g->force_bn == 0 && rf::gemm_ps_eligible(g, pl->swap != 0, pl->splits, pl->bn, pl->grid_x * pl->grid_y)
-                ? RF_GEMM_PERSISTENT : RF_GEMM_TILE;
+  *form = rf::gemm_ps_form(g, pl->swap != 0, pl->splits, pl->bn, pl->grid_x * pl->grid_y);
+  *kernel = *form ? RF_GEMM_PERSISTENT : RF_GEMM_TILE;
   return RF_OK;
 }
 
 static int run_gemm(const RfGemm* g, cudaStream_t stream, bool w8) {
   int rc = check_gemm(g);
   if (rc) return rc;
-  int kernel;
+  int kernel, form;
   GemmPlan pl;
-  rc = route_gemm(g, &kernel, &pl);
+  rc = route_gemm(g, &kernel, &pl, &form);
   if (rc) return rc;
   if (kernel == RF_GEMM_SMALL) return rf::gemm_small_run(g, stream);
   if (kernel == RF_GEMM_STREAM_K) return rf::launch_gemm_sk(g, stream);
   if (kernel == RF_GEMM_ROWS) return rf::launch_gemm_rows(g, stream);
-  if (kernel == RF_GEMM_PERSISTENT) return rf::launch_gemm_ps(g, stream);
+  if (kernel == RF_GEMM_PERSISTENT) return rf::launch_gemm_ps(g, form, stream);
   if (w8 && g->w_bits != 4 && !pl.swap && g->M > 256 && g->w_packed && g->w_scratch && g->force_splits == 0 && g->force_bn == 0) {
     // Large token counts are compute-bound: widen the int8 weight image once into the caller's scratch (a pass
     // over the weights costs a few per cent of the GEMM) and run the 16-bit kernels, whose main loop has no
@@ -1562,10 +1557,19 @@ extern "C" int rf_gemm_takes_norm(const RfGemm* g) { return g && check_gemm(g) =
 extern "C" int rf_gemm_kernel(const RfGemm* g) {
   int rc = check_gemm(g);
   if (rc) return rc;
-  int kernel;
+  int kernel, form;
   GemmPlan pl;
-  rc = route_gemm(g, &kernel, &pl);
+  rc = route_gemm(g, &kernel, &pl, &form);
   return rc ? rc : kernel;
+}
+
+extern "C" int rf_gemm_pair_cols(const RfGemm* g) {
+  int rc = check_gemm(g);
+  if (rc) return rc;
+  int kernel, form;
+  GemmPlan pl;
+  rc = route_gemm(g, &kernel, &pl, &form);
+  return rc ? rc : form == 2 ? rf::gemm_pair_cols(g) : 0;
 }
 
 extern "C" int rf_gemm_plan_info(const RfGemm* g, int32_t* out) {
@@ -1577,7 +1581,7 @@ extern "C" int rf_gemm_plan_info(const RfGemm* g, int32_t* out) {
   if (rc) return rc;
   out[0] = pl.swap; out[1] = pl.bn; out[2] = pl.splits; out[3] = pl.stages; out[4] = pl.grid_x; out[5] = pl.grid_y;
   out[6] = (int32_t)pl.smem_bytes; out[7] = pl.k_blocks;
-  out[8] = (!g->w_int8 && g->force_splits == 0 && g->force_bn == 0 && rf::gemm_ps_eligible(g, pl.swap != 0, pl.splits, pl.bn, pl.grid_x * pl.grid_y)) ? 1 : 0;
+  out[8] = rf::gemm_ps_form(g, pl.swap != 0, pl.splits, pl.bn, pl.grid_x * pl.grid_y) ? 1 : 0;
   if (!g->w_int8 && rf::gemm_sk_eligible(g, nullptr)) out[8] = 2;   // persistent stream-K kernel
   out[9] = (g->ar_world > 1 && !pl.swap && g->M > 256) ? 1 : 0;
   return RF_OK;

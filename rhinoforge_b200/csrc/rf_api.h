@@ -118,6 +118,8 @@ int rf_gemm_takes_norm(const RfGemm* g);  // host-only: can this GEMM take the s
 // RF_GEMM_PERSISTENT is either form, one CTA to a tile or two.)
 enum { RF_GEMM_TILE = 0, RF_GEMM_PERSISTENT = 1, RF_GEMM_STREAM_K = 2, RF_GEMM_ROWS = 3, RF_GEMM_SMALL = 4 };
 int rf_gemm_kernel(const RfGemm* g);
+// Columns of a tile (of a GLU pair: of its result) where that is the persistent kernel with two CTAs to a tile, 0 anywhere else.  Host-only.
+int rf_gemm_pair_cols(const RfGemm* g);
 // Launch plan of a shape on the tcgen05 tile kernels without launching (rf_gemm_kernel says whether one of them takes it): out[10] = {swap, bn, splits, stages, grid_x, grid_y, smem bytes, k_blocks,
 // persistent kernel, two-shot all-reduce}.  Host-only.
 int rf_gemm_plan_info(const RfGemm* g, int32_t* out);

@@ -58,7 +58,8 @@ def gemm_plan(M: int, N_out: int, K: int, *, dtype: torch.dtype = torch.float16,
               int8: bool = False, force_splits: int = 0) -> Optional[dict]:
     """The launch plan the library would pick for ``[M, K] x [N_out, K]^T`` - swap-AB, tile width, K splits, ring stages,
     grid, shared memory, persistent / two-shot form - and ``kernel``, the family that runs (of :data:`GEMM_KERNELS`; the other entries are the
-    plan of the tcgen05 tile kernels, which only ``tile`` and ``persistent`` launch).  A host-side query (no device, no launch); ``None`` when the native
+    plan of the tcgen05 tile kernels, which only ``tile`` and ``persistent`` launch), and ``pair_cols``, the columns of a tile where that is the
+    persistent kernel with two CTAs to a tile (else 0).  A host-side query (no device, no launch); ``None`` when the native
     library is not built."""
     if not N.available():
         return None
@@ -74,7 +75,8 @@ def gemm_plan(M: int, N_out: int, K: int, *, dtype: torch.dtype = torch.float16,
     out = (C.c_int32 * len(GEMM_PLAN_KEYS))()
     if N.lib().rf_gemm_plan_info(C.byref(g), out) != 0:
         return None
-    return dict(zip(GEMM_PLAN_KEYS, (int(v) for v in out)), kernel=GEMM_KERNELS[N.lib().rf_gemm_kernel(C.byref(g))])
+    return dict(zip(GEMM_PLAN_KEYS, (int(v) for v in out)), kernel=GEMM_KERNELS[N.lib().rf_gemm_kernel(C.byref(g))],
+                pair_cols=N.lib().rf_gemm_pair_cols(C.byref(g)))
 
 
 def gemm(x: torch.Tensor, w: torch.Tensor, *, out: Optional[torch.Tensor] = None,
