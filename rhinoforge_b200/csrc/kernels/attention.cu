@@ -994,10 +994,14 @@ extern "C" int rf_attn_decode(const RfAttn* a, rf_stream_t stream) {
   RF_ATTN_DISPATCH(launch_decode)
 }
 
+namespace rf {
+bool rope_vec_on();      // rope_kv.cu
+}
+
 // Whether rf_attn_decode_insert takes the pair: one row per sequence that sees its whole cache, heads and operands that the 16-byte form of
 // rf_qk_norm_rope_kv takes with one position axis, at most 16 query heads to a K/V head, and nothing that wants the rotated rows themselves.
 extern "C" int rf_attn_decode_inserts(const RfAttn* a, const RfRopeKv* r) {
-  if (!a || !r || !a->k_pool || a->num_seqs <= 0 || a->rows_per_seq > 1 || a->pos || a->slot || a->window > 0 || a->chunk > 0 || a->keep_first > 0) return 0;
+  if (!rf::rope_vec_on() || !a || !r || !a->k_pool || a->num_seqs <= 0 || a->rows_per_seq > 1 || a->pos || a->slot || a->window > 0 || a->chunk > 0 || a->keep_first > 0) return 0;
   if ((a->hd != 64 && a->hd != 128 && a->hd != 256) || a->Hkv <= 0 || a->Hq % a->Hkv || a->Hq / a->Hkv > 16) return 0;
   if (r->qkv != a->q || r->ld != a->ldq || r->tokens != a->num_seqs || r->Hq != a->Hq || r->Hkv != a->Hkv || r->hd != a->hd || r->dtype != a->dtype) return 0;
   if (r->k_pool != a->k_pool || r->v_pool != a->v_pool || r->page_table != a->page_table || r->pt_stride != a->pt_stride) return 0;

@@ -251,6 +251,14 @@ __global__ void __launch_bounds__(256) qk_norm_rope_kv_vec_kernel(const RfRopeKv
 
 using namespace rf;
 
+namespace rf {
+// RF_ROPE_VEC=0: heads are normalised, rotated and inserted by the scalar kernel everywhere.
+bool rope_vec_on() {
+  static const bool on = [] { const char* e = getenv("RF_ROPE_VEC"); return !(e && e[0] == '0'); }();
+  return on;
+}
+}
+
 extern "C" int rf_qk_norm_rope_kv(const RfRopeKv* a, rf_stream_t stream) {
   RF_SKIP_IF_REPLAYING();
   RF_REQUIRE(a && a->qkv, "rope_kv: null arguments");
@@ -269,8 +277,8 @@ extern "C" int rf_qk_norm_rope_kv(const RfRopeKv* a, rf_stream_t stream) {
   }
   const size_t smem = (size_t)warps * a->hd * sizeof(float);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  // the common geometries take the 16-byte kernel (RF_ROPE_VEC=0: never)
-  static const bool vec_on = [] { const char* e = getenv("RF_ROPE_VEC"); return !(e && e[0] == '0'); }();
+  // the common geometries take the 16-byte kernel
+  const bool vec_on = rf::rope_vec_on();
   const bool aligned = a->ld % 8 == 0 && (reinterpret_cast<uintptr_t>(a->qkv) & 15) == 0 &&
                        (!a->q_out || (a->ldq % 8 == 0 && (reinterpret_cast<uintptr_t>(a->q_out) & 15) == 0)) &&
                        (!a->k_pool || ((reinterpret_cast<uintptr_t>(a->k_pool) | reinterpret_cast<uintptr_t>(a->v_pool)) & 15) == 0) &&
