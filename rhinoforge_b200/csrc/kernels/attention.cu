@@ -163,10 +163,11 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
   // by row: the row's own position bounds its keys and its sequence's slot owns the pages
   const int owner = p.pos && p.seq_of_row ? p.seq_of_row[seq] : seq;
   const int pt_row = p.slot ? p.slot[owner] : owner;
-  // the first stage's page numbers are asked for beside the length, not behind it, where pages are read in order
+  // the first stage's page numbers are asked for beside the length, not behind it, where pages are read in order (a row that sees nothing need
+  // have no pages: its table row may be negative)
   int early_page = -1;
   const int kvlen = p.pos ? p.pos[seq] + 1 : p.kv_len[seq];
-  if (warp == 4 && lane < 4 && p.paged && p.window <= 0 && p.chunk <= 0 && split * p.pages_per_split + lane < p.pt_stride)
+  if (warp == 4 && lane < 4 && pt_row >= 0 && p.paged && p.window <= 0 && p.chunk <= 0 && split * p.pages_per_split + lane < p.pt_stride)
     early_page = p.page_table[(size_t)pt_row * p.pt_stride + split * p.pages_per_split + lane];
   int kvlo = p.chunk > 0 && kvlen > 0 ? (kvlen - 1) / p.chunk * p.chunk : 0;
   if (p.window > 0) kvlo = max(kvlo, kvlen - p.window);

@@ -1162,6 +1162,26 @@ def test_attn_decode_inserts(dt, hd, Hq, Hkv, rot, lens, mode, status):
 
 
 @pytest.mark.parametrize("dt", DT)
+@pytest.mark.parametrize("hd", [64, 128, 256])
+@pytest.mark.parametrize("longest", [40, 1500])
+def test_attn_decode_of_a_row_without_pages(dt, hd, longest, status):
+    """Rows that see nothing (position -1, no table row: -1) beside rows that do: zeros for them, the others as without them, one and several splits."""
+    from rhinoforge_b200.ops import kernels as K_
+    Hq, Hkv, maxp = 8, 2, (longest + 15) // 16
+    g = torch.Generator(device="cuda").manual_seed(hd)
+    q = torch.randn(4, Hq * hd, device="cuda", generator=g).to(dt)
+    kp, vp = torch.randn(2, 2 * maxp, Hkv, 16, hd, device="cuda", generator=g).to(dt)
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")
+    pt = torch.randperm(2 * maxp, device="cuda", generator=g).to(torch.int32).view(2, maxp)
+    pos, slot = [longest - 1, -1, 6, -1], [1, -1, 0, -1]
+    run = lambda rows: K_.attention_rows(q[rows].contiguous(), K_.rows(i32([pos[r] for r in rows]), slot=i32([slot[r] for r in rows]), page_table=pt), kp, vp, Hq=Hq,
+                                         Hkv=Hkv, hd=hd, scale=hd ** -0.5, max_kv=longest)
+    got, want = run([0, 1, 2, 3]), run([0, 2])
+    torch.testing.assert_close(got[[0, 2]].float(), want.float(), rtol=0, atol=2e-3 if dt == torch.float16 else 1.6e-2)     # other splits: one rounding of values below 1
+    assert not got[[1, 3]].any()
+
+
+@pytest.mark.parametrize("dt", DT)
 @pytest.mark.parametrize("hd,Hq,Hkv", [(64, 8, 2), (128, 16, 8), (256, 8, 1)])
 @pytest.mark.parametrize("lens", [[33, 16, 7], [1500, 700, 15]])
 def test_attn_decode_inserts_nothing_into_a_page_of_nobody(dt, hd, Hq, Hkv, lens, status):
