@@ -841,15 +841,16 @@ static DecodeSplitPlan plan_decode_split(int num_seqs, int rows_per_seq, int Hq,
   return pl;
 }
 
-// Clusters of `size` CTAs of the kernel that the current device holds at once (asked once per kernel, device and size)
+// Clusters of `size` CTAs of the kernel that the current device holds at once (asked once per kernel, device, size and group: the inserting form's
+// shared memory grows with the query heads of a group, up to 16)
 template <typename T, int HD, bool INSERT>
-static long clusters_resident(int size, size_t smem) {
-  static std::atomic<int> known[64][9];
+static long clusters_resident(int size, int group, size_t smem) {
+  static std::atomic<int> known[64][9][17];
   auto kfn = attn_decode_kernel<T, HD, INSERT>;
   const int dev = device_ordinal();
   const bool track = dev >= 0 && dev < 64;
   if (track) {
-    const int n = known[dev][size].load(std::memory_order_relaxed);
+    const int n = known[dev][size][group].load(std::memory_order_relaxed);
     if (n > 0) return n - 1;
   }
   cudaLaunchConfig_t cfg = {};
@@ -863,7 +864,7 @@ static long clusters_resident(int size, size_t smem) {
     (void)cudaGetLastError();
     n = 0;
   }
-  if (track) known[dev][size].store(n + 1, std::memory_order_relaxed);
+  if (track) known[dev][size][group].store(n + 1, std::memory_order_relaxed);
   return n;
 }
 
@@ -898,7 +899,7 @@ static int launch_decode_as(const RfAttn* a, AttnParams& p, const AttnInsert& in
   for (int n = splits; splits <= 8 && n > 1 && 2 * n >= splits; --n) {
     const int pages = n == splits ? pl.pages_per_split : round_up(ceil_div(pl.max_pages, n), 4), parts = ceil_div(pl.max_pages, pages);
     if (n < splits && pages * HD > 48 * 128 && 15 * busiest(parts, pages) > (HD == 256 ? 19 : 18) * busiest(splits, pl.pages_per_split)) break;
-    if (parts > 1 && (long)a->Hkv * p.g_tiles * a->num_seqs < clusters_resident<T, HD, INSERT>(parts, smem)) {
+    if (parts > 1 && (long)a->Hkv * p.g_tiles * a->num_seqs < clusters_resident<T, HD, INSERT>(parts, INSERT ? std::min(p.G, 16) : 0, smem)) {
       p.cluster = 1;
       splits = parts;
       p.pages_per_split = pages;
