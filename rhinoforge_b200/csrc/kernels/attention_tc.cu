@@ -161,7 +161,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
     // the warp reads 32 page numbers at a time, one elected lane issues the copies
     constexpr int kPagesPerBlock = KVB / 16, kBlocksPerFetch = 32 / kPagesPerBlock;
     const bool lead = elect_one();
-    if (lead) {
+    if (lead && nblk > 0) {                                 // nobody would wait for it without keys
       mbar_arrive_expect_tx(&ctl->q_full, (uint32_t)(tiles * G::kQTile));
       for (int t = 0; t < tiles; ++t)
 #pragma unroll

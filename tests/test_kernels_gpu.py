@@ -1062,6 +1062,24 @@ def test_attn_prefill_two_tiles(dt, hd, Hq, Hkv, mode, status):
 
 
 @pytest.mark.parametrize("dt", DT)
+@pytest.mark.parametrize("hd", [64, 128, 256])
+@pytest.mark.parametrize("causal", [False, True])
+def test_attn_prefill_of_sequences_without_keys(dt, hd, causal, status):
+    """Query rows of a sequence that has no keys come out as zeros, beside one that has; more rows than a tile."""
+    from rhinoforge_b200.ops import kernels as K_
+    heads, q_lens, kv_lens = 4, [200, 300, 5], [200, 0, 0]
+    i32 = lambda l: torch.tensor(l, dtype=torch.int32, device="cuda")
+    q, k, v = (torch.randn(sum(q_lens), heads * hd, device="cuda").to(dt) for _ in range(3))
+    out = torch.full_like(q, 7.0)
+    K_.attention_prefill(q, out, Hq=heads, Hkv=heads, hd=hd, q_start=i32([0, 200, 500]), q_len=i32(q_lens), kv_len=i32(kv_lens), kv_start=i32([0, 200, 200]),
+                         max_q_len=300, k=k, v=v, causal=causal, status=status)
+    assert not out[200:].any()
+    h = lambda t: t[:200].view(200, heads, hd).transpose(0, 1)
+    mask = torch.ones(200, 200, dtype=torch.bool, device="cuda")
+    _close(out[:200], _sdpa_ref(h(q), h(k), h(v), mask.tril() if causal else mask).transpose(0, 1).reshape(200, heads * hd), dt)
+
+
+@pytest.mark.parametrize("dt", DT)
 @pytest.mark.parametrize("heads,lens", [(2, [16, 1, 65]), (16, [256, 256, 256]), (32, [300, 513, 129, 64])])
 @pytest.mark.parametrize("mode", ["full", "causal", "mask"])
 def test_attn_prefill_heads_of_80(dt, heads, lens, mode, status):
