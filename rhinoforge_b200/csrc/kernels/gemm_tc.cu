@@ -1581,7 +1581,9 @@ extern "C" int rf_gemm_plan_info(const RfGemm* g, int32_t* out) {
   if (rc) return rc;
   out[0] = pl.swap; out[1] = pl.bn; out[2] = pl.splits; out[3] = pl.stages; out[4] = pl.grid_x; out[5] = pl.grid_y;
   out[6] = (int32_t)pl.smem_bytes; out[7] = pl.k_blocks;
-  out[8] = rf::gemm_ps_form(g, pl.swap != 0, pl.splits, pl.bn, pl.grid_x * pl.grid_y) ? 1 : 0;
+  int kernel, form;
+  GemmPlan routed;
+  out[8] = route_gemm(g, &kernel, &routed, &form) == RF_OK && kernel == RF_GEMM_PERSISTENT ? 1 : 0;
   if (!g->w_int8 && rf::gemm_sk_eligible(g, nullptr)) out[8] = 2;   // persistent stream-K kernel
   out[9] = (g->ar_world > 1 && !pl.swap && g->M > 256) ? 1 : 0;
   return RF_OK;
