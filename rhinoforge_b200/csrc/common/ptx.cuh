@@ -124,7 +124,8 @@ static __device__ __noinline__ void role_gives_up(int32_t* gave_up, int32_t* sta
 //   * a role that writes what others may still use (copies into a ring, a new accumulator, stores, arrivals) starts nothing more;
 //   * the MMA role alone goes on through the k blocks of an accumulator whose operands did not come: it writes nothing but that accumulator, and
 //     whoever is told that it is complete looks at `gave_up` before taking it.  A test or a vote between barrier and MMA would cost every launch
-//     (prefill attention, a chain of such waits, 2 to 10 per cent);
+//     (prefill attention, a chain of such waits, 2 to 10 per cent).  It gives no ring stage back any more, whose copies may still be under way: a
+//     barrier armed again with bytes of its phase outstanding has no meaning;
 //   * the teardown waits for what was started (settle_copies, settle_mmas).
 // `peer`: the flag of the pair's other CTA (a shared::cluster address), 0 for none.
 __device__ __forceinline__ bool role_wait(uint64_t* bar, uint32_t parity, uint64_t* limit_ns, int32_t* gave_up, int32_t* status, int32_t code,

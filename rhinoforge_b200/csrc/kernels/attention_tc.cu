@@ -262,7 +262,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
             if (j + 1 == nblk_t[t]) umma_commit(&ctl->o_full[t]);
           }
         }
-        if (lead) umma_commit(&ctl->kv_empty[s]);                     // every tile's products with this block
+        if (lead && limit) umma_commit(&ctl->kv_empty[s]);            // every tile's products with this block
         s = s_next;
         if (++s_next == stages) { s_next = 0; ph_next ^= 1u; }
       }

@@ -199,7 +199,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
             pair_umma_f16(acc, ad, bd, idesc, kb ? 1u : 0u);
 #pragma unroll
             for (int k = 1; k < kPrBK / 16; ++k) pair_umma_f16(acc, ad + 2 * k, bd + 2 * k, idesc, 1u);
-            pair_umma_commit(&ctl->empty[s]);
+            if (limit) pair_umma_commit(&ctl->empty[s]);
           }
           at += stage_step;
           if (++s == p.stages) { s = 0; at = 0; phase ^= 1u; }

@@ -274,7 +274,7 @@ gemm_ps_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
               if (DUAL) umma_f16(acc + h * half_cols + bn, da + (h * (kPsATile >> 4) + 2 * k), db + (b_second + 2 * k), idesc, accum);
             }
           }
-          umma_commit(&ctl->empty[s]);
+          if (limit) umma_commit(&ctl->empty[s]);
         }
         at += stage_step;
         if (++s == p.stages) { s = 0; at = 0; phase ^= 1u; }

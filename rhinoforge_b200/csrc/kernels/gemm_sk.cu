@@ -207,7 +207,7 @@ gemm_sk_kernel(const __grid_constant__ CUtensorMap tmX, const GemmSkParams p) {
             umma_f16(acc, dw + 2 * k, dx + 2 * k, idesc, accum);
             if (DUAL) umma_f16(acc + bn, dw + 2 * k + (kSkWBlock >> 4), dx + 2 * k, idesc, accum);
           }
-          umma_commit(&ctl->empty[s]);
+          if (limit) umma_commit(&ctl->empty[s]);
         }
         at += stage_step;
         if (++s == p.stages) { s = 0; at = 0; phase ^= 1u; }

@@ -372,7 +372,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
           umma_f16(tmem_base, da + 2 * k, db + 2 * k, idesc, acc);
           if (DUAL) umma_f16(tmem_base + bn, da + 2 * k + (SWAP ? a_second : 0u), db + 2 * k + (SWAP ? 0u : b_second), idesc, acc);
         }
-        umma_commit(&ctl->empty[s]);
+        if (limit) umma_commit(&ctl->empty[s]);
       }
       at += stage_step;
       if (++s == p.stages) { s = 0; at = 0; ph ^= 1u; }
