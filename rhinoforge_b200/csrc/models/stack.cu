@@ -481,7 +481,7 @@ static int forward(Stack& s, const RfStackForward& f, cudaStream_t st) {
       const bool needed = a.q_norm_w || a.rot_dim > 0 || c.paged_kv;
       if (needed) {
         RF_REQUIRE(f.pos != nullptr, "forward: positions are required");
-        if (f.decode && !twin_qk) {
+        if (f.decode && f.own_pages && !twin_qk) {
           insert = a;
           one_insert = true;
           continue;

@@ -138,6 +138,9 @@ typedef struct RfStackForward {
   // accordingly; positions, cache rows and the attention mask are per row, so the order is free.
   int32_t twin_split;
   int32_t rows_per_seq;                    // decode: query rows of every sequence (0: 1), which all see its kv_len keys (attention layers only)
+  // decode: 1 where no row reads a page that this step writes for another row.  Only then may a row's new key and value be put away by the CTAs that
+  // read its pages; with 0 they are ahead of attention, for rows that share pages (two new tokens of a sequence given as two rows, say).
+  int32_t own_pages;
 } RfStackForward;
 
 int64_t rf_stack_create(const RfStackConfig* cfg);

@@ -282,7 +282,8 @@ typedef struct RfAttn {
 int rf_attn_prefill(const RfAttn* a, rf_stream_t stream);
 int rf_attn_decode(const RfAttn* a, rf_stream_t stream);
 // rf_qk_norm_rope_kv(r) and rf_attn_decode(a) in one launch, for the pairs that rf_attn_decode_inserts returns 1 for (others are refused): decode
-// steps of one row per sequence, a->q the QKV buffer.  The rows of that buffer stay as the GEMM left them.
+// steps of one row per sequence, a->q the QKV buffer.  The rows of that buffer stay as the GEMM left them.  No row may read a page that another
+// one's token goes to: nothing orders the two in a launch.
 int rf_attn_decode_inserts(const RfAttn* a, const RfRopeKv* r);
 int rf_attn_decode_insert(const RfAttn* a, const RfRopeKv* r, rf_stream_t stream);
 uint64_t rf_attn_decode_scratch_bytes(int num_seqs, int Hq, int hd);

@@ -739,7 +739,7 @@ class DecoderEngine:
     def _decode_step(self, B: int, logits_out: Optional[torch.Tensor] = None) -> None:
         self._embed(self.ids[:B], B)
         f = N.RfStackForward()
-        f.hidden, f.tokens, f.decode = self.hidden.data_ptr(), B, 1
+        f.hidden, f.tokens, f.decode, f.own_pages = self.hidden.data_ptr(), B, 1, 1      # the pool gives no page to two sequences
         f.pos, f.pos_stride = self.pos.data_ptr(), self.pos_stride
         f.cos, f.sin = self.cos.data_ptr(), self.sin.data_ptr()
         f.axis_of_freq = None if self.axis is None else self.axis.data_ptr()

@@ -201,9 +201,10 @@ class NativeStack:
                 mod: Optional[torch.Tensor] = None, rows_per_mod: int = 1, layer_range=None,
                 deepstack: Optional[Sequence[Optional[torch.Tensor]]] = None,
                 deepstack_rows: Optional[torch.Tensor] = None, taps: Optional[Dict[int, torch.Tensor]] = None,
-                kv_start: Optional[torch.Tensor] = None, twin_split: int = 0, rows_per_seq: int = 1) -> torch.Tensor:
+                kv_start: Optional[torch.Tensor] = None, twin_split: int = 0, rows_per_seq: int = 1, own_pages: bool = False) -> torch.Tensor:
         """Run the layer loop in place on ``hidden`` ``[tokens, hidden]`` (all metadata int32, device).  ``decode`` with ``rows_per_seq`` > 1:
-        every sequence has that many query rows, each of which sees all of the sequence's ``kv_len`` keys."""
+        every sequence has that many query rows, each of which sees all of the sequence's ``kv_len`` keys.  ``own_pages``: no row of a decode step
+        reads a page that the step writes for another row (a launch less per layer)."""
         f = N.RfStackForward()
         T = hidden.shape[0]
         f.hidden, f.tokens, f.decode = hidden.data_ptr(), T, int(decode)
@@ -226,7 +227,7 @@ class NativeStack:
             f.mod, f.rows_per_mod = mod.data_ptr(), rows_per_mod
         if layer_range is not None:
             f.layer_begin, f.layer_end = layer_range
-        f.twin_split, f.rows_per_seq = int(twin_split), int(rows_per_seq)
+        f.twin_split, f.rows_per_seq, f.own_pages = int(twin_split), int(rows_per_seq), int(own_pages)
         keep = []
         if deepstack is not None:
             ptrs = torch.tensor([0 if t is None else t.data_ptr() for t in deepstack], dtype=torch.int64)

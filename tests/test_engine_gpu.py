@@ -207,3 +207,46 @@ def test_prompts_that_end_beside_others_and_in_the_last_page(slots):
         assert (logits[s].float() - want[0].float()).abs().max().item() < 6e-3
         assert first[s] == f[0] or (want[0, f[0]] - want[0, first[s]]).item() < 6e-3
     one.close()
+
+
+@pytest.mark.parametrize("dtype,tol", [(torch.float16, 4e-3), (torch.bfloat16, 3.2e-2)])     # eight roundings
+def test_rows_of_one_sequence_see_each_other_in_a_decode_step(dtype, tol):
+    """Two new tokens of a sequence as two rows over the same pages: as one after the other.  Rows with pages of their own: the same bits whether a row's
+    token is put away ahead of attention or within it."""
+    import ctypes as C
+    from rhinoforge_b200 import _native as N
+    from rhinoforge_b200.models.decoder import tiny_config
+    cfg = tiny_config()
+    _, eng = _oracle_and_engine(cfg, dtype, max_batch=2, max_seq_len=64)
+    g = torch.Generator().manual_seed(7)
+    prompts = [torch.randint(0, cfg.vocab_size, (L,), generator=g) for L in (3, 5)]
+    a, b, other = (int(t) for t in torch.randperm(cfg.vocab_size, generator=g)[:3])
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")
+
+    def step(tokens, slots, pos, own=0):
+        n, ids, p, kl, pt = len(tokens), i32(tokens), i32(pos), i32([q + 1 for q in pos]), eng.cache.page_table[slots].contiguous()
+        eng._embed(ids, n)
+        f = N.RfStackForward()
+        f.hidden, f.tokens, f.decode, f.own_pages, f.num_seqs = eng.hidden.data_ptr(), n, 1, own, n
+        f.pos, f.pos_stride, f.cos, f.sin, f.kv_len, f.max_q_len, f.max_kv_len = p.data_ptr(), 1, eng.cos.data_ptr(), eng.sin.data_ptr(), kl.data_ptr(), 1, 64
+        f.page_table, f.pt_stride, f.pool_pages = pt.data_ptr(), pt.stride(0), eng.cache.num_pages
+        N.check(N.lib().rf_stack_forward(eng.handle, C.byref(f), eng._stream()), "rf_stack_forward")
+        return eng.hidden[:n].clone().float()
+
+    eng.prefill(prompts)
+    both = step([a, b], [0, 0], [3, 4])
+    eng.prefill(prompts)
+    one_by_one = torch.cat((step([a], [0], [3]), step([b], [0], [4])))
+    eng.prefill(prompts)
+    step([other], [0], [3])
+    without = step([b], [0], [4])
+    far = lambda x, y: float((x - y).norm() / y.norm())
+    assert far(without[0], one_by_one[1]) > 4 * tol, "the second token does not depend on the first: the test shows nothing"
+    assert far(both[0], one_by_one[0]) < tol and far(both[1], one_by_one[1]) < tol
+    out = []
+    for own in (0, 1):
+        eng.prefill(prompts)
+        out.append(step([a, b], [0, 1], [3, 5], own))
+    assert torch.equal(*out)
+    eng.check_status()
+    eng.close()
