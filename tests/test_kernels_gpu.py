@@ -1506,3 +1506,38 @@ def test_rmsnorm_around_the_line_between_block_and_warp(dt, H, mod):
             _close(K_.rmsnorm(x[:rows], None, 1e-6, mod=m), (n * (1 + m[:, :H].float()) + m[:, H:2 * H].float())[:rows], dt, scale=2.0)
         else:
             _close(K_.rmsnorm(x[:rows], w, 1e-6), (n * w.float())[:rows], dt, scale=2.0)
+
+
+@pytest.mark.parametrize("dt", DT)
+@pytest.mark.parametrize("M,N,K,extra,dual,cols", [(257, 1032, 72, True, False, 128), (2087, 4104, 72, False, False, 192), (2087, 4104, 72, True, False, 192), (1538, 1288, 1032, False, False, 192),
+                                                   (2819, 4104, 72, False, False, 256), (2819, 4104, 1032, True, False, 256), (129, 2048, 2048, False, False, 128), (200, 2056, 1160, True, False, 128),
+                                                   (256, 3080, 1160, True, True, 128), (600, 1288, 520, False, True, 128), (300, 2568, 1032, True, True, 128)])
+def test_gemm_cta_pairs_of_every_width(dt, M, N, K, extra, dual, cols, status):
+    """Tiles of 128, 192 and 256 columns by name, bare and with scale, bias, row scale and residual: 192 columns begin at all four offsets of a 128-row weight block
+    and end inside one; GLU pairs; 129 to 256 rows, which have one row tile."""
+    import ctypes as C
+    from rhinoforge_b200 import _native as N_
+    from rhinoforge_b200.ops import kernels as K_
+    rows = 2 * N if dual else N
+    x = (torch.randn(M, K, device="cuda") * 0.5).to(dt)
+    w = (torch.randn(rows, K, device="cuda") / K ** 0.5).to(dt)
+    b, sc, rs = torch.randn(rows, device="cuda").to(dt), (torch.rand(rows, device="cuda") + 0.5).to(dt), torch.rand(M, device="cuda") + 0.5
+    r, out = torch.randn(M, N, device="cuda").to(dt), torch.full((M + 1, N + 8), 7.0, device="cuda").to(dt)
+    wp = K_.pack_weight(w, 2 if dual else 1)
+    g = N_.RfGemm()
+    g.x, g.w, g.out, g.M, g.N, g.K, g.ldx, g.ldw, g.ldo, g.force_swap, g.w_packed = x.data_ptr(), wp.data_ptr(), out.data_ptr(), M, N, K, K, K, N + 8, -1, 1
+    if extra:
+        g.bias, g.scale, g.row_scale, g.residual, g.ldr = b.data_ptr(), sc.data_ptr(), rs.data_ptr(), r.data_ptr(), N
+    if dual:
+        g.dual_offset, g.act = N, 1
+    assert N_.lib().rf_gemm_pair_cols(C.byref(g)) == cols
+    z = x.float() @ w.float().t()
+    if extra:
+        z = z * rs[:, None] * sc.float() + b.float()
+    ref = torch.nn.functional.silu(z[:, :N]) * z[:, N:] if dual else z
+    if extra:
+        ref = ref + r.float()
+    kw = dict(bias=b, scale=sc, row_scale=rs, residual=r) if extra else {}
+    K_.gemm(x, wp, packed_shape=(rows, K), out=out[:M, :N], status=status, **kw, **(dict(act="silu_mul", dual=True) if dual else {}))
+    _close(out[:M, :N], ref, dt, scale=2.0 if extra else 1.0)
+    assert bool((out[M:] == 7.0).all()) and bool((out[:, N:] == 7.0).all())
