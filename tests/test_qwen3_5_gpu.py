@@ -410,3 +410,31 @@ def test_conv1d_of_a_few_tokens(dt, off, L):
     y = K.causal_conv1d(x, w, st, q_start=z, q_len=ql, max_q_len=L, slot=z)
     assert _rel(y, ref) < (4e-3 if dt == torch.float16 else 2e-2)
     assert torch.equal(st[0].float(), full[-3:].to(dt).float())
+
+
+@pytest.mark.parametrize("dt", DT)
+@pytest.mark.parametrize("off", [0, 2])
+@pytest.mark.parametrize("lens", [[3], [4], [5], [63, 64, 65], [65, 1, 3, 4, 5, 8, 31, 32, 33, 63, 64, 2] * 12])
+def test_conv1d_of_ragged_sequences(dt, off, lens):
+    """Around the four tokens that are asked for together and a block's 32 or (the last case: at least three blocks an SM) 64; rows on their 16-byte
+    boundary and two values behind it."""
+    from rhinoforge_b200.ops import kernels as K
+    Cc, n, T = 1032, len(lens), sum(lens)
+    if n > 100 and 2 * n * 2 < 3 * torch.cuda.get_device_properties(0).multi_processor_count:
+        pytest.skip("more SMs than the last case was made for")
+    x = torch.randn(T, Cc + 8, device="cuda").to(dt)[:, off:off + Cc]
+    st, w = torch.randn(n, 3, Cc, device="cuda").to(dt), (torch.randn(Cc, 4, device="cuda") * 0.5).to(dt)
+    ql = torch.tensor(lens, dtype=torch.int32, device="cuda")
+    q0 = (torch.cumsum(ql, 0) - ql).int()
+    slot = torch.arange(n - 1, -1, -1, dtype=torch.int32, device="cuda")
+    ref, want, o = torch.empty(T, Cc, device="cuda"), torch.empty_like(st), 0
+    for s, L in enumerate(lens):
+        full = torch.cat((st[n - 1 - s].float(), x[o:o + L].float()), 0)
+        ref[o:o + L] = F.silu(F.conv1d(full.t()[None], w.float()[:, None], groups=Cc)[0].t())
+        want[n - 1 - s] = full[-3:].to(dt)
+        o += L
+    out = torch.full((T + 1, Cc + 8), 7.0, device="cuda").to(dt)
+    K.causal_conv1d(x, w, st, q_start=q0, q_len=ql, max_q_len=max(lens), slot=slot, out=out[:T, off:off + Cc])
+    assert _rel(out[:T, off:off + Cc], ref) < (4e-3 if dt == torch.float16 else 2e-2)
+    assert bool((out[T:] == 7.0).all()) and bool((out[:, :off] == 7.0).all()) and bool((out[:, off + Cc:] == 7.0).all())
+    assert torch.equal(st, want)
